@@ -312,26 +312,6 @@ def run_ours(a, ws, rank, local):
         torch.cuda.synchronize()
         fp64_256 = e0.elapsed_time(e1)
         beta256_err = float(np.max(np.linalg.norm(b256 - b256_64, axis=1) / np.linalg.norm(b256_64, axis=1)))
-        # the same batch with the slab contraction on the tensor cores (P <= 32)
-        tc256 = None
-        if P <= 32:
-            tuned_tc = ctx.proj_kernel()
-            ctx.set_proj_kernel(True)
-            btc = ctx.project_batch(sh256, mg.PREC_SPLIT)
-            t_tc = []
-            for _ in range(2):
-                flush.zero_()
-                torch.cuda.synchronize()
-                e0, e1 = torch.cuda.Event(enable_timing=True), torch.cuda.Event(enable_timing=True)
-                e0.record(stream)
-                ctx.project_batch(sh256, mg.PREC_SPLIT)
-                e1.record(stream)
-                torch.cuda.synchronize()
-                t_tc.append(e0.elapsed_time(e1))
-            ctx.set_proj_kernel(tuned_tc)
-            tc256 = {"ms": float(min(t_tc)), "beta_max_rel_err_vs_fp64": float(np.max(
-                np.linalg.norm(btc - b256_64, axis=1) / np.linalg.norm(b256_64, axis=1))),
-                     "kernel": "k_project_slab_tc (tcgen05, BF16 three-piece operands)"}
         go64 = extra.get("fp64_gamma_ortho_ms", go_ms)
         gos = extra.get("split_gamma_ortho_ms", go_ms)
         extra["projection_256_shapes"] = {
@@ -339,8 +319,7 @@ def run_ours(a, ws, rank, local):
             "split_ms": p256, "split_projections_per_s": 256.0 / (p256 * 1e-3),
             "fp64_ms": fp64_256, "split_beta_max_rel_err_vs_fp64": beta256_err,
             "split_vs_fp64_gamma_ortho_plus_256_projections": (go64 + fp64_256) / (gos + p256),
-            "kernel": "k_project_slab_tc" if ctx.proj_kernel() else "k_project_slab_f32 (CUDA cores)",
-            "tensor_core_form": tc256}
+            "kernel": "k_project_f32 (tcgen05, BF16 three-piece operands)"}
 
     # roofline of the dominant kernel of the timed step: the tridiagonalisation's
     # panel kernel (the FP64 matrix-vector product over the trailing matrix of

@@ -2,9 +2,8 @@
 //
 // Two kernels have launch parameters whose best value depends on the problem
 // size and the GPU:
-//   * the FP32 projection slab kernel: shapes per CTA (8 or 4) and the grid
-//     form (one CTA per (slab, shape group), or a persistent grid of 1 or 2
-//     CTAs per SM taking work items from a counter);
+//   * the FP32 projection kernel: shapes per work item (8 or 4) and row teams
+//     per SM (1, 2, or 0 for as many as fit);
 //   * the FP64 Gamma kernel: mu steps staged per shared-memory load (KC).
 // modal_autotune times every candidate with CUDA events on the context stream
 // on the context's own basis (a fixed synthetic batch of 16 shapes for the
@@ -147,8 +146,7 @@ modal_status modal_autotune(modal_ctx *c, const char *cache_path)
     const std::string arch = arch_tag(c->device);
     const int P = c->P;
 
-    // ---- projection slab kernel: tensor-core kernel (P <= 32), or the CUDA-core
-    // kernel with (shapes per CTA, persistent CTAs per SM)
+    // ---- FP32 projection kernel: shapes per work item, row teams per SM
     const std::string kp = "proj2 " + arch + " lmax=" + std::to_string(c->lmax) + " P=" + std::to_string(P);
     int pv[3] = {0, 0, 0};
     if (cache_lookup(cache_path, kp, pv, 3)) {
@@ -161,8 +159,7 @@ modal_status modal_autotune(modal_ctx *c, const char *cache_path)
         tune_shapes(c->lmax, tab, sh);
         struct Cand { int sg, cpb, tc; };
         std::vector<Cand> cands;
-        if (P <= 32) cands.push_back({0, 0, 1});
-        for (int sg : (P <= 32) ? std::vector<int>{8, 4} : std::vector<int>{4})
+        for (int sg : {8, 4})
             for (int cpb : {0, 1, 2}) cands.push_back({sg, cpb, 0});
         float best = 1e30f;
         Cand b = cands[0];

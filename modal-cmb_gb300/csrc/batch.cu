@@ -55,7 +55,7 @@ void batch_release(modal_ctx *c)
 static std::vector<const void *> batch_ptrs(const modal_ctx *c)
 {
     return {c->q.ptr, c->cl.ptr, c->vl.ptr, c->triples.ptr, c->slab_order.ptr, c->shape_tab.ptr, c->shape_desc.ptr,
-            c->scratch.ptr, c->beta.ptr};
+            c->scratch.ptr, c->beta.ptr, c->pf_sched.ptr};
 }
 
 static bool batch_matches(const BatchGraph &g, const modal_ctx *c, int S, const modal_shape *shapes, modal_prec prec)
@@ -63,6 +63,8 @@ static bool batch_matches(const BatchGraph &g, const modal_ctx *c, int S, const 
     if (!g.exec || g.S != S || g.prec != (int)prec || g.lmin != c->lmin || g.lmax != c->lmax || g.P != c->P ||
         g.N != c->N || g.sg != c->proj_sg || g.cpb != c->proj_cpb || g.tc != c->proj_tc)
         return false;
+    // the slab schedule on the device may by now be another range's
+    if (prec == MODAL_PREC_SPLIT && (c->pf_lmin != c->lmin || c->pf_lmax != c->lmax)) return false;
     for (int s = 0; s < S; s++)
         if (g.kinds[s] != shapes[s].kind || (shapes[s].kind == MODAL_SHAPE_SEPARABLE && g.nterms[s] != shapes[s].nterms))
             return false;

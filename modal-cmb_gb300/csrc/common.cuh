@@ -68,6 +68,10 @@ struct modal_ctx {
     modal::DevBuf shape_tab;   // separable tables
     modal::DevBuf shape_desc;  // device shape descriptors
     modal::DevBuf slab_order;  // projection slab schedule
+    // FP32 projection: weight-table offsets and slab order of (pf_lmin, pf_lmax); table length in 128 floats
+    modal::DevBuf pf_sched;
+    int pf_lmin = -1, pf_lmax = -1;
+    long long pf_total = 0;
     modal::DevBuf split;       // split-precision Gamma: operand pieces, T table, per-P tables
     int split_P = -1;          // layout the tables in `split` were uploaded for: P, K padding, buffer
     long split_key = -1;
@@ -195,7 +199,7 @@ struct DShape {
     int kind, nterms;
     long tab_off;  // FP64 tables: [term][f, g, h][l] from this double offset
     double c1, c2, c3, sigma;
-    long tab_off_f = 0;  // FP32 form: [parity of l][l / 2][term][f, g, h, 0] from this float offset
+    long tab_off_f = 0;  // FP32 form (k_pf_tab's layout) from this float offset
 };
 
 // Internal shape kind of the 3D transfer Gamma: the radial integral s_n(l1,l2,l3)
@@ -215,16 +219,15 @@ struct ProjPlan {
     modal_prec prec = MODAL_PREC_FP64;
     long tab_total = 0;
     std::vector<DShape> desc;
-    int SG = 8, CPL = 1, cpb = 0, nsm = 0, fpt = 0;
-    size_t smem = 0, o_q = 0, o_v = 0, o_t = 0, o_s = 0, o_F = 0, o_B = 0, o_c = 0, o_w = 0, o_sb = 0;
-    long long npts = 0;  // tetrapyd points (FP32 weight table entries)
+    int fpt = 0;
+    size_t smem = 0, o_B = 0, o_w = 0, o_sb = 0;
+    long long npts = 0;  // tetrapyd points (FP64 weight table entries)
+    // FP32 form (project_f32.cu): shapes per work item, operand columns, groups of 8 lattice points
+    // per parity of the B operand, segments of the slab reduction, buffer offsets
+    int SG = 4, NC = 32, M8 = 0, QR = 0, nseg = 1, nsm = 0, teams = 1;
+    size_t team_smem = 0, o_q = 0, o_v = 0, o_g = 0, o_t = 0, o_s = 0, o_F = 0, o_bq = 0;
     long tabf_total = 0;  // floats of the FP32 separable tables
     RadialArgs ra;        // radial shapes (3D transfer Gamma only)
-    int max_nterms = 0;
-    bool tc = false;        // tensor-core slab kernel (FP32 form, P <= 32)
-    int Mpad = 0;           // compact k entries per row of its BF16 q pieces
-    size_t o_bq = 0, o_perm = 0;
-    std::vector<int> perm;  // shape order of its work items (by kind and term count)
 };
 // plan: validate, size every buffer, upload the slab schedule (may allocate);
 // stage: copy shape tables/descriptors to the device; record: enqueue the
@@ -232,6 +235,9 @@ struct ProjPlan {
 modal_status proj_plan(modal_ctx *ctx, int S, const modal_shape *shapes, modal_prec prec, ProjPlan &pl);
 modal_status proj_stage(modal_ctx *ctx, const ProjPlan &pl, const modal_shape *shapes);
 modal_status proj_record(modal_ctx *ctx, const ProjPlan &pl);
+// The same two steps of the single-precision form (project_f32.cu).
+modal_status pf_plan(modal_ctx *ctx, ProjPlan &pl);
+modal_status pf_record(modal_ctx *ctx, const ProjPlan &pl);
 
 // Frees the captured batched-projection graph and its pinned staging buffers.
 void batch_release(modal_ctx *ctx);

@@ -35,6 +35,7 @@ __device__ __forceinline__ bool mbar_try(uint32_t bar, uint32_t parity)
 // Bounded wait: false when `budget` clock64 cycles ran out or another role aborted.
 __device__ __forceinline__ bool mbar_wait(uint32_t bar, uint32_t parity, volatile int *abort_flag, long long budget)
 {
+    if (mbar_try(bar, parity)) return true;
     const long long t0 = clock64();
     while (!mbar_try(bar, parity)) {
         if (*abort_flag) return false;

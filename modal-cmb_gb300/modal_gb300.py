@@ -353,11 +353,11 @@ class Context:
         _check(lib().modal_set_pca_floor(self.h, float(floor)))
 
     def set_proj_kernel(self, tensor_cores):
-        """FP32 projection kernel: True = tcgen05 tensor cores (P <= 32), False = CUDA cores."""
+        """FP32 projection kernel preference (one kernel: both settings give the same result)."""
         _check(lib().modal_set_proj_kernel(self.h, 1 if tensor_cores else 0))
 
     def proj_kernel(self):
-        """True when the FP32 projection of the current basis runs on the tensor cores."""
+        """The preference set by set_proj_kernel, where P <= 32."""
         v = ctypes.c_int()
         _check(lib().modal_get_proj_kernel(self.h, ctypes.byref(v)))
         return bool(v.value)

@@ -1,0 +1,70 @@
+"""The single-precision projection kernel at the edges of its tiling, against
+the FP64 projection of the same shapes: row blocks of 128 rows per parity (the
+second block opens at l_max = 258), chunks of 32 lattice points, operand widths
+of 16, 32, 48 and 64 basis columns, passes of four terms, one shape per item and
+partly filled items.
+
+Tolerance.  Each shape value carries about ten FP32 roundings of 2^-24, its
+product with the basis is exact to 2^-24, and the sums over rows and slabs round
+at 2^-24 of partial sums that exceed the result by a modest factor (the
+oscillating basis): 1e-6 relative per shape for P <= 32 and 2e-6 beyond, the
+bounds the FP32 form has always been held to."""
+import numpy as np
+import pytest
+from conftest import rel_fro
+
+pytestmark = pytest.mark.gpu
+
+
+def _ctx(mg, lmin, lmax, P):
+    cl = mg.synthetic_cl(lmax)
+    c = mg.Context(0)
+    c.set_basis(lmin, lmax, mg.weighted_q(mg.legendre_q(lmin, lmax, P), cl, lmin))
+    c.set_modes(mg.mode_triples(P))
+    c.set_spectrum(cl)
+    return c
+
+
+@pytest.mark.parametrize("lmin,lmax,P,terms,S", [
+    (2, 3, 2, 1, 1), (2, 17, 3, 4, 2), (5, 64, 16, 5, 3), (2, 257, 17, 1, 1), (2, 258, 16, 4, 5), (3, 259, 8, 8, 2),
+    (2, 300, 33, 2, 3), (2, 130, 48, 3, 2), (2, 131, 49, 1, 9), (2, 90, 64, 4, 1), (2, 515, 4, 2, 4)])
+def test_f32_projection_edges(mg, lmin, lmax, P, terms, S):
+    shapes = mg.separable_shapes(lmax, S, seed=7, tmin=terms, tmax=terms) + mg.bump_shapes(2, seed=8)
+    with _ctx(mg, lmin, lmax, P) as c:
+        b64 = c.project(shapes, mg.PREC_FP64)
+        b32 = c.project(shapes, mg.PREC_SPLIT)
+        again = c.project(shapes, mg.PREC_SPLIT)
+        batch = c.project_batch(shapes, mg.PREC_SPLIT)
+    assert np.array_equal(b32, again) and np.array_equal(b32, batch)
+    for s in range(len(shapes)):
+        assert rel_fro(b32[s], b64[s]) <= (1e-6 if P <= 32 else 2e-6), (s, rel_fro(b32[s], b64[s]))
+
+
+def test_f32_projection_ignores_table_entries_below_lmin(mg):
+    """l < l_min takes no part: infinities and NaN there (a power law at l = 0) leave the result alone."""
+    lmax = 60
+    shapes = mg.separable_shapes(lmax, 3, seed=9, tmin=1, tmax=3)
+    dirty = [dict(s, tab=s["tab"].copy()) for s in shapes]
+    for s in dirty:
+        s["tab"][:, :, 0] = np.inf
+        s["tab"][:, :, 1] = np.nan
+    with _ctx(mg, 2, lmax, 5) as c:
+        clean = c.project(shapes, mg.PREC_SPLIT)
+        got = c.project(dirty, mg.PREC_SPLIT)
+    assert np.array_equal(got, clean)
+
+
+def test_f32_batch_replays_after_another_range(mg):
+    """The captured batch uses the slab schedule of its own range: a projection at another l_max in
+    between makes it plan again."""
+    q1, tr, cl = mg.workload(150, 6)
+    q2, _, cl2 = mg.workload(90, 6)
+    shapes = mg.config_shapes(150, ("mix", 6, 1, 2), seed=3)
+    with _ctx(mg, 2, 150, 6) as c:
+        first = c.project_batch(shapes, mg.PREC_SPLIT)
+        c.set_basis(2, 90, q2)
+        c.set_spectrum(cl2)
+        c.project(mg.config_shapes(90, ("mix", 6, 1, 2), seed=4), mg.PREC_SPLIT)
+        c.set_basis(2, 150, q1)
+        c.set_spectrum(cl)
+        assert np.array_equal(c.project_batch(shapes, mg.PREC_SPLIT), first)
