@@ -133,7 +133,8 @@ modal_status legendre_table_dev(modal_ctx *ctx, int nmu, int lmax, const double 
     MODAL_TRY(launched(ctx, "pl_factors"));
     const size_t smem = sizeof(double) * 3 * (size_t)(lmax + 1);
     if (smem > 200 * 1024) { set_error("legendre table: lmax = %d too large", lmax); return MODAL_ERR_ARG; }
-    MODAL_CUDA(cudaFuncSetAttribute(k_legendre_table, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem));
+    // the limit, not this call's size: the allocation-free entry point launches the kernel with its own size
+    MODAL_CUDA(cudaFuncSetAttribute(k_legendre_table, cudaFuncAttributeMaxDynamicSharedMemorySize, 200 * 1024));
     k_legendre_table<<<ceil_div(nmu, 32 * PL_WPB), 32 * PL_WPB, smem, ctx->stream>>>(nmu, lmax, d_mu, pw, d_pl);
     return launched(ctx, "legendre_table");
 }
