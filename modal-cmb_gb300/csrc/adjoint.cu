@@ -28,6 +28,7 @@
 //   J = (1/S) sum_s (<S_s,S_s> - beta_s^T alpha_s) / <S_s,S_s>
 //   dJ/dGamma = sum_s c_s alpha_s alpha_s^T, dJ/dbeta_s = -2 c_s alpha_s, c_s = 1/(S <S_s,S_s>).
 #include <algorithm>
+#include <cmath>
 #include <vector>
 #include "common.cuh"
 
@@ -616,9 +617,15 @@ modal_status modal_adjoint_residual(modal_ctx *c, int S, const modal_shape *shap
             set_error("modal_adjoint_residual: shape %d has <S,S> = %g", s, hn2[s]);
             return MODAL_ERR_ARG;
         }
-        double ba = 0.0;
-        for (int n = 0; n < N; n++) ba += hb[(size_t)s * N + n] * ha[(size_t)s * N + n];
-        Jv += (hn2[s] - ba) / hn2[s];
+        // beta . alpha with the rounding of every product and sum carried along: J is differenced by
+        // optimisers, and the N plain roundings are the largest part of its noise
+        double ba = 0.0, lo = 0.0;
+        for (int n = 0; n < N; n++) {
+            const double x = hb[(size_t)s * N + n], y = ha[(size_t)s * N + n], pr = x * y, t = ba + pr, z = t - ba;
+            lo += std::fma(x, y, -pr) + ((ba - (t - z)) + (pr - z));
+            ba = t;
+        }
+        Jv += ((hn2[s] - ba) - lo) / hn2[s];
         cs[s] = 1.0 / ((double)S * hn2[s]);
     }
     if (J) *J = Jv / S;

@@ -162,7 +162,7 @@ void modal_ctx_destroy(modal_ctx *c)
     if (c->stream) cudaStreamSynchronize(c->stream);
     DevBuf *bufs[] = {&c->q, &c->triples, &c->mu, &c->w, &c->pl, &c->mt, &c->gamma, &c->chol, &c->linv,
                       &c->orthol, &c->lambdal, &c->norm, &c->info, &c->cl, &c->vl, &c->beta, &c->alpha,
-                      &c->modesr, &c->scratch, &c->scratch2, &c->shape_tab, &c->shape_desc, &c->slab_order, &c->pf_sched,
+                      &c->modesr, &c->trip, &c->scratch, &c->scratch2, &c->shape_tab, &c->shape_desc, &c->slab_order, &c->pf_sched,
                       &c->split, &c->tr_x, &c->tr_qt, &c->tr_prim, &c->tr_mt, &c->tr_v, &c->tr_out,
                       &c->adj, &c->adj2, &c->adj3, &c->prune, &c->gemm_part, &c->qe, &c->me, &c->tri_pol, &c->gamma_pol,
                       &c->tr_qte, &c->tr_we, &c->tr_mte, &c->prim, &c->eigw, &c->ozw, &c->ozerr, &c->ozrun};

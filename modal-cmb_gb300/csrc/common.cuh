@@ -64,6 +64,7 @@ struct modal_ctx {
     modal::DevBuf alpha;    // [S][N]
     modal::DevBuf modesr;   // [S][N]
     modal::DevBuf scratch;  // general work area
+    modal::DevBuf trip;     // triple products: operand rows and T (triple.cu)
     modal::DevBuf scratch2;
     modal::DevBuf shape_tab;   // separable tables
     modal::DevBuf shape_desc;  // device shape descriptors

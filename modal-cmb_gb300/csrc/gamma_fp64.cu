@@ -10,32 +10,38 @@
 //  mt[k][i][j] (mu-major, so one mu step of the whole P x P table is one
 //  contiguous block).
 #include "common.cuh"
+#include "triple.cuh"
 
 namespace modal {
 
 // --------------------------------------------------------------------------
-// l-contraction, FP64 SIMT GEMM over l: out tile 64 (mu) x 32 (p<=q pairs).
-// Summation over l in ascending order, as the reference.
+// l-contraction, FP64 SIMT GEMM over l: out tile 8R (mu) x 32 (p<=q pairs),
+// bound by the FP64 pipe (the tile's loads hide behind it).  Summation over l in
+// ascending order, as the reference, whatever the tile.
 // --------------------------------------------------------------------------
-constexpr int MIJ_BK = 64, MIJ_BU = 32, MIJ_LC = 16;
+constexpr int MIJ_BU = 32, MIJ_LC = 16;
 
-__global__ void __launch_bounds__(256) k_mij_fp64(int nmu, int lmin, int lmax, int P, int npair,
+template <int R>
+__device__ __forceinline__ void mij_tile(int nmu, int lmin, int lmax, int P, int npair,
                                                   const double *__restrict__ pl, const double *__restrict__ q,
                                                   const int2 *__restrict__ pairs, double *__restrict__ mt)
 {
+    constexpr int MIJ_BK = 8 * R;
     __shared__ double sPl[MIJ_LC][MIJ_BK];
     __shared__ double sV[MIJ_LC][MIJ_BU];
     const int tid = threadIdx.x, tx = tid & 31, ty = tid >> 5;
     const int k0 = blockIdx.x * MIJ_BK, u0 = blockIdx.y * MIJ_BU;
     const int L = lmax - lmin + 1;
-    double acc[8];
+    double acc[R];
 #pragma unroll
-    for (int r = 0; r < 8; r++) acc[r] = 0.0;
+    for (int r = 0; r < R; r++) acc[r] = 0.0;
 
     for (int l0 = 0; l0 < L; l0 += MIJ_LC) {
 #pragma unroll
-        for (int t = 0; t < (MIJ_LC * MIJ_BK) / 256; t++) {
-            int e = tid + 256 * t, lr = e / MIJ_BK, kc = e % MIJ_BK;
+        for (int t = 0; t < (MIJ_LC * MIJ_BK + 255) / 256; t++) {
+            int e = tid + 256 * t;
+            if (e >= MIJ_LC * MIJ_BK) break;
+            int lr = e / MIJ_BK, kc = e % MIJ_BK;
             int l = l0 + lr, k = k0 + kc;
             sPl[lr][kc] = (l < L && k < nmu) ? pl[(size_t)(lmin + l) * nmu + k] : 0.0;
         }
@@ -55,7 +61,7 @@ __global__ void __launch_bounds__(256) k_mij_fp64(int nmu, int lmin, int lmax, i
         for (int lr = 0; lr < MIJ_LC; lr++) {
             double vv = sV[lr][tx];
 #pragma unroll
-            for (int r = 0; r < 8; r++) acc[r] = fma(sPl[lr][ty + 8 * r], vv, acc[r]);
+            for (int r = 0; r < R; r++) acc[r] = fma(sPl[lr][ty + 8 * r], vv, acc[r]);
         }
         __syncthreads();
     }
@@ -63,7 +69,7 @@ __global__ void __launch_bounds__(256) k_mij_fp64(int nmu, int lmin, int lmax, i
     if (u >= npair) return;
     const int2 pq = pairs[u];
 #pragma unroll
-    for (int r = 0; r < 8; r++) {
+    for (int r = 0; r < R; r++) {
         int k = k0 + ty + 8 * r;
         if (k < nmu) {
             double *blk = mt + (size_t)k * P * P;
@@ -71,6 +77,23 @@ __global__ void __launch_bounds__(256) k_mij_fp64(int nmu, int lmin, int lmax, i
             blk[pq.y * P + pq.x] = acc[r];
         }
     }
+}
+
+// The 64-node tile under the name that the allocation-free entry point launches, and the tile of 8R
+// nodes for the regular path.
+__global__ void __launch_bounds__(256) k_mij_fp64(int nmu, int lmin, int lmax, int P, int npair, const double *__restrict__ pl,
+                                                  const double *__restrict__ q, const int2 *__restrict__ pairs,
+                                                  double *__restrict__ mt)
+{
+    mij_tile<8>(nmu, lmin, lmax, P, npair, pl, q, pairs, mt);
+}
+
+template <int R>
+__global__ void __launch_bounds__(256) k_mij_fp64_r(int nmu, int lmin, int lmax, int P, int npair,
+                                                    const double *__restrict__ pl, const double *__restrict__ q,
+                                                    const int2 *__restrict__ pairs, double *__restrict__ mt)
+{
+    mij_tile<R>(nmu, lmin, lmax, P, npair, pl, q, pairs, mt);
 }
 
 // M table [nmu][P][P] of a basis q[L][P] on lmin..lmax (T or E) into out.
@@ -87,9 +110,19 @@ modal_status mij_table_dev(modal_ctx *ctx, const double *q, int lmin, int lmax, 
     if (e == cudaSuccess) e = cudaStreamSynchronize(ctx->stream);
     delete[] h;
     if (e != cudaSuccess) { set_error("mij pairs: %s", cudaGetErrorString(e)); return MODAL_ERR_CUDA; }
-    dim3 grid(ceil_div(ctx->nmu, MIJ_BK), ceil_div(npair, MIJ_BU));
-    k_mij_fp64<<<grid, 256, 0, ctx->stream>>>(ctx->nmu, lmin, lmax, P, npair, ctx->pl.as<double>(), q,
-                                              ctx->scratch.as<int2>(), out.as<double>());
+    // smaller mu tiles until there are two CTAs per SM: with 24 CTAs (l <= 500, P = 10) the 64-node tile
+    // took 295 us, the FP64 pipe of 128 SMs idle
+    int nsm = 0, R = 8;
+    MODAL_CUDA(cudaDeviceGetAttribute(&nsm, cudaDevAttrMultiProcessorCount, ctx->device));
+    while (R > 1 && (long)ceil_div(ctx->nmu, 8 * R) * ceil_div(npair, MIJ_BU) < 2L * nsm) R /= 2;
+    auto run = [&](auto kern) {
+        kern<<<dim3(ceil_div(ctx->nmu, 8 * R), ceil_div(npair, MIJ_BU)), 256, 0, ctx->stream>>>(
+            ctx->nmu, lmin, lmax, P, npair, ctx->pl.as<double>(), q, ctx->scratch.as<int2>(), out.as<double>());
+    };
+    if (R == 8) run(k_mij_fp64);
+    else if (R == 4) run(k_mij_fp64_r<4>);
+    else if (R == 2) run(k_mij_fp64_r<2>);
+    else run(k_mij_fp64_r<1>);
     return launched(ctx, "mij_fp64");
 }
 
@@ -185,6 +218,12 @@ modal_status gamma_fp64_dev(modal_ctx *ctx, int mu0, int nmu)
     MODAL_TRY(ensure(ctx->scratch2, sizeof(double) * nmu));
     k_wgt48<<<ceil_div(nmu, 256), 256, 0, ctx->stream>>>(nmu, ctx->w.as<double>() + mu0, ctx->scratch2.as<double>());
     MODAL_TRY(launched(ctx, "wgt48"));
+    // the distinct products of three M entries, or (few modes of a large basis) the permanents of the
+    // pairs: full lists at l <= 2000 take 102 ms on the first against 645 ms on the second at P = 30
+    if (triple_wins(0.5 * N * (N + 1.0), 0.5 * P * (P + 1.0))) {
+        const modal_status st = gamma_triple_dev(ctx, mu0, nmu, ctx->scratch2.as<double>());
+        if (st != MODAL_ERR_NOMEM) return st;
+    }
     int KC = (96 * 1024) / (P * P * 8);
     if (KC < 1) KC = 1;
     if (KC > 32) KC = 32;

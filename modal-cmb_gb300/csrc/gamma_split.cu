@@ -26,6 +26,7 @@
 #include <vector>
 #include "common.cuh"
 #include "dfbits.cuh"
+#include "triple.cuh"
 
 namespace modal {
 
@@ -111,45 +112,6 @@ __global__ void __launch_bounds__(256) k_slice_y(int UV, int UVpad, int K, int K
     }
 }
 
-// Gamma_mn = sum over the six orderings of T[lo][vt(mid, hi)] (sorted pair
-// indices lo <= mid <= hi; vt(v, t) = vbase[v] + t - v, the row order of Y).
-// One thread per (m, n) of a 32 x 32 tile with tile(m) <= tile(n).
-__global__ void __launch_bounds__(256) k_gamma_gather64(int N, int P, int U, long ldT, const int *__restrict__ triples,
-                                                        const int *__restrict__ pidx, const long long *__restrict__ vbase,
-                                                        const double *__restrict__ T, double *__restrict__ gamma)
-{
-    const int tm = blockIdx.y, tn = blockIdx.x;
-    if (tm > tn) return;
-    extern __shared__ unsigned char gsm[];
-    long long *sbase = reinterpret_cast<long long *>(gsm);
-    int *sp = reinterpret_cast<int *>(sbase + U);
-    for (int e = threadIdx.x; e < U; e += 256) sbase[e] = vbase[e];
-    for (int e = threadIdx.x; e < P * P; e += 256) sp[e] = pidx[e];
-    __syncthreads();
-    const int tx = threadIdx.x & 31, ty = threadIdx.x >> 5;
-    const int n = tn * 32 + tx;
-    if (n >= N) return;
-    const int n0 = triples[3 * n], n1 = triples[3 * n + 1], n2 = triples[3 * n + 2];
-    const int perm[6][3] = {{0, 1, 2}, {1, 2, 0}, {2, 0, 1}, {2, 1, 0}, {1, 0, 2}, {0, 2, 1}};
-    for (int r = 0; r < 4; r++) {
-        const int m = tm * 32 + ty + 8 * r;
-        if (m >= N || m > n) continue;
-        const int mm[3] = {triples[3 * m], triples[3 * m + 1], triples[3 * m + 2]};
-        const int nn[3] = {n0, n1, n2};
-        double g = 0.0;
-#pragma unroll
-        for (int s = 0; s < 6; s++) {
-            const int x = sp[mm[0] * P + nn[perm[s][0]]];
-            const int y = sp[mm[1] * P + nn[perm[s][1]]];
-            const int z = sp[mm[2] * P + nn[perm[s][2]]];
-            const int lo = min(x, min(y, z)), hi = max(x, max(y, z)), mid = x + y + z - lo - hi;
-            g += T[(size_t)lo * ldT + sbase[mid] + (hi - mid)];
-        }
-        gamma[(size_t)m * N + n] = g;
-        gamma[(size_t)n * N + m] = g;
-    }
-}
-
 }  // namespace
 
 modal_status gamma_split_dev(modal_ctx *ctx, int mu0, int nmu)
@@ -161,22 +123,18 @@ modal_status gamma_split_dev(modal_ctx *ctx, int mu0, int nmu)
     const long UVpad = (long)ceil_div(UV, SP_TILE) * SP_TILE;
     const int Kpad = ceil_div(nmu, 64) * 64;
 
-    // host tables: pairs, pair index, (v,t) rows and their bases, output tiles
+    // host tables: pairs, (v,t) rows, output tiles
     std::vector<int2> pairs(U);
-    std::vector<int> pidx((size_t)P * P);
     {
         int u = 0;
         for (int p = 0; p < P; p++)
-            for (int q = p; q < P; q++) { pairs[u] = make_int2(p, q); pidx[p * P + q] = pidx[q * P + p] = u; u++; }
+            for (int q = p; q < P; q++) pairs[u++] = make_int2(p, q);
     }
-    std::vector<long long> vbase(U);
     std::vector<int2> vtp(UV);
     {
         long r = 0;
-        for (int v = 0; v < U; v++) {
-            vbase[v] = r;
+        for (int v = 0; v < U; v++)
             for (int t = v; t < U; t++) vtp[r++] = make_int2(v, t);
-        }
     }
     std::vector<int2> tiles;
     for (long j = 0; j < UVpad / SP_TILE; j++) {
@@ -190,8 +148,6 @@ modal_status gamma_split_dev(modal_ctx *ctx, int mu0, int nmu)
     size_t o = 0;
     // the host tables first: their offsets depend on P alone
     const size_t o_pairs = o; o += al((size_t)U * sizeof(int2));
-    const size_t o_pidx = o; o += al((size_t)P * P * 4);
-    const size_t o_vbase = o; o += al((size_t)U * 8);
     const size_t o_vtp = o; o += al((size_t)UV * sizeof(int2));
     const size_t o_qp = o; o += al((size_t)U * L * 8);
     const size_t o_x = o; o += al((size_t)U * Kpad * 8);
@@ -209,8 +165,6 @@ modal_status gamma_split_dev(modal_ctx *ctx, int mu0, int nmu)
     // the host tables depend on P only; a reallocated buffer has lost them
     if (ctx->split_P != P || ctx->split_ptr != ctx->split.ptr || ctx->split_bytes != ctx->split.bytes) {
         MODAL_CUDA(cudaMemcpyAsync(b + o_pairs, pairs.data(), U * sizeof(int2), cudaMemcpyHostToDevice, ctx->stream));
-        MODAL_CUDA(cudaMemcpyAsync(b + o_pidx, pidx.data(), pidx.size() * 4, cudaMemcpyHostToDevice, ctx->stream));
-        MODAL_CUDA(cudaMemcpyAsync(b + o_vbase, vbase.data(), U * 8, cudaMemcpyHostToDevice, ctx->stream));
         MODAL_CUDA(cudaMemcpyAsync(b + o_vtp, vtp.data(), UV * sizeof(int2), cudaMemcpyHostToDevice, ctx->stream));
         MODAL_CUDA(cudaStreamSynchronize(ctx->stream));
         ctx->split_P = P;
@@ -251,14 +205,7 @@ modal_status gamma_split_dev(modal_ctx *ctx, int mu0, int nmu)
     }
     // 3. Gamma from the sorted-triple entries of T
     MODAL_TRY(ensure(ctx->gamma, sizeof(double) * (size_t)N * N));
-    const size_t gsm = (size_t)U * 8 + (size_t)P * P * 4;
-    MODAL_CUDA(cudaFuncSetAttribute(k_gamma_gather64, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)gsm));
-    const int nt = ceil_div(N, 32);
-    k_gamma_gather64<<<dim3(nt, nt), 256, gsm, ctx->stream>>>(N, P, U, UV, ctx->triples.as<int>(),
-                                                                reinterpret_cast<const int *>(b + o_pidx),
-                                                                reinterpret_cast<const long long *>(b + o_vbase), T,
-                                                                ctx->gamma.as<double>());
-    MODAL_TRY(launched(ctx, "gamma_gather64"));
+    MODAL_TRY(gamma_gather_dev(ctx, U, T));
     return oz_check(ctx);
 }
 
