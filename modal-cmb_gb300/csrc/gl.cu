@@ -4,67 +4,115 @@
 
 namespace modal {
 
+// n / c for a small positive integer c and r = 1 / c rounded: Markstein's correction of n r (P. W.
+// Markstein, "Computation of elementary functions on the IBM RISC System/6000 processor", IBM J.
+// Res. Develop. 34 (1990)).  Three dependent operations instead of a division's dozen, and the same
+// bits: the residual is exact, and a quotient by c < 2^13 is never within 2^-14 ulp of a midpoint.
+__device__ __forceinline__ double div_small(double n, double c, double r)
+{
+    const double q = n * r;
+    return fma(fma(-q, c, n), r, q);
+}
+
 // ---------------------------------------------------------------------------
 // Gauss-Legendre nodes/weights (replaces asy, gl_integration.c:46-168; same
-// ascending symmetric layout).  One thread per positive root.  Newton in
-// theta (x = cos theta) from Tricomi's guess; P_n(cos theta) by the
-// three-term recurrence in differences D_l = P_l - P_{l-1} with
-// y = 1 - x = 2 sin^2(theta/2):
+// ascending symmetric layout).  One thread per positive root theta (x = cos theta), from Olver's
+// uniform expansion in the zeros of J_0 (DLMF 18.16(v)): psi = j_{0,k} / (n + 1/2),
+//     theta = psi + (psi cot psi - 1) / (8 psi (n + 1/2)^2),
+// within 1e-11 of the root (relative) for n >= 751.  P_n(cos theta) by the three-term recurrence
+// in differences D_l = P_l - P_{l-1} with y = 1 - x = 2 sin^2(theta/2):
 //     D_{l+1} = (l D_l - (2l+1) y P_l) / (l+1),  P_{l+1} = P_l + D_{l+1},
-// which stays accurate next to x = 1, where the small endpoint weights carry
-// a large share of the Gamma integrand.  w = 2 sin^2 theta / (n (P_{n-1} - x P_n))^2.
-// Newton stops after 30 iterations at most.
+// which stays accurate next to x = 1, where the small endpoint weights carry a large share of the
+// Gamma integrand.  With f(theta) = P_n(cos theta), df = -n Q / sin theta, Q = P_{n-1} - x P_n, and
+// Legendre's equation d2f = -cot df - n(n+1) f (and its derivative for d3f), a step d = -f/df that is
+// small enough is completed to third order and the derivative carried to the root,
+//     w = 2 / df(theta + d)^2,
+// so that one recurrence per root does for n >= 31 (two for smaller n; 30 at most).
+// The bound is that recurrence: n steps of six dependent FP64 operations, one warp per SM.
+// n = 3001: 47.4 -> 1.06 ms per call (the Newton iteration before this ran until a step fell below
+// 1e-17, about 20 recurrences, with a full division per step); weights as accurate as before (4e-14).
 // ---------------------------------------------------------------------------
+constexpr int GL_CH = 256;  // reciprocals staged per chunk of the recurrence
+
+// P_n and Q at cos(theta) for every thread of the block (uniform control flow).
 __device__ __forceinline__ void leg_diff(int n, double th, double &Pn, double &Q)
 {
-    double s = sin(0.5 * th);
-    double y = 2.0 * s * s;
-    double P = 1.0, D = 0.0;
-    for (int l = 0; l < n; l++) {
-        double Dn = (l * D - (2.0 * l + 1.0) * y * P) / (l + 1.0);
-        P += Dn;
-        D = Dn;
+    __shared__ double rec[GL_CH];
+    const double s = sin(0.5 * th), y = 2.0 * s * s;
+    double P = 1.0, D = 0.0, l = 0.0;
+    for (int c0 = 0; c0 < n; c0 += GL_CH) {
+        __syncthreads();
+        for (int i = threadIdx.x; i < GL_CH; i += blockDim.x) rec[i] = 1.0 / (double)(c0 + i + 1);
+        __syncthreads();
+        const int m = min(GL_CH, n - c0);
+#pragma unroll 4
+        for (int i = 0; i < m; i++) {
+            const double t = (2.0 * l + 1.0) * y, l1 = l + 1.0;
+            D = div_small(fma(l, D, -(t * P)), l1, rec[i]);
+            P += D;
+            l = l1;
+        }
     }
     Pn = P;
     Q = -D + y * P;
+}
+
+// Olver's approximation of the k-th root (k = 1 next to theta = 0).
+__device__ __forceinline__ double gl_guess(int n, int k)
+{
+    // the first zeros of J_0, then McMahon's expansion
+    const double j0[8] = {2.4048255576957728, 5.5200781102863106, 8.6537279129110122, 11.791534439014281,
+                          14.930917708487785, 18.071063967910922, 21.211636629879259, 24.352471530749303};
+    const double b = (k - 0.25) * 3.14159265358979323846, e = 1.0 / (8.0 * b), e2 = e * e;
+    const double j = k <= 8 ? j0[k - 1] : b + e * (1.0 - e2 * (124.0 / 3.0 - e2 * (120928.0 / 15.0)));
+    const double v = n + 0.5, ps = j / v;
+    return ps + (ps * cos(ps) / sin(ps) - 1.0) / (8.0 * ps * v * v);
 }
 
 __global__ void k_gl_nodes(int n, double *mu, double *w)
 {
     const int half = n / 2;
     const int k = blockIdx.x * blockDim.x + threadIdx.x + 1;  // root index 1..half (+ middle)
-    if (k <= half) {
-        const double pi = 3.141592653589793238462643383279502884;
-        double th = pi * (4.0 * k - 1.0) / (4.0 * n + 2.0);
-        double x0 = (1.0 - (n - 1.0) / (8.0 * (double)n * n * n)) * cos(th);
-        th = acos(x0);
-        double Pn, Q;
-        for (int it = 0; it < 30; it++) {
-            leg_diff(n, th, Pn, Q);
-            double dth = Pn * sin(th) / (n * Q);
-            th += dth;
-            if (fabs(dth) <= 1e-17 * th) break;
+    const bool root = k <= half, mid = k == half + 1 && (n & 1);
+    double th = root ? gl_guess(n, k) : 1.5707963267948966192313216916397514, wk = 0.0;
+    bool open = root || mid;
+    for (int it = 0; it < 30; it++) {
+        double f, Q;
+        leg_diff(n, th, f, Q);
+        if (open && mid) {
+            wk = 2.0 / ((double)n * n * Q * Q);
+            open = false;
+        } else if (open) {
+            const double st = sin(th), f1 = -n * Q / st, d = -f / f1;
+            if ((fabs(d) <= 1e-6 * th && n * fabs(d) <= 1e-5) || it == 29) {
+                const double nn = (double)n * (n + 1.0), cot = cos(th) / st, f2 = -cot * f1 - nn * f,
+                             f3 = f1 / (st * st) - cot * f2 - nn * f1;
+                const double dd = d - f2 / (2.0 * f1) * d * d, g = f1 + dd * (f2 + 0.5 * dd * f3);
+                th += dd;
+                wk = 2.0 / (g * g);
+                open = false;
+            } else {
+                th += d;
+            }
         }
-        leg_diff(n, th, Pn, Q);
-        double st = sin(th);
-        double wk = 2.0 * st * st / ((double)n * n * Q * Q);
-        double x = cos(th);
+        if (!__syncthreads_or(open)) break;
+    }
+    if (root) {
+        const double x = cos(th);
         mu[n - k] = x;
         mu[k - 1] = -x;
         w[n - k] = wk;
         w[k - 1] = wk;
-    } else if (k == half + 1 && (n & 1)) {
-        double Pn, Q;
-        leg_diff(n, 1.5707963267948966192313216916397514, Pn, Q);
+    } else if (mid) {
         mu[half] = 0.0;
-        w[half] = 2.0 / ((double)n * n * Q * Q);
+        w[half] = wk;
     }
 }
 
 modal_status gl_nodes_dev(modal_ctx *ctx, int n, double *d_mu, double *d_w)
 {
-    int threads = 64;
-    int roots = n / 2 + 1;
+    const int threads = 32;  // one warp per SM: the roots' recurrences share an SM's FP64 pipe otherwise
+    const int roots = n / 2 + 1;
     k_gl_nodes<<<ceil_div(roots, threads), threads, 0, ctx->stream>>>(n, d_mu, d_w);
     return launched(ctx, "gl_nodes");
 }
@@ -85,43 +133,49 @@ __global__ void k_pl_factors(int lmax, double *pw)
 }
 
 // One thread per node, so that the n_mu independent recurrences spread over as
-// many warps as possible: the recurrence is serial in l and GB300's FP64 rate
-// per SM is low, so the length of the FP64 dependency chain, not the bytes
-// written, sets the time (~1.45 ms for 3001 nodes to l = 2000: 33 GB/s of
-// table).  The arithmetic is gsl_sf_legendre_Pl's upward recurrence exactly,
-// (x (2l-1) P_{l-1} - (l-1) P_{l-2}) / l, with the integer factors read as
-// doubles from shared memory (the same values, so the same bits; it saves
-// three integer-to-FP64 conversions per step, 10%).  Folding the division into
-// precomputed reciprocals is faster but moves the table by ~1e-12 at l = 500
-// (the roundings accumulate coherently along l), which would show in Gamma's
-// 1e-12 parity with the reference.
+// many warps as possible: the recurrence is serial in l, so the length of the FP64
+// dependency chain, not the bytes written, sets the time.  The arithmetic is
+// gsl_sf_legendre_Pl's upward recurrence, (x (2l-1) P_{l-1} - (l-1) P_{l-2}) / l, the division by
+// Markstein's correction (div_small: the same bits), which leaves four dependent operations per
+// step instead of about fifteen.
+// 1802 nodes to l = 1201: 576 -> 345 us, bit-identical.
 constexpr int PL_WPB = 1;  // warps per block (measured: 1 and 4 give the same time; the chains do not contend)
 __global__ void __launch_bounds__(32 * PL_WPB) k_legendre_table(int nmu, int lmax, const double *__restrict__ mu,
                                                                 const double *__restrict__ pw, double *__restrict__ pl)
 {
-    extern __shared__ double tab[];  // [lmax+1][3]: 2l - 1, l - 1, l
+    // [lmax+1][3]: 2l - 1, 1/l, (2l+1)^{2/3}: loads, where conversions would take turns on the FP64
+    // pipe and a global load of the factor would stall the chain
+    extern __shared__ double tab[];
     for (int l = threadIdx.x; l <= lmax; l += blockDim.x) {
         tab[3 * l] = (double)(2 * l - 1);
-        tab[3 * l + 1] = (double)(l - 1);
-        tab[3 * l + 2] = (double)l;
+        tab[3 * l + 1] = l > 0 ? 1.0 / (double)l : 0.0;
+        tab[3 * l + 2] = pw[l];
     }
     __syncthreads();
     const int k = blockIdx.x * blockDim.x + threadIdx.x;
     if (k >= nmu) return;
     const double x = mu[k];
-    const bool xp1 = (x == 1.0), xm1 = (x == -1.0);
-    pl[k] = pw[0];
-    if (lmax >= 1) pl[(size_t)nmu + k] = pw[1] * x;
-    double pm2 = 1.0, pm1 = x;
-    for (int l = 2; l <= lmax; l++) {
-        const double pr = (x * tab[3 * l] * pm1 - tab[3 * l + 1] * pm2) / tab[3 * l + 2];
+    const bool edge = x == 1.0 || x == -1.0;  // exact values there
+    double *o = pl + k;
+    o[0] = tab[2];
+    if (lmax >= 1) o[nmu] = tab[5] * x;
+    double pm2 = 1.0, pm1 = x, c1 = 1.0;
+    if (lmax >= 2) {
+        // P_2 in closed form, as GSL; the recurrence goes on from its own value
+        const double pr = div_small(fma(x * tab[6], pm1, -(c1 * pm2)), 2.0, tab[7]);
         pm2 = pm1;
         pm1 = pr;
-        double p = pr;
-        if (l == 2) p = 0.5 * (3.0 * x * x - 1.0);
-        else if (xp1) p = 1.0;
-        else if (xm1) p = (l & 1) ? -1.0 : 1.0;
-        pl[(size_t)l * nmu + k] = pw[l] * p;
+        c1 = 2.0;
+        o[2 * (size_t)nmu] = tab[8] * (0.5 * (3.0 * x * x - 1.0));
+    }
+#pragma unroll 4
+    for (int l = 3; l <= lmax; l++) {
+        const double c = c1 + 1.0;
+        const double pr = div_small(fma(x * tab[3 * l], pm1, -(c1 * pm2)), c, tab[3 * l + 1]);
+        pm2 = pm1;
+        pm1 = pr;
+        c1 = c;
+        o[(size_t)l * nmu] = tab[3 * l + 2] * (edge ? (x > 0.0 || !(l & 1) ? 1.0 : -1.0) : pr);
     }
 }
 

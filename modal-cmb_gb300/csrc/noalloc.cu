@@ -151,12 +151,12 @@ extern "C" modal_status modal_gamma_fp64_noalloc(int lmin, int lmax, int P, cons
     const double *mu = d_nodes, *w = d_weights;
     if (own_nodes) {
         double *mu_s = reinterpret_cast<double *>(base + off_mu), *w_s = reinterpret_cast<double *>(base + off_w);
-        k_gl_nodes<<<ceil_div(nmu / 2 + 1, 64), 64, 0, s>>>(nmu, mu_s, w_s);
+        k_gl_nodes<<<ceil_div(nmu / 2 + 1, 32), 32, 0, s>>>(nmu, mu_s, w_s);
         mu = mu_s;
         w = w_s;
     }
     k_pl_factors<<<ceil_div(lmax + 1, 256), 256, 0, s>>>(lmax, pw);
-    // the table kernel keeps its integer factors in 3 (lmax + 1) doubles of shared
+    // the table kernel keeps its factors in 3 (lmax + 1) doubles of shared
     // memory (at most 24 KB for the problems the scratch array admits)
     k_legendre_table<<<ceil_div(nmu, 32), 32, sizeof(double) * 3 * (size_t)(lmax + 1), s>>>(nmu, lmax, mu, pw, pl);
     k_noalloc_pairs<<<1, 1, 0, s>>>(P, pairs, status);
