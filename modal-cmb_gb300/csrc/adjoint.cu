@@ -21,8 +21,9 @@
 //   dq_r(l)    += sum_k pl_l(k) sum_q (dM[r][q](k) + dM[q][r](k)) q_q(l)
 //   dB_e[q](k)  = sum_{s,n} Gb_sn w_k/(48 pi) sum_t sum_{a,b: e=(s,t,a), n_b=q} cof_ab(B(k))
 //   dq_q(l)    += sum_k pl_l(k) sum_e f~_e(l) dB_e[q](k)
-// The Gamma adjoint recomputes M(mu_k) from the Legendre table and q inside each
-// CTA instead of reading a stored copy.  Objectives built on these:
+// For full mode lists the Gamma adjoint runs over the distinct products of three M entries
+// (gamma_triple_vjp_dev); few modes of a large basis keep the cofactors, one CTA per node, which
+// recomputes M(mu_k) from the Legendre table and q.  Objectives built on these:
 //   alpha_s = Gamma^{-1} beta_s = lambda^T lambda beta_s  (the orthogonalisation's factor)
 //   dL/dbeta_s = u_s, dL/dGamma = -sum_s u_s alpha_s^T,   u_s = Gamma^{-1} dL/dalpha_s
 //   J = (1/S) sum_s (<S_s,S_s> - beta_s^T alpha_s) / <S_s,S_s>
@@ -31,6 +32,7 @@
 #include <cmath>
 #include <vector>
 #include "common.cuh"
+#include "triple.cuh"
 
 namespace modal {
 
@@ -113,13 +115,14 @@ __global__ void __launch_bounds__(128) k_beta_gl(int N, int nmu, LegInfo li, con
                                                  const double *__restrict__ w, const double *__restrict__ BK,
                                                  double *__restrict__ beta)
 {
-    const int s = blockIdx.y;
+    // nodes of split z only; its sums go to beta + z S N
+    const int s = blockIdx.y, kper = (nmu + gridDim.z - 1) / gridDim.z, k0 = blockIdx.z * kper, k1 = min(nmu, k0 + kper);
     const int n = blockIdx.x * blockDim.x + threadIdx.x;
     if (n >= N) return;
     const int P = li.P, e0 = li.leg0[s], T = li.nterm[s];
     const int nb[3] = {triples[3 * n], triples[3 * n + 1], triples[3 * n + 2]};
     double acc = 0.0;
-    for (int k = 0; k < nmu; k++) {
+    for (int k = k0; k < k1; k++) {
         const double *Bk = BK + (size_t)k * li.stride;
         double sk = 0.0;
         for (int t = 0; t < T; t++) {
@@ -132,7 +135,17 @@ __global__ void __launch_bounds__(128) k_beta_gl(int N, int nmu, LegInfo li, con
         }
         acc = fma(w[k] * kInv48Pi, sk, acc);
     }
-    beta[(size_t)s * N + n] = acc;
+    beta[((size_t)blockIdx.z * li.nshape + s) * N + n] = acc;
+}
+
+// beta[e] = sum over the node splits (in order)
+__global__ void k_beta_sum(long n, int Z, const double *__restrict__ part, double *__restrict__ beta)
+{
+    const long e = (long)blockIdx.x * blockDim.x + threadIdx.x;
+    if (e >= n) return;
+    double s = part[e];
+    for (int z = 1; z < Z; z++) s += part[(size_t)z * n + e];
+    beta[e] = s;
 }
 
 // norm2[s] = <S_s,S_s>: one CTA per shape, threads over mu nodes, tree reduction.
@@ -222,41 +235,83 @@ __global__ void __launch_bounds__(256) k_gamma_vjp(int N, int P, int nmu, int lm
     for (int e = threadIdx.x; e < PP; e += blockDim.x) dM[(size_t)k * PP + e] = sD[e];
 }
 
-// Projection adjoint, one CTA per mu node k: B(k) staged in shared memory,
-// dB(k) accumulated there.
-__global__ void __launch_bounds__(256) k_beta_vjp(int N, int nmu, LegInfo li, int E, const int *__restrict__ triples,
-                                                  const double *__restrict__ BK, const double *__restrict__ w,
-                                                  const double *__restrict__ Gb, double *__restrict__ dB)
+// Projection adjoint.  With the symmetric tensor of shape s
+//   Gs[q][q'][q''] = sum_n Gb_sn sum over the six orderings of mode n of delta(q q' q'', ordering),
+// the term (s, t) contributes sum_k w_k/(48 pi) sum Gs B_0[q] B_1[q'] B_2[q''], so its three
+// gradients need two FMAs per entry of Gs and node instead of nine cofactors and nine shared-memory
+// additions per mode.  Bound by the FP64 pipe: 364 modes at P = 12, 48 terms, 1501 nodes in 0.84 ms
+// (6.1 ms with the cofactors).
+__global__ void k_beta_tensor(int S, int N, int P, const int *__restrict__ triples, const double *__restrict__ Gb,
+                              double *__restrict__ Gs)
+{
+    const long e = (long)blockIdx.x * blockDim.x + threadIdx.x;
+    if (e >= (long)S * N) return;
+    const int s = (int)(e / N), n = (int)(e - (long)s * N);
+    const double g = Gb[e];
+    if (g == 0.0) return;
+    const int b[3] = {triples[3 * n], triples[3 * n + 1], triples[3 * n + 2]};
+    const int perm[6][3] = {{0, 1, 2}, {1, 2, 0}, {2, 0, 1}, {2, 1, 0}, {1, 0, 2}, {0, 2, 1}};
+    double *G = Gs + (size_t)s * P * P * P;
+#pragma unroll
+    for (int x = 0; x < 6; x++) atomicAdd(&G[(b[perm[x][0]] * P + b[perm[x][1]]) * P + b[perm[x][2]]], g);
+}
+
+// One thread per (term, node): grid (ceil(nmu / 64), terms), 64 threads; the legs and two gradients
+// in shared memory [5][P][64].  term_shape[j], term_leg[j]: shape and first leg of term j.
+constexpr int BV_T = 64;
+__global__ void __launch_bounds__(BV_T) k_beta_vjp(int nmu, int P, int E, int stride, const int *__restrict__ term_shape,
+                                                   const int *__restrict__ term_leg, const double *__restrict__ BK,
+                                                   const double *__restrict__ w, const double *__restrict__ Gs,
+                                                   double *__restrict__ dB)
 {
     extern __shared__ double sm[];
-    const int k = blockIdx.x, P = li.P, EP = E * P;
-    double *sB = sm, *sD = sm + EP;
-    for (int e = threadIdx.x; e < EP; e += blockDim.x) { sB[e] = BK[(size_t)k * li.stride + e]; sD[e] = 0.0; }
-    __syncthreads();
-    const double wk = w[k] * kInv48Pi;
-    const long SN = (long)li.nshape * N;
-    for (long e = threadIdx.x; e < SN; e += blockDim.x) {
-        const double g = Gb[e];
-        if (g == 0.0) continue;
-        const int s = (int)(e / N), n = (int)(e - (long)s * N);
-        const int nb[3] = {triples[3 * n], triples[3 * n + 1], triples[3 * n + 2]};
-        const int e0 = li.leg0[s], T = li.nterm[s];
-        const double gw = g * wk;
-        for (int t = 0; t < T; t++) {
-            const int lg = e0 + 3 * t;
-            double a[3][3];
-#pragma unroll
-            for (int x = 0; x < 3; x++)
-#pragma unroll
-                for (int y = 0; y < 3; y++) a[x][y] = sB[(lg + x) * P + nb[y]];
-#pragma unroll
-            for (int x = 0; x < 3; x++)
-#pragma unroll
-                for (int y = 0; y < 3; y++) atomicAdd(&sD[(lg + x) * P + nb[y]], gw * cof3(a, x, y));
-        }
+    const int t = threadIdx.x, k = blockIdx.x * BV_T + t, leg = term_leg[blockIdx.y];
+    if (k >= nmu) return;
+    double *b0 = sm + t, *b1 = b0 + P * BV_T, *b2 = b1 + P * BV_T, *d1 = b2 + P * BV_T, *d2 = d1 + P * BV_T;
+    const double *B = BK + (size_t)k * stride + (size_t)leg * P;
+    for (int q = 0; q < P; q++) {
+        b0[q * BV_T] = B[q];
+        b1[q * BV_T] = B[P + q];
+        b2[q * BV_T] = B[2 * P + q];
+        d1[q * BV_T] = d2[q * BV_T] = 0.0;
     }
-    __syncthreads();
-    for (int e = threadIdx.x; e < EP; e += blockDim.x) dB[(size_t)k * EP + e] = sD[e];
+    const double wk = w[k] * kInv48Pi;
+    const double *G = Gs + (size_t)term_shape[blockIdx.y] * P * P * P;
+    double *out = dB + ((size_t)k * E + leg) * P;
+    for (int q = 0; q < P; q++) {
+        const double x = b0[q * BV_T];
+        double d0 = 0.0;
+        for (int r = 0; r < P; r++) {
+            const double y = b1[r * BV_T], xy = x * y, *g = G + (size_t)(q * P + r) * P;
+            double a = 0.0;
+#pragma unroll 4
+            for (int u = 0; u < P; u++) {
+                const double gv = __ldg(g + u);
+                a = fma(gv, b2[u * BV_T], a);
+                d2[u * BV_T] = fma(gv, xy, d2[u * BV_T]);
+            }
+            d0 = fma(a, y, d0);
+            d1[r * BV_T] = fma(a, x, d1[r * BV_T]);
+        }
+        out[q] = wk * d0;
+    }
+    for (int q = 0; q < P; q++) {
+        out[P + q] = wk * d1[q * BV_T];
+        out[2 * P + q] = wk * d2[q * BV_T];
+    }
+}
+
+// dq[l][r] += sum_c Z[l][(r, c)] q[l][c], the diagonal pair twice      (Z = pl^T dX, one column per pair)
+__global__ void k_dq_pairs(int L, int P, int U, const double *__restrict__ Z, const double *__restrict__ q,
+                           double *__restrict__ dq)
+{
+    const int e = blockIdx.x * blockDim.x + threadIdx.x;
+    if (e >= L * P) return;
+    const int l = e / P, r = e - l * P;
+    const double *z = Z + (size_t)l * U;
+    double acc = 0.0;
+    for (int c = 0; c < P; c++) acc = fma(c == r ? 2.0 * z[pair_rank(r, c, P)] : z[pair_rank(r, c, P)], q[(size_t)l * P + c], acc);
+    dq[e] += acc;
 }
 
 // dq[l][r] += sum_c (Z[l][r*P+c] + Z[l][c*P+r]) q[l][c]      (Z = pl^T dM)
@@ -313,6 +368,7 @@ __global__ void k_scale_rows(int S, int N, const double *__restrict__ a, const d
 struct AdjFwd {
     int S = 0, E = 0, ncolB = 0, ncolK = 0;
     LegInfo li{};
+    const int *term_shape = nullptr, *term_leg = nullptr;  // [E / 3] shape and first leg of each term
     double *BK = nullptr;     // [nmu][ncolB + ncolK]
     double *vecs = nullptr;   // [P + E][L]
     double *beta = nullptr;   // [S][N]
@@ -326,7 +382,7 @@ inline size_t al256(size_t b) { return (b + 255) & ~(size_t)255; }
 modal_status adj_forward(modal_ctx *c, int S, const modal_shape *shapes, AdjFwd &f)
 {
     const int lmin = c->lmin, lmax = c->lmax, L = c->L, P = c->P, N = c->N, nmu = c->nmu;
-    std::vector<int> leg0(S), nterm(S), kb(S);
+    std::vector<int> leg0(S), nterm(S), kb(S), tshape, tleg;
     std::vector<long> leg_off;
     long tab_total = 0;
     int E = 0, ncolK = 0;
@@ -338,6 +394,10 @@ modal_status adj_forward(modal_ctx *c, int S, const modal_shape *shapes, AdjFwd 
         leg0[s] = E;
         nterm[s] = shapes[s].nterms;
         kb[s] = ncolK;
+        for (int t = 0; t < shapes[s].nterms; t++) {
+            tshape.push_back(s);
+            tleg.push_back(E + 3 * t);
+        }
         for (int t = 0; t < shapes[s].nterms; t++)
             for (int a = 0; a < 3; a++) leg_off.push_back(tab_total + ((long)t * 3 + a) * (lmax + 1));
         tab_total += (long)shapes[s].nterms * 3 * (lmax + 1);
@@ -368,6 +428,7 @@ modal_status adj_forward(modal_ctx *c, int S, const modal_shape *shapes, AdjFwd 
     const size_t o_leg0 = o; o += al256(sizeof(int) * S);
     const size_t o_nt = o; o += al256(sizeof(int) * S);
     const size_t o_kb = o; o += al256(sizeof(int) * S);
+    const size_t o_ts = o; o += al256(sizeof(int) * (size_t)E);
     const size_t o_wl = o; o += al256(sizeof(double) * (lmax + 1));
     const size_t o_vecs = o; o += al256(sizeof(double) * (size_t)(P + E) * L);
     const size_t o_BK = o; o += al256(sizeof(double) * (size_t)nmu * ncol);
@@ -388,6 +449,11 @@ modal_status adj_forward(modal_ctx *c, int S, const modal_shape *shapes, AdjFwd 
     MODAL_CUDA(cudaMemcpyAsync(b + o_leg0, leg0.data(), sizeof(int) * S, cudaMemcpyHostToDevice, c->stream));
     MODAL_CUDA(cudaMemcpyAsync(b + o_nt, nterm.data(), sizeof(int) * S, cudaMemcpyHostToDevice, c->stream));
     MODAL_CUDA(cudaMemcpyAsync(b + o_kb, kb.data(), sizeof(int) * S, cudaMemcpyHostToDevice, c->stream));
+    MODAL_CUDA(cudaMemcpyAsync(b + o_ts, tshape.data(), sizeof(int) * tshape.size(), cudaMemcpyHostToDevice, c->stream));
+    MODAL_CUDA(cudaMemcpyAsync(b + o_ts + sizeof(int) * tshape.size(), tleg.data(), sizeof(int) * tleg.size(),
+                               cudaMemcpyHostToDevice, c->stream));
+    f.term_shape = reinterpret_cast<const int *>(b + o_ts);
+    f.term_leg = f.term_shape + tshape.size();
     double *wl = reinterpret_cast<double *>(b + o_wl);
     f.vecs = reinterpret_cast<double *>(b + o_vecs);
     f.BK = reinterpret_cast<double *>(b + o_BK);
@@ -412,9 +478,16 @@ modal_status adj_forward(modal_ctx *c, int S, const modal_shape *shapes, AdjFwd 
     f.li.leg0 = reinterpret_cast<const int *>(b + o_leg0);
     f.li.nterm = reinterpret_cast<const int *>(b + o_nt);
     f.li.kb = reinterpret_cast<const int *>(b + o_kb);
-    const dim3 g2(ceil_div(N, 128), S);
-    k_beta_gl<<<g2, 128, 0, c->stream>>>(N, nmu, f.li, c->triples.as<int>(), c->w.as<double>(), f.BK, f.beta);
+    // one thread per (shape, mode) alone fills a fifth of the GPU at 32 shapes and 364 modes: split the nodes
+    int nsm = 0;
+    MODAL_CUDA(cudaDeviceGetAttribute(&nsm, cudaDevAttrMultiProcessorCount, c->device));
+    const int Zn = (int)std::max<long>(1, std::min<long>(std::min(16, nmu / 64), 8L * nsm / ((long)ceil_div(N, 128) * S)));
+    MODAL_TRY(ensure(c->trip, sizeof(double) * (size_t)Zn * S * N));
+    const dim3 g2(ceil_div(N, 128), S, Zn);
+    k_beta_gl<<<g2, 128, 0, c->stream>>>(N, nmu, f.li, c->triples.as<int>(), c->w.as<double>(), f.BK, c->trip.as<double>());
     MODAL_TRY(launched(c, "beta_gl"));
+    k_beta_sum<<<ceil_div((long)S * N, 256), 256, 0, c->stream>>>((long)S * N, Zn, c->trip.as<double>(), f.beta);
+    MODAL_TRY(launched(c, "beta_sum"));
     k_norm_gl<<<S, 128, 0, c->stream>>>(nmu, f.li, c->w.as<double>(), f.BK, f.norm2);
     MODAL_TRY(launched(c, "norm_gl"));
     // the host-side tables above are pageable and go out of scope on return
@@ -425,7 +498,23 @@ modal_status adj_forward(modal_ctx *c, int S, const modal_shape *shapes, AdjFwd 
 // dq (device [L][P], accumulated) += VJP of Gamma for the upstream G [N][N] (device).
 modal_status gamma_vjp_dev(modal_ctx *c, const double *G, double *dq)
 {
-    const int P = c->P, PP = P * P, nmu = c->nmu, L = c->L;
+    const int P = c->P, PP = P * P, nmu = c->nmu, L = c->L, U = P * (P + 1) / 2;
+    // by distinct triple products where that takes fewer FP64 instructions (U^3/2 per node against
+    // about 45 per pair of modes, and nine shared-memory additions): the full list of 364 modes at
+    // P = 12, n_mu = 1501 takes 1 ms instead of 49
+    if (0.5 * U * (U * (U + 1.0)) < 45.0 * c->N * (double)c->N && 4.0 * U * U * (U + 1.0) <= 16e9) {
+        MODAL_TRY(mt_ready(c));
+        MODAL_TRY(ensure(c->adj2, sizeof(double) * ((size_t)nmu + L) * U));
+        double *dX = c->adj2.as<double>(), *Z = dX + (size_t)nmu * U;
+        const modal_status st = gamma_triple_vjp_dev(c, G, dX);
+        if (st == MODAL_OK) {
+            MODAL_TRY(dgemm_splitk(c, L, U, nmu, c->pl.as<double>() + (size_t)c->lmin * nmu, nmu, false, dX, U, false, Z, U, 0,
+                                   false));
+            k_dq_pairs<<<ceil_div((long)L * P, 256), 256, 0, c->stream>>>(L, P, U, Z, c->q.as<double>(), dq);
+            return launched(c, "dq_pairs");
+        }
+        if (st != MODAL_ERR_NOMEM) return st;
+    }
     const size_t smem = sizeof(double) * (2 * (size_t)PP + (size_t)GV_LC * P + GV_LC);
     if (smem > 200 * 1024) { set_error("adjoint: P=%d too large for the Gamma adjoint", P); return MODAL_ERR_ARG; }
     MODAL_TRY(ensure(c->adj2, sizeof(double) * ((size_t)nmu * PP + (size_t)L * PP)));
@@ -452,9 +541,15 @@ modal_status beta_vjp_dev(modal_ctx *c, const AdjFwd &f, const double *Gb, doubl
     }
     MODAL_TRY(ensure(c->adj2, sizeof(double) * ((size_t)nmu * EP + (size_t)L * EP)));
     double *dB = c->adj2.as<double>(), *Z2 = dB + (size_t)nmu * EP;
-    MODAL_CUDA(cudaFuncSetAttribute(k_beta_vjp, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem));
-    k_beta_vjp<<<nmu, 256, smem, c->stream>>>(c->N, nmu, f.li, E, c->triples.as<int>(), f.BK, c->w.as<double>(), Gb,
-                                              dB);
+    const size_t PPP = (size_t)P * P * P, vs = sizeof(double) * 5 * (size_t)P * BV_T;
+    MODAL_TRY(ensure(c->trip, sizeof(double) * f.S * PPP));
+    double *Gs = c->trip.as<double>();
+    MODAL_CUDA(cudaMemsetAsync(Gs, 0, sizeof(double) * f.S * PPP, c->stream));
+    k_beta_tensor<<<ceil_div((long)f.S * c->N, 256), 256, 0, c->stream>>>(f.S, c->N, P, c->triples.as<int>(), Gb, Gs);
+    MODAL_TRY(launched(c, "beta_tensor"));
+    MODAL_CUDA(cudaFuncSetAttribute(k_beta_vjp, cudaFuncAttributeMaxDynamicSharedMemorySize, 5 * 64 * BV_T * 8));
+    k_beta_vjp<<<dim3(ceil_div(nmu, BV_T), E / 3), BV_T, vs, c->stream>>>(nmu, P, E, f.li.stride, f.term_shape, f.term_leg, f.BK,
+                                                                         c->w.as<double>(), Gs, dB);
     MODAL_TRY(launched(c, "beta_vjp"));
     MODAL_TRY(dgemm(c, L, EP, nmu, 1.0, c->pl.as<double>() + (size_t)c->lmin * nmu, nmu, false, dB, EP, false, 0.0,
                     Z2, EP, 0));

@@ -145,6 +145,113 @@ __global__ void __launch_bounds__(256) k_gamma_gather(int N, int P, int U, long 
     }
 }
 
+// X^T[u][k] = M_ab(mu_k), u = (a, b), from the symmetric P x P rows of the M table.
+__global__ void k_triple_cols(int K, int U, int P, const double *__restrict__ mt, double *__restrict__ XT)
+{
+    const long e = (long)blockIdx.x * blockDim.x + threadIdx.x;
+    if (e >= (long)K * U) return;
+    const int u = (int)(e / K), k = (int)(e - (long)u * K);
+    int a, b;
+    tri_unrank(u, P, a, b);
+    XT[e] = mt[(size_t)k * P * P + a * P + b];
+}
+
+// Adjoint of the gather: T[sorted triple] += G_mn for each of the six terms of every (m, n).
+__global__ void k_gamma_scatter(int N, int P, int U, long ldT, const int *__restrict__ triples, const double *__restrict__ G,
+                                double *__restrict__ T)
+{
+    const long e = (long)blockIdx.x * blockDim.x + threadIdx.x;
+    if (e >= (long)N * N) return;
+    const int m = (int)(e / N), n = (int)(e - (long)m * N);
+    const double g = G[e];
+    if (g == 0.0) return;
+    const int mm[3] = {triples[3 * m], triples[3 * m + 1], triples[3 * m + 2]};
+    const int nn[3] = {triples[3 * n], triples[3 * n + 1], triples[3 * n + 2]};
+    const int perm[6][3] = {{0, 1, 2}, {1, 2, 0}, {2, 0, 1}, {2, 1, 0}, {1, 0, 2}, {0, 2, 1}};
+#pragma unroll
+    for (int s = 0; s < 6; s++)
+        atomicAdd(&T[triple_at(pair_rank(mm[0], nn[perm[s][0]], P), pair_rank(mm[1], nn[perm[s][1]], P),
+                               pair_rank(mm[2], nn[perm[s][2]], P), U, ldT)],
+                  g);
+}
+
+// Adjoint of the contraction over nodes: part[z][a][k] = sum over pairs r = (v, t) of split z of
+//   mult(a; {a, v, t}) T[{a, v, t}] X_v(k) X_t(k),
+// mult the number of times a stands in the sorted triple (d/dX_a of X_u X_v X_t).  Tile 32 a x 64 k,
+// 16 pairs per stage; one FP64 FMA per (a, r, k), the products X_v X_t formed once per tile.
+__global__ void __launch_bounds__(256) k_triple_vjp(int U, int UV, int K, int rper, const double *__restrict__ XT,
+                                                    const double *__restrict__ T, double *__restrict__ part)
+{
+    __shared__ __align__(16) double sC[TP_KC][TP_BU];
+    __shared__ double sY[TP_KC][TP_BV];
+    const int tid = threadIdx.x, lane = tid & 31, warp = tid >> 5;
+    const int k0 = blockIdx.x * TP_BV, a0 = blockIdx.y * TP_BU;
+    const int r0 = blockIdx.z * rper, r1 = min(UV, r0 + rper);
+    const int kc = min(k0 + (tid & 63), K - 1), ac = min(a0 + lane, U - 1);
+    double acc[4][2];
+#pragma unroll
+    for (int i = 0; i < 4; i++) acc[i][0] = acc[i][1] = 0.0;
+    for (int rb = r0; rb < r1; rb += TP_KC) {
+        __syncthreads();
+#pragma unroll
+        for (int i = 0; i < 2; i++) {
+            const int r = rb + warp + 8 * i;
+            double c = 0.0;
+            if (r < r1) {
+                int v, t;
+                tri_unrank(r, U, v, t);
+                c = T[triple_at(ac, v, t, U, UV)] * (double)(1 + (ac == v) + (ac == t));
+            }
+            sC[warp + 8 * i][lane] = c;
+        }
+#pragma unroll
+        for (int i = 0; i < 4; i++) {
+            const int r = rb + (tid >> 6) + 4 * i;
+            double y = 0.0;
+            if (r < r1) {
+                int v, t;
+                tri_unrank(r, U, v, t);
+                y = XT[(size_t)v * K + kc] * XT[(size_t)t * K + kc];
+            }
+            sY[(tid >> 6) + 4 * i][tid & 63] = y;
+        }
+        __syncthreads();
+        const int rn = min(TP_KC, r1 - rb);
+#pragma unroll 4
+        for (int rr = 0; rr < rn; rr++) {
+            const double2 ca = *reinterpret_cast<const double2 *>(&sC[rr][4 * warp]);
+            const double2 cb = *reinterpret_cast<const double2 *>(&sC[rr][4 * warp + 2]);
+            const double c[4] = {ca.x, ca.y, cb.x, cb.y}, y0 = sY[rr][lane], y1 = sY[rr][lane + 32];
+#pragma unroll
+            for (int i = 0; i < 4; i++) {
+                acc[i][0] = fma(c[i], y0, acc[i][0]);
+                acc[i][1] = fma(c[i], y1, acc[i][1]);
+            }
+        }
+    }
+    part += (size_t)blockIdx.z * U * K;
+#pragma unroll
+    for (int i = 0; i < 4; i++) {
+        const int a = a0 + 4 * warp + i;
+        if (a >= U) break;
+#pragma unroll
+        for (int c = 0; c < 2; c++)
+            if (k0 + lane + 32 * c < K) part[(size_t)a * K + k0 + lane + 32 * c] = acc[i][c];
+    }
+}
+
+// dX[k][u] = w_k/(48 pi) sum over the splits of part[z][u][k]
+__global__ void k_triple_vjp_sum(int U, int K, int Z, const double *__restrict__ w, const double *__restrict__ part,
+                                 double *__restrict__ dX)
+{
+    const long e = (long)blockIdx.x * blockDim.x + threadIdx.x;
+    if (e >= (long)U * K) return;
+    const int u = (int)(e / K), k = (int)(e - (long)u * K);
+    double s = 0.0;
+    for (int z = 0; z < Z; z++) s += part[(size_t)z * U * K + e];
+    dX[(size_t)k * U + u] = w[k] / (48e0 * 3.14159265358979323846) * s;
+}
+
 }  // namespace
 
 bool triple_wins(double pairs, double U)
@@ -211,6 +318,33 @@ modal_status gamma_triple_dev(modal_ctx *ctx, int mu0, int nmu, const double *wg
     MODAL_TRY(triple_dev(ctx, U, nmu, kper, X, Z, T, U * UV));
     MODAL_TRY(triple_sum_dev(ctx, U * UV, Zn, U * UV, T));
     return gamma_gather_dev(ctx, U, T);
+}
+
+// dX[nmu][U] = dL/dX of Gamma's M entries for an upstream G[N][N] = dL/dGamma (device).
+modal_status gamma_triple_vjp_dev(modal_ctx *ctx, const double *G, double *dX)
+{
+    const int P = ctx->P, U = P * (P + 1) / 2, K = ctx->nmu, N = ctx->N;
+    const size_t UV = (size_t)U * (U + 1) / 2;
+    int nsm = 0;
+    MODAL_CUDA(cudaDeviceGetAttribute(&nsm, cudaDevAttrMultiProcessorCount, ctx->device));
+    // pair splits: about six CTAs per SM
+    const long tiles = (long)ceil_div(K, TP_BV) * ceil_div(U, TP_BU);
+    const int want = (int)std::max<long>(1, std::min<long>(std::min<long>(32, ceil_div((long)UV, 4 * TP_KC)), 6L * nsm / tiles));
+    const int rper = ceil_div(ceil_div((long)UV, want), TP_KC) * TP_KC, Zn = ceil_div((long)UV, rper);
+    auto al = [](size_t b) { return (b + 255) & ~(size_t)255; };
+    const size_t ox = al(sizeof(double) * U * UV), op = ox + al(sizeof(double) * (size_t)U * K);
+    MODAL_TRY(ensure(ctx->trip, op + sizeof(double) * Zn * (size_t)U * K));
+    uint8_t *b = ctx->trip.as<uint8_t>();
+    double *T = reinterpret_cast<double *>(b), *XT = reinterpret_cast<double *>(b + ox), *part = reinterpret_cast<double *>(b + op);
+    MODAL_CUDA(cudaMemsetAsync(T, 0, sizeof(double) * U * UV, ctx->stream));
+    k_gamma_scatter<<<ceil_div((long)N * N, 256), 256, 0, ctx->stream>>>(N, P, U, (long)UV, ctx->triples.as<int>(), G, T);
+    MODAL_TRY(launched(ctx, "gamma_scatter"));
+    k_triple_cols<<<ceil_div((long)K * U, 256), 256, 0, ctx->stream>>>(K, U, P, ctx->mt.as<double>(), XT);
+    MODAL_TRY(launched(ctx, "triple_cols"));
+    k_triple_vjp<<<dim3(ceil_div(K, TP_BV), ceil_div(U, TP_BU), Zn), 256, 0, ctx->stream>>>(U, (int)UV, K, rper, XT, T, part);
+    MODAL_TRY(launched(ctx, "triple_vjp"));
+    k_triple_vjp_sum<<<ceil_div((long)K * U, 256), 256, 0, ctx->stream>>>(U, K, Zn, ctx->w.as<double>(), part, dX);
+    return launched(ctx, "triple_vjp_sum");
 }
 
 }  // namespace modal

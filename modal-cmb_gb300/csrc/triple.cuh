@@ -47,5 +47,6 @@ modal_status triple_sum_dev(modal_ctx *ctx, size_t n, int Z, size_t zstride, dou
 // ctx->gamma from T[U][U(U+1)/2].
 modal_status gamma_gather_dev(modal_ctx *ctx, int U, const double *T);
 modal_status gamma_triple_dev(modal_ctx *ctx, int mu0, int nmu, const double *wg);
+modal_status gamma_triple_vjp_dev(modal_ctx *ctx, const double *G, double *dX);
 
 }  // namespace modal
