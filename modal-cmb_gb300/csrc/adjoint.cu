@@ -44,6 +44,8 @@ constexpr double kInv48Pi = 1.0 / (48.0 * 3.14159265358979323846);
 // vecs holds per-l rows [nvec][L].  Tile: 64 mu nodes x 32 columns, 16 l per stage.
 constexpr int AJ_BK = 64, AJ_BC = 32, AJ_LC = 16;
 
+// FOLD: antisymmetric nodes, even and odd l summed apart at the first half of the nodes (as mij_tile).
+template <bool FOLD>
 __global__ void __launch_bounds__(256) k_lcontract(int nmu, int lmin, int lmax, int ncol, const double *__restrict__ pl,
                                                    const double *__restrict__ vecs, const int *__restrict__ ca,
                                                    const int *__restrict__ cb, double *__restrict__ out)
@@ -52,16 +54,17 @@ __global__ void __launch_bounds__(256) k_lcontract(int nmu, int lmin, int lmax, 
     __shared__ double sV[AJ_LC][AJ_BC];
     const int tid = threadIdx.x, tx = tid & 31, ty = tid >> 5;
     const int k0 = blockIdx.x * AJ_BK, c0 = blockIdx.y * AJ_BC;
-    const int L = lmax - lmin + 1;
-    double acc[8];
+    constexpr int NA = FOLD ? 2 : 1;
+    const int L = lmax - lmin + 1, nk = FOLD ? (nmu + 1) / 2 : nmu;
+    double acc[NA][8];
 #pragma unroll
-    for (int r = 0; r < 8; r++) acc[r] = 0.0;
+    for (int r = 0; r < 8; r++) acc[0][r] = acc[NA - 1][r] = 0.0;
     for (int l0 = 0; l0 < L; l0 += AJ_LC) {
 #pragma unroll
         for (int t = 0; t < (AJ_LC * AJ_BK) / 256; t++) {
             const int e = tid + 256 * t, lr = e / AJ_BK, kc = e % AJ_BK;
             const int l = l0 + lr, k = k0 + kc;
-            sPl[lr][kc] = (l < L && k < nmu) ? pl[(size_t)(lmin + l) * nmu + k] : 0.0;
+            sPl[lr][kc] = (l < L && k < nk) ? pl[(size_t)(lmin + l) * nmu + k] : 0.0;
         }
 #pragma unroll
         for (int t = 0; t < (AJ_LC * AJ_BC) / 256; t++) {
@@ -74,7 +77,7 @@ __global__ void __launch_bounds__(256) k_lcontract(int nmu, int lmin, int lmax, 
         for (int lr = 0; lr < AJ_LC; lr++) {
             const double vv = sV[lr][tx];
 #pragma unroll
-            for (int r = 0; r < 8; r++) acc[r] = fma(sPl[lr][ty + 8 * r], vv, acc[r]);
+            for (int r = 0; r < 8; r++) acc[lr & (NA - 1)][r] = fma(sPl[lr][ty + 8 * r], vv, acc[lr & (NA - 1)][r]);
         }
         __syncthreads();
     }
@@ -83,7 +86,10 @@ __global__ void __launch_bounds__(256) k_lcontract(int nmu, int lmin, int lmax, 
 #pragma unroll
     for (int r = 0; r < 8; r++) {
         const int k = k0 + ty + 8 * r;
-        if (k < nmu) out[(size_t)k * ncol + c] = acc[r];
+        if (k >= nk) continue;
+        const double E = acc[(lmin & 1) ? NA - 1 : 0][r], O = FOLD ? acc[(lmin & 1) ? 0 : NA - 1][r] : 0.0;
+        out[(size_t)k * ncol + c] = FOLD ? E + O : acc[0][r];
+        if (FOLD && nmu - 1 - k != k) out[(size_t)(nmu - 1 - k) * ncol + c] = E - O;
     }
 }
 
@@ -301,6 +307,45 @@ __global__ void __launch_bounds__(BV_T) k_beta_vjp(int nmu, int P, int E, int st
     }
 }
 
+// In place over the rows of D[nmu][ncol]: row k < nmu / 2 becomes D_k + D_{nmu-1-k}, row nmu-1-k becomes
+// D_{nmu-1-k} - D_k; a middle row stays.
+__global__ void k_fold_nodes(int nmu, int ncol, double *__restrict__ D)
+{
+    const long e = (long)blockIdx.x * blockDim.x + threadIdx.x;
+    if (e >= (long)(nmu / 2) * ncol) return;
+    const long k = e / ncol, c = e - k * ncol;
+    double *a = D + k * ncol + c, *b = D + (nmu - 1 - k) * ncol + c;
+    const double x = *a, y = *b;
+    *a = x + y;
+    *b = y - x;
+}
+
+// Z[l - lmin][c] = sum_k pl[l][k] D[k][c], D overwritten.  Antisymmetric nodes: P_l(-x) = (-1)^l P_l(x)
+// leaves the sums (even l) or differences (odd l) of mirrored rows against half the nodes.
+modal_status pl_contract(modal_ctx *c, int ncol, double *D, double *Z)
+{
+    const int nmu = c->nmu, L = c->L, lmin = c->lmin;
+    const double *pl = c->pl.as<double>() + (size_t)lmin * nmu;
+    if (!c->gl_sym) return dgemm_splitk(c, L, ncol, nmu, pl, nmu, false, D, ncol, false, Z, ncol, 0, false);
+    k_fold_nodes<<<ceil_div((long)(nmu / 2) * ncol, 256), 256, 0, c->stream>>>(nmu, ncol, D);
+    MODAL_TRY(launched(c, "fold_nodes"));
+    for (int p = 0; p < 2; p++) {
+        const int rows = (L - p + 1) / 2, even = !((lmin + p) & 1);
+        // even l: the sums against the first half, the middle included; odd l: the differences against
+        // the second half (the middle value is zero)
+        const int K = even ? (nmu + 1) / 2 : nmu / 2;
+        if (rows <= 0) continue;
+        double *z = Z + (size_t)p * ncol;
+        const double *a = pl + (size_t)p * nmu + (even ? 0 : nmu - nmu / 2), *d = D + (even ? 0 : (size_t)(nmu - nmu / 2) * ncol);
+        if (K <= 0) {
+            MODAL_CUDA(cudaMemset2DAsync(z, sizeof(double) * 2 * ncol, 0, sizeof(double) * ncol, rows, c->stream));
+            continue;
+        }
+        MODAL_TRY(dgemm_splitk(c, rows, ncol, K, a, 2 * nmu, false, d, ncol, false, z, 2 * ncol, 0, false));
+    }
+    return MODAL_OK;
+}
+
 // dq[l][r] += sum_c Z[l][(r, c)] q[l][c], the diagonal pair twice      (Z = pl^T dX, one column per pair)
 __global__ void k_dq_pairs(int L, int P, int U, const double *__restrict__ Z, const double *__restrict__ q,
                            double *__restrict__ dq)
@@ -465,11 +510,14 @@ modal_status adj_forward(modal_ctx *c, int S, const modal_shape *shapes, AdjFwd 
         L, lmin, P, E, c->q.as<double>(), wl, reinterpret_cast<const double *>(b + o_tab),
         reinterpret_cast<const long *>(b + o_loff), f.vecs);
     MODAL_TRY(launched(c, "adj_vecs"));
-    const dim3 g1(ceil_div(nmu, AJ_BK), ceil_div(ncol, AJ_BC));
+    const dim3 g1(ceil_div(c->gl_sym ? (nmu + 1) / 2 : nmu, AJ_BK), ceil_div(ncol, AJ_BC));
     if (g1.y > 65535) { set_error("adjoint: %d projection columns exceed one launch", ncol); return MODAL_ERR_ARG; }
-    k_lcontract<<<g1, 256, 0, c->stream>>>(nmu, lmin, lmax, ncol, c->pl.as<double>(), f.vecs,
-                                           reinterpret_cast<const int *>(b + o_ca),
-                                           reinterpret_cast<const int *>(b + o_cb), f.BK);
+    auto contract = [&](auto kern) {
+        kern<<<g1, 256, 0, c->stream>>>(nmu, lmin, lmax, ncol, c->pl.as<double>(), f.vecs,
+                                        reinterpret_cast<const int *>(b + o_ca), reinterpret_cast<const int *>(b + o_cb), f.BK);
+    };
+    if (c->gl_sym) contract(k_lcontract<true>);
+    else contract(k_lcontract<false>);
     MODAL_TRY(launched(c, "lcontract_legs"));
     f.li.nshape = S;
     f.li.P = P;
@@ -481,7 +529,7 @@ modal_status adj_forward(modal_ctx *c, int S, const modal_shape *shapes, AdjFwd 
     // one thread per (shape, mode) alone fills a fifth of the GPU at 32 shapes and 364 modes: split the nodes
     int nsm = 0;
     MODAL_CUDA(cudaDeviceGetAttribute(&nsm, cudaDevAttrMultiProcessorCount, c->device));
-    const int Zn = (int)std::max<long>(1, std::min<long>(std::min(16, nmu / 64), 8L * nsm / ((long)ceil_div(N, 128) * S)));
+    const int Zn = (int)std::max<long>(1, std::min<long>(std::min(4, nmu / 64), 8L * nsm / ((long)ceil_div(N, 128) * S)));
     MODAL_TRY(ensure(c->trip, sizeof(double) * (size_t)Zn * S * N));
     const dim3 g2(ceil_div(N, 128), S, Zn);
     k_beta_gl<<<g2, 128, 0, c->stream>>>(N, nmu, f.li, c->triples.as<int>(), c->w.as<double>(), f.BK, c->trip.as<double>());
@@ -508,8 +556,7 @@ modal_status gamma_vjp_dev(modal_ctx *c, const double *G, double *dq)
         double *dX = c->adj2.as<double>(), *Z = dX + (size_t)nmu * U;
         const modal_status st = gamma_triple_vjp_dev(c, G, dX);
         if (st == MODAL_OK) {
-            MODAL_TRY(dgemm_splitk(c, L, U, nmu, c->pl.as<double>() + (size_t)c->lmin * nmu, nmu, false, dX, U, false, Z, U, 0,
-                                   false));
+            MODAL_TRY(pl_contract(c, U, dX, Z));
             k_dq_pairs<<<ceil_div((long)L * P, 256), 256, 0, c->stream>>>(L, P, U, Z, c->q.as<double>(), dq);
             return launched(c, "dq_pairs");
         }
@@ -524,8 +571,7 @@ modal_status gamma_vjp_dev(modal_ctx *c, const double *G, double *dq)
                                                c->pl.as<double>(), c->q.as<double>(), c->w.as<double>(), G, dM);
     MODAL_TRY(launched(c, "gamma_vjp"));
     // Z[l][pq] = sum_k pl[lmin+l][k] dM[k][pq]
-    MODAL_TRY(dgemm(c, L, PP, nmu, 1.0, c->pl.as<double>() + (size_t)c->lmin * nmu, nmu, false, dM, PP, false, 0.0, Z,
-                    PP, 0));
+    MODAL_TRY(pl_contract(c, PP, dM, Z));
     k_dq_gamma<<<ceil_div((long)L * P, 256), 256, 0, c->stream>>>(L, P, Z, c->q.as<double>(), dq);
     return launched(c, "dq_gamma");
 }
@@ -551,8 +597,7 @@ modal_status beta_vjp_dev(modal_ctx *c, const AdjFwd &f, const double *Gb, doubl
     k_beta_vjp<<<dim3(ceil_div(nmu, BV_T), E / 3), BV_T, vs, c->stream>>>(nmu, P, E, f.li.stride, f.term_shape, f.term_leg, f.BK,
                                                                          c->w.as<double>(), Gs, dB);
     MODAL_TRY(launched(c, "beta_vjp"));
-    MODAL_TRY(dgemm(c, L, EP, nmu, 1.0, c->pl.as<double>() + (size_t)c->lmin * nmu, nmu, false, dB, EP, false, 0.0,
-                    Z2, EP, 0));
+    MODAL_TRY(pl_contract(c, EP, dB, Z2));
     k_dq_beta<<<ceil_div((long)L * P, 256), 256, 0, c->stream>>>(L, P, E, Z2, f.vecs + (size_t)P * L, dq);
     return launched(c, "dq_beta");
 }

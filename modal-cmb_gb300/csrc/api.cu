@@ -361,6 +361,8 @@ modal_status modal_set_gl(modal_ctx *c, int nmu, const double *nodes, const doub
     MODAL_TRY(h2d(c, c->mu, nodes, sizeof(double) * nmu));
     MODAL_TRY(h2d(c, c->w, weights, sizeof(double) * nmu));
     c->gl_n = -1;
+    c->gl_sym = true;
+    for (int k = 0; k < nmu && c->gl_sym; k++) c->gl_sym = nodes[k] == -nodes[nmu - 1 - k];
     MODAL_TRY(sync(c));
     c->have_user_gl = true;
     c->have_glint = c->have_gamma = c->have_ortho = false;
@@ -382,6 +384,7 @@ modal_status modal_init_glint(modal_ctx *c)
             StageTimer t(c, MODAL_T_GL);
             MODAL_TRY(gl_nodes_dev(c, c->nmu, c->mu.as<double>(), c->w.as<double>()));
             c->gl_n = c->nmu;
+            c->gl_sym = true;
         }
     }
     MODAL_TRY(ensure(c->pl, sizeof(double) * (size_t)(lmax_all + 1) * c->nmu));

@@ -79,6 +79,7 @@ struct modal_ctx {
     void *split_ptr = nullptr;
     size_t split_bytes = 0;
     int gl_n = -1;             // n of the GPU quadrature held in mu/w (-1: none or caller-supplied)
+    bool gl_sym = false;       // nodes exactly antisymmetric: mu[n-1-k] = -mu[k] (the l-contractions fold the halves)
 
     // late x primordial transfer Gamma
     int tr_Pp = 0, tr_xsize = 0, tr_Nprim = 0;

@@ -15,26 +15,30 @@
 namespace modal {
 
 // --------------------------------------------------------------------------
-// l-contraction, FP64 SIMT GEMM over l: out tile 8R (mu) x 32 (p<=q pairs),
-// bound by the FP64 pipe (the tile's loads hide behind it).  Summation over l in
-// ascending order, as the reference, whatever the tile.
+// l-contraction, FP64 SIMT GEMM over l: out tile 8R (mu) x 32 (p<=q pairs), bound by the FP64 pipe
+// (the tile's loads hide behind it).  FOLD: the quadrature is antisymmetric, so with
+// P_l(-x) = (-1)^l P_l(x) (exact in the table) the sums over even and over odd l at the first half of
+// the nodes give both halves, E + O and E - O, at half the FMAs; else the sum over l in ascending
+// order, as the reference.
 // --------------------------------------------------------------------------
 constexpr int MIJ_BU = 32, MIJ_LC = 16;
 
-template <int R>
-__device__ __forceinline__ void mij_tile(int nmu, int lmin, int lmax, int P, int npair,
-                                                  const double *__restrict__ pl, const double *__restrict__ q,
-                                                  const int2 *__restrict__ pairs, double *__restrict__ mt)
+template <int R, bool FOLD>
+__device__ __forceinline__ void mij_tile(int nmu, int lmin, int lmax, int P, int npair, const double *__restrict__ pl,
+                                         const double *__restrict__ q, const int2 *__restrict__ pairs,
+                                         double *__restrict__ mt)
 {
-    constexpr int MIJ_BK = 8 * R;
+    constexpr int MIJ_BK = 8 * R, NA = FOLD ? 2 : 1;
     __shared__ double sPl[MIJ_LC][MIJ_BK];
     __shared__ double sV[MIJ_LC][MIJ_BU];
     const int tid = threadIdx.x, tx = tid & 31, ty = tid >> 5;
-    const int k0 = blockIdx.x * MIJ_BK, u0 = blockIdx.y * MIJ_BU;
+    const int k0 = blockIdx.x * MIJ_BK, u0 = blockIdx.y * MIJ_BU, nk = FOLD ? (nmu + 1) / 2 : nmu;
     const int L = lmax - lmin + 1;
-    double acc[R];
+    double acc[NA][R];
 #pragma unroll
-    for (int r = 0; r < R; r++) acc[r] = 0.0;
+    for (int p = 0; p < NA; p++)
+#pragma unroll
+        for (int r = 0; r < R; r++) acc[p][r] = 0.0;
 
     for (int l0 = 0; l0 < L; l0 += MIJ_LC) {
 #pragma unroll
@@ -43,7 +47,7 @@ __device__ __forceinline__ void mij_tile(int nmu, int lmin, int lmax, int P, int
             if (e >= MIJ_LC * MIJ_BK) break;
             int lr = e / MIJ_BK, kc = e % MIJ_BK;
             int l = l0 + lr, k = k0 + kc;
-            sPl[lr][kc] = (l < L && k < nmu) ? pl[(size_t)(lmin + l) * nmu + k] : 0.0;
+            sPl[lr][kc] = (l < L && k < nk) ? pl[(size_t)(lmin + l) * nmu + k] : 0.0;
         }
 #pragma unroll
         for (int t = 0; t < (MIJ_LC * MIJ_BU) / 256; t++) {
@@ -61,20 +65,29 @@ __device__ __forceinline__ void mij_tile(int nmu, int lmin, int lmax, int P, int
         for (int lr = 0; lr < MIJ_LC; lr++) {
             double vv = sV[lr][tx];
 #pragma unroll
-            for (int r = 0; r < R; r++) acc[r] = fma(sPl[lr][ty + 8 * r], vv, acc[r]);
+            for (int r = 0; r < R; r++) acc[lr & (NA - 1)][r] = fma(sPl[lr][ty + 8 * r], vv, acc[lr & (NA - 1)][r]);
         }
         __syncthreads();
     }
     const int u = u0 + tx;
     if (u >= npair) return;
     const int2 pq = pairs[u];
+    auto put = [&](int k, double v) {
+        double *blk = mt + (size_t)k * P * P;
+        blk[pq.x * P + pq.y] = v;
+        blk[pq.y * P + pq.x] = v;
+    };
 #pragma unroll
     for (int r = 0; r < R; r++) {
-        int k = k0 + ty + 8 * r;
-        if (k < nmu) {
-            double *blk = mt + (size_t)k * P * P;
-            blk[pq.x * P + pq.y] = acc[r];
-            blk[pq.y * P + pq.x] = acc[r];
+        const int k = k0 + ty + 8 * r;
+        if (k >= nk) continue;
+        if (!FOLD) {
+            put(k, acc[0][r]);
+        } else {
+            // the sums start at lmin: acc[0] holds its parity
+            const double E = acc[(lmin & 1) ? NA - 1 : 0][r], O = acc[(lmin & 1) ? 0 : NA - 1][r];
+            put(k, E + O);
+            if (nmu - 1 - k != k) put(nmu - 1 - k, E - O);
         }
     }
 }
@@ -85,7 +98,7 @@ __global__ void __launch_bounds__(256) k_mij_fp64(int nmu, int lmin, int lmax, i
                                                   const double *__restrict__ q, const int2 *__restrict__ pairs,
                                                   double *__restrict__ mt)
 {
-    mij_tile<8>(nmu, lmin, lmax, P, npair, pl, q, pairs, mt);
+    mij_tile<8, false>(nmu, lmin, lmax, P, npair, pl, q, pairs, mt);
 }
 
 template <int R>
@@ -93,7 +106,14 @@ __global__ void __launch_bounds__(256) k_mij_fp64_r(int nmu, int lmin, int lmax,
                                                     const double *__restrict__ pl, const double *__restrict__ q,
                                                     const int2 *__restrict__ pairs, double *__restrict__ mt)
 {
-    mij_tile<R>(nmu, lmin, lmax, P, npair, pl, q, pairs, mt);
+    mij_tile<R, false>(nmu, lmin, lmax, P, npair, pl, q, pairs, mt);
+}
+
+__global__ void __launch_bounds__(256) k_mij_fp64_fold(int nmu, int lmin, int lmax, int P, int npair,
+                                                       const double *__restrict__ pl, const double *__restrict__ q,
+                                                       const int2 *__restrict__ pairs, double *__restrict__ mt)
+{
+    mij_tile<8, true>(nmu, lmin, lmax, P, npair, pl, q, pairs, mt);
 }
 
 // M table [nmu][P][P] of a basis q[L][P] on lmin..lmax (T or E) into out.
@@ -111,15 +131,20 @@ modal_status mij_table_dev(modal_ctx *ctx, const double *q, int lmin, int lmax, 
     delete[] h;
     if (e != cudaSuccess) { set_error("mij pairs: %s", cudaGetErrorString(e)); return MODAL_ERR_CUDA; }
     // smaller mu tiles until there are two CTAs per SM: with 24 CTAs (l <= 500, P = 10) the 64-node tile
-    // took 295 us, the FP64 pipe of 128 SMs idle
+    // took 295 us, the FP64 pipe of 128 SMs idle.  Folded where half the nodes still fill the GPU with
+    // full tiles (l <= 2000, P = 30: 6.1 -> 3.1 ms); below that it would only leave fewer CTAs, and the
+    // sum keeps the reference's order.
     int nsm = 0, R = 8;
     MODAL_CUDA(cudaDeviceGetAttribute(&nsm, cudaDevAttrMultiProcessorCount, ctx->device));
-    while (R > 1 && (long)ceil_div(ctx->nmu, 8 * R) * ceil_div(npair, MIJ_BU) < 2L * nsm) R /= 2;
+    const bool fold = ctx->gl_sym && (long)ceil_div((ctx->nmu + 1) / 2, 64) * ceil_div(npair, MIJ_BU) >= 2L * nsm;
+    const int nk = fold ? (ctx->nmu + 1) / 2 : ctx->nmu;
+    while (R > 1 && (long)ceil_div(nk, 8 * R) * ceil_div(npair, MIJ_BU) < 2L * nsm) R /= 2;
     auto run = [&](auto kern) {
-        kern<<<dim3(ceil_div(ctx->nmu, 8 * R), ceil_div(npair, MIJ_BU)), 256, 0, ctx->stream>>>(
+        kern<<<dim3(ceil_div(nk, 8 * R), ceil_div(npair, MIJ_BU)), 256, 0, ctx->stream>>>(
             ctx->nmu, lmin, lmax, P, npair, ctx->pl.as<double>(), q, ctx->scratch.as<int2>(), out.as<double>());
     };
-    if (R == 8) run(k_mij_fp64);
+    if (fold) run(k_mij_fp64_fold);
+    else if (R == 8) run(k_mij_fp64);
     else if (R == 4) run(k_mij_fp64_r<4>);
     else if (R == 2) run(k_mij_fp64_r<2>);
     else run(k_mij_fp64_r<1>);

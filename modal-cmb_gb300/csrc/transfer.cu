@@ -76,29 +76,31 @@ constexpr int TR_BK = 64, TR_BU = 32, TR_LC = 16;
 
 // With v2/qt2 (polarised E side): the transfer factor is v_l qt - v2_l qt2.
 // qt and qt2 rows have stride qstride (lmax_T + 1).
+// FOLD: antisymmetric nodes, even and odd l summed apart at the first half of the nodes (as mij_tile).
+template <bool FOLD>
 __global__ void __launch_bounds__(256) k_mij_transfer(int nmu, int lmin, int lmax, int P, int Pp,
                                                       const double *__restrict__ pl, const double *__restrict__ q,
                                                       const double *__restrict__ v, const double *__restrict__ qt,
-                                                      double *__restrict__ mt2, const double *__restrict__ v2 = nullptr,
-                                                      const double *__restrict__ qt2 = nullptr, int qstride = 0)
+                                                      double *__restrict__ mt2, const double *__restrict__ v2,
+                                                      const double *__restrict__ qt2, int qstride)
 {
+    constexpr int NA = FOLD ? 2 : 1;
     __shared__ double sPl[TR_LC][TR_BK];
     __shared__ double sV[TR_LC][TR_BU];
     const int tid = threadIdx.x, tx = tid & 31, ty = tid >> 5;
     const int k0 = blockIdx.x * TR_BK, u0 = blockIdx.y * TR_BU, xi = blockIdx.z;
-    const int L = lmax - lmin + 1, nu = Pp * P;
-    if (qstride == 0) qstride = lmax + 1;
+    const int L = lmax - lmin + 1, nu = Pp * P, nk = FOLD ? (nmu + 1) / 2 : nmu;
     const double *qtx = qt + (size_t)xi * Pp * qstride;
     const double *qtx2 = qt2 ? qt2 + (size_t)xi * Pp * qstride : nullptr;
-    double acc[8];
+    double acc[NA][8];
 #pragma unroll
-    for (int r = 0; r < 8; r++) acc[r] = 0.0;
+    for (int r = 0; r < 8; r++) acc[0][r] = acc[NA - 1][r] = 0.0;
     for (int l0 = 0; l0 < L; l0 += TR_LC) {
 #pragma unroll
         for (int t = 0; t < (TR_LC * TR_BK) / 256; t++) {
             int e = tid + 256 * t, lr = e / TR_BK, kc = e % TR_BK;
             int l = l0 + lr, k = k0 + kc;
-            sPl[lr][kc] = (l < L && k < nmu) ? pl[(size_t)(lmin + l) * nmu + k] : 0.0;
+            sPl[lr][kc] = (l < L && k < nk) ? pl[(size_t)(lmin + l) * nmu + k] : 0.0;
         }
 #pragma unroll
         for (int t = 0; t < (TR_LC * TR_BU) / 256; t++) {
@@ -118,7 +120,7 @@ __global__ void __launch_bounds__(256) k_mij_transfer(int nmu, int lmin, int lma
         for (int lr = 0; lr < TR_LC; lr++) {
             double vv = sV[lr][tx];
 #pragma unroll
-            for (int r = 0; r < 8; r++) acc[r] = fma(sPl[lr][ty + 8 * r], vv, acc[r]);
+            for (int r = 0; r < 8; r++) acc[lr & (NA - 1)][r] = fma(sPl[lr][ty + 8 * r], vv, acc[lr & (NA - 1)][r]);
         }
         __syncthreads();
     }
@@ -126,8 +128,11 @@ __global__ void __launch_bounds__(256) k_mij_transfer(int nmu, int lmin, int lma
     if (u >= nu) return;
 #pragma unroll
     for (int r = 0; r < 8; r++) {
-        int k = k0 + ty + 8 * r;
-        if (k < nmu) mt2[((size_t)xi * nmu + k) * nu + u] = acc[r];
+        const int k = k0 + ty + 8 * r;
+        if (k >= nk) continue;
+        const double E = acc[(lmin & 1) ? NA - 1 : 0][r], O = FOLD ? acc[(lmin & 1) ? 0 : NA - 1][r] : 0.0;
+        mt2[((size_t)xi * nmu + k) * nu + u] = FOLD ? E + O : acc[0][r];
+        if (FOLD && nmu - 1 - k != k) mt2[((size_t)xi * nmu + nmu - 1 - k) * nu + u] = E - O;
     }
 }
 
@@ -293,6 +298,20 @@ __global__ void __launch_bounds__(256) k_gamma_transfer_pol(int N, int Nprim, in
 
 using namespace modal;
 
+// mt2 of the late basis q on lmin..lmax; the transfer factor is v qt, or v qt - v2 qt2.
+static modal_status mij_transfer_dev(modal_ctx *c, int lmin, int lmax, int P, const double *q, const double *v,
+                                     const double *qt, double *mt2, const double *v2, const double *qt2)
+{
+    const int nu = c->tr_Pp * P, nk = c->gl_sym ? (c->nmu + 1) / 2 : c->nmu;
+    const dim3 g(ceil_div(nk, TR_BK), ceil_div(nu, TR_BU), c->tr_xsize);
+    auto run = [&](auto kern) {
+        kern<<<g, 256, 0, c->stream>>>(c->nmu, lmin, lmax, P, c->tr_Pp, c->pl.as<double>(), q, v, qt, mt2, v2, qt2, c->lmax + 1);
+    };
+    if (c->gl_sym) run(k_mij_transfer<true>);
+    else run(k_mij_transfer<false>);
+    return launched(c, "mij_transfer");
+}
+
 extern "C" modal_status modal_set_transfer(modal_ctx *c, int Pp, int xsize, const double *xvec, const double *qtilde,
                                            int Nprim, const int *prim)
 {
@@ -345,10 +364,8 @@ extern "C" modal_status modal_gamma_transfer(modal_ctx *c, double deltaphi, doub
     StageTimer t(c, MODAL_T_GAMMA);
     k_transfer_weight<<<ceil_div(c->lmax + 1, 256), 256, 0, c->stream>>>(c->lmax, c->cl.as<double>(), c->tr_v.as<double>());
     MODAL_TRY(launched(c, "transfer_weight"));
-    dim3 gm(ceil_div(nmu, TR_BK), ceil_div(nu, TR_BU), xsize);
-    k_mij_transfer<<<gm, 256, 0, c->stream>>>(nmu, c->lmin, c->lmax, P, Pp, c->pl.as<double>(), c->q.as<double>(),
-                                              c->tr_v.as<double>(), c->tr_qt.as<double>(), c->tr_mt.as<double>());
-    MODAL_TRY(launched(c, "mij_transfer"));
+    MODAL_TRY(mij_transfer_dev(c, c->lmin, c->lmax, P, c->q.as<double>(), c->tr_v.as<double>(), c->tr_qt.as<double>(),
+                               c->tr_mt.as<double>(), nullptr, nullptr));
     int KC = (96 * 1024) / (nu * 8);
     if (KC < 1) KC = 1;
     if (KC > 32) KC = 32;
@@ -457,15 +474,11 @@ extern "C" modal_status modal_gamma_transfer_pol(modal_ctx *c, double deltaphi, 
     StageTimer t(c, MODAL_T_GAMMA);
     k_transfer_weight<<<ceil_div(c->lmax + 1, 256), 256, 0, c->stream>>>(c->lmax, c->cl.as<double>(), c->tr_v.as<double>());
     MODAL_TRY(launched(c, "transfer_weight"));
-    dim3 gT(ceil_div(nmu, TR_BK), ceil_div(nuT, TR_BU), xsize), gE(ceil_div(nmu, TR_BK), ceil_div(nuE, TR_BU), xsize);
-    k_mij_transfer<<<gT, 256, 0, c->stream>>>(nmu, c->lmin, c->lmax, P, Pp, c->pl.as<double>(), c->q.as<double>(),
-                                              c->tr_v.as<double>(), c->tr_qt.as<double>(), c->tr_mt.as<double>());
-    MODAL_TRY(launched(c, "mij_transfer"));
+    MODAL_TRY(mij_transfer_dev(c, c->lmin, c->lmax, P, c->q.as<double>(), c->tr_v.as<double>(), c->tr_qt.as<double>(),
+                               c->tr_mt.as<double>(), nullptr, nullptr));
     const double *wq = c->tr_we.as<double>(), *wl = wq + (c->lmax + 1);
-    k_mij_transfer<<<gE, 256, 0, c->stream>>>(nmu, c->lmin_e, c->lmax_e, PE, Pp, c->pl.as<double>(), c->qe.as<double>(),
-                                              wq, c->tr_qte.as<double>(), c->tr_mte.as<double>(), wl,
-                                              c->tr_qt.as<double>(), c->lmax + 1);
-    MODAL_TRY(launched(c, "mij_transfer_e"));
+    MODAL_TRY(mij_transfer_dev(c, c->lmin_e, c->lmax_e, PE, c->qe.as<double>(), wq, c->tr_qte.as<double>(),
+                               c->tr_mte.as<double>(), wl, c->tr_qt.as<double>()));
     int nsm = 0;
     MODAL_CUDA(cudaDeviceGetAttribute(&nsm, cudaDevAttrMultiProcessorCount, c->device));
     const long tiles = (long)ceil_div(Nprim, 32) * ceil_div(N, 32);

@@ -277,7 +277,7 @@ int triple_splits(const modal_ctx *ctx, int U, long K)
     // tiles with work: about a third of all, never fewer than one column of them; six CTAs per SM
     // even out the last wave, and a split costs one more pass over T
     const long tiles = std::max<long>(ceil_div(UV, TP_BV), (long)ceil_div(UV, TP_BV) * ceil_div(U, TP_BU) / 3);
-    return (int)std::max<long>(1, std::min<long>(std::min<long>(ceil_div(K, 4 * TP_KC), 32), 6L * nsm / tiles));
+    return (int)std::max<long>(1, std::min<long>(std::min<long>(ceil_div(K, 8 * TP_KC), 32), 6L * nsm / tiles));
 }
 
 modal_status triple_dev(modal_ctx *ctx, int U, int K, int kper, const double *X, const double *Z, double *T, size_t zstride)
