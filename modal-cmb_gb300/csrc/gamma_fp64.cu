@@ -244,7 +244,7 @@ modal_status gamma_fp64_dev(modal_ctx *ctx, int mu0, int nmu)
     k_wgt48<<<ceil_div(nmu, 256), 256, 0, ctx->stream>>>(nmu, ctx->w.as<double>() + mu0, ctx->scratch2.as<double>());
     MODAL_TRY(launched(ctx, "wgt48"));
     // the distinct products of three M entries, or (few modes of a large basis) the permanents of the
-    // pairs: full lists at l <= 2000 take 102 ms on the first against 645 ms on the second at P = 30
+    // pairs: full lists at l <= 2000 take 98 ms on the first against 665 ms on the second at P = 30
     if (triple_wins(0.5 * N * (N + 1.0), 0.5 * P * (P + 1.0))) {
         const modal_status st = gamma_triple_dev(ctx, mu0, nmu, ctx->scratch2.as<double>());
         if (st != MODAL_ERR_NOMEM) return st;

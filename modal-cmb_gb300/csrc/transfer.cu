@@ -16,6 +16,7 @@
 #include <cmath>
 #include <vector>
 #include "common.cuh"
+#include "triple.cuh"
 
 namespace modal {
 
@@ -215,6 +216,55 @@ __global__ void k_sum_groups(long n, int G, long stride, double *__restrict__ ou
     out[e] = s;
 }
 
+// The transfer Gamma from the distinct products of three M entries (triple.cu, U = Pp P entries per
+// node and radial sample).  The spline integral is linear, so the samples x >= 10 form one sum over
+// (x, k) with weights c_x x^2 w_k, T_sum; each of the first ten keeps its own T_x, because the reference
+// drops y_x there when |y_x| > 1e-18 (calculate_gamma.c:803-804).
+// w2[xi nmu + k] = x^2 w_k for the first nx samples, c_x x^2 w_k beyond
+__global__ void k_transfer_node_weights(int nmu, int xsize, int nx, const double *__restrict__ w,
+                                        const double *__restrict__ xvec, const double *__restrict__ cx,
+                                        double *__restrict__ w2)
+{
+    const long e = (long)blockIdx.x * blockDim.x + threadIdx.x;
+    if (e >= (long)nmu * xsize) return;
+    const int xi = (int)(e / nmu), k = (int)(e - (long)xi * nmu);
+    const double x2 = xvec[xi] * xvec[xi];
+    w2[e] = (xi < nx ? x2 : cx[xi] * x2) * w[k];
+}
+
+// out[m][n]: six entries of T_sum and, one x at a time, of the first nx tables with the zero rule.
+// T: [nx] tables of the first samples, then T_sum (if last), zstride apart.
+__global__ void __launch_bounds__(256) k_transfer_gather(int N, int Nprim, int P, int U, long ldT, int nx, int last, size_t zstride,
+                                                         const int *__restrict__ triples, const int *__restrict__ prim,
+                                                         const double *__restrict__ cx, const double *__restrict__ T,
+                                                         double scale, double *__restrict__ out)
+{
+    const long e = (long)blockIdx.x * blockDim.x + threadIdx.x;
+    if (e >= (long)N * Nprim) return;
+    const int m = (int)(e / Nprim), n = (int)(e - (long)m * Nprim);
+    const int q[3] = {triples[3 * m], triples[3 * m + 1], triples[3 * m + 2]};
+    const int p[3] = {prim[3 * n] * P, prim[3 * n + 1] * P, prim[3 * n + 2] * P};
+    const int perm[6][3] = {{0, 1, 2}, {1, 2, 0}, {2, 0, 1}, {2, 1, 0}, {1, 0, 2}, {0, 2, 1}};
+    size_t at[6];
+#pragma unroll
+    for (int s = 0; s < 6; s++) at[s] = triple_at(p[0] + q[perm[s][0]], p[1] + q[perm[s][1]], p[2] + q[perm[s][2]], U, ldT);
+    double res = 0.0;
+    for (int x = 0; x < nx; x++) {
+        double y = 0.0;
+#pragma unroll
+        for (int s = 0; s < 6; s++) y += T[x * zstride + at[s]];
+        if (fabs(y) > 1e-18) y = 0.0;
+        res = fma(cx[x], y, res);
+    }
+    if (last) {
+        double y = 0.0;
+#pragma unroll
+        for (int s = 0; s < 6; s++) y += T[(size_t)nx * zstride + at[s]];
+        res += y;
+    }
+    out[e] = res * scale;
+}
+
 // Polarised points (gamma_2d_pt_TTE/TEE/EEE, calculate_gamma.c:558-687): the
 // 3x3 block has rows = primordial legs and columns = late legs, column b taken
 // from the T table (b < nT: FORM 1 TTE nT = 2, FORM 2 TEE nT = 1) or the E
@@ -312,6 +362,36 @@ static modal_status mij_transfer_dev(modal_ctx *c, int lmin, int lmax, int P, co
     return launched(c, "mij_transfer");
 }
 
+// tr_out[N][Nprim] from the distinct products.
+static modal_status transfer_triple_dev(modal_ctx *c, double scale)
+{
+    const int xsize = c->tr_xsize, nmu = c->nmu, U = c->tr_Pp * c->P, N = c->N, Nprim = c->tr_Nprim;
+    const int nx = std::min(10, xsize), K2 = (xsize - nx) * nmu;
+    const size_t UV = (size_t)U * (U + 1) / 2, n = U * UV;
+    const int kper = K2 > 0 ? ceil_div(K2, triple_splits(c, U, K2)) : 1, Zn = K2 > 0 ? ceil_div(K2, kper) : 0;
+    const long K = (long)xsize * nmu;
+    auto al = [](size_t b) { return (b + 255) & ~(size_t)255; };
+    const size_t oz = al(sizeof(double) * K * U), ow = 2 * oz, ot = ow + al(sizeof(double) * K);
+    MODAL_TRY(ensure(c->trip, ot + sizeof(double) * (nx + Zn) * n));
+    uint8_t *b = c->trip.as<uint8_t>();
+    double *X = reinterpret_cast<double *>(b), *Z = reinterpret_cast<double *>(b + oz), *w2 = reinterpret_cast<double *>(b + ow),
+           *T = reinterpret_cast<double *>(b + ot);
+    const double *cx = c->tr_x.as<double>() + xsize;
+    k_transfer_node_weights<<<ceil_div(K, 256), 256, 0, c->stream>>>(nmu, xsize, nx, c->w.as<double>(), c->tr_x.as<double>(), cx, w2);
+    MODAL_TRY(launched(c, "transfer_node_weights"));
+    MODAL_TRY(triple_rows_dev(c, K, U, 0, c->tr_mt.as<double>(), U, w2, X, Z));
+    MODAL_TRY(triple_dev(c, U, nx * nmu, nmu, X, Z, T, n));
+    if (K2 > 0) {
+        const size_t o = (size_t)nx * nmu * U;
+        MODAL_TRY(triple_dev(c, U, K2, kper, X + o, Z + o, T + nx * n, n));
+        MODAL_TRY(triple_sum_dev(c, n, Zn, n, T + nx * n));
+    }
+    k_transfer_gather<<<ceil_div((long)N * Nprim, 256), 256, 0, c->stream>>>(
+        N, Nprim, c->P, U, (long)UV, nx, K2 > 0, n, c->triples.as<int>(), c->tr_prim.as<int>(), cx, T, scale,
+        c->tr_out.as<double>());
+    return launched(c, "transfer_gather");
+}
+
 extern "C" modal_status modal_set_transfer(modal_ctx *c, int Pp, int xsize, const double *xvec, const double *qtilde,
                                            int Nprim, const int *prim)
 {
@@ -366,11 +446,29 @@ extern "C" modal_status modal_gamma_transfer(modal_ctx *c, double deltaphi, doub
     MODAL_TRY(launched(c, "transfer_weight"));
     MODAL_TRY(mij_transfer_dev(c, c->lmin, c->lmax, P, c->q.as<double>(), c->tr_v.as<double>(), c->tr_qt.as<double>(),
                                c->tr_mt.as<double>(), nullptr, nullptr));
+    const double scale = deltaphi * deltaphi / (8.0 * 3.14159265358979323846);
+    auto finish = [&]() -> modal_status {
+        t.stop();
+        if (gamma_t)
+            MODAL_CUDA(cudaMemcpyAsync(gamma_t, c->tr_out.ptr, sizeof(double) * (size_t)N * Nprim, cudaMemcpyDeviceToHost,
+                                       c->stream));
+        MODAL_CUDA(cudaStreamSynchronize(c->stream));
+        return MODAL_OK;
+    };
     int KC = (96 * 1024) / (nu * 8);
     if (KC < 1) KC = 1;
     if (KC > 32) KC = 32;
     const size_t smem = sizeof(double) * ((size_t)KC + (size_t)KC * nu);
     if (smem > 200 * 1024) { set_error("modal_gamma_transfer: Pp*P=%d too large for the tile", nu); return MODAL_ERR_ARG; }
+    // the distinct products, or (few modes) the permanents of the pairs: 816 x 120 modes at P = 16, Pp = 8,
+    // 32 samples and l <= 600 take 24 ms on the first, 55 ms on the second.  Up to eleven and a few more
+    // tables of 8 U^2 (U+1) / 2 bytes: at most 16 GB
+    if (triple_wins((double)N * Nprim, nu) && 4.0 * nu * nu * (nu + 1.0) * 42 <= 16e9 &&
+        (double)xsize * nmu * nu < 2e9) {
+        const modal_status st = transfer_triple_dev(c, scale);
+        if (st == MODAL_OK) return finish();
+        if (st != MODAL_ERR_NOMEM) return st;
+    }
     MODAL_CUDA(cudaFuncSetAttribute(k_gamma_transfer, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem));
     // the (primordial x late) tiles alone fill about two thirds of the SMs at the
     // benchmark sizes: split the radial samples into groups so that the grid holds
@@ -384,7 +482,6 @@ extern "C" modal_status modal_gamma_transfer(modal_ctx *c, double deltaphi, doub
     XG = ceil_div(xsize, xs);
     MODAL_TRY(ensure(c->tr_out, sizeof(double) * (size_t)XG * N * Nprim));
     dim3 gg(ceil_div(Nprim, 32), ceil_div(N, 32), XG);
-    const double scale = deltaphi * deltaphi / (8.0 * 3.14159265358979323846);
     k_gamma_transfer<<<gg, 256, smem, c->stream>>>(N, Nprim, P, Pp, nmu, xsize, xs, KC, c->triples.as<int>(),
                                                    c->tr_prim.as<int>(), c->tr_mt.as<double>(), c->w.as<double>(),
                                                    c->tr_x.as<double>(), c->tr_x.as<double>() + xsize, scale,
@@ -395,12 +492,7 @@ extern "C" modal_status modal_gamma_transfer(modal_ctx *c, double deltaphi, doub
         k_sum_groups<<<ceil_div(n, 256), 256, 0, c->stream>>>(n, XG, n, c->tr_out.as<double>());
         MODAL_TRY(launched(c, "sum_groups"));
     }
-    t.stop();
-    if (gamma_t)
-        MODAL_CUDA(cudaMemcpyAsync(gamma_t, c->tr_out.ptr, sizeof(double) * (size_t)N * Nprim, cudaMemcpyDeviceToHost,
-                                   c->stream));
-    MODAL_CUDA(cudaStreamSynchronize(c->stream));
-    return MODAL_OK;
+    return finish();
 }
 
 // E-side weights of calculate_gamma.c:142-183 on the host, divided by the

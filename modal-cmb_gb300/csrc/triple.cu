@@ -12,7 +12,9 @@
 // Bound: the FP64 pipe, one warp instruction per 16 cycles and SM on GB300, which hides every load
 // of these kernels; so the tiles only serve to keep the number of FP64 instructions near one per
 // product: 32 u x 64 (v,t) per CTA, the products Z_v X_t formed once per tile (1/32 extra), tiles
-// with no u <= v skipped.  l <= 2000, P = 30 (U = 465): 1.7e7 products, 5.3e10 FMAs.
+// with no u <= v skipped, and within a tile the warps (4 u each) with none.
+// Measured: l <= 2000, P = 30 (U = 465, 1.7e7 products, 5.1e10 FMAs): a new basis in 98 ms, 665 ms by
+// permanents.
 #include <algorithm>
 #include <cmath>
 #include <vector>
@@ -83,7 +85,7 @@ __global__ void __launch_bounds__(256) k_triple(int U, int UV, int K, int kper, 
         for (int i = 0; i < 4; i++) sY[(tid >> 6) + 4 * i][tid & 63] = rz[i] * ry[i];
         __syncthreads();
         if (kb + TP_KC < k1) fetch(kb + TP_KC);
-        const int kn = min(TP_KC, k1 - kb);
+        const int kn = u0 + 4 * warp <= vl ? min(TP_KC, k1 - kb) : 0;  // a warp past every v leaves the pipe to the others
 #pragma unroll 4
         for (int kk = 0; kk < kn; kk++) {
             const double2 xa = *reinterpret_cast<const double2 *>(&sX[kk][4 * warp]);
