@@ -7,11 +7,12 @@
 // 1. Householder tridiagonalisation A = Q T Q^T (lower, blocked; the algorithm
 //    of LAPACK's dsytrd/dlatrd).  Each panel of TRD_NB columns is one
 //    cooperative launch, one CTA per SM, each CTA owning a block of rows kept
-//    in shared memory; the CTAs meet at a grid barrier twice per column: (a) finish the previous column's w vector and update the
-//    next column with the panel's rank-2c correction, reduce its norm; (b)
-//    form the reflector and the product y = A v over the trailing matrix (the
-//    matrix-vector product that bounds this stage, summed in double-float
-//    FP32 arithmetic over a (head, tail) copy of the trailing matrix).  After
+//    in shared memory; the CTAs meet at a grid barrier twice per column: (a) finish
+//    the previous column's w vector, update the next column with the panel's
+//    rank-2c correction, reduce its norm and its products with the panel; (b)
+//    form the reflector and the product y = A v over the trailing matrix (summed
+//    in double-float FP32 arithmetic over a (head, tail) copy of the trailing
+//    matrix) while four warps form the FP64 sums that the next column needs.  After
 //    a panel, A22 -= V W^T + W V^T on the lower triangle as an FP64-accurate
 //    tensor-core product (ozgemm.cu), and the trailing block's double-float
 //    copy is refreshed from it.
@@ -41,8 +42,9 @@ namespace {
 
 constexpr int TRD_NB = 32;                 // panel width
 constexpr int DC_DEFL_SMEM = 216 * 1024;    // shared memory of the deflation's serial loop (bytes)
-constexpr int TRD_THREADS = 512;           // 16 warps per CTA
+constexpr int TRD_THREADS = 512;           // 16 warps per CTA for the matrix-vector product
 constexpr int TRD_WARPS = TRD_THREADS / 32;
+constexpr int TRD_AUX = 128;               // 4 more for the panel's own sums
 constexpr int VLD = TRD_NB + 1;            // shared-memory row stride of V, W (odd: no bank conflicts across rows)
 constexpr int LDP = 2 * TRD_NB;            // panel row: V (TRD_NB columns) then W
 constexpr int PCOMP = 2 * TRD_NB + 2;      // partial components: p[NB], q[NB], y.v, |x|^2
@@ -74,22 +76,17 @@ __device__ __forceinline__ double warp_max(double v)
     return v;
 }
 
-// Grid barrier for a cooperative launch (all CTAs co-resident), one per phase:
-// bar[0] counts arrivals, bar[1] is the generation.  Measured faster here
-// than per-CTA flag words that every CTA polls (152 x 152 pollers on a few L2
-// lines).  Memory ordering by release/acquire atomics at GPU scope instead of
-// full fences: each CTA's arrival is an acq_rel add (its writes, ordered before
-// it by __syncthreads, are released; the last arrival acquires every earlier
-// one), the last arrival releases the generation, the others acquire it.
-// Bounded: a wait that runs out of its clock64 budget sets *err, and every CTA
-// returns false once *err is set.
-__device__ __forceinline__ unsigned atom_add_acq_rel_gpu(unsigned *p, unsigned v)
-{
-    unsigned old;
-    asm volatile("atom.add.acq_rel.gpu.global.u32 %0, [%1], %2;" : "=r"(old) : "l"(p), "r"(v) : "memory");
-    return old;
-}
-
+// Grid barrier for a cooperative launch (all CTAs co-resident): one counter that
+// only grows.  A CTA's arrival is a releasing add of one (its writes, ordered
+// before it by __syncthreads), and the CTA waits until the counter, read with
+// acquire, reaches `target`: the arrivals of every barrier so far, which the caller
+// counts across launches.  An arrival and a poll are all that lie on the path: 1,500
+// cycles (27 CTAs) to 2,350 (152), where a counter that the last arrival resets, a
+// generation word that it then raises and an error word read in every poll cost 3,000
+// more.  Flag words or packets per CTA that every CTA polls are slower: 4,600 cycles at
+// 52 CTAs and 8,400 at 152 (152 x 152 pollers on a few L2 lines).
+// Bounded: a wait that runs out of its clock64 budget sets *err; the others look at
+// *err every 256 polls, and every CTA returns false.
 __device__ __forceinline__ unsigned ld_acquire_gpu(const unsigned *p)
 {
     unsigned v;
@@ -97,28 +94,28 @@ __device__ __forceinline__ unsigned ld_acquire_gpu(const unsigned *p)
     return v;
 }
 
-__device__ bool grid_barrier(unsigned *bar, int *err)
+__device__ __forceinline__ bool grid_barrier(unsigned *bar, unsigned target, int *err)
 {
+    __shared__ int s_ok;
     __syncthreads();
     if (threadIdx.x == 0) {
-        const unsigned g = ld_acquire_gpu(bar + 1);
-        const unsigned arrived = atom_add_acq_rel_gpu(bar, 1u);
-        if (arrived == gridDim.x - 1) {
-            atomicExch(bar, 0u);
-            atom_add_acq_rel_gpu(bar + 1, 1u);
-        } else {
-            const long long t0 = clock64();
-            while (ld_acquire_gpu(bar + 1) == g) {
-                if (*(volatile int *)err) break;
-                if (clock64() - t0 > BAR_CYCLES) {
-                    atomicExch(err, 1);
-                    break;
-                }
+        asm volatile("red.release.gpu.global.add.u32 [%0], 1;" :: "l"(bar) : "memory");
+        int ok = 1;
+        unsigned polls = 0;
+        const long long t0 = clock64();
+        while ((int)(ld_acquire_gpu(bar) - target) < 0) {
+            if (++polls & 255) continue;
+            if (*(volatile int *)err) { ok = 0; break; }
+            if (clock64() - t0 > BAR_CYCLES) {
+                atomicExch(err, 1);
+                ok = 0;
+                break;
             }
         }
+        s_ok = ok;
     }
     __syncthreads();
-    return *(volatile int *)err == 0;
+    return s_ok != 0;
 }
 
 // ------------------------------------------------------------------ stage 1
@@ -132,30 +129,29 @@ struct TrdArgs {
     double *d, *e, *tau;
     double *a, *y;  // [n] work vectors
     double *part;   // [PCOMP][grid] per-CTA partial sums
-    unsigned *bar;  // grid barrier: arrivals, generation
+    unsigned *bar;  // grid barrier: arrivals so far
+    unsigned bar0;  // arrivals of the launches before this one
     int *err;
 };
 
-// Sum over the grid of component `comp` of the partials, by one warp (fixed order).
+// Sum over the grid of component `comp` of the partials, by one warp (fixed order:
+// two chains per lane; six loads in flight).
 __device__ __forceinline__ double grid_total(const double *part, int comp, int lane)
 {
-    double s0 = 0.0, s1 = 0.0;
-    const double *p = part + (size_t)comp * gridDim.x;
-    int b = lane;
-    for (; b + 32 < (int)gridDim.x; b += 64) {
-        s0 += p[b];
-        s1 += p[b + 32];
+    const int G = gridDim.x;
+    double s[2] = {0.0, 0.0};
+    const double *p = part + (size_t)comp * G;
+    for (int b0 = 0; b0 < G; b0 += 192) {
+        double v[6];
+#pragma unroll
+        for (int u = 0; u < 6; u++) v[u] = b0 + lane + 32 * u < G ? p[b0 + lane + 32 * u] : 0.0;
+#pragma unroll
+        for (int u = 0; u < 6; u++)
+            if (b0 + 32 * u < G) s[u & 1] += v[u];
     }
-    if (b < (int)gridDim.x) s0 += p[b];
-    return warp_sum(s0 + s1);
+    return warp_sum(s[0] + s[1]);
 }
 
-// Panel of the tridiagonalisation (dlatrd, lower) as one cooperative launch.
-// The CTA owns a fixed block of rows [rb0, rb1) of [j0, n) for the whole panel
-// and keeps their V, W, y and updated-column entries in shared memory; only
-// reductions over all rows and the head row of each reflector go through
-// global memory.  Shared memory: v (n doubles) | V rows | W rows (R x NB each) | y | a.
-// x = head + tail with |x - head - tail| <= 2^-48 |x|
 // (head, tail) floats of x: the bits of (RN(x), RN(x - RN(x))), by integer
 // arithmetic where it covers x (dfbits.cuh), else by FP64 conversions
 __device__ __forceinline__ float2 df_split(double x)
@@ -166,322 +162,336 @@ __device__ __forceinline__ float2 df_split(double x)
     return make_float2(h, __double2float_rn(x - (double)h));
 }
 
-__global__ void __launch_bounds__(TRD_THREADS, 1) k_trd_panel(TrdArgs g)
+// Panel of the tridiagonalisation (dlatrd, lower) as one cooperative launch.
+// The CTA owns a fixed block of rows [rb0, rb1) of [j0, n) for the whole panel
+// and keeps their V, W, y and updated-column entries in shared memory; only
+// reductions over all rows and the head row of each reflector go through
+// global memory.  Shared memory: v (n doubles) | V rows | W rows (R x NB each) | y | a |
+// the rows' sums | the rows' products.
+//
+// What bounds it: the bytes of the trailing matrix in the product (19,400 cycles per
+// column on average over n = 4,960, 3,300 over n = 816), and the chain of FP64 sums and
+// two grid barriers around it (an FP64 operation takes 65 cycles, its warp instruction
+// 16 cycles of an SM's pipe, so an instruction that 16 warps repeat costs 256).  With
+// v = (1, scale a), p = V^T v and q = W^T v are sums over the updated column a, which is
+// known before the first barrier: they are summed there with |a|^2, and everything that
+// follows from them - p.q, the head row's correction, each row's V q + W p and the next
+// column's update but for its last term - is formed by four warps of their own while the
+// others stream the matrix.  After the product only y.v crosses the grid, and each row's
+// FP64 arithmetic is one thread's, once.  The sums between the barriers by all warps, with
+// the slower barrier, took 136.6 ms over the 155 panels of n = 4,960; this 94.1 ms.
+__global__ void __launch_bounds__(TRD_THREADS + TRD_AUX, 1) k_trd_panel(TrdArgs g)
 {
     extern __shared__ double sm[];
-    __shared__ double s_pq[2 * TRD_NB + 2];
-    __shared__ double s_vi[TRD_NB], s_wi[TRD_NB];
-    __shared__ double s_red[TRD_WARPS];
-    __shared__ double s_scal[4];
-    __shared__ double s_pp[8][2 * TRD_NB + 1];  // partial dot products per row group
+    __shared__ double s_pq[2 * TRD_NB];  // p, q of the current reflector
+    __shared__ double s_vw[2 * TRD_NB];  // V, W of the next column's row
+    __shared__ double s_scal[8];
+    __shared__ double s_pp[8][2 * TRD_NB];  // partial dot products per row group
+    enum { KYV = 0, WHEAD = 1, SCALE = 2, TAU = 3, PQ = 4, HV = 5 };
 
     const int n = g.n, tid = threadIdx.x, lane = tid & 31, warp = tid >> 5;
     const int G = gridDim.x, b = blockIdx.x;
     const int R = (n - g.j0 + G - 1) / G;
     const int rb0 = min(n, g.j0 + b * R), rb1 = min(n, rb0 + R);
     float *svh = reinterpret_cast<float *>(sm), *svl = svh + n;  // the column a as head, tail (v = scale a)
-    double *Vs = sm + n, *Ws = Vs + (size_t)R * VLD, *ys = Ws + (size_t)R * VLD, *as = ys + R;
-    for (int e = tid; e < 2 * R * VLD; e += blockDim.x) Vs[e] = 0.0;
+    double *Vs = sm + n, *Ws = Vs + (size_t)R * VLD, *ys = Ws + (size_t)R * VLD, *as = ys + R, *pas = as + R,
+           *pbs = pas + R;
+    float2 *yhl = reinterpret_cast<float2 *>(pbs + R);  // the rows' products as (head, tail)
+#pragma unroll 1
+    for (int e = tid; e < 2 * R * VLD; e += TRD_THREADS + TRD_AUX) Vs[e] = 0.0;
     __syncthreads();
 
-    double apre = 0.0;  // this thread's row of the next column of A, loaded one phase early
+    if (*(volatile int *)g.err) return;  // an earlier panel gave up
+    unsigned arrived = g.bar0;
+    const int at = tid - TRD_THREADS;  // the auxiliary warps' thread number
+    double apre = 0.0;  // an auxiliary thread's row of the next column of A, loaded one phase early
     for (int c = 0; c <= g.nbp; c++) {
         const int i = g.j0 + c;  // column reduced now; head row of reflector c - 1
-        const int x0 = max(rb0, i);
-        double nrm = 0.0;
-        // ---------------- phase X: finish w of column c - 1, update column i
+        const int cp = c - 1, x0 = max(rb0, i);
+        // ---------------- phase X: w of column c - 1, column i, and their sums over the rows
         if (c > 0) {
-            const int cp = c - 1;
-            const int ncomp = 2 * cp + 1;
-            // the head row's V, W entries and y, loaded before the reduction so that their
-            // latency overlaps it (written before the last grid barrier)
-            double vi = 0.0, wi = 0.0, yi = 0.0, taup = 0.0;
             if (warp == 0) {
-                if (lane < c) {
-                    vi = g.V[(size_t)i * LDP + lane];
-                    wi = g.W[(size_t)i * LDP + lane];
-                }
-                yi = g.y[i];
-                taup = g.tau[i - 1];
-            }
-            {   // grid sums of the previous phase's partials, 8 threads per component
-                const int ci = tid >> 3, sub = tid & 7;
-                double s = 0.0;
-                if (ci < ncomp) {
-                    const int comp = ci < cp ? ci : (ci < 2 * cp ? TRD_NB + (ci - cp) : 2 * TRD_NB);
-                    const double *pp = g.part + (size_t)comp * G;
-                    // four independent chains (GB300's FP64 additions have a long latency)
-                    double s4[4] = {0.0, 0.0, 0.0, 0.0};
-                    int bb = sub;
-                    for (; bb + 24 < G; bb += 32)
-#pragma unroll
-                        for (int u = 0; u < 4; u++) s4[u] += pp[bb + 8 * u];
-                    if (bb < G) s4[0] += pp[bb];
-                    if (bb + 8 < G) s4[1] += pp[bb + 8];
-                    if (bb + 16 < G) s4[2] += pp[bb + 16];
-                    s = (s4[0] + s4[1]) + (s4[2] + s4[3]);
-                }
-                s += __shfl_xor_sync(0xffffffffu, s, 1);
-                s += __shfl_xor_sync(0xffffffffu, s, 2);
-                s += __shfl_xor_sync(0xffffffffu, s, 4);
-                if (ci < ncomp && sub == 0) s_pq[ci] = s;  // p[0..cp), q[0..cp), y.v
-            }
-            __syncthreads();
-            const double *p = s_pq, *q = s_pq + cp;
-            if (warp == 0) {
-                double pq = 0.0, hv = 0.0;
-                if (lane < cp) {
-                    pq = p[lane] * q[lane];
-                    hv = vi * q[lane] + wi * p[lane];
-                }
-                pq = warp_sum(pq);
-                hv = warp_sum(hv);
-                const double yvc = s_pq[2 * cp] - 2.0 * pq;  // (corrected y).v
+                const double yi = g.y[i], tau = s_scal[TAU];
+                const double yv = grid_total(g.part, 2 * TRD_NB, lane) - 2.0 * s_scal[PQ];  // (corrected y).v
+                const double kyv = 0.5 * tau * tau * yv;
                 // w of row i (head row: v = 1 there), computed by every CTA alike
-                const double whead = taup * (yi - hv) - 0.5 * taup * taup * yvc;
-                if (lane == 0) { s_scal[0] = yvc; s_scal[1] = whead; s_scal[3] = taup; }
-                if (c < g.nbp && lane < c) {
-                    s_vi[lane] = vi;
-                    s_wi[lane] = (lane == cp) ? whead : wi;
-                }
+                if (lane == 0) { s_scal[KYV] = kyv; s_scal[WHEAD] = tau * (yi - s_scal[HV]) - kyv; }
             }
             __syncthreads();
-            const double taup_all = s_scal[3];
-            const double yvc = s_scal[0], whead = s_scal[1];
-            // four threads per row: the row's w entry and its updated column entry, each a sum
-            // over the panel's columns, the threads taking every fourth term in two chains and
-            // adding through two shuffles (short FP64 dependency chains on few warps: the FP64
-            // pipe of an SM takes one warp instruction per 16 cycles on GB300)
-            const int nrows = rb1 - x0, sub = tid & 3;
-            for (int rb = 0; rb < nrows; rb += TRD_THREADS / 4) {
-                const int rr = rb + (tid >> 2), r = x0 + rr;
-                const bool ok = rr < nrows;
-                const int lr = ok ? r - rb0 : 0;
-                const double *Vr = Vs + (size_t)lr * VLD, *Wr = Ws + (size_t)lr * VLD;
-                double a0 = 0.0, a1 = 0.0;
-                if (ok)
-                    for (int t = sub; t < cp; t += 8) {
-                        a0 = fma(Vr[t], q[t], fma(Wr[t], p[t], a0));
-                        if (t + 4 < cp) a1 = fma(Vr[t + 4], q[t + 4], fma(Wr[t + 4], p[t + 4], a1));
-                    }
-                double pa = a0 + a1;
-                pa += __shfl_xor_sync(0xffffffffu, pa, 1);
-                pa += __shfl_xor_sync(0xffffffffu, pa, 2);
-                const double wr = ok ? ((r == i) ? whead : taup_all * (ys[lr] - pa) - 0.5 * taup_all * taup_all * yvc * Vr[cp]) : 0.0;
+        }
+        if (at >= 0) {  // a thread per row
+            const double kyv = s_scal[KYV], whead = s_scal[WHEAD], tau = s_scal[TAU];
+#pragma unroll 1
+            for (int r = x0 + at; r < rb1; r += TRD_AUX) {
+                const int lr = r - rb0;
+                double pb = 0.0;
+                if (c > 0) {
+                    const double vc = Vs[(size_t)lr * VLD + cp];
+                    const double wr = (r == i) ? whead : tau * (ys[lr] - pas[lr]) - kyv * vc;
+                    Ws[(size_t)lr * VLD + cp] = wr;
+                    g.W[(size_t)r * LDP + cp] = wr;
+                    pb = pbs[lr] + fma(vc, whead, wr);  // v of row i is 1 in the last column
+                }
                 if (c < g.nbp) {
-                    double b0 = 0.0, b1 = 0.0;
-                    if (ok)
-                        for (int t = sub; t < c; t += 8) {
-                            b0 = fma(Vr[t], s_wi[t], fma(t == cp ? wr : Wr[t], s_vi[t], b0));
-                            if (t + 4 < c) b1 = fma(Vr[t + 4], s_wi[t + 4], fma(t + 4 == cp ? wr : Wr[t + 4], s_vi[t + 4], b1));
+                    const double x = ((r == x0 + at && c > 0) ? apre : g.A[(size_t)r * n + i]) - pb;
+                    as[lr] = x;
+                    g.a[r] = x;
+                    g.ahl[r] = df_split(x);
+                }
+            }
+        }
+        if (c == g.nbp) break;
+        __syncthreads();
+        // over this CTA's rows below the next head row: |x|^2, and V[:, t].x, W[:, t].x (t < c),
+        // all components at once: thread (group gq of 8, component), the groups added through
+        // shared memory
+        const int z0 = max(rb0, i + 2);
+        if (at < 0) {
+            const int gq = tid >> 6, comp = tid & 63;
+            const double *col = comp < TRD_NB ? Vs + comp : Ws + (comp - TRD_NB);
+            if ((comp & 31) < c) {
+                double sp = 0.0;
+#pragma unroll 1
+                for (int lr = z0 + gq - rb0; lr < rb1 - rb0; lr += 8) sp = fma(col[(size_t)lr * VLD], as[lr], sp);
+                s_pp[gq][comp] = sp;
+            }
+        } else if (warp == TRD_WARPS) {
+            double s = 0.0;
+#pragma unroll 1
+            for (int lr = z0 + lane - rb0; lr < rb1 - rb0; lr += 32) s = fma(as[lr], as[lr], s);
+            s = warp_sum(s);
+            if (lane == 0) g.part[(size_t)(2 * TRD_NB + 1) * G + b] = s;
+        }
+        if (c > 0) {
+            __syncthreads();
+            if (tid < 2 * TRD_NB && (tid & 31) < c)
+                g.part[(size_t)tid * G + b] = ((s_pp[0][tid] + s_pp[1][tid]) + (s_pp[2][tid] + s_pp[3][tid])) +
+                                              ((s_pp[4][tid] + s_pp[5][tid]) + (s_pp[6][tid] + s_pp[7][tid]));
+        }
+        if (!grid_barrier(g.bar, arrived += G, g.err)) return;
+
+        // ---------------- phase Y: reflector of column i, y = A v on the trailing matrix
+        const int m = n - i - 1;  // trailing size
+        const int y0 = max(rb0, i + 1);
+        if (at >= 0) {
+            // the auxiliary warps, while the others form the product: p = V^T v, q = W^T v, and for
+            // the rows what the next column's w and update take from the columns before this one
+            if (c + 1 < g.nbp && y0 + at < rb1) apre = g.A[(size_t)(y0 + at) * n + i + 1];
+            const int comp = at >> 1, half = at & 1;
+            const bool on = (comp & 31) < c;
+            double s = 0.0, head = 0.0;
+            if (on) {
+                head = g.V[(size_t)(i + 1) * LDP + comp];  // V, then W, of row i + 1 (where v is 1)
+                const double *pp = g.part + (size_t)comp * G;
+                double s4[4] = {0.0, 0.0, 0.0, 0.0};
+#pragma unroll 1
+                for (int b0 = half; b0 < G; b0 += 32) {  // sixteen loads in flight, four chains
+                    double v[16];
+#pragma unroll
+                    for (int u = 0; u < 16; u++) v[u] = b0 + 2 * u < G ? pp[b0 + 2 * u] : 0.0;
+#pragma unroll
+                    for (int u = 0; u < 16; u++) s4[u & 3] += v[u];
+                }
+                s = (s4[0] + s4[1]) + (s4[2] + s4[3]);
+            }
+            s += __shfl_xor_sync(0xffffffffu, s, 1);
+            asm volatile("bar.sync 2, %0;" :: "n"(TRD_AUX + 32) : "memory");  // the reflector's scale
+            if (half == 0) {
+                s_pq[comp] = on ? fma(s_scal[SCALE], s, head) : 0.0;
+                s_vw[comp] = on ? head : 0.0;
+            }
+            asm volatile("bar.sync 3, %0;" :: "n"(TRD_AUX) : "memory");
+            if (warp == TRD_WARPS) {
+                const double p = s_pq[lane], q = s_pq[TRD_NB + lane];
+                const double pq = warp_sum(p * q);
+                const double hv = warp_sum(s_vw[lane] * q + s_vw[TRD_NB + lane] * p);
+                if (lane == 0) { s_scal[PQ] = pq; s_scal[HV] = hv; }
+            } else {
+                // four threads per row, each every fourth column
+                const int a1 = at - 32, sub = a1 & 3;
+#pragma unroll 1
+                for (int rr = 0; rr < rb1 - y0; rr += (TRD_AUX - 32) / 4) {
+                    const int lr = y0 - rb0 + rr + (a1 >> 2);
+                    double pa = 0.0, pb = 0.0;
+                    if (lr < rb1 - rb0) {
+                        const double *Vr = Vs + (size_t)lr * VLD, *Wr = Ws + (size_t)lr * VLD;
+#pragma unroll 2
+                        for (int t = sub; t < c; t += 4) {
+                            const double v = Vr[t], w = Wr[t];
+                            pa = fma(v, s_pq[TRD_NB + t], fma(w, s_pq[t], pa));
+                            pb = fma(v, s_vw[TRD_NB + t], fma(w, s_vw[t], pb));
                         }
-                    double pb = b0 + b1;
+                    }
+                    pa += __shfl_xor_sync(0xffffffffu, pa, 1);
                     pb += __shfl_xor_sync(0xffffffffu, pb, 1);
+                    pa += __shfl_xor_sync(0xffffffffu, pa, 2);
                     pb += __shfl_xor_sync(0xffffffffu, pb, 2);
-                    if (ok && sub == 0) {
-                        const double x = ((rb == 0) ? apre : g.A[(size_t)r * n + i]) - pb;
-                        as[lr] = x;
-                        g.a[r] = x;
-                        g.ahl[r] = df_split(x);
-                        if (r >= i + 2) nrm += x * x;
+                    if (lr < rb1 - rb0 && sub == 0) { pas[lr] = pa; pbs[lr] = pb; }
+                }
+            }
+        } else {
+            if (warp == 0) {
+                const double alpha = (lane < 2) ? g.a[i + 1] : 0.0;  // issued before the reduction
+                const double sig = grid_total(g.part, 2 * TRD_NB + 1, lane);
+                if (lane < 2) {
+                    // lane 0 divides for scale, lane 1 for tau
+                    double beta = alpha, quot = 0.0;
+                    if (sig != 0.0) {
+                        beta = -copysign(sqrt(alpha * alpha + sig), alpha);
+                        quot = (lane ? beta - alpha : 1.0) / (lane ? beta : alpha - beta);
+                    }
+                    s_scal[SCALE + lane] = quot;
+                    if (b == 0) {
+                        if (lane == 0) {
+                            g.d[i] = g.a[i];
+                            g.e[i] = beta;
+                        } else
+                            g.tau[i] = quot;
                     }
                 }
                 __syncwarp();
-                if (ok && sub == 0) {
-                    Ws[(size_t)lr * VLD + cp] = wr;
-                    g.W[(size_t)r * LDP + cp] = wr;
+                asm volatile("bar.arrive 2, %0;" :: "n"(TRD_AUX + 32) : "memory");
+            } else {
+                // v = (1, scale a[i+2..n)): the gemv uses a as double-float pairs, its rows take scale
+                // at the end; the other warps stage it meanwhile
+#pragma unroll 4
+                for (int k = tid - 32; k < m; k += TRD_THREADS - 32) {
+                    const float2 h = (k == 0) ? make_float2(0.f, 0.f) : g.ahl[i + 1 + k];
+                    svh[k] = h.x;
+                    svl[k] = h.y;
                 }
             }
-            if (c == g.nbp) break;
-        } else {
-            for (int r = x0 + tid; r < rb1; r += blockDim.x) {
-                const double x = g.A[(size_t)r * n + i];
-                as[r - rb0] = x;
-                g.a[r] = x;
-                g.ahl[r] = df_split(x);
-                if (r >= i + 2) nrm += x * x;
-            }
-        }
-        if (x0 + 8 * warp < rb1) nrm = warp_sum(nrm);  // only the warps that hold rows
-        if (lane == 0) s_red[warp] = nrm;
-        __syncthreads();
-        if (tid == 0) {
-            double s4[4];
+            asm volatile("bar.sync 1, %0;" :: "n"(TRD_THREADS) : "memory");
+            // warp per row: sum_{k>=1} A[r][i+1+k] a[i+1+k] in double-float FP32 arithmetic
+            // (products split exactly by FMA, heads added by TwoSum): about 2^-47 relative to
+            // sum |A a|, at the FP32 rate instead of GB300's FP64 rate
+            const int nrw = (rb1 - y0 - warp + TRD_WARPS - 1) / TRD_WARPS;  // this warp's rows
+#pragma unroll 1
+            for (int rk = 0; rk < nrw; rk++) {
+                const int r = y0 + warp + TRD_WARPS * ((c & 1) ? nrw - 1 - rk : rk);
+                const float2 *Ar = g.Ahl + (size_t)r * n + i + 1;
+                // elements k = kb.. as 16-byte pairs (four loads of 512 B per warp in flight);
+                // an unaligned element k = 1 and an odd last element go to lane 0
+                const int kb = (((size_t)r * n + i + 2) & 1) ? 2 : 1;
+                const int npair = (m - kb) / 2;
+                const float4 *A4 = reinterpret_cast<const float4 *>(Ar + kb);
+                const float *vbh = svh + kb, *vbl = svl + kb;  // scalar shared-memory reads (kb may be odd)
+                float sh[8], sl[8];
 #pragma unroll
-            for (int u = 0; u < 4; u++)
-                s4[u] = (s_red[u] + s_red[u + 4]) + (s_red[u + 8] + s_red[u + 12]);
-            g.part[(size_t)(2 * TRD_NB + 1) * G + b] = (s4[0] + s4[1]) + (s4[2] + s4[3]);
-        }
-        if (!grid_barrier(g.bar, g.err)) return;
-
-        // ---------------- phase Y: reflector of column i, y = A v on the trailing matrix
-        {   // the next column's A entry of this thread's row (A does not change during the panel;
-            // rows of four threads, the first keeps it)
-            const int rn = max(rb0, i + 1) + (tid >> 2);
-            if ((tid & 3) == 0 && c + 1 < g.nbp && rn < rb1) apre = g.A[(size_t)rn * n + i + 1];
-        }
-        if (warp == 0) {
-            const double alpha = (lane == 0) ? g.a[i + 1] : 0.0;  // issued before the reduction
-            const double sig = grid_total(g.part, 2 * TRD_NB + 1, lane);
-            if (lane == 0) {
-                double beta, tau, scale;
-                if (sig == 0.0) {
-                    beta = alpha; tau = 0.0; scale = 0.0;
-                } else {
-                    beta = -copysign(sqrt(alpha * alpha + sig), alpha);
-                    tau = (beta - alpha) / beta;
-                    scale = 1.0 / (alpha - beta);
-                }
-                s_scal[2] = scale;
-                if (b == 0) {
-                    g.d[i] = g.a[i];
-                    g.e[i] = beta;
-                    g.tau[i] = tau;
-                }
-            }
-        }
-        __syncthreads();
-        const double scale = s_scal[2];
-        const int m = n - i - 1;  // trailing size
-        // v = (1, scale a[i+2..n)): the gemv uses a as double-float pairs and applies scale at the end
-        for (int k = tid; k < m; k += blockDim.x) {
-            const float2 h = (k == 0) ? make_float2(0.f, 0.f) : g.ahl[i + 1 + k];
-            svh[k] = h.x;
-            svl[k] = h.y;
-        }
-        __syncthreads();
-        const int y0 = max(rb0, i + 1);
-        // warp per row: y[r] = A[r][i+1] + scale sum_{k>=1} A[r][i+1+k] a[i+1+k], the sum in
-        // double-float FP32 arithmetic (products split exactly by FMA, heads added by TwoSum):
-        // about 2^-47 relative to sum |A a|, at the FP32 rate instead of GB300's FP64 rate
-        const int nrw = (rb1 - y0 - warp + TRD_WARPS - 1) / TRD_WARPS;  // this warp's rows
-        for (int rk = 0; rk < nrw; rk++) {
-            const int r = y0 + warp + TRD_WARPS * ((c & 1) ? nrw - 1 - rk : rk);
-            const float2 *Ar = g.Ahl + (size_t)r * n + i + 1;
-            // elements k = kb.. as 16-byte pairs (four loads of 512 B per warp in flight);
-            // an unaligned element k = 1 and an odd last element go to lane 0
-            const int kb = (((size_t)r * n + i + 2) & 1) ? 2 : 1;
-            const int npair = (m - kb) / 2;
-            const float4 *A4 = reinterpret_cast<const float4 *>(Ar + kb);
-            const float *vbh = svh + kb, *vbl = svl + kb;  // scalar shared-memory reads (kb may be odd)
-            float sh[8], sl[8];
+                for (int u = 0; u < 8; u++) { sh[u] = 0.f; sl[u] = 0.f; }
+                auto acc = [&](float ah, float al, float vh, float vl, float &h, float &l) {
+                    const float p = ah * vh;
+                    float e = fmaf(ah, vh, -p);
+                    e = fmaf(ah, vl, e);
+                    e = fmaf(al, vh, e);
+                    const float t = h + p, bp = t - h;
+                    l += ((h - (t - bp)) + (p - bp)) + e;
+                    h = t;
+                };
+                // eight 16-byte loads in flight per lane, the last partial block predicated; odd
+                // columns walk the rows backwards, so they start on the data the previous column
+                // read last (still in L2)
+                const int nfull = npair / (8 * 32);
+                const bool tail = nfull * (8 * 32) < npair;
+                const bool back = c & 1;
+                auto block_tail = [&]() {  // the last partial block, four loads at a time
+#pragma unroll 1
+                    for (int h = 0; h < 2; h++) {
+                        const int j = nfull * (8 * 32) + 128 * h + lane;
+                        if (j - lane >= npair) break;
+                        float4 x[4];
 #pragma unroll
-            for (int u = 0; u < 8; u++) { sh[u] = 0.f; sl[u] = 0.f; }
-            auto acc = [&](float ah, float al, float vh, float vl, float &h, float &l) {
-                const float p = ah * vh;
-                float e = fmaf(ah, vh, -p);
-                e = fmaf(ah, vl, e);
-                e = fmaf(al, vh, e);
-                const float t = h + p, bp = t - h;
-                l += ((h - (t - bp)) + (p - bp)) + e;
-                h = t;
-            };
-            // eight 16-byte loads in flight per lane, the last partial block predicated; odd
-            // columns walk the rows backwards, so they start on the data the previous column
-            // read last (still in L2)
-            const int nfull = npair / (8 * 32);
-            auto block = [&](int jb, bool tail) {
-                const int j = jb * (8 * 32) + lane;
-                float4 x[8];
+                        for (int u = 0; u < 4; u++)
+                            x[u] = j + 32 * u < npair ? A4[j + 32 * u] : make_float4(0.f, 0.f, 0.f, 0.f);
 #pragma unroll
-                for (int u = 0; u < 8; u++)
-                    x[u] = (!tail || j + 32 * u < npair) ? A4[j + 32 * u] : make_float4(0.f, 0.f, 0.f, 0.f);
+                        for (int u = 0; u < 4; u++)
+                            if (j + 32 * u < npair) {
+                                const int e = 2 * (j + 32 * u);
+                                acc(x[u].x, x[u].y, vbh[e], vbl[e], sh[2 * u], sl[2 * u]);
+                                acc(x[u].z, x[u].w, vbh[e + 1], vbl[e + 1], sh[2 * u + 1], sl[2 * u + 1]);
+                            }
+                    }
+                };
+#pragma unroll 1
+                for (int t = 0; t < nfull + 1; t++) {
+                    const int jb = back ? nfull - t : t;
+                    if (jb == nfull) {
+                        if (tail) block_tail();
+                        continue;
+                    }
+                    const int j = jb * (8 * 32) + lane;
+                    float4 x[8];
 #pragma unroll
-                for (int u = 0; u < 8; u++) {
-                    if (!tail || j + 32 * u < npair) {
+                    for (int u = 0; u < 8; u++) x[u] = A4[j + 32 * u];
+#pragma unroll
+                    for (int u = 0; u < 8; u++) {
                         const int e = 2 * (j + 32 * u);
                         acc(x[u].x, x[u].y, vbh[e], vbl[e], sh[2 * (u & 3)], sl[2 * (u & 3)]);
                         acc(x[u].z, x[u].w, vbh[e + 1], vbl[e + 1], sh[2 * (u & 3) + 1], sl[2 * (u & 3) + 1]);
                     }
                 }
-            };
-            const bool tail = nfull * (8 * 32) < npair;
-            if (c & 1) {
-                if (tail) block(nfull, true);
-                for (int jb = nfull - 1; jb >= 0; jb--) block(jb, false);
-            } else {
-                for (int jb = 0; jb < nfull; jb++) block(jb, false);
-                if (tail) block(nfull, true);
-            }
-            if (lane == 0) {
-                if (kb == 2 && m > 1) {
-                    const float2 x = Ar[1];
-                    acc(x.x, x.y, svh[1], svl[1], sh[2], sl[2]);
-                }
-                if (kb + 2 * npair < m) {
-                    const int k = kb + 2 * npair;
-                    const float2 x = Ar[k];
-                    acc(x.x, x.y, svh[k], svl[k], sh[3], sl[3]);
-                }
-            }
-            // the lane's eight (head, tail) sums combined in double-FP32 (TwoSum), so that only
-            // one conversion and the warp sum use the FP64 pipe (one warp instruction per 16
-            // cycles of an SM on GB300)
-            float hh = sh[0], hl = sl[0];
-#pragma unroll
-            for (int u = 1; u < 8; u++) {
-                const float t = hh + sh[u], bp = t - hh;
-                const float e = ((hh - (t - bp)) + (sh[u] - bp)) + (hl + sl[u]);
-                hh = t + e;
-                hl = e - (hh - t);
-            }
-            // the warp's sum in double-FP32 as well (short FP32 dependency chains instead of
-            // FP64 ones), converted once
-#pragma unroll
-            for (int o = 16; o > 0; o >>= 1) {
-                const float oh = __shfl_xor_sync(0xffffffffu, hh, o), ol = __shfl_xor_sync(0xffffffffu, hl, o);
-                const float t = hh + oh, bp = t - hh;
-                const float e = ((hh - (t - bp)) + (oh - bp)) + (hl + ol);
-                hh = t + e;
-                hl = e - (hh - t);
-            }
-            const double ssum = (double)hh + (double)hl;
-            if (lane == 0) {
-                const float2 a0 = Ar[0];
-                const double s = fma(scale, ssum, (double)a0.x + (double)a0.y);
-                const int lr = r - rb0;
-                const double vr = (r == i + 1) ? 1.0 : as[lr] * scale;
-                ys[lr] = s;
-                g.y[r] = s;
-                Vs[(size_t)lr * VLD + c] = vr;
-                g.V[(size_t)r * LDP + c] = vr;
-            }
-        }
-        __syncthreads();
-        // partials over this CTA's rows: p_t = V[:,t].v, q_t = W[:,t].v (t < c), y.v;
-        // all components at once: thread (group gq of 8, component t), the 8 groups'
-        // sums added in order through shared memory
-        const int ncomp = 2 * c + 1;
-        {
-            const int gq = tid >> 6;
-            double sp[2] = {0.0, 0.0};
-            for (int r = y0 + gq; r < rb1; r += 8) {
-                const int lr = r - rb0;
-                const double vr = Vs[(size_t)lr * VLD + c];  // v of the row, stored with the product
-#pragma unroll
-                for (int h = 0; h < 2; h++) {
-                    const int t = (tid & 63) + 64 * h;
-                    if (t < ncomp) {
-                        const double x = t < c ? Vs[(size_t)lr * VLD + t]
-                                               : (t < 2 * c ? Ws[(size_t)lr * VLD + (t - c)] : ys[lr]);
-                        sp[h] += x * vr;
+                if (lane == 0) {
+                    if (kb == 2 && m > 1) {
+                        const float2 x = Ar[1];
+                        acc(x.x, x.y, svh[1], svl[1], sh[2], sl[2]);
+                    }
+                    if (kb + 2 * npair < m) {
+                        const int k = kb + 2 * npair;
+                        const float2 x = Ar[k];
+                        acc(x.x, x.y, svh[k], svl[k], sh[3], sl[3]);
                     }
                 }
-            }
+                // the lane's eight (head, tail) sums combined in double-FP32 (TwoSum), so that only
+                // one conversion and the warp sum use the FP64 pipe (one warp instruction per 16
+                // cycles of an SM on GB300)
+                float hh = sh[0], hl = sl[0];
 #pragma unroll
-            for (int h = 0; h < 2; h++) {
-                const int t = (tid & 63) + 64 * h;
-                if (t < ncomp) s_pp[gq][t] = sp[h];
-            }
-            __syncthreads();
-            if (tid < ncomp) {
-                double sum = 0.0;
-                for (int q8 = 0; q8 < 8; q8++) sum += s_pp[q8][tid];
-                const int comp = tid < c ? tid : (tid < 2 * c ? TRD_NB + (tid - c) : 2 * TRD_NB);
-                g.part[(size_t)comp * G + b] = sum;
+                for (int u = 1; u < 8; u++) {
+                    const float t = hh + sh[u], bp = t - hh;
+                    const float e = ((hh - (t - bp)) + (sh[u] - bp)) + (hl + sl[u]);
+                    hh = t + e;
+                    hl = e - (hh - t);
+                }
+                // the warp's sum in double-FP32 as well (short FP32 dependency chains instead of
+                // FP64 ones), converted once
+#pragma unroll
+                for (int o = 16; o > 0; o >>= 1) {
+                    const float oh = __shfl_xor_sync(0xffffffffu, hh, o), ol = __shfl_xor_sync(0xffffffffu, hl, o);
+                    const float t = hh + oh, bp = t - hh;
+                    const float e = ((hh - (t - bp)) + (oh - bp)) + (hl + ol);
+                    hh = t + e;
+                    hl = e - (hh - t);
+                }
+                if (lane == 0) yhl[r - rb0] = make_float2(hh, hl);
             }
         }
-        if (!grid_barrier(g.bar, g.err)) return;
+        float2 af[2] = {};  // column i + 1 of the rows the last step takes, in flight over the wait
+        if (warp == TRD_WARPS)
+#pragma unroll
+            for (int u = 0; u < 2; u++)
+                if (y0 + lane + 32 * u < rb1) af[u] = g.Ahl[(size_t)(y0 + lane + 32 * u) * n + i + 1];
+        __syncthreads();
+        // the rows' y = A[r][i+1] + scale times the product, v, and y.v, by one warp: an FP64
+        // instruction here is one for all rows, where in the product it would be one per row
+        if (warp == TRD_WARPS) {
+            const double scale = s_scal[SCALE];
+            double yv = 0.0;
+#pragma unroll 1
+            for (int r = y0 + lane, u = 0; r < rb1; r += 32, u++) {
+                const int lr = r - rb0;
+                const float2 a0 = u == 0 ? af[0] : u == 1 ? af[1] : g.Ahl[(size_t)r * n + i + 1], h = yhl[lr];
+                const double y = fma(scale, (double)h.x + (double)h.y, (double)a0.x + (double)a0.y);
+                const double vr = (r == i + 1) ? 1.0 : as[lr] * scale;
+                ys[lr] = y;
+                if (r == i + 1) g.y[r] = y;
+                Vs[(size_t)lr * VLD + c] = vr;
+                g.V[(size_t)r * LDP + c] = vr;
+                yv = fma(y, vr, yv);
+            }
+            yv = warp_sum(yv);
+            if (lane == 0) g.part[(size_t)(2 * TRD_NB) * G + b] = yv;
+        }
+        if (!grid_barrier(g.bar, arrived += G, g.err)) return;
     }
 }
 
@@ -1211,12 +1221,12 @@ static modal_status trd_run(modal_ctx *ctx, int n, double *A, SyevPtrs &p, int n
     auto grid_of = [&](int rows) { return std::max(1, std::min(std::min(nsm, 1024), ceil_div(rows, 16))); };
     int Rmax = 1;
     for (int j0 = 0; j0 < n - 1; j0 += TRD_NB) Rmax = std::max(Rmax, ceil_div(n - j0, grid_of(n - j0)));
-    // v (n) + this CTA's V and W rows (Rmax x NB each) + y and a (Rmax each)
-    const size_t smem = sizeof(double) * ((size_t)n + (size_t)Rmax * (2 * VLD + 2));
-    if (smem > 200 * 1024) { set_error("eigensolver: n = %d exceeds the panel kernel's shared memory", n); return MODAL_ERR_ARG; }
+    // v (n) + this CTA's V and W rows (Rmax x NB each) + five numbers per row
+    const size_t smem = sizeof(double) * ((size_t)n + (size_t)Rmax * (2 * VLD + 5));
+    if (smem - sizeof(double) * 3 * (size_t)Rmax > 200 * 1024) { set_error("eigensolver: n = %d exceeds the panel kernel's shared memory", n); return MODAL_ERR_ARG; }
     MODAL_CUDA(cudaFuncSetAttribute(k_trd_panel, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem));
     int per_sm = 0;
-    MODAL_CUDA(cudaOccupancyMaxActiveBlocksPerMultiprocessor(&per_sm, k_trd_panel, TRD_THREADS, smem));
+    MODAL_CUDA(cudaOccupancyMaxActiveBlocksPerMultiprocessor(&per_sm, k_trd_panel, TRD_THREADS + TRD_AUX, smem));
     if (per_sm < 1) { set_error("eigensolver: panel kernel does not fit on an SM"); return MODAL_ERR_CUDA; }
     MODAL_CUDA(cudaMemsetAsync(p.err, 0, 2 * sizeof(int), ctx->stream));
     MODAL_CUDA(cudaMemsetAsync(p.bar, 0, 2 * sizeof(unsigned), ctx->stream));
@@ -1231,6 +1241,7 @@ static modal_status trd_run(modal_ctx *ctx, int n, double *A, SyevPtrs &p, int n
     oz.slices = OZ_SLICES;
     oz.lower = 1;
     oz.check = false;
+    unsigned arrived = 0;  // at the grid barrier, by the panels so far
     for (int pi = 0; pi < npanel; pi++) {
         const int j0 = pi * TRD_NB;
         const int nbp = std::min(TRD_NB, n - 1 - j0);  // reflectors 0 .. n-2
@@ -1239,12 +1250,13 @@ static modal_status trd_run(modal_ctx *ctx, int n, double *A, SyevPtrs &p, int n
         g.A = A; g.Ahl = p.Ahl; g.ahl = p.ahl; g.n = n; g.j0 = j0; g.nbp = nbp;
         g.V = p.P;
         g.W = p.P + TRD_NB;
-        g.d = p.d; g.e = p.e; g.tau = p.tau; g.a = p.a; g.y = p.y; g.part = p.part; g.bar = p.bar; g.err = p.err;
+        g.d = p.d; g.e = p.e; g.tau = p.tau; g.a = p.a; g.y = p.y; g.part = p.part; g.bar = p.bar; g.bar0 = arrived; g.err = p.err;
         void *args[] = {&g};
         const int G = grid_of(n - j0);
+        arrived += 2u * nbp * G;
         {
             StageTimer tp(ctx, MODAL_T_EIG_PANEL);
-            MODAL_CUDA(cudaLaunchCooperativeKernel((const void *)k_trd_panel, dim3(G), dim3(TRD_THREADS), args, smem,
+            MODAL_CUDA(cudaLaunchCooperativeKernel((const void *)k_trd_panel, dim3(G), dim3(TRD_THREADS + TRD_AUX), args, smem,
                                                    ctx->stream));
             MODAL_TRY(launched(ctx, "trd_panel"));
         }
