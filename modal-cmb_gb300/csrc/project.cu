@@ -11,7 +11,7 @@
 //   B[a][b][c] = sum_i q_a(i) sum_j q_b(j) sum_k f(i,j,k) q_c(k)
 //   beta_r     = (1/6) sum over the six orderings s of B[p_s1][p_s2][p_s3]
 // for mode r = (p1,p2,p3).  That is O(points * P) instead of O(points * N).
-// One CTA per slab l1 = i; the tetrapyd rows j are processed JC at a time:
+// One CTA per shape and slab l1 = i; the tetrapyd rows j are processed JC at a time:
 //   phase 1: f(i,j,k) for the JC rows into shared memory (shape evaluated here)
 //   phase 2: H[j][c] = sum_k f(i,j,k) q_c(k)
 //   phase 3: F_i[b][c] += sum_j q_b(j) H[j][c]          (registers)
@@ -21,28 +21,6 @@
 #include "common.cuh"
 
 namespace modal {
-
-__device__ __forceinline__ double d_permsix(int i, int j, int k)
-{
-    if (i == k && i == j) return 1.0;
-    if (i == j || j == k || i == k) return 3.0;
-    return 6.0;
-}
-
-// calculate_geometric (calculate_geometric.c:59-92) for a point already known
-// to satisfy parity and the triangle condition.
-__device__ __forceinline__ double d_geo(int l1, int l2, int l3)
-{
-    double s1 = l1 + l2 + l3 + 1.0, s3 = l1 + l2 + l3 + 1.0 / 3.0, s6 = l1 + l2 + l3 + 1.0 / 6.0;
-    double s13 = l2 + l3 - l1 + 1.0 / 3.0, s23 = l3 + l1 - l2 + 1.0 / 3.0, s33 = l1 + l2 - l3 + 1.0 / 3.0;
-    double s16 = l2 + l3 - l1 + 1.0 / 6.0, s26 = l3 + l1 - l2 + 1.0 / 6.0, s36 = l1 + l2 - l3 + 1.0 / 6.0;
-    const double ipi = 0.318309886183790671537767526745028724;
-    double fact = ipi * ipi / 2.0;
-    double p1 = fact * ((2.0 * l1 + 1.0) * (2.0 * l2 + 1.0) * (2.0 * l3 + 1.0)) / s1;
-    double p2 = s3 / (s13 * s23 * s33);
-    double p3 = sqrt(s16 * s26 * s36 / s6);
-    return p1 * p2 * p3;
-}
 
 // s_n(i,j,k) / (wq_i wq_j wq_k) of calculate_sijk_TTT (calculate_gamma_3d.c:813-860):
 // the trapezium integral (integrate, :783-811) over x of x^2 (1/6) sum over the six
@@ -135,8 +113,8 @@ __device__ __forceinline__ double d_shape(const DShape &s, const double *__restr
 }
 
 // A separable shape on a fixed row (i, j), FP64: with the row coefficients
-//   c[t] = (f_t(i) g_t(j) + f_t(j) g_t(i), f_t(i) h_t(j) + f_t(j) h_t(i), g_t(i) h_t(j) + g_t(j) h_t(i))
-// the value at k is (1/6) sum_t (c0 h_t(k) + c1 g_t(k) + c2 f_t(k)): three loads
+//   c[t] = (f_t(i) g_t(j) + f_t(j) g_t(i), f_t(i) h_t(j) + f_t(j) h_t(i), g_t(i) h_t(j) + g_t(j) h_t(i)) / 6
+// the value at k is sum_t (c0 h_t(k) + c1 g_t(k) + c2 f_t(k)): three loads
 // and three FMAs per term instead of the six-ordering sum.
 constexpr int PJ_TCOEF64 = 8;  // terms per shape with row coefficients (more: d_shape)
 
@@ -150,16 +128,25 @@ __device__ __forceinline__ double d_sep_rows(const DShape &s, const double *__re
         acc = fma(c[3 * t + 1], f[stride + k], acc);
         acc = fma(c[3 * t + 2], f[k], acc);
     }
-    return acc * (1.0 / 6.0);
+    return acc;
 }
 
-// v_l = (2l+1)^{-1/3} w_l, w_l = (2l+1)^{1/6}/sqrt(C_l + N_l/b_l^2), w_0 = w_1 = 0
+// 1D factors of the point weight permsix h~^2 prod (2l+1)^{-1/3} w_l:
+//   h~^2(l1,l2,l3) = gL(L) g(L - 2 l1) g(L - 2 l2) g(L - 2 l3) prod (2l+1), L = l1 + l2 + l3 (always even),
+//   g(x) = sqrt(x + 1/6) / (x + 1/3), gL(L) = (L + 1/3) / (2 pi^2 (L + 1) sqrt(L + 1/6))
+// (calculate_geometric.c:59-92 regrouped), w_l = (2l+1)^{1/6} / sqrt(C_l + N_l/b_l^2), w_0 = w_1 = 0
 // (calculate_mode_3D.c:53-62, get_weight :283-290).
-__global__ void k_vl(int lmax, const double *__restrict__ cl, double *__restrict__ vl)
+// v[l] = (2l+1)^{2/3} w_l for l <= lmax, then g[h] = g(2h) and gl[h] = gL(2h) for h < vl_nh.
+__host__ __device__ inline int vl_nh(int lmax) { return 3 * lmax / 2 + 1; }
+inline size_t vl_count(int lmax) { return (size_t)(lmax + 1) + 2 * (size_t)vl_nh(lmax); }
+__global__ void k_vl(int lmax, const double *__restrict__ cl, double *__restrict__ v)
 {
-    int l = blockIdx.x * blockDim.x + threadIdx.x;
-    if (l > lmax) return;
-    vl[l] = (l < 2) ? 0.0 : pow(2.0 * l + 1.0, -1.0 / 3.0) * (pow(2.0 * l + 1.0, 1.0 / 6.0) / sqrt(cl[l]));
+    const int h = blockIdx.x * blockDim.x + threadIdx.x, nh = vl_nh(lmax);
+    if (h <= lmax) v[h] = (h < 2) ? 0.0 : cbrt(2.0 * h + 1.0) * sqrt(2.0 * h + 1.0) / sqrt(cl[h]);
+    if (h >= nh) return;
+    const double x = 2.0 * h;
+    v[lmax + 1 + h] = sqrt(x + 1.0 / 6.0) / (x + 1.0 / 3.0);
+    v[lmax + 1 + nh + h] = (x + 1.0 / 3.0) / ((x + 1.0) * sqrt(x + 1.0 / 6.0)) * 0.050660591821168885722;
 }
 
 constexpr int JC = 8;
@@ -210,8 +197,9 @@ __global__ void k_slab_base(int lmin, int lmax, long long *__restrict__ base)
     if (t == 255) base[L] = part[255];
 }
 
-// FP64 form of the weight table: the same products in the same order as the
-// FP64 point weight, so the projection is unchanged to the last bit.
+// Point weights in slab and row order, from their 1D factors: seven FP64 multiplications per
+// point, which bound it.  At l <= 1000: 0.69 ms; the closed form's quotients and square root
+// took 6.3 ms.  Relative error of a weight (rms, units of 2^-53): 2.9, the closed form 3.9.
 __global__ void __launch_bounds__(256) k_weight_table_fp64(int lmin, int lmax, const double *__restrict__ vl,
                                                            const long long *__restrict__ base, double *__restrict__ Wd)
 {
@@ -222,17 +210,27 @@ __global__ void __launch_bounds__(256) k_weight_table_fp64(int lmin, int lmax, c
     if (kend < k0) return;
     const int n = (kend - k0) / 2 + 1;
     double *row = Wd + base[blockIdx.x] + tet_row_offset(i, j, lmax);
-    const double vi = vl[i], vj = vl[j];
+    const double *vk = vl + k0;
+    const double *gl = vl + lmax + 1 + vl_nh(lmax) + (i + j + k0) / 2;
+    const double *g1 = vl + lmax + 1 + (j + k0 - i) / 2, *g2 = vl + lmax + 1 + (i + k0 - j) / 2,
+                 *g3 = vl + lmax + 1 + (i + j - k0) / 2;
+    const double vij = vl[i] * vl[j];
     for (int m = lane; m < n; m += 32) {
-        const int k = k0 + 2 * m;
-        row[m] = d_permsix(i, j, k) * d_geo(i, j, k) * vi * vj * vl[k];
+        const double perm = (i == j && m == 0 && ip == 0) ? 1.0 : (i == j || (m == 0 && ip == 0)) ? 3.0 : 6.0;
+        row[m] = (perm * (gl[m] * g1[m])) * (g2[m] * g3[-m]) * (vij * vk[2 * m]);
     }
 }
 
+// One CTA per shape and slab (a shape's slabs in decreasing size).  Bound by the FP64 pipe, one
+// warp instruction per 16 cycles of an SM: per point 3 per term and one for the weighted shape
+// value, P for the contraction over k, P^2 per row for the one over j; the sums over k run in
+// four chains (an FP64 operation takes 65 cycles), and a row's points are one warp's.  At
+// l <= 1000, P = 20, four shapes of two terms: 10.3 ms (9.4 ms of FP64 instructions); one CTA per
+// slab that takes the shapes in turn, one chain per sum: 13.1 ms.
 template <int FPT>
-__global__ void __launch_bounds__(256) k_project_slab_fp64(int lmin, int lmax, int P, int S, int KMAX,
+__global__ void __launch_bounds__(256) k_project_slab_fp64(int lmin, int lmax, int P, int KMAX,
                                                             const int *__restrict__ slab_order,
-                                                            const double *__restrict__ q, const double *__restrict__ vl,
+                                                            const double *__restrict__ q,
                                                             const DShape *__restrict__ shapes,
                                                             const double *__restrict__ tab,
                                                             const double *__restrict__ Wd,
@@ -246,94 +244,99 @@ __global__ void __launch_bounds__(256) k_project_slab_fp64(int lmin, int lmax, i
     double *V = Cf + JC * PJ_TCOEF64 * 3;  // radial shapes: [JC][3][X] row factors, then [X] trapezium weights
     const int XR = ra.xsize;
     double *TW = V + (size_t)JC * 3 * XR;
-    const int slab = slab_order[blockIdx.x];
+    const int s = blockIdx.x, slab = slab_order[blockIdx.y];
     const int i = lmin + slab;
-    const int tid = threadIdx.x;
+    const int tid = threadIdx.x, lane = tid & 31, warp = tid >> 5;
     const int PP = P * P, L = lmax - lmin + 1, stride = lmax + 1;
     const int par = i & 1;
-    for (int s = 0; s < S; s++) {
-        const DShape sh = shapes[s];
-        double Facc[FPT];
+    const DShape sh = shapes[s];
+    double Facc[FPT];
 #pragma unroll
-        for (int t = 0; t < FPT; t++) Facc[t] = 0.0;
-        const bool radial = sh.kind == SHAPE_RADIAL;
-        const bool rowc = sh.kind == MODAL_SHAPE_SEPARABLE && sh.nterms <= PJ_TCOEF64;
-        for (int j0 = i; j0 <= lmax; j0 += JC) {
-            if (rowc) {
-                for (int e = tid; e < JC * sh.nterms; e += 256) {
-                    const int jj = e / sh.nterms, t = e - jj * sh.nterms, j = min(j0 + jj, lmax);
-                    const double *f = tab + sh.tab_off + (long)t * 3 * stride, *g = f + stride, *h = g + stride;
-                    double *c = Cf + ((size_t)jj * PJ_TCOEF64 + t) * 3;
-                    c[0] = f[i] * g[j] + f[j] * g[i];  // with h(k)
-                    c[1] = f[i] * h[j] + f[j] * h[i];  // with g(k)
-                    c[2] = g[i] * h[j] + g[j] * h[i];  // with f(k)
-                }
-                __syncthreads();
-            }
-            if (radial) {
-                const int a1 = ra.prim[3 * sh.nterms], a2 = ra.prim[3 * sh.nterms + 1], a3 = ra.prim[3 * sh.nterms + 2];
-                for (int e = tid; e < JC * XR; e += 256) {
-                    const int jj = e / XR, x = e - jj * XR, j = min(j0 + jj, lmax);
-                    const double *qx = ra.qt + (size_t)x * ra.Pp * ra.L1;
-                    const double p1 = qx[(size_t)a1 * ra.L1 + i], p2 = qx[(size_t)a2 * ra.L1 + i],
-                                 p3 = qx[(size_t)a3 * ra.L1 + i], p4 = qx[(size_t)a1 * ra.L1 + j],
-                                 p5 = qx[(size_t)a2 * ra.L1 + j], p6 = qx[(size_t)a3 * ra.L1 + j];
-                    const double g = ra.x[x] * ra.x[x] * (1.0 / 6.0);
-                    double *u = V + (size_t)jj * 3 * XR;
-                    u[x] = g * (p2 * p6 + p3 * p5);           // with q~_{a1}(k)
-                    u[XR + x] = g * (p3 * p4 + p1 * p6);      // with q~_{a2}(k)
-                    u[2 * XR + x] = g * (p1 * p5 + p2 * p4);  // with q~_{a3}(k)
-                }
-                for (int x = tid; x < XR; x += 256) TW[x] = trap_w(ra, x);
-                __syncthreads();
-            }
-            for (int e = tid; e < JC * KMAX; e += 256) {
-                int jj = e / KMAX, kk = e - jj * KMAX, j = j0 + jj;
-                double val = 0.0;
-                if (j <= lmax) {
-                    int k = j + par + 2 * kk, k1 = min(i + j, lmax);
-                    if (k <= k1)
-                        val = Wd[sbase[slab] + tet_row_offset(i, j, lmax) + kk] *
-                              (radial ? d_radial_rows(ra, sh.nterms, i, j, k, V + (size_t)jj * 3 * XR, TW)
-                               : rowc ? d_sep_rows(sh, tab, stride, k, Cf + (size_t)jj * PJ_TCOEF64 * 3)
-                                      : d_shape(sh, tab, stride, i, j, k, ra));
-                }
-                f[e] = val;
-            }
-            __syncthreads();
-            for (int e = tid; e < JC * P; e += 256) {
-                int jj = e / P, c = e - jj * P, j = j0 + jj;
-                double acc = 0.0;
-                if (j <= lmax) {
-                    int kf = j + par, k1 = min(i + j, lmax);
-                    int nk = (k1 >= kf) ? (k1 - kf) / 2 + 1 : 0;
-                    const double *fr = f + jj * KMAX;
-                    const double *qc = q + (size_t)(kf - lmin) * P + c;
-                    for (int kk = 0; kk < nk; kk++) acc = fma(fr[kk], qc[(size_t)2 * kk * P], acc);
-                }
-                H[e] = acc;
-            }
-            __syncthreads();
-#pragma unroll
-            for (int t = 0; t < FPT; t++) {
-                int e = tid + 256 * t;
-                if (e < PP) {
-                    int b = e / P, c = e - b * P;
-                    double a = 0.0;
-                    for (int jj = 0; jj < JC; jj++) {
-                        int j = j0 + jj;
-                        if (j <= lmax) a = fma(q[(size_t)(j - lmin) * P + b], H[jj * P + c], a);
-                    }
-                    Facc[t] += a;
-                }
+    for (int t = 0; t < FPT; t++) Facc[t] = 0.0;
+    const bool radial = sh.kind == SHAPE_RADIAL;
+    const bool rowc = sh.kind == MODAL_SHAPE_SEPARABLE && sh.nterms <= PJ_TCOEF64;
+    for (int j0 = i; j0 <= lmax; j0 += JC) {
+        if (rowc) {
+            for (int e = tid; e < JC * sh.nterms; e += 256) {
+                const int jj = e / sh.nterms, t = e - jj * sh.nterms, j = min(j0 + jj, lmax);
+                const double *f = tab + sh.tab_off + (long)t * 3 * stride, *g = f + stride, *h = g + stride;
+                double *c = Cf + ((size_t)jj * PJ_TCOEF64 + t) * 3;
+                c[0] = (f[i] * g[j] + f[j] * g[i]) * (1.0 / 6.0);  // with h(k)
+                c[1] = (f[i] * h[j] + f[j] * h[i]) * (1.0 / 6.0);  // with g(k)
+                c[2] = (g[i] * h[j] + g[j] * h[i]) * (1.0 / 6.0);  // with f(k)
             }
             __syncthreads();
         }
+        if (radial) {
+            const int a1 = ra.prim[3 * sh.nterms], a2 = ra.prim[3 * sh.nterms + 1], a3 = ra.prim[3 * sh.nterms + 2];
+            for (int e = tid; e < JC * XR; e += 256) {
+                const int jj = e / XR, x = e - jj * XR, j = min(j0 + jj, lmax);
+                const double *qx = ra.qt + (size_t)x * ra.Pp * ra.L1;
+                const double p1 = qx[(size_t)a1 * ra.L1 + i], p2 = qx[(size_t)a2 * ra.L1 + i],
+                             p3 = qx[(size_t)a3 * ra.L1 + i], p4 = qx[(size_t)a1 * ra.L1 + j],
+                             p5 = qx[(size_t)a2 * ra.L1 + j], p6 = qx[(size_t)a3 * ra.L1 + j];
+                const double g = ra.x[x] * ra.x[x] * (1.0 / 6.0);
+                double *u = V + (size_t)jj * 3 * XR;
+                u[x] = g * (p2 * p6 + p3 * p5);           // with q~_{a1}(k)
+                u[XR + x] = g * (p3 * p4 + p1 * p6);      // with q~_{a2}(k)
+                u[2 * XR + x] = g * (p1 * p5 + p2 * p4);  // with q~_{a3}(k)
+            }
+            for (int x = tid; x < XR; x += 256) TW[x] = trap_w(ra, x);
+            __syncthreads();
+        }
+        {   // a warp per row
+            const int jj = warp, j = j0 + jj, k0 = j + par;
+            const int nk = j <= lmax && min(i + j, lmax) >= k0 ? (min(i + j, lmax) - k0) / 2 + 1 : 0;
+            if (nk > 0) {
+                const double *w = Wd + sbase[slab] + tet_row_offset(i, j, lmax);
+                for (int kk = lane; kk < nk; kk += 32) {
+                    const int k = k0 + 2 * kk;
+                    f[jj * KMAX + kk] = w[kk] * (radial ? d_radial_rows(ra, sh.nterms, i, j, k, V + (size_t)jj * 3 * XR, TW)
+                                                 : rowc ? d_sep_rows(sh, tab, stride, k, Cf + (size_t)jj * PJ_TCOEF64 * 3)
+                                                        : d_shape(sh, tab, stride, i, j, k, ra));
+                }
+            }
+        }
+        __syncthreads();
+        for (int e = tid; e < JC * P; e += 256) {
+            const int jj = e / P, c = e - jj * P, j = j0 + jj;
+            double acc[4] = {0.0, 0.0, 0.0, 0.0};
+            if (j <= lmax) {
+                const int kf = j + par, k1 = min(i + j, lmax), nk = (k1 >= kf) ? (k1 - kf) / 2 + 1 : 0;
+                const double *fr = f + jj * KMAX;
+                const double *qc = q + (size_t)(kf - lmin) * P + c;
+                int kk = 0;
+                for (; kk + 4 <= nk; kk += 4)
+#pragma unroll
+                    for (int u = 0; u < 4; u++) acc[u] = fma(fr[kk + u], qc[(size_t)2 * (kk + u) * P], acc[u]);
+#pragma unroll
+                for (int u = 0; u < 3; u++)
+                    if (kk + u < nk) acc[u] = fma(fr[kk + u], qc[(size_t)2 * (kk + u) * P], acc[u]);
+            }
+            H[e] = (acc[0] + acc[1]) + (acc[2] + acc[3]);
+        }
+        __syncthreads();
 #pragma unroll
         for (int t = 0; t < FPT; t++) {
-            int e = tid + 256 * t;
-            if (e < PP) Fbuf[((size_t)s * L + slab) * PP + e] = Facc[t];
+            const int e = tid + 256 * t;
+            if (e < PP) {
+                const int b = e / P, c = e - b * P, nj = min(JC, lmax - j0 + 1);
+                const double *qb = q + (size_t)(j0 - lmin) * P + b;
+                double a = 0.0;
+                if (nj == JC) {
+#pragma unroll
+                    for (int jj = 0; jj < JC; jj++) a = fma(qb[(size_t)jj * P], H[jj * P + c], a);
+                } else
+                    for (int jj = 0; jj < nj; jj++) a = fma(qb[(size_t)jj * P], H[jj * P + c], a);
+                Facc[t] += a;
+            }
         }
+        // H is written again only after the next rows' points; Cf, V and f before that are not read here
+    }
+#pragma unroll
+    for (int t = 0; t < FPT; t++) {
+        const int e = tid + 256 * t;
+        if (e < PP) Fbuf[((size_t)s * L + slab) * PP + e] = Facc[t];
     }
 }
 
@@ -348,9 +351,19 @@ __global__ void k_project_B(int L, int P, int S, const double *__restrict__ q, c
     int rem = (int)(e - (size_t)s * P * PP);
     int a = rem / PP, bc = rem - a * PP;
     const double *F = Fbuf + (size_t)s * L * PP + bc;
-    double acc = 0.0;
-    for (int l = 0; l < L; l++) acc = fma(q[(size_t)l * P + a], F[(size_t)l * PP], acc);
-    B[e] = acc;
+    // eight loads in flight, four chains (the loop is one thread's and bound by latency:
+    // 0.25 ms at l <= 1000, P = 20, four shapes; 0.35 ms as one chain)
+    double acc[4] = {0.0, 0.0, 0.0, 0.0};
+    int l = 0;
+    for (; l + 8 <= L; l += 8) {
+        double x[8];
+#pragma unroll
+        for (int u = 0; u < 8; u++) x[u] = F[(size_t)(l + u) * PP];
+#pragma unroll
+        for (int u = 0; u < 8; u++) acc[u & 3] = fma(q[(size_t)(l + u) * P + a], x[u], acc[u & 3]);
+    }
+    for (; l < L; l++) acc[0] = fma(q[(size_t)l * P + a], F[(size_t)l * PP], acc[0]);
+    B[e] = (acc[0] + acc[1]) + (acc[2] + acc[3]);
 }
 
 // beta[s][r] = (1/6) sum of B over the six orderings of mode r's triple
@@ -417,7 +430,7 @@ modal_status proj_plan(modal_ctx *ctx, int S, const modal_shape *shapes, modal_p
     }
     MODAL_TRY(ensure(ctx->shape_tab, sizeof(double) * (size_t)(tab_total > 0 ? tab_total : 1)));
     MODAL_TRY(ensure(ctx->shape_desc, sizeof(DShape) * (size_t)S));
-    MODAL_TRY(ensure(ctx->vl, sizeof(double) * (lmax + 1)));
+    MODAL_TRY(ensure(ctx->vl, sizeof(double) * vl_count(lmax)));
     MODAL_TRY(ensure(ctx->beta, sizeof(double) * (size_t)S * N));
     if (prec == MODAL_PREC_SPLIT) {
         MODAL_TRY(pf_plan(ctx, pl));
@@ -473,7 +486,7 @@ modal_status proj_record(modal_ctx *ctx, const ProjPlan &pl)
 {
     const int lmin = ctx->lmin, lmax = ctx->lmax, L = ctx->L, P = ctx->P, N = ctx->N, PP = P * P, S = pl.S;
     if (pl.prec == MODAL_PREC_SPLIT) return pf_record(ctx, pl);
-    k_vl<<<ceil_div(lmax + 1, 256), 256, 0, ctx->stream>>>(lmax, ctx->cl.as<double>(), ctx->vl.as<double>());
+    k_vl<<<ceil_div(vl_nh(lmax), 256), 256, 0, ctx->stream>>>(lmax, ctx->cl.as<double>(), ctx->vl.as<double>());
     MODAL_TRY(launched(ctx, "vl"));
     uint8_t *b8 = ctx->scratch.as<uint8_t>();
     double *Fbuf = reinterpret_cast<double *>(b8);
@@ -486,9 +499,9 @@ modal_status proj_record(modal_ctx *ctx, const ProjPlan &pl)
     MODAL_TRY(launched(ctx, "weight_table_fp64"));
     const int KMAX = (lmax - lmin) / 2 + 2;
     auto run = [&](auto kern) -> modal_status {
-        kern<<<L, 256, pl.smem, ctx->stream>>>(lmin, lmax, P, S, KMAX, ctx->slab_order.as<int>(), ctx->q.as<double>(),
-                                               ctx->vl.as<double>(), ctx->shape_desc.as<DShape>(),
-                                               ctx->shape_tab.as<double>(), Wd, sbase, Fbuf, pl.ra);
+        kern<<<dim3(S, L), 256, pl.smem, ctx->stream>>>(lmin, lmax, P, KMAX, ctx->slab_order.as<int>(), ctx->q.as<double>(),
+                                                        ctx->shape_desc.as<DShape>(), ctx->shape_tab.as<double>(), Wd,
+                                                        sbase, Fbuf, pl.ra);
         return launched(ctx, "project_slab_fp64");
     };
     if (pl.fpt <= 1) MODAL_TRY(run(k_project_slab_fp64<1>));
