@@ -55,6 +55,15 @@ DFB_HD int clz64(uint64_t a)
 #endif
 }
 
+// x = f 2^e for the float f of bits u, exactly: zero and normal floats, |e| <= 890.
+DFB_HD bool scaled(uint32_t u, int e, double *x)
+{
+    const uint32_t m = u & 0x7fffffffu, sg = u & 0x80000000u;
+    const uint32_t hi = (m >> 3) + ((896u + (uint32_t)e) << 20);  // exponent rebiased, top 20 significand bits
+    *x = from64(m == 0u ? (uint64_t)sg << 32 : (uint64_t)(sg | hi) << 32 | (uint64_t)(u << 29));
+    return m == 0u || (m - 0x00800000u < 0x7f000000u && (uint32_t)e + 890u <= 1780u);
+}
+
 // Head and tail of x as floats: hi = RN(x), lo = RN(x - hi) (round to nearest
 // even, the bits of __double2float_rn(x) and __double2float_rn(x - (double)hi)).
 // Covers zero and |x| in [2^-74, 2^127) (both parts then normal floats);

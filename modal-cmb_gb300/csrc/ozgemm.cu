@@ -21,23 +21,33 @@
 //   products with p + q >= s dropped (below 2^{-7s} of the leading term).
 //
 // The exact block sums are added in double-FP32 ("double-float": an FP32
-// head and tail, Knuth's TwoSum) kept in tensor memory; the tile is converted
+// head and tail, Knuth's TwoSum) kept in registers; the tile is converted
 // to FP64 once at the end.  Accuracy: about 2^-48 relative to max|row| max|col|
 // per K block, the class of an FP64 GEMM over K = 5000 terms.
 //
 // Kernel k_oz_gemm: persistent, one CTA per SM over the output tiles
 // (128 x 128); warp 0 TMA producer (8-stage ring of 16 KB: an A-slice and a
 // B-slice chunk of 32 K, 64-byte swizzle), warp 1 MMA issuer (tcgen05.mma
-// kind::f16, M = N = 128, K = 16) and TMEM owner, warps 2-5 epilogue.  TMEM:
-// two FP32 accumulators (columns 0-255, the epilogue drains one while the next
-// group fills the other) and the double-float sums (columns 256-511).  Every
-// mbarrier wait is bounded; on expiry the CTA flags an error, stops, drains its
-// copies, frees TMEM and returns (MODAL_ERR_TIMEOUT).
+// kind::f16, M = N = 128, K = 16) and TMEM owner, warps 4-11 epilogue (64 columns
+// of 32 rows each, the sums in 128 registers).  TMEM: four FP32 accumulators, two
+// groups that the epilogue drains while the next two fill.  Two groups at a time
+// take half as many operand copies as one (20 instead of 36 pairs of slices for
+// s = 8).  Every mbarrier wait is bounded; on expiry the CTA flags an error, stops,
+// drains its copies, frees TMEM and returns (MODAL_ERR_TIMEOUT).
+//
+// What bounds it: for a short K (the trailing updates of the tridiagonalisation,
+// K = 64) the epilogue's instructions, 80 per 32 elements and tile after packing two
+// columns per FP32 instruction and building the FP64 results as bit patterns; for a
+// long K the operand copies.  One group at a time, four epilogue warps, sums in
+// tensor memory and results by FP64 conversions: trailing update of 4,928 rows
+// 361 -> 186 us, of a merge's 4,960 x 4,960 x 2,480 product 2.54 -> 2.10 ms, the 220 products
+// of an eigendecomposition of n = 4,960 42.1 -> 25.1 ms.
 #include <cuda.h>
 #include <cuda_fp16.h>
 #include <cudaTypedefs.h>
 #include <algorithm>
 #include <mutex>
+#include <type_traits>
 #include <vector>
 #include "common.cuh"
 #include "dfbits.cuh"
@@ -54,10 +64,13 @@ constexpr int OZ_MAXS = 8;
 constexpr uint32_t OZ_A_BYTES = OZ_BM * OZ_BK * 2;  // 8 KB
 constexpr uint32_t OZ_B_BYTES = OZ_BN * OZ_BK * 2;  // 8 KB
 constexpr uint32_t OZ_STAGE_BYTES = OZ_A_BYTES + OZ_B_BYTES;
-constexpr uint32_t OZ_STAGING = 4 * 32 * 33 * 8;  // epilogue: 32 x 32 FP64 per warp (+1 column pad)
+constexpr int OZ_EW = 8;                          // epilogue warps: 32 rows x 64 columns of the tile each
+constexpr int OZ_THREADS = 128 + 32 * OZ_EW;      // after one warpgroup of copies and products
+constexpr int OZ_RIO = 56, OZ_REPI = 216;         // registers of that one and of the epilogue's, out of 168 each
+static_assert(128 * OZ_RIO + 32 * OZ_EW * OZ_REPI <= OZ_THREADS * 168, "registers of the launch");
+constexpr uint32_t OZ_STAGING = OZ_EW * 32 * 33 * 8;  // epilogue: 32 x 32 double-floats per warp (+1 column pad)
 constexpr uint32_t OZ_SMEM = OZ_STAGES * OZ_STAGE_BYTES + 1024 + 256 + OZ_STAGING;
 constexpr uint32_t OZ_TMEM_COLS = 512;
-constexpr uint32_t OZ_SUM_COL = 256;  // first column of the double-float sums
 constexpr long long OZ_WAIT = 1ll << 31;  // ~1 s of clock64 per wait
 constexpr uint32_t OZ_IDESC = idesc_f16(OZ_BM, OZ_BN);
 
@@ -168,19 +181,65 @@ struct OzArgs {
     int *err;
 };
 
-// double-float a + b (Knuth's TwoSum, then renormalised)
-__device__ __forceinline__ void df_add(float &hi, float &lo, float b)
+// Pairs of floats (packed arithmetic).
+using f2 = unsigned long long;
+__device__ __forceinline__ f2 pk(float a, float b)
 {
-    const float s = hi + b;
-    const float bb = s - hi;
-    const float e = (hi - (s - bb)) + (b - bb);
-    const float t = lo + e;
-    hi = s + t;
-    lo = t - (hi - s);
+    f2 v;
+    asm("mov.b64 %0, {%1, %2};" : "=l"(v) : "f"(a), "f"(b));
+    return v;
+}
+__device__ __forceinline__ float2 upk(f2 v)
+{
+    float2 x;
+    asm("mov.b64 {%0, %1}, %2;" : "=f"(x.x), "=f"(x.y) : "l"(v));
+    return x;
+}
+__device__ __forceinline__ f2 add2(f2 a, f2 b)
+{
+    f2 v;
+    asm("add.rn.f32x2 %0, %1, %2;" : "=l"(v) : "l"(a), "l"(b));
+    return v;
+}
+__device__ __forceinline__ f2 sub2(f2 a, f2 b)
+{
+    f2 v;
+    asm("sub.rn.f32x2 %0, %1, %2;" : "=l"(v) : "l"(a), "l"(b));
+    return v;
+}
+__device__ __forceinline__ f2 mul2(f2 a, f2 b)
+{
+    f2 v;
+    asm("mul.rn.f32x2 %0, %1, %2;" : "=l"(v) : "l"(a), "l"(b));
+    return v;
 }
 
-__global__ void __launch_bounds__(192, 1) k_oz_gemm(const __grid_constant__ CUtensorMap tmA,
-                                                   const __grid_constant__ CUtensorMap tmB, OzArgs a)
+// double-float a + b (Knuth's TwoSum, then renormalised), two at a time
+__device__ __forceinline__ void df_add2(f2 &hi, f2 &lo, f2 b)
+{
+    const f2 s = add2(hi, b);
+    const f2 bb = sub2(s, hi);
+    const f2 e = add2(sub2(hi, sub2(s, bb)), sub2(b, bb));
+    const f2 t = add2(lo, e);
+    hi = add2(s, t);
+    lo = sub2(t, sub2(hi, s));
+}
+
+// (h + l) 2^er 2^en where the bit patterns do not reach.  A call of its own: inlined, its FP64
+// instructions are executed for every element and thrown away.
+__device__ __noinline__ double oz_join_far(float h, float l, int er, int en)
+{
+    return ((double)h + (double)l) * ldexp(1.0, er) * ldexp(1.0, en);
+}
+
+// The digit products of one K block run in groups of equal p + q = g, two groups
+// g = gh - 1, gh at a time (group 0 alone when s is odd): A's digit p then meets B's digits
+// gh - p and gh - 1 - p, the second of which is the first of p + 1.  A stage of the ring
+// holds (A_p, B_{gh-1-p}) and keeps its B for the next stage's products.
+__device__ __forceinline__ int oz_first_group(int s) { return (s & 1) ? 0 : 1; }
+
+__global__ void __launch_bounds__(OZ_THREADS, 1) k_oz_gemm(const __grid_constant__ CUtensorMap tmA,
+                                                           const __grid_constant__ CUtensorMap tmB, OzArgs a)
 {
     extern __shared__ uint8_t smem_raw[];
     uint8_t *smem = reinterpret_cast<uint8_t *>((reinterpret_cast<uintptr_t>(smem_raw) + 1023) & ~(uintptr_t)1023);
@@ -188,7 +247,7 @@ __global__ void __launch_bounds__(192, 1) k_oz_gemm(const __grid_constant__ CUte
     uint64_t *full = bars, *empty = bars + OZ_STAGES, *afull = bars + 2 * OZ_STAGES, *aempty = afull + 2;
     volatile uint32_t *tmem_slot = reinterpret_cast<volatile uint32_t *>(bars + 2 * OZ_STAGES + 4);
     volatile int *abort_flag = reinterpret_cast<volatile int *>(bars + 2 * OZ_STAGES + 5);
-    double *stage = reinterpret_cast<double *>(smem + OZ_STAGES * OZ_STAGE_BYTES + 256);
+    float2 *stage = reinterpret_cast<float2 *>(smem + OZ_STAGES * OZ_STAGE_BYTES + 256);
 
     const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
     const int s = a.s;
@@ -199,7 +258,7 @@ __global__ void __launch_bounds__(192, 1) k_oz_gemm(const __grid_constant__ CUte
         }
         for (int b = 0; b < 2; b++) {
             mbar_init(smem_u32(&afull[b]), 1);
-            mbar_init(smem_u32(&aempty[b]), 4);
+            mbar_init(smem_u32(&aempty[b]), OZ_EW);
         }
         *abort_flag = 0;
         asm volatile("fence.mbarrier_init.release.cluster;" ::: "memory");
@@ -212,95 +271,130 @@ __global__ void __launch_bounds__(192, 1) k_oz_gemm(const __grid_constant__ CUte
     tc_fence_after();
     const uint32_t tmem = *tmem_slot;
 
-    if (warp == 0) {
-        if (lane == 0) {
-            long g = 0;
-            bool stop = false;
-            for (int t = blockIdx.x; t < a.ntiles && !stop; t += gridDim.x) {
-                const int4 tile = a.tiles[t];
-                const int m0 = tile.x * OZ_BM, n0 = tile.y * OZ_BN;
-                const int kb0 = tile.z * a.kper, kb1 = min(a.nkb, kb0 + a.kper);
-                for (int kb = kb0; kb < kb1 && !stop; kb++) {
-                    const int kbeg = kb * OZ_KB, nkc = min(OZ_KB, a.Kpad - kbeg) / OZ_BK;
-                    for (int gg = 0; gg < s && !stop; gg++)
-                        for (int p = 0; p <= gg && !stop; p++)
-                            for (int kc = 0; kc < nkc; kc++, g++) {
-                                const int st = (int)(g % OZ_STAGES);
-                                const long it = g / OZ_STAGES;
-                                if (it > 0 && !mbar_wait(smem_u32(&empty[st]), (uint32_t)((it - 1) & 1), abort_flag, OZ_WAIT)) {
-                                    if (!*abort_flag) { *abort_flag = 1; atomicCAS(a.err, 0, 1); }
-                                    stop = true;
-                                    break;
-                                }
-                                uint8_t *sp = smem + (size_t)st * OZ_STAGE_BYTES;
-                                const uint32_t fb = smem_u32(&full[st]);
-                                mbar_expect_tx(fb, OZ_STAGE_BYTES);
+    if (warp < 4) {
+        asm volatile("setmaxnreg.dec.sync.aligned.u32 %0;" ::"n"(OZ_RIO));
+        if (warp == 0) {
+            if (lane == 0) {
+                long g = 0;
+                bool stop = false;
+                // the next stage: digit p of A (p >= 0) and digit q of B (q >= 0), columns k .. k + 31
+                auto load = [&](int p, int q, int m0, int n0, int k) {
+                    const int st = (int)(g % OZ_STAGES);
+                    const long it = g / OZ_STAGES;
+                    if (it > 0 && !mbar_wait(smem_u32(&empty[st]), (uint32_t)((it - 1) & 1), abort_flag, OZ_WAIT)) {
+                        if (!*abort_flag) { *abort_flag = 1; atomicCAS(a.err, 0, 1); }
+                        return false;
+                    }
+                    uint8_t *sp = smem + (size_t)st * OZ_STAGE_BYTES;
+                    const uint32_t fb = smem_u32(&full[st]);
+                    mbar_expect_tx(fb, (p >= 0 ? OZ_A_BYTES : 0u) + (q >= 0 ? OZ_B_BYTES : 0u));
+                    if (p >= 0) tma_load_2d(smem_u32(sp), &tmA, k, p * a.Mpad + m0, fb);
+                    if (q >= 0) tma_load_2d(smem_u32(sp + OZ_A_BYTES), &tmB, k, q * a.Npad + n0, fb);
+                    g++;
+                    return true;
+                };
+                for (int t = blockIdx.x; t < a.ntiles && !stop; t += gridDim.x) {
+                    const int4 tile = a.tiles[t];
+                    const int m0 = tile.x * OZ_BM, n0 = tile.y * OZ_BN;
+                    const int kb0 = tile.z * a.kper, kb1 = min(a.nkb, kb0 + a.kper);
+                    for (int kb = kb0; kb < kb1 && !stop; kb++) {
+                        const int kbeg = kb * OZ_KB, nkc = min(OZ_KB, a.Kpad - kbeg) / OZ_BK;
+                        for (int gh = oz_first_group(s); gh < s && !stop; gh += 2)
+                            for (int kc = 0; kc < nkc && !stop; kc++) {
                                 const int k = kbeg + kc * OZ_BK;
-                                tma_load_2d(smem_u32(sp), &tmA, k, p * a.Mpad + m0, fb);
-                                tma_load_2d(smem_u32(sp + OZ_A_BYTES), &tmB, k, (gg - p) * a.Npad + n0, fb);
+                                if (gh > 0) stop = !load(-1, gh, m0, n0, k);
+                                for (int p = 0; p <= gh && !stop; p++) stop = !load(p, gh > 0 ? gh - 1 - p : 0, m0, n0, k);
                             }
+                    }
+                }
+                // drain: the copies of the last stages must land before the CTA exits
+                for (long h = (g > OZ_STAGES ? g - OZ_STAGES : 0); h < g; h++) {
+                    const int st = (int)(h % OZ_STAGES);
+                    const long long t0 = clock64();
+                    while (!mbar_try(smem_u32(&full[st]), (uint32_t)((h / OZ_STAGES) & 1)) && clock64() - t0 < OZ_WAIT) {
+                    }
                 }
             }
-            // drain: the copies of the last stages must land before the CTA exits
-            for (long h = (g > OZ_STAGES ? g - OZ_STAGES : 0); h < g; h++) {
-                const int st = (int)(h % OZ_STAGES);
-                const long long t0 = clock64();
-                while (!mbar_try(smem_u32(&full[st]), (uint32_t)((h / OZ_STAGES) & 1)) && clock64() - t0 < OZ_WAIT) {
-                }
-            }
-        }
-    } else if (warp == 1) {
-        if (lane == 0) {
-            long g = 0, u = 0;
-            bool stop = false;
-            for (int t = blockIdx.x; t < a.ntiles && !stop; t += gridDim.x) {
-                const int kb0 = a.tiles[t].z * a.kper, kb1 = min(a.nkb, kb0 + a.kper);
-                for (int kb = kb0; kb < kb1 && !stop; kb++) {
-                    const int kbeg = kb * OZ_KB, nkc = min(OZ_KB, a.Kpad - kbeg) / OZ_BK;
-                    for (int gg = 0; gg < s && !stop; gg++, u++) {
-                        const int buf = (int)(u & 1);
-                        const long use = u >> 1;
-                        if (use > 0 && !mbar_wait(smem_u32(&aempty[buf]), (uint32_t)((use - 1) & 1), abort_flag, OZ_WAIT)) {
-                            if (!*abort_flag) { *abort_flag = 1; atomicCAS(a.err, 0, 4); }
-                            stop = true;
-                            break;
-                        }
-                        tc_fence_after();
-                        const uint32_t d = tmem + (uint32_t)(buf * OZ_BN);
-                        uint32_t accf = 0;
-                        for (int p = 0; p <= gg && !stop; p++)
-                            for (int kc = 0; kc < nkc; kc++, g++) {
-                                const int st = (int)(g % OZ_STAGES);
-                                const long it = g / OZ_STAGES;
-                                if (!mbar_wait(smem_u32(&full[st]), (uint32_t)(it & 1), abort_flag, OZ_WAIT)) {
-                                    if (!*abort_flag) { *abort_flag = 1; atomicCAS(a.err, 0, 2); }
-                                    stop = true;
-                                    break;
-                                }
-                                tc_fence_after();
-                                const uint32_t sa = smem_u32(smem + (size_t)st * OZ_STAGE_BYTES), sb = sa + OZ_A_BYTES;
+        } else if (warp == 1) {
+            if (lane == 0) {
+                long g = 0, u = 0;
+                bool stop = false;
+                uint32_t sa = 0;
+                auto wait = [&]() {  // the next stage has landed
+                    const int st = (int)(g % OZ_STAGES);
+                    if (!mbar_wait(smem_u32(&full[st]), (uint32_t)((g / OZ_STAGES) & 1), abort_flag, OZ_WAIT)) {
+                        if (!*abort_flag) { *abort_flag = 1; atomicCAS(a.err, 0, 2); }
+                        return false;
+                    }
+                    tc_fence_after();
+                    sa = smem_u32(smem + (size_t)st * OZ_STAGE_BYTES);
+                    g++;
+                    return true;
+                };
+                auto mma = [&](uint32_t d, uint32_t ax, uint32_t bx, uint32_t acc) {
 #pragma unroll
-                                for (int kk = 0; kk < OZ_BK / 16; kk++) {
-                                    umma_f16(d, desc_sw64(sa + kk * 32), desc_sw64(sb + kk * 32), OZ_IDESC, accf);
-                                    accf = 1;
-                                }
-                                umma_commit(smem_u32(&empty[st]));
+                    for (int kk = 0; kk < OZ_BK / 16; kk++) {
+                        umma_f16(d, desc_sw64(ax + kk * 32), desc_sw64(bx + kk * 32), OZ_IDESC, acc);
+                        acc = 1;
+                    }
+                };
+                for (int t = blockIdx.x; t < a.ntiles && !stop; t += gridDim.x) {
+                    const int kb0 = a.tiles[t].z * a.kper, kb1 = min(a.nkb, kb0 + a.kper);
+                    for (int kb = kb0; kb < kb1 && !stop; kb++) {
+                        const int kbeg = kb * OZ_KB, nkc = min(OZ_KB, a.Kpad - kbeg) / OZ_BK;
+                        for (int gh = oz_first_group(s); gh < s && !stop; gh += 2, u++) {
+                            const int buf = (int)(u & 1);
+                            const long use = u >> 1;
+                            if (use > 0 && !mbar_wait(smem_u32(&aempty[buf]), (uint32_t)((use - 1) & 1), abort_flag, OZ_WAIT)) {
+                                if (!*abort_flag) { *abort_flag = 1; atomicCAS(a.err, 0, 4); }
+                                stop = true;
+                                break;
                             }
-                        if (!stop) umma_commit(smem_u32(&afull[buf]));
+                            tc_fence_after();
+                            // accumulators of groups gh - 1 and gh
+                            const uint32_t dl = tmem + (uint32_t)(2 * buf * OZ_BN), dh = dl + OZ_BN;
+                            for (int kc = 0; kc < nkc; kc++) {
+                                if (gh == 0) {
+                                    stop = !wait();
+                                    if (stop) break;
+                                    mma(dh, sa, sa + OZ_A_BYTES, kc > 0);
+                                    umma_commit(smem_u32(&empty[(g - 1) % OZ_STAGES]));
+                                    continue;
+                                }
+                                stop = !wait();
+                                if (stop) break;
+                                uint32_t bprev = sa + OZ_A_BYTES;
+                                for (int p = 0; p <= gh; p++) {
+                                    stop = !wait();
+                                    if (stop) break;
+                                    mma(dh, sa, bprev, kc > 0 || p > 0);
+                                    bprev = sa + OZ_A_BYTES;
+                                    if (p < gh) mma(dl, sa, bprev, kc > 0 || p > 0);
+                                    umma_commit(smem_u32(&empty[(g - 2) % OZ_STAGES]));  // the stage before: its B is done
+                                }
+                                if (stop) break;
+                                umma_commit(smem_u32(&empty[(g - 1) % OZ_STAGES]));
+                            }
+                            if (!stop) umma_commit(smem_u32(&afull[buf]));
+                        }
                     }
                 }
             }
         }
     } else {
-        // epilogue: warps 2..5 own TMEM lanes 32*(warp % 4) .. +31 (rows of the tile)
-        const int lb = (warp & 3) * 32;
-        const uint32_t trow = (uint32_t)lb << 16;
+        asm volatile("setmaxnreg.inc.sync.aligned.u32 %0;" ::"n"(OZ_REPI));
+        // epilogue: the warp's TMEM lanes are 32*(warp % 4) .. +31 (rows of the tile), its columns a half
+        const int ew = warp - 4, lb = (warp & 3) * 32, cb = (ew >> 2) * 64;
+        const uint32_t trow = ((uint32_t)lb << 16) + (uint32_t)cb;
         long u = 0;
         bool stop = false;
         for (int t = blockIdx.x; t < a.ntiles && !stop; t += gridDim.x) {
             const int kb0 = a.tiles[t].z * a.kper, kb1 = min(a.nkb, kb0 + a.kper);
+            f2 hs[32], ls[32];  // the row's double-float sums, columns in pairs
+#pragma unroll
+            for (int j = 0; j < 32; j++) hs[j] = ls[j] = 0ull;
             for (int kb = kb0; kb < kb1 && !stop; kb++) {
-                for (int gg = 0; gg < s; gg++, u++) {
+                for (int gh = oz_first_group(s); gh < s; gh += 2, u++) {
                     const int buf = (int)(u & 1);
                     const long use = u >> 1;
                     if (!mbar_wait(smem_u32(&afull[buf]), (uint32_t)(use & 1), abort_flag, OZ_WAIT)) {
@@ -309,44 +403,22 @@ __global__ void __launch_bounds__(192, 1) k_oz_gemm(const __grid_constant__ CUte
                         break;
                     }
                     tc_fence_after();
-                    const float scale = ldexpf(1.0f, -7 * gg);
-                    const bool first = (kb == kb0 && gg == 0);
-                    for (int c0 = 0; c0 < OZ_BN; c0 += 32) {
-                        uint32_t v[32], hl[32];
-                        tmem_ld32(tmem + trow + (uint32_t)(buf * OZ_BN + c0), v);
-                        if (!first) {
-                            tmem_ld32(tmem + trow + OZ_SUM_COL + (uint32_t)(2 * c0), hl);       // heads, tails of 16 columns
-                            uint32_t hl2[32];
-                            tmem_ld32(tmem + trow + OZ_SUM_COL + (uint32_t)(2 * c0 + 32), hl2);  // the next 16
+#pragma unroll 1
+                    for (int gi = gh > 0 ? 0 : 1; gi < 2; gi++) {
+                        const float sc = __int_as_float((127 - 7 * (gh - 1 + gi)) << 23);
+                        const f2 scale = pk(sc, sc);
+                        const uint32_t ta = tmem + trow + (uint32_t)((2 * buf + gi) * OZ_BN);
+#pragma unroll
+                        for (int c0 = 0; c0 < 64; c0 += 32) {
+                            uint32_t v[32];
+                            tmem_ld32(ta + c0, v);
                             tmem_wait_ld();
 #pragma unroll
-                            for (int j = 0; j < 16; j++) {
-                                float h = __uint_as_float(hl[2 * j]), l = __uint_as_float(hl[2 * j + 1]);
-                                df_add(h, l, __uint_as_float(v[j]) * scale);
-                                hl[2 * j] = __float_as_uint(h);
-                                hl[2 * j + 1] = __float_as_uint(l);
-                                float h2 = __uint_as_float(hl2[2 * j]), l2 = __uint_as_float(hl2[2 * j + 1]);
-                                df_add(h2, l2, __uint_as_float(v[16 + j]) * scale);
-                                hl2[2 * j] = __float_as_uint(h2);
-                                hl2[2 * j + 1] = __float_as_uint(l2);
-                            }
-                            tmem_st32(tmem + trow + OZ_SUM_COL + (uint32_t)(2 * c0), hl);
-                            tmem_st32(tmem + trow + OZ_SUM_COL + (uint32_t)(2 * c0 + 32), hl2);
-                        } else {
-                            tmem_wait_ld();
-                            uint32_t h1[32], h2[32];
-#pragma unroll
-                            for (int j = 0; j < 16; j++) {
-                                h1[2 * j] = __float_as_uint(__uint_as_float(v[j]) * scale);
-                                h1[2 * j + 1] = 0u;
-                                h2[2 * j] = __float_as_uint(__uint_as_float(v[16 + j]) * scale);
-                                h2[2 * j + 1] = 0u;
-                            }
-                            tmem_st32(tmem + trow + OZ_SUM_COL + (uint32_t)(2 * c0), h1);
-                            tmem_st32(tmem + trow + OZ_SUM_COL + (uint32_t)(2 * c0 + 32), h2);
+                            for (int j = 0; j < 32; j += 2)
+                                df_add2(hs[(c0 + j) / 2], ls[(c0 + j) / 2],
+                                        mul2(pk(__uint_as_float(v[j]), __uint_as_float(v[j + 1])), scale));
                         }
                     }
-                    tmem_wait_st();
                     tc_fence_before();
                     __syncwarp();
                     if (lane == 0) mbar_arrive(smem_u32(&aempty[buf]));
@@ -354,52 +426,76 @@ __global__ void __launch_bounds__(192, 1) k_oz_gemm(const __grid_constant__ CUte
             }
             if (stop) break;
             // the tile's result: C = beta C + alpha 2^{eA + eB - 12} (head + tail), or the
-            // unscaled partial of this K split.  Each warp stages its 32 rows x 32
-            // columns in shared memory and writes them row by row, coalesced.
+            // unscaled partial of this K split.  Each warp stages 32 rows x 32 columns of sums
+            // in shared memory and writes them row by row, coalesced.  The scaled parts are built
+            // as FP64 bit patterns, so an element costs one FP64 addition, and one more where
+            // C is added to (conversions and scalings on the FP64 pipe made it six).
             const int4 tile = a.tiles[t];
             const int mrow = tile.x * OZ_BM + lb;
-            const int n0 = tile.y * OZ_BN;
-            const int m = mrow + lane;
-            const double rs = ldexp(1.0, ((m < a.M) ? a.ea[m] : 0) - 12);
+            const int em = (mrow + lane < a.M) ? a.ea[mrow + lane] - 12 : 0;
             const bool split = a.part != nullptr;
-            double *st = stage + (size_t)(warp - 2) * 32 * 33;
-            for (int c0 = 0; c0 < OZ_BN; c0 += 32) {
-                uint32_t h1[32], h2[32];
-                tmem_ld32(tmem + trow + OZ_SUM_COL + (uint32_t)(2 * c0), h1);
-                tmem_ld32(tmem + trow + OZ_SUM_COL + (uint32_t)(2 * c0 + 32), h2);
-                tmem_wait_ld();
+            float2 *st = stage + (size_t)ew * 32 * 33;
 #pragma unroll
-                for (int j = 0; j < 16; j++) {
-                    st[lane * 33 + j] = ((double)__uint_as_float(h1[2 * j]) + (double)__uint_as_float(h1[2 * j + 1])) * rs;
-                    st[lane * 33 + 16 + j] = ((double)__uint_as_float(h2[2 * j]) + (double)__uint_as_float(h2[2 * j + 1])) * rs;
+            for (int c0 = 0; c0 < 64; c0 += 32) {
+#pragma unroll
+                for (int j = 0; j < 32; j += 2) {
+                    const float2 h = upk(hs[(c0 + j) / 2]), l = upk(ls[(c0 + j) / 2]);
+                    st[lane * 33 + j] = make_float2(h.x, l.x);
+                    st[lane * 33 + j + 1] = make_float2(h.y, l.y);
                 }
                 __syncwarp();
-                const int n = n0 + c0 + lane;
-                const double cs = (n < a.N) ? ldexp(1.0, a.eb[n]) : 0.0;
-                // the C values of 16 rows are loaded together before any store (one round
-                // trip per 16 rows instead of one per row)
+                const int n = tile.y * OZ_BN + cb + c0 + lane;
+                const int en = (n < a.N) ? a.eb[n] : 0;
+                // FORM 0: +-result or partial, 1: C +- result, 2: any alpha and beta.  The C values of
+                // 16 rows are loaded together before any store (one round trip per 16 rows instead
+                // of one per row)
+                auto emit = [&](auto form, auto inside) {
+                    constexpr int FORM = decltype(form)::value;
+                    constexpr bool INSIDE = decltype(inside)::value;  // no element to leave out
+                    const long ld = split ? a.N : a.ldc;
+                    double *base = (split ? a.part + (size_t)tile.z * a.M * a.N : a.C) + (size_t)mrow * ld + n;
+                    const unsigned long long sg = (!split && a.alpha < 0.0) ? 1ull << 63 : 0ull;
 #pragma unroll 1
-                for (int r0 = 0; r0 < 32; r0 += 16) {
-                    double cv[16];
+                    for (int r0 = 0; r0 < 32; r0 += 16, base += 16 * ld) {
+                        double cv[16];
 #pragma unroll
-                    for (int rr = 0; rr < 16; rr++) {
-                        const int mm = mrow + r0 + rr;
-                        const bool ok = !split && a.beta != 0.0 && mm < a.M && n < a.N && !(a.lower && n > mm);
-                        cv[rr] = ok ? a.C[(size_t)mm * a.ldc + n] : 0.0;
-                    }
+                        for (int rr = 0; rr < 16; rr++) {
+                            const int mm = mrow + r0 + rr;
+                            const bool ok = INSIDE || (mm < a.M && n < a.N && !(a.lower && n > mm));
+                            cv[rr] = (FORM == 1 || (FORM == 2 && a.beta != 0.0)) && ok ? base[rr * ld] : 0.0;
+                        }
 #pragma unroll
-                    for (int rr = 0; rr < 16; rr++) {
-                        const int mm = mrow + r0 + rr;
-                        if (mm >= a.M || n >= a.N || (a.lower && n > mm)) continue;
-                        const double v = st[(r0 + rr) * 33 + lane] * cs;
-                        if (split) a.part[((size_t)tile.z * a.M + mm) * a.N + n] = v;
-                        else a.C[(size_t)mm * a.ldc + n] = (a.beta == 0.0) ? a.alpha * v : fma(a.beta, cv[rr], a.alpha * v);
+                        for (int rr = 0; rr < 16; rr++) {
+                            const int mm = mrow + r0 + rr, e = __shfl_sync(0xffffffffu, em, r0 + rr) + en;
+                            const float2 x = st[(r0 + rr) * 33 + lane];
+                            if (!INSIDE && (mm >= a.M || n >= a.N || (a.lower && n > mm))) continue;
+                            double xh, xl, v;
+                            const bool near = dfb::scaled(__float_as_uint(x.x), e, &xh) & dfb::scaled(__float_as_uint(x.y), e, &xl);
+                            v = xh + xl;
+                            if (!near) v = oz_join_far(x.x, x.y, e - en, en);
+                            if (FORM < 2) v = __longlong_as_double((long long)((unsigned long long)__double_as_longlong(v) ^ sg));
+                            if (FORM == 1) v = cv[rr] + v;
+                            if (FORM == 2) v = fma(a.beta, cv[rr], a.alpha * v);
+                            base[rr * ld] = v;
+                        }
                     }
-                }
+                };
+                // (warp-uniform) every element of the 32 x 32 block is one of C's
+                const int nl = tile.y * OZ_BN + cb + c0 + 31;
+                const bool in = mrow + 31 < a.M && nl < a.N && !(a.lower && nl > mrow);
+                constexpr std::integral_constant<bool, true> yes{};
+                constexpr std::integral_constant<bool, false> no{};
+                const bool unit = a.alpha == 1.0 || a.alpha == -1.0;
+                if (split || (unit && a.beta == 0.0)) {
+                    if (in) emit(std::integral_constant<int, 0>{}, yes);
+                    else emit(std::integral_constant<int, 0>{}, no);
+                } else if (unit && a.beta == 1.0) {
+                    if (in) emit(std::integral_constant<int, 1>{}, yes);
+                    else emit(std::integral_constant<int, 1>{}, no);
+                } else
+                    emit(std::integral_constant<int, 2>{}, no);
                 __syncwarp();
             }
-            tc_fence_before();
-            __syncwarp();
         }
     }
     tc_fence_before();
@@ -549,7 +645,7 @@ modal_status oz_run(modal_ctx *ctx, const OzOperand &A, const OzOperand &B, int 
     const int grid = std::max(1, std::min(g.ntiles, nsm));
     {
         StageTimer t(ctx, MODAL_T_TC);
-        k_oz_gemm<<<grid, 192, OZ_SMEM, ctx->stream>>>(ma, mb, g);
+        k_oz_gemm<<<grid, OZ_THREADS, OZ_SMEM, ctx->stream>>>(ma, mb, g);
         MODAL_TRY(launched(ctx, "oz_gemm"));
     }
     if (ks > 1) {
