@@ -26,9 +26,10 @@
 // per K block, the class of an FP64 GEMM over K = 5000 terms.
 //
 // Kernel k_oz_gemm: persistent, one CTA per SM over the output tiles
-// (128 x 128); warp 0 TMA producer (8-stage ring of 16 KB: an A-slice and a
-// B-slice chunk of 32 K, 64-byte swizzle), warp 1 MMA issuer (tcgen05.mma
-// kind::f16, M = N = 128, K = 16) and TMEM owner, warps 4-11 epilogue (64 columns
+// (128 x 128); warp 0 TMA producer (5-stage ring of 32 KB: an A-slice and a
+// B-slice chunk of 64 K, 128-byte swizzle), warp 1 MMA issuer (tcgen05.mma
+// kind::f16, M = 128, N = 256 over the B chunks of two neighbouring stages, or 128
+// where the ring wraps) and TMEM owner, warps 4-11 epilogue (64 columns
 // of 32 rows each, the sums in 128 registers).  TMEM: four FP32 accumulators, two
 // groups that the epilogue drains while the next two fill.  Two groups at a time
 // take half as many operand copies as one (20 instead of 36 pairs of slices for
@@ -38,10 +39,13 @@
 // What bounds it: for a short K (the trailing updates of the tridiagonalisation,
 // K = 64) the epilogue's instructions, 80 per 32 elements and tile after packing two
 // columns per FP32 instruction and building the FP64 results as bit patterns; for a
-// long K the operand copies.  One group at a time, four epilogue warps, sums in
-// tensor memory and results by FP64 conversions: trailing update of 4,928 rows
-// 361 -> 186 us, of a merge's 4,960 x 4,960 x 2,480 product 2.54 -> 2.10 ms, the 220 products
-// of an eigendecomposition of n = 4,960 42.1 -> 25.1 ms.
+// long K shared memory, which the copies write and the products read (an A chunk met with
+// two B chunks by one instruction is read once; rows of 128 bytes instead of 64 halve the
+// copies' requests).  Measured, one group at a time, four epilogue warps, sums in tensor memory,
+// results by FP64 conversions -> two groups, eight warps, registers, bit patterns -> chunks of
+// 64 K and N = 256: trailing update of 4,928 rows 361 -> 186 -> 170 us, a merge's 4,960 x 4,960 x
+// 2,480 product 2.54 -> 2.10 -> 1.41 ms, the 220 products of an eigendecomposition of n = 4,960
+// 42.1 -> 25.1 -> 20.4 ms.
 #include <cuda.h>
 #include <cuda_fp16.h>
 #include <cudaTypedefs.h>
@@ -59,20 +63,20 @@ namespace {
 
 using namespace tc;
 
-constexpr int OZ_BM = 128, OZ_BN = 128, OZ_BK = 32, OZ_KB = 512, OZ_STAGES = 8;
+constexpr int OZ_BM = 128, OZ_BN = 128, OZ_BK = 64, OZ_KB = 512, OZ_STAGES = 5;
 constexpr int OZ_MAXS = 8;
-constexpr uint32_t OZ_A_BYTES = OZ_BM * OZ_BK * 2;  // 8 KB
-constexpr uint32_t OZ_B_BYTES = OZ_BN * OZ_BK * 2;  // 8 KB
+constexpr uint32_t OZ_A_BYTES = OZ_BM * OZ_BK * 2;  // 16 KB
+constexpr uint32_t OZ_B_BYTES = OZ_BN * OZ_BK * 2;  // 16 KB
 constexpr uint32_t OZ_STAGE_BYTES = OZ_A_BYTES + OZ_B_BYTES;
 constexpr int OZ_EW = 8;                          // epilogue warps: 32 rows x 64 columns of the tile each
 constexpr int OZ_THREADS = 128 + 32 * OZ_EW;      // after one warpgroup of copies and products
 constexpr int OZ_RIO = 56, OZ_REPI = 216;         // registers of that one and of the epilogue's, out of 168 each
 static_assert(128 * OZ_RIO + 32 * OZ_EW * OZ_REPI <= OZ_THREADS * 168, "registers of the launch");
-constexpr uint32_t OZ_STAGING = OZ_EW * 32 * 33 * 8;  // epilogue: 32 x 32 double-floats per warp (+1 column pad)
+constexpr uint32_t OZ_STAGING = OZ_EW * 32 * 32 * 8;  // epilogue: 32 x 32 double-floats per warp, (r, c) at 32 r + (c ^ r)
 constexpr uint32_t OZ_SMEM = OZ_STAGES * OZ_STAGE_BYTES + 1024 + 256 + OZ_STAGING;
 constexpr uint32_t OZ_TMEM_COLS = 512;
 constexpr long long OZ_WAIT = 1ll << 31;  // ~1 s of clock64 per wait
-constexpr uint32_t OZ_IDESC = idesc_f16(OZ_BM, OZ_BN);
+constexpr uint32_t OZ_IDESC = idesc_f16(OZ_BM, OZ_BN), OZ_IDESC2 = idesc_f16(OZ_BM, 2 * OZ_BN);
 
 // ------------------------------------------------------------------ slicing
 // Rows of op(X), R x K: element (r, k) = trans ? X[k*ld + r] : X[r*ld + k].
@@ -277,7 +281,7 @@ __global__ void __launch_bounds__(OZ_THREADS, 1) k_oz_gemm(const __grid_constant
             if (lane == 0) {
                 long g = 0;
                 bool stop = false;
-                // the next stage: digit p of A (p >= 0) and digit q of B (q >= 0), columns k .. k + 31
+                // the next stage: digit p of A (p >= 0) and digit q of B (q >= 0), columns k .. k + 63
                 auto load = [&](int p, int q, int m0, int n0, int k) {
                     const int st = (int)(g % OZ_STAGES);
                     const long it = g / OZ_STAGES;
@@ -285,11 +289,11 @@ __global__ void __launch_bounds__(OZ_THREADS, 1) k_oz_gemm(const __grid_constant
                         if (!*abort_flag) { *abort_flag = 1; atomicCAS(a.err, 0, 1); }
                         return false;
                     }
-                    uint8_t *sp = smem + (size_t)st * OZ_STAGE_BYTES;
+                    uint8_t *sa = smem + (size_t)st * OZ_A_BYTES, *sb = smem + OZ_STAGES * OZ_A_BYTES + (size_t)st * OZ_B_BYTES;
                     const uint32_t fb = smem_u32(&full[st]);
                     mbar_expect_tx(fb, (p >= 0 ? OZ_A_BYTES : 0u) + (q >= 0 ? OZ_B_BYTES : 0u));
-                    if (p >= 0) tma_load_2d(smem_u32(sp), &tmA, k, p * a.Mpad + m0, fb);
-                    if (q >= 0) tma_load_2d(smem_u32(sp + OZ_A_BYTES), &tmB, k, q * a.Npad + n0, fb);
+                    if (p >= 0) tma_load_2d(smem_u32(sa), &tmA, k, p * a.Mpad + m0, fb);
+                    if (q >= 0) tma_load_2d(smem_u32(sb), &tmB, k, q * a.Npad + n0, fb);
                     g++;
                     return true;
                 };
@@ -319,7 +323,7 @@ __global__ void __launch_bounds__(OZ_THREADS, 1) k_oz_gemm(const __grid_constant
             if (lane == 0) {
                 long g = 0, u = 0;
                 bool stop = false;
-                uint32_t sa = 0;
+                uint32_t sa = 0, sb = 0;
                 auto wait = [&]() {  // the next stage has landed
                     const int st = (int)(g % OZ_STAGES);
                     if (!mbar_wait(smem_u32(&full[st]), (uint32_t)((g / OZ_STAGES) & 1), abort_flag, OZ_WAIT)) {
@@ -327,14 +331,15 @@ __global__ void __launch_bounds__(OZ_THREADS, 1) k_oz_gemm(const __grid_constant
                         return false;
                     }
                     tc_fence_after();
-                    sa = smem_u32(smem + (size_t)st * OZ_STAGE_BYTES);
+                    sa = smem_u32(smem + (size_t)st * OZ_A_BYTES);
+                    sb = smem_u32(smem + OZ_STAGES * OZ_A_BYTES + (size_t)st * OZ_B_BYTES);
                     g++;
                     return true;
                 };
-                auto mma = [&](uint32_t d, uint32_t ax, uint32_t bx, uint32_t acc) {
+                auto mma = [&](uint32_t d, uint32_t ax, uint32_t bx, uint32_t idesc, uint32_t acc) {
 #pragma unroll
                     for (int kk = 0; kk < OZ_BK / 16; kk++) {
-                        umma_f16(d, desc_sw64(ax + kk * 32), desc_sw64(bx + kk * 32), OZ_IDESC, acc);
+                        umma_f16(d, desc_sw128(ax + kk * 32), desc_sw128(bx + kk * 32), idesc, acc);
                         acc = 1;
                     }
                 };
@@ -351,25 +356,30 @@ __global__ void __launch_bounds__(OZ_THREADS, 1) k_oz_gemm(const __grid_constant
                                 break;
                             }
                             tc_fence_after();
-                            // accumulators of groups gh - 1 and gh
-                            const uint32_t dl = tmem + (uint32_t)(2 * buf * OZ_BN), dh = dl + OZ_BN;
+                            // accumulators of groups gh and gh - 1
+                            const uint32_t dh = tmem + (uint32_t)(2 * buf * OZ_BN), dl = dh + OZ_BN;
                             for (int kc = 0; kc < nkc; kc++) {
                                 if (gh == 0) {
                                     stop = !wait();
                                     if (stop) break;
-                                    mma(dh, sa, sa + OZ_A_BYTES, kc > 0);
+                                    mma(dh, sa, sb, OZ_IDESC, kc > 0);
                                     umma_commit(smem_u32(&empty[(g - 1) % OZ_STAGES]));
                                     continue;
                                 }
                                 stop = !wait();
                                 if (stop) break;
-                                uint32_t bprev = sa + OZ_A_BYTES;
+                                uint32_t bprev = sb;
                                 for (int p = 0; p <= gh; p++) {
                                     stop = !wait();
                                     if (stop) break;
-                                    mma(dh, sa, bprev, kc > 0 || p > 0);
-                                    bprev = sa + OZ_A_BYTES;
-                                    if (p < gh) mma(dl, sa, bprev, kc > 0 || p > 0);
+                                    // both groups' products as one, where this stage's B follows the one before
+                                    if (p < gh && sb == bprev + OZ_B_BYTES)
+                                        mma(dh, sa, bprev, OZ_IDESC2, kc > 0 || p > 0);
+                                    else {
+                                        mma(dh, sa, bprev, OZ_IDESC, kc > 0 || p > 0);
+                                        if (p < gh) mma(dl, sa, sb, OZ_IDESC, kc > 0 || p > 0);
+                                    }
+                                    bprev = sb;
                                     umma_commit(smem_u32(&empty[(g - 2) % OZ_STAGES]));  // the stage before: its B is done
                                 }
                                 if (stop) break;
@@ -407,7 +417,7 @@ __global__ void __launch_bounds__(OZ_THREADS, 1) k_oz_gemm(const __grid_constant
                     for (int gi = gh > 0 ? 0 : 1; gi < 2; gi++) {
                         const float sc = __int_as_float((127 - 7 * (gh - 1 + gi)) << 23);
                         const f2 scale = pk(sc, sc);
-                        const uint32_t ta = tmem + trow + (uint32_t)((2 * buf + gi) * OZ_BN);
+                        const uint32_t ta = tmem + trow + (uint32_t)((2 * buf + 1 - gi) * OZ_BN);
 #pragma unroll
                         for (int c0 = 0; c0 < 64; c0 += 32) {
                             uint32_t v[32];
@@ -434,14 +444,14 @@ __global__ void __launch_bounds__(OZ_THREADS, 1) k_oz_gemm(const __grid_constant
             const int mrow = tile.x * OZ_BM + lb;
             const int em = (mrow + lane < a.M) ? a.ea[mrow + lane] - 12 : 0;
             const bool split = a.part != nullptr;
-            float2 *st = stage + (size_t)ew * 32 * 33;
+            float2 *st = stage + (size_t)ew * 32 * 32;
 #pragma unroll
             for (int c0 = 0; c0 < 64; c0 += 32) {
 #pragma unroll
                 for (int j = 0; j < 32; j += 2) {
                     const float2 h = upk(hs[(c0 + j) / 2]), l = upk(ls[(c0 + j) / 2]);
-                    st[lane * 33 + j] = make_float2(h.x, l.x);
-                    st[lane * 33 + j + 1] = make_float2(h.y, l.y);
+                    st[lane * 32 + (j ^ lane)] = make_float2(h.x, l.x);
+                    st[lane * 32 + ((j + 1) ^ lane)] = make_float2(h.y, l.y);
                 }
                 __syncwarp();
                 const int n = tile.y * OZ_BN + cb + c0 + lane;
@@ -467,7 +477,7 @@ __global__ void __launch_bounds__(OZ_THREADS, 1) k_oz_gemm(const __grid_constant
 #pragma unroll
                         for (int rr = 0; rr < 16; rr++) {
                             const int mm = mrow + r0 + rr, e = __shfl_sync(0xffffffffu, em, r0 + rr) + en;
-                            const float2 x = st[(r0 + rr) * 33 + lane];
+                            const float2 x = st[(r0 + rr) * 32 + (lane ^ (r0 + rr))];
                             if (!INSIDE && (mm >= a.M || n >= a.N || (a.lower && n > mm))) continue;
                             double xh, xl, v;
                             const bool near = dfb::scaled(__float_as_uint(x.x), e, &xh) & dfb::scaled(__float_as_uint(x.y), e, &xl);
@@ -539,7 +549,7 @@ modal_status oz_encoder()
     return MODAL_OK;
 }
 
-// 2D FP16 map over [rows][Kpad], box [box_rows][32], 64-byte swizzle.
+// 2D FP16 map over [rows][Kpad], box [box_rows][64], 128-byte swizzle.
 modal_status oz_map(CUtensorMap *m, const void *base, long rows, int Kpad, int box_rows)
 {
     cuuint64_t dims[2] = {(cuuint64_t)Kpad, (cuuint64_t)rows};
@@ -547,7 +557,7 @@ modal_status oz_map(CUtensorMap *m, const void *base, long rows, int Kpad, int b
     cuuint32_t box[2] = {(cuuint32_t)OZ_BK, (cuuint32_t)box_rows};
     cuuint32_t estr[2] = {1, 1};
     CUresult r = g_oz_encode(m, CU_TENSOR_MAP_DATA_TYPE_FLOAT16, 2, const_cast<void *>(base), dims, strides, box, estr,
-                             CU_TENSOR_MAP_INTERLEAVE_NONE, CU_TENSOR_MAP_SWIZZLE_64B, CU_TENSOR_MAP_L2_PROMOTION_L2_256B,
+                             CU_TENSOR_MAP_INTERLEAVE_NONE, CU_TENSOR_MAP_SWIZZLE_128B, CU_TENSOR_MAP_L2_PROMOTION_L2_256B,
                              CU_TENSOR_MAP_FLOAT_OOB_FILL_NONE);
     if (r != CUDA_SUCCESS) { set_error("cuTensorMapEncodeTiled failed (%d)", (int)r); return MODAL_ERR_CUDA; }
     return MODAL_OK;

@@ -57,16 +57,16 @@ __device__ __forceinline__ void tma_load_2d(uint32_t dst, const void *map, int c
         : "memory");
 }
 
-// Shared-memory matrix descriptor: K-major, 64-byte swizzle (64-byte rows of
-// 32 FP16), 8-row groups 512 B apart.
-__device__ __forceinline__ uint64_t desc_sw64(uint32_t saddr)
+// Shared-memory matrix descriptor: K-major, 128-byte swizzle (128-byte rows of
+// 64 FP16), 8-row groups 1024 B apart.
+__device__ __forceinline__ uint64_t desc_sw128(uint32_t saddr)
 {
     uint64_t d = 0;
     d |= (uint64_t)((saddr & 0x3FFFF) >> 4);  // start address
     d |= (uint64_t)1 << 16;                   // leading byte offset (unused for this layout)
-    d |= (uint64_t)(512 >> 4) << 32;          // stride byte offset
+    d |= (uint64_t)(1024 >> 4) << 32;         // stride byte offset
     d |= (uint64_t)1 << 46;                   // descriptor version
-    d |= (uint64_t)4 << 61;                   // 64-byte swizzle
+    d |= (uint64_t)2 << 61;                   // 128-byte swizzle
     return d;
 }
 
