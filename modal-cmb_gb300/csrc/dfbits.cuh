@@ -146,6 +146,19 @@ DFB_HD bool scaled_rint(double x, int sh, long long *F)
     return true;
 }
 
+// F = x 2^sh rounded to the nearest integer (halves away from zero) where |x 2^sh| < 2^55:
+// the significand with three bits below, shifted once, rounded in its last bit.  Zeros and
+// what rounds to zero by its exponent alone are covered.
+DFB_HD bool near_int(double x, int sh, long long *F)
+{
+    const uint64_t u = bits64(x);
+    const int e11 = (int)((u >> 52) & 2047u), sft = 1077 - sh - e11;
+    const uint64_t W = (((u & 0xfffffffffffffull) | (1ull << 52)) << 3) >> (sft > 63 ? 63 : sft < 0 ? 0 : sft);
+    const int64_t q = (int64_t)((W + 1) >> 1), m = (int64_t)u >> 63;
+    *F = (q ^ m) - m;
+    return e11 != 2047 && sft >= 0 && (e11 != 0 || sft > 63);
+}
+
 // max(m, |x|) on the bit patterns (m the bits of a non-negative double): for
 // non-negative doubles the unsigned integer order is the numeric order.  NaNs
 // are skipped, as fmax skips them; infinities count.  Start from 0 (+0.0).

@@ -26,6 +26,7 @@
 #include <vector>
 #include "common.cuh"
 #include "dfbits.cuh"
+#include "ozdigits.cuh"
 #include "triple.cuh"
 
 namespace modal {
@@ -66,50 +67,70 @@ __global__ void k_weight_rows(int U, int K, int Kpad, const double *__restrict__
 }
 
 // Digits of the rows Y_vt(k) = (wk[k] X_v(k)) X_t(k) = Z_v(k) X_t(k) (one FP64
-// product), one warp per row: the row's exponent from its maximum, then s
-// balanced 7-bit digits of y 2^{6 - e + 7(s-1)} rounded to an integer (the
-// ozgemm.cu layout: out[p][r][k], FP16).  Rows >= UV are zero.  The maximum
-// and the scaled rounding run on the bit patterns (integer instructions), so
-// the FP64 pipe sees one multiply per element and pass.
-__global__ void __launch_bounds__(256) k_slice_y(int UV, int UVpad, int K, int Kpad, const int2 *__restrict__ vt,
-                                                 const double *__restrict__ X, const double *__restrict__ Z, long ldx,
-                                                 int s, __half *__restrict__ out, int *__restrict__ ey)
+// product), a CTA per row: the row's exponent from its maximum, then s balanced
+// 7-bit digits of y 2^{6 - e + 7(s-1)} rounded to an integer (ozdigits.cuh;
+// ozgemm.cu layout: out[p][r][k], FP16).  Rows >= UV are zero.  The products stay
+// in registers between the two passes up to SY_N pairs per thread (K <= 3072, what a
+// quadrature for l <= 2000 has), and are formed again beyond.  Bound by its integer
+// instructions and the 14 bytes per element it writes (0.7 ms): 1.57 ms at U = 465, K = 3,001;
+// a warp per row with two FP64 products per element, carried digits and conversions 2.58 ms.
+constexpr int SY_T = 128, SY_N = 12;
+__global__ void __launch_bounds__(SY_T) k_slice_y(long UV, int K, int Kpad, const int2 *__restrict__ vt,
+                                                  const double *__restrict__ X, const double *__restrict__ Z, long ldx,
+                                                  int s, size_t plane, __half2 *__restrict__ out, int *__restrict__ ey)
 {
-    const long r = ((long)blockIdx.x * blockDim.x + threadIdx.x) >> 5;
-    const int lane = threadIdx.x & 31;
-    if (r >= UVpad) return;
-    const size_t plane = (size_t)UVpad * Kpad;
-    __half *o = out + (size_t)r * Kpad;
+    const long r = blockIdx.x;
+    const int tid = threadIdx.x, n2 = Kpad / 2;  // pairs of elements of the row
+    __half2 *o = out + (size_t)r * n2;
     if (r >= UV) {
-        for (int k = lane; k < Kpad; k += 32)
-            for (int p = 0; p < s; p++) o[p * plane + k] = __int2half_rn(0);
-        if (lane == 0) ey[r] = 0;
+        for (int k = tid; k < n2; k += SY_T)
+            for (int p = 0; p < s; p++) o[p * plane + k] = __half2half2(__int2half_rn(0));
+        if (tid == 0) ey[r] = 0;
         return;
     }
     const int2 p2 = vt[r];
-    const double *zv = Z + (size_t)p2.x * ldx, *xt = X + (size_t)p2.y * ldx;
+    const double2 *zv = reinterpret_cast<const double2 *>(Z + (size_t)p2.x * ldx);
+    const double2 *xt = reinterpret_cast<const double2 *>(X + (size_t)p2.y * ldx);
+    auto prod = [&](int k) {  // zero beyond the nodes (X is not set there)
+        const double2 z = zv[k], x = xt[k];
+        return make_double2(2 * k < K ? z.x * x.x : 0.0, 2 * k + 1 < K ? z.y * x.y : 0.0);
+    };
+    const bool keep = n2 <= SY_T * SY_N;
+    double2 y[SY_N];
     unsigned long long mb = 0ull;
-    for (int k = lane; k < K; k += 32) mb = dfb::absmax_bits(mb, zv[k] * xt[k]);
+    if (keep) {
+#pragma unroll
+        for (int i = 0; i < SY_N; i++)
+            if (tid + SY_T * i < n2) {
+                y[i] = prod(tid + SY_T * i);
+                mb = dfb::absmax_bits(dfb::absmax_bits(mb, y[i].x), y[i].y);
+            }
+    } else
+        for (int k = tid; k < n2; k += SY_T) {
+            const double2 v = prod(k);
+            mb = dfb::absmax_bits(dfb::absmax_bits(mb, v.x), v.y);
+        }
+    __shared__ unsigned long long smax[SY_T / 32];
 #pragma unroll
     for (int off = 16; off > 0; off >>= 1) mb = max(mb, __shfl_xor_sync(0xffffffffu, mb, off));
-    const double m = __longlong_as_double((long long)mb);
-    const int e = (m > 0.0 && isfinite(m)) ? ilogb(m) + 1 : 0;
-    if (lane == 0) ey[r] = e;
+    if ((tid & 31) == 0) smax[tid >> 5] = mb;
+    __syncthreads();
+#pragma unroll
+    for (int w = 0; w < SY_T / 32; w++) mb = max(mb, smax[w]);
+    // ilogb of the maximum (a normal number's exponent field), 0 for a row of zeros or infinities
+    const int f = (int)(mb >> 52);
+    const int e = (mb == 0ull || f == 2047) ? 0 : f > 0 ? f - 1022 : ilogb(__longlong_as_double((long long)mb)) + 1;
+    if (tid == 0) ey[r] = e;
     const int sh = 6 - e + 7 * (s - 1);
-    for (int k = lane; k < Kpad; k += 32) {
-        const double y = (k < K) ? zv[k] * xt[k] : 0.0;
-        long long F;
-        if (!dfb::scaled_rint(y, sh, &F)) {
-            const double ys = ldexp(y, sh);
-            F = isfinite(ys) ? __double2ll_rn(ys) : 0ll;
+    if (keep) {
+#pragma unroll
+        for (int i = 0; i < SY_N; i++)
+            if (tid + SY_T * i < n2) ozd::store2(y[i].x, y[i].y, sh, s, o + tid + SY_T * i, plane);
+    } else
+        for (int k = tid; k < n2; k += SY_T) {
+            const double2 v = prod(k);
+            ozd::store2(v.x, v.y, sh, s, o + k, plane);
         }
-        for (int p = s - 1; p > 0; p--) {
-            const long long d = ((F + 64) & 127) - 64;
-            o[p * plane + k] = __int2half_rn((int)d);
-            F = (F - d) >> 7;
-        }
-        o[k] = __int2half_rn((int)F);
-    }
 }
 
 }  // namespace
@@ -193,9 +214,9 @@ modal_status gamma_split_dev(modal_ctx *ctx, int mu0, int nmu)
     double *Z = reinterpret_cast<double *>(b + o_z);
     k_weight_rows<<<ceil_div((long)U * Kpad, 256), 256, 0, ctx->stream>>>(U, nmu, Kpad, X, wk, Z);
     MODAL_TRY(launched(ctx, "weight_rows"));
-    k_slice_y<<<ceil_div(UVpad * 32, 256), 256, 0, ctx->stream>>>((int)UV, (int)UVpad, nmu, Kpad,
-                                                                   reinterpret_cast<const int2 *>(b + o_vtp), X, Z, Kpad,
-                                                                   SP_SLICES_G, ys.slices, ys.ex);
+    k_slice_y<<<(unsigned)UVpad, SY_T, 0, ctx->stream>>>(UV, nmu, Kpad, reinterpret_cast<const int2 *>(b + o_vtp), X, Z,
+                                                         Kpad, SP_SLICES_G, (size_t)UVpad * Kpad / 2,
+                                                         reinterpret_cast<__half2 *>(ys.slices), ys.ex);
     MODAL_TRY(launched(ctx, "slice_y"));
     oz.slices = SP_SLICES_G;
     oz.ksplit = 1;

@@ -55,6 +55,7 @@
 #include <vector>
 #include "common.cuh"
 #include "dfbits.cuh"
+#include "ozdigits.cuh"
 #include "tc_ptx.cuh"
 
 namespace modal {
@@ -137,7 +138,6 @@ __global__ void __launch_bounds__(256) k_oz_slice(int R, int K, int Rpad, int Kp
     __shared__ double tile[32][33];
     __shared__ int sexp[32];
     const int r0 = blockIdx.x * 32, kb = blockIdx.y * kchunk, ke = min(Kpad, kb + kchunk);
-    const int tx = threadIdx.x & 31, ty = threadIdx.x >> 5;
     if (threadIdx.x < 32) {
         const int r = r0 + threadIdx.x;
         const int e = ex[r];
@@ -149,25 +149,12 @@ __global__ void __launch_bounds__(256) k_oz_slice(int R, int K, int Rpad, int Kp
     for (int k0 = kb; k0 < ke; k0 += 32) {
         if (k0 < K) oz_load_tile(tile, X, ld, trans, R, K, r0, k0);
         __syncthreads();
-        for (int rr = ty; rr < 32; rr += 8) {
-            const int r = r0 + rr, k = k0 + tx;
-            // F = x 2^{6 - e + 7(s-1)} rounded to an integer, |F| < 2^55 (from the bits
-            // of x; FP64 instructions only outside that route's range); its balanced
-            // base-128 digits, least significant first, are exact integer operations
-            const double x = (k0 < K) ? tile[rr][tx] : 0.0;
-            const int sh = 6 - sexp[rr] + 7 * (s - 1);
-            long long F;
-            if (!dfb::scaled_rint(x, sh, &F)) {
-                const double y = ldexp(x, sh);
-                F = isfinite(y) ? __double2ll_rn(y) : 0ll;
-            }
-            __half *o = out + (size_t)r * Kpad + k;
-            for (int p = s - 1; p > 0; p--) {
-                const long long d = ((F + 64) & 127) - 64;
-                o[p * plane] = __int2half_rn((int)d);
-                F = (F - d) >> 7;
-            }
-            o[0] = __int2half_rn((int)F);
+        // two neighbouring columns per thread
+        const int c = 2 * (threadIdx.x & 15);
+        for (int rr = threadIdx.x >> 4; rr < 32; rr += 16) {
+            const double x0 = (k0 < K) ? tile[rr][c] : 0.0, x1 = (k0 < K) ? tile[rr][c + 1] : 0.0;
+            ozd::store2(x0, x1, 6 - sexp[rr] + 7 * (s - 1), s,
+                        reinterpret_cast<__half2 *>(out + (size_t)(r0 + rr) * Kpad + k0 + c), plane / 2);
         }
         __syncthreads();
     }

