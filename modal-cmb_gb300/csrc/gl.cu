@@ -1,6 +1,7 @@
 // gl.cu -- Gauss-Legendre quadrature, the P_l(mu) table, the shifted Legendre
 // basis and the asymptotic geometric factor, all FP64 on the GPU.
 #include "common.cuh"
+#include "legendre.cuh"
 
 namespace modal {
 
@@ -28,30 +29,48 @@ __device__ __forceinline__ double div_small(double n, double c, double r)
 // small enough is completed to third order and the derivative carried to the root,
 //     w = 2 / df(theta + d)^2,
 // so that one recurrence per root does for n >= 31 (two for smaller n; 30 at most).
-// The bound is that recurrence: n steps of six dependent FP64 operations, one warp per SM.
-// n = 3001: 47.4 -> 1.06 ms per call (the Newton iteration before this ran until a step fell below
-// 1e-17, about 20 recurrences, with a full division per step); weights as accurate as before (4e-14).
+// The bound is that recurrence: a quarter of an SM takes one FP64 warp instruction per 64 cycles, so
+// it counts instructions of one warp.  The warp that recurs has six per step; a second one, on
+// another quarter, prepares l, 1/(l+1) and (2l+1) y a chunk ahead (nine in one warp: n = 1501
+// 448 us, now 324 us, the same bits; n = 3001 by a Newton iteration of about 20
+// recurrences with a full division per step: 47.4 ms).
 // ---------------------------------------------------------------------------
-constexpr int GL_CH = 256;  // reciprocals staged per chunk of the recurrence
+constexpr int GL_CH = 32;  // steps per chunk of the recurrence
 
-// P_n and Q at cos(theta) for every thread of the block (uniform control flow).
+// P_n and Q at cos(theta) for the 32 threads of warp 0, th on both warps (uniform control flow; 64 threads).
 __device__ __forceinline__ void leg_diff(int n, double th, double &Pn, double &Q)
 {
-    __shared__ double rec[GL_CH];
+    __shared__ double rec[2][GL_CH], num[2][GL_CH + 1], tt[2][GL_CH][32];
+    const int lane = threadIdx.x & 31;
+    const bool ahead = threadIdx.x >= 32;
     const double s = sin(0.5 * th), y = 2.0 * s * s;
-    double P = 1.0, D = 0.0, l = 0.0;
-    for (int c0 = 0; c0 < n; c0 += GL_CH) {
-        __syncthreads();
-        for (int i = threadIdx.x; i < GL_CH; i += blockDim.x) rec[i] = 1.0 / (double)(c0 + i + 1);
-        __syncthreads();
-        const int m = min(GL_CH, n - c0);
+    double P = 1.0, D = 0.0;
+    auto prepare = [&](int c0) {
+        const int b = (c0 / GL_CH) & 1;
+        const double l1 = (double)(c0 + lane + 1);
+        rec[b][lane] = 1.0 / l1;
+        num[b][lane + 1] = l1;
+        if (lane == 0) num[b][0] = l1 - 1.0;
+        __syncwarp();
 #pragma unroll 4
-        for (int i = 0; i < m; i++) {
-            const double t = (2.0 * l + 1.0) * y, l1 = l + 1.0;
-            D = div_small(fma(l, D, -(t * P)), l1, rec[i]);
-            P += D;
-            l = l1;
+        for (int i = 0; i < GL_CH; i++) tt[b][i][lane] = (num[b][i] + num[b][i + 1]) * y;
+    };
+    __syncthreads();
+    if (ahead) prepare(0);
+    __syncthreads();
+    for (int c0 = 0; c0 < n; c0 += GL_CH) {
+        if (ahead) {
+            if (c0 + GL_CH < n) prepare(c0 + GL_CH);
+        } else {
+            const int b = (c0 / GL_CH) & 1;
+            const int m = min(GL_CH, n - c0);
+#pragma unroll 8
+            for (int i = 0; i < m; i++) {
+                D = div_small(fma(num[b][i], D, -(tt[b][i][lane] * P)), num[b][i + 1], rec[b][i]);
+                P += D;
+            }
         }
+        __syncthreads();
     }
     Pn = P;
     Q = -D + y * P;
@@ -69,16 +88,21 @@ __device__ __forceinline__ double gl_guess(int n, int k)
     return ps + (ps * cos(ps) / sin(ps) - 1.0) / (8.0 * ps * v * v);
 }
 
-__global__ void k_gl_nodes(int n, double *mu, double *w)
+__global__ void __launch_bounds__(GL_THREADS) k_gl_nodes(int n, double *mu, double *w)
 {
     const int half = n / 2;
-    const int k = blockIdx.x * blockDim.x + threadIdx.x + 1;  // root index 1..half (+ middle)
-    const bool root = k <= half, mid = k == half + 1 && (n & 1);
+    __shared__ double s_th[32];
+    const int lane = threadIdx.x & 31;
+    const bool first = threadIdx.x < 32;        // warp 0 holds the roots, warp 1 works ahead for it
+    const int k = blockIdx.x * 32 + lane + 1;  // root index 1..half (+ middle)
+    const bool root = first && k <= half, mid = first && k == half + 1 && (n & 1);
     double th = root ? gl_guess(n, k) : 1.5707963267948966192313216916397514, wk = 0.0;
     bool open = root || mid;
     for (int it = 0; it < 30; it++) {
         double f, Q;
-        leg_diff(n, th, f, Q);
+        if (first) s_th[lane] = th;
+        __syncthreads();
+        leg_diff(n, s_th[lane], f, Q);
         if (open && mid) {
             wk = 2.0 / ((double)n * n * Q * Q);
             open = false;
@@ -111,9 +135,9 @@ __global__ void k_gl_nodes(int n, double *mu, double *w)
 
 modal_status gl_nodes_dev(modal_ctx *ctx, int n, double *d_mu, double *d_w)
 {
-    const int threads = 32;  // one warp per SM: the roots' recurrences share an SM's FP64 pipe otherwise
+    const int threads = 32;  // roots per block: one recurring warp per SM
     const int roots = n / 2 + 1;
-    k_gl_nodes<<<ceil_div(roots, threads), threads, 0, ctx->stream>>>(n, d_mu, d_w);
+    k_gl_nodes<<<ceil_div(roots, threads), GL_THREADS, 0, ctx->stream>>>(n, d_mu, d_w);
     return launched(ctx, "gl_nodes");
 }
 
@@ -136,46 +160,84 @@ __global__ void k_pl_factors(int lmax, double *pw)
 // many warps as possible: the recurrence is serial in l, so the length of the FP64
 // dependency chain, not the bytes written, sets the time.  The arithmetic is
 // gsl_sf_legendre_Pl's upward recurrence, (x (2l-1) P_{l-1} - (l-1) P_{l-2}) / l, the division by
-// Markstein's correction (div_small: the same bits), which leaves four dependent operations per
-// step instead of about fifteen.
-// 1802 nodes to l = 1201: 576 -> 345 us, bit-identical.
-constexpr int PL_WPB = 1;  // warps per block (measured: 1 and 4 give the same time; the chains do not contend)
-__global__ void __launch_bounds__(32 * PL_WPB) k_legendre_table(int nmu, int lmax, const double *__restrict__ mu,
-                                                                const double *__restrict__ pw, double *__restrict__ pl)
+// Markstein's correction (div_small: the same bits).  A quarter of an SM takes one FP64 warp
+// instruction per 64 cycles, so the time is a warp's instruction count: warp 0 recurs (five per
+// step), warp 1 forms x (2l-1) a chunk of PL_CH steps ahead, warp 2 scales and stores the chunk
+// before.  1802 nodes to l = 1201: 244 us, all eight in one warp 363 us, with a full division 576 us; the same
+// bits throughout.
+constexpr int PL_CH = 16;
+__global__ void __launch_bounds__(PL_THREADS) k_legendre_table(int nmu, int lmax, const double *__restrict__ mu,
+                                                               const double *__restrict__ pw, double *__restrict__ pl)
 {
-    // [lmax+1][3]: 2l - 1, 1/l, (2l+1)^{2/3}: loads, where conversions would take turns on the FP64
+    // [lmax+1][3]: l, 1/l, (2l+1)^{2/3}: loads, where conversions would take turns on the FP64
     // pipe and a global load of the factor would stall the chain
     extern __shared__ double tab[];
+    __shared__ double st[2][PL_CH][32], sp[2][PL_CH][32];
     for (int l = threadIdx.x; l <= lmax; l += blockDim.x) {
-        tab[3 * l] = (double)(2 * l - 1);
+        tab[3 * l] = (double)l;
         tab[3 * l + 1] = l > 0 ? 1.0 / (double)l : 0.0;
         tab[3 * l + 2] = pw[l];
     }
     __syncthreads();
-    const int k = blockIdx.x * blockDim.x + threadIdx.x;
-    if (k >= nmu) return;
-    const double x = mu[k];
+    const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31, k = blockIdx.x * 32 + lane;
+    const double x = k < nmu ? mu[k] : 0.0;
     const bool edge = x == 1.0 || x == -1.0;  // exact values there
     double *o = pl + k;
-    o[0] = tab[2];
-    if (lmax >= 1) o[nmu] = tab[5] * x;
     double pm2 = 1.0, pm1 = x, c1 = 1.0;
-    if (lmax >= 2) {
-        // P_2 in closed form, as GSL; the recurrence goes on from its own value
-        const double pr = div_small(fma(x * tab[6], pm1, -(c1 * pm2)), 2.0, tab[7]);
-        pm2 = pm1;
-        pm1 = pr;
-        c1 = 2.0;
-        o[2 * (size_t)nmu] = tab[8] * (0.5 * (3.0 * x * x - 1.0));
-    }
+    auto ahead = [&](int c) {  // x (2l - 1) of chunk c
+        for (int i = 0; i < PL_CH; i++) {
+            const int l = 3 + c * PL_CH + i;
+            if (l <= lmax) st[c & 1][i][lane] = x * (double)(2 * l - 1);
+        }
+    };
+    if (warp == 0) {
+        if (k < nmu) {
+            o[0] = tab[2];
+            if (lmax >= 1) o[nmu] = tab[5] * x;
+        }
+        if (lmax >= 2) {
+            // P_2 in closed form, as GSL; the recurrence goes on from its own value
+            const double pr = div_small(fma(x * 3.0, pm1, -(c1 * pm2)), 2.0, tab[7]);
+            pm2 = pm1;
+            pm1 = pr;
+            c1 = 2.0;
+            if (k < nmu) o[2 * (size_t)nmu] = tab[8] * (0.5 * (3.0 * x * x - 1.0));
+        }
+    } else if (warp == 1)
+        ahead(0);
+    __syncthreads();
+    const int nc = lmax >= 3 ? (lmax - 3) / PL_CH + 1 : 0;  // chunks of l = 3 .. lmax
+    for (int c = 0; c <= nc; c++) {
+        const int l0 = 3 + c * PL_CH;
+        if (warp == 0) {
+            if (c < nc) {
+                const int m = min(PL_CH, lmax - l0 + 1);
+                auto step = [&](int i) {
+                    const double cl = tab[3 * (l0 + i)];
+                    const double pr = div_small(fma(st[c & 1][i][lane], pm1, -(c1 * pm2)), cl, tab[3 * (l0 + i) + 1]);
+                    pm2 = pm1;
+                    pm1 = pr;
+                    c1 = cl;
+                    sp[c & 1][i][lane] = pr;
+                };
+                if (m == PL_CH) {
+#pragma unroll
+                    for (int i = 0; i < PL_CH; i++) step(i);
+                } else
+                    for (int i = 0; i < m; i++) step(i);
+            }
+        } else if (warp == 1) {
+            if (c + 1 < nc) ahead(c + 1);
+        } else if (c > 0 && k < nmu) {
+            const int b0 = l0 - PL_CH, m = min(PL_CH, lmax - b0 + 1);
 #pragma unroll 4
-    for (int l = 3; l <= lmax; l++) {
-        const double c = c1 + 1.0;
-        const double pr = div_small(fma(x * tab[3 * l], pm1, -(c1 * pm2)), c, tab[3 * l + 1]);
-        pm2 = pm1;
-        pm1 = pr;
-        c1 = c;
-        o[(size_t)l * nmu] = tab[3 * l + 2] * (edge ? (x > 0.0 || !(l & 1) ? 1.0 : -1.0) : pr);
+            for (int i = 0; i < m; i++) {
+                const int l = b0 + i;
+                const double pr = sp[(c - 1) & 1][i][lane];
+                o[(size_t)l * nmu] = tab[3 * l + 2] * (edge ? (x > 0.0 || !(l & 1) ? 1.0 : -1.0) : pr);
+            }
+        }
+        __syncthreads();
     }
 }
 
@@ -186,10 +248,10 @@ modal_status legendre_table_dev(modal_ctx *ctx, int nmu, int lmax, const double 
     k_pl_factors<<<ceil_div(lmax + 1, 256), 256, 0, ctx->stream>>>(lmax, pw);
     MODAL_TRY(launched(ctx, "pl_factors"));
     const size_t smem = sizeof(double) * 3 * (size_t)(lmax + 1);
-    if (smem > 200 * 1024) { set_error("legendre table: lmax = %d too large", lmax); return MODAL_ERR_ARG; }
+    if (smem > PL_SMEM_MAX) { set_error("legendre table: lmax = %d too large", lmax); return MODAL_ERR_ARG; }
     // the limit, not this call's size: the allocation-free entry point launches the kernel with its own size
-    MODAL_CUDA(cudaFuncSetAttribute(k_legendre_table, cudaFuncAttributeMaxDynamicSharedMemorySize, 200 * 1024));
-    k_legendre_table<<<ceil_div(nmu, 32 * PL_WPB), 32 * PL_WPB, smem, ctx->stream>>>(nmu, lmax, d_mu, pw, d_pl);
+    MODAL_CUDA(cudaFuncSetAttribute(k_legendre_table, cudaFuncAttributeMaxDynamicSharedMemorySize, PL_SMEM_MAX));
+    k_legendre_table<<<ceil_div(nmu, 32), PL_THREADS, smem, ctx->stream>>>(nmu, lmax, d_mu, pw, d_pl);
     return launched(ctx, "legendre_table");
 }
 

@@ -31,15 +31,14 @@
 // gamma_fp64.cu); only the buffers differ.
 #include <mutex>
 #include "common.cuh"
+#include "legendre.cuh"
 
 #define MODAL_NOALLOC_MAX_DEVICES 64
 
 namespace modal {
 
 // Kernels defined in gl.cu and gamma_fp64.cu.
-__global__ void k_gl_nodes(int n, double *mu, double *w);
 __global__ void k_pl_factors(int lmax, double *pw);
-__global__ void k_legendre_table(int nmu, int lmax, const double *mu, const double *pw, double *pl);
 __global__ void k_mij_fp64(int nmu, int lmin, int lmax, int P, int npair, const double *pl, const double *q,
                            const int2 *pairs, double *mt);
 __global__ void k_wgt48(int nmu, const double *w, double *wg);
@@ -151,14 +150,14 @@ extern "C" modal_status modal_gamma_fp64_noalloc(int lmin, int lmax, int P, cons
     const double *mu = d_nodes, *w = d_weights;
     if (own_nodes) {
         double *mu_s = reinterpret_cast<double *>(base + off_mu), *w_s = reinterpret_cast<double *>(base + off_w);
-        k_gl_nodes<<<ceil_div(nmu / 2 + 1, 32), 32, 0, s>>>(nmu, mu_s, w_s);
+        k_gl_nodes<<<ceil_div(nmu / 2 + 1, 32), GL_THREADS, 0, s>>>(nmu, mu_s, w_s);
         mu = mu_s;
         w = w_s;
     }
     k_pl_factors<<<ceil_div(lmax + 1, 256), 256, 0, s>>>(lmax, pw);
-    // the table kernel keeps its factors in 3 (lmax + 1) doubles of shared
-    // memory (at most 24 KB for the problems the scratch array admits)
-    k_legendre_table<<<ceil_div(nmu, 32), 32, sizeof(double) * 3 * (size_t)(lmax + 1), s>>>(nmu, lmax, mu, pw, pl);
+    // the table kernel keeps its factors in 3 (lmax + 1) doubles of shared memory beside its own
+    MODAL_CUDA(cudaFuncSetAttribute(k_legendre_table, cudaFuncAttributeMaxDynamicSharedMemorySize, PL_SMEM_MAX));
+    k_legendre_table<<<ceil_div(nmu, 32), PL_THREADS, sizeof(double) * 3 * (size_t)(lmax + 1), s>>>(nmu, lmax, mu, pw, pl);
     k_noalloc_pairs<<<1, 1, 0, s>>>(P, pairs, status);
     k_noalloc_triples<<<ceil_div(3L * N, 256), 256, 0, s>>>(N, P, d_triples, triples, status);
     dim3 gm(ceil_div(nmu, NA_MIJ_BK), ceil_div(npair, NA_MIJ_BU));

@@ -564,7 +564,7 @@ __global__ void k_panel_post(int n, int j0, int nbp, const double *__restrict__ 
 // triangle.  Bound by the FP64 pipe (about NBB^3 / 6 multiply-adds per block over 16
 // CTAs).  Measured at n = 816 (4 blocks): 0.22 ms; one CTA per block taking the columns
 // in turn, each entry one thread's serial sum, took 3.65 ms.
-constexpr int LARFT_ROWS = 4, LARFT_WARPS = 4;
+constexpr int LARFT_ROWS = 4, LARFT_WARPS = 1;
 __global__ void __launch_bounds__(32 * LARFT_WARPS) k_larft(int nv, const double *__restrict__ G, long ldg,
                                                             const double *__restrict__ tau, double *__restrict__ T)
 {
