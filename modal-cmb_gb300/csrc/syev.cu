@@ -35,6 +35,7 @@
 #include <vector>
 #include "common.cuh"
 #include "dfbits.cuh"
+#include "ozdigits.cuh"
 
 namespace modal {
 
@@ -540,16 +541,40 @@ __global__ void k_copy_last_diag(const double *A, int n, double *d)
     if (threadIdx.x == 0 && blockIdx.x == 0) d[n - 1] = A[(size_t)(n - 1) * n + (n - 1)];
 }
 
-// After a panel: Psw = [W V] (the halves of the panel rows swapped, for
-// A22 -= [V W] [W V]^T) and the panel's reflectors into columns j0.. of VA.
-__global__ void k_panel_post(int n, int j0, int nbp, const double *__restrict__ P, double *__restrict__ Psw,
-                             double *__restrict__ VA, long ldva)
+// After a panel: its reflectors into columns j0.. of VA, and the operands of the trailing update
+// A22 -= [V W] [W V]^T as digits (ozgemm.cu layout, K = LDP): the rows from j0 + nbp on, to `pad`
+// rows, with one exponent per row, since [W V] is [V W] with its halves swapped.  Eight threads per
+// row of P.  One launch where a copy of the swapped panel, two exponent and two slicing kernels took
+// five: over the 155 panels of n = 4,960, 1.25 ms instead of 4.2 ms.
+__global__ void __launch_bounds__(256) k_panel_post(int n, int j0, int nbp, int pad, const double *__restrict__ P,
+                                                    double *__restrict__ VA, long ldva, __half *__restrict__ sa,
+                                                    __half *__restrict__ sb, int *__restrict__ ex)
 {
-    const size_t e = (size_t)blockIdx.x * blockDim.x + threadIdx.x;
-    if (e >= (size_t)n * LDP) return;
-    const int r = (int)(e / LDP), c = (int)(e % LDP);
-    Psw[e] = P[(size_t)r * LDP + (c < TRD_NB ? c + TRD_NB : c - TRD_NB)];
-    if (c < nbp) VA[(size_t)r * ldva + j0 + c] = P[e];
+    const int r = j0 + blockIdx.x * 32 + (threadIdx.x >> 3), c = 8 * (threadIdx.x & 7), q = r - j0 - nbp;
+    double x[8];
+    unsigned long long mb = 0ull;
+#pragma unroll
+    for (int u = 0; u < 8; u++) {
+        x[u] = r < n ? P[(size_t)r * LDP + c + u] : 0.0;
+        mb = dfb::absmax_bits(mb, x[u]);
+    }
+    if (r < n && c < TRD_NB)
+#pragma unroll
+        for (int u = 0; u < 8; u++)
+            if (c + u < nbp) VA[(size_t)r * ldva + j0 + c + u] = x[u];
+#pragma unroll
+    for (int o = 1; o < 8; o <<= 1) mb = max(mb, __shfl_xor_sync(0xffffffffu, mb, o));
+    if (q < 0 || q >= pad) return;
+    const int f = (int)(mb >> 52);  // exponent field of the row's maximum; 0 for rows of zeros or infinities
+    const int e = (mb == 0ull || f == 2047) ? 0 : f > 0 ? f - 1022 : ilogb(__longlong_as_double((long long)mb)) + 1;
+    if (c == 0) ex[q] = e;
+    const size_t plane = (size_t)pad * LDP / 2;
+    __half2 *oa = reinterpret_cast<__half2 *>(sa + (size_t)q * LDP + c), *ob = reinterpret_cast<__half2 *>(sb + (size_t)q * LDP + (c ^ TRD_NB));
+#pragma unroll
+    for (int u = 0; u < 8; u += 2) {
+        ozd::store2(x[u], x[u + 1], 6 - e + 7 * (OZ_SLICES - 1), OZ_SLICES, oa + u / 2, plane);
+        ozd::store2(x[u], x[u + 1], 6 - e + 7 * (OZ_SLICES - 1), OZ_SLICES, ob + u / 2, plane);
+    }
 }
 
 // Compact-WY factor of a block of reflectors (LAPACK dlarft, forward, columnwise):
@@ -1114,7 +1139,7 @@ static void build_tree(int a, int b, int lev, std::vector<std::vector<int3>> &ou
 
 // Carve the eigensolver's workspace out of ctx->eigw for size n.
 struct SyevPtrs {
-    double *P, *Psw, *VA, *GB, *TB, *TW, *TT, *d, *e, *tau, *a, *y, *part;
+    double *P, *VA, *GB, *TB, *TW, *TT, *d, *e, *tau, *a, *y, *part;
     float2 *Ahl, *ahl;
     long ldva;
     unsigned *bar;
@@ -1138,7 +1163,6 @@ static size_t carve(uint8_t *base, int n, int npanel, int nlev, int nmerge, Syev
     p.P = (double *)take(sizeof(double) * (size_t)n * LDP);
     p.Ahl = (float2 *)take(sizeof(float2) * NN);
     p.ahl = (float2 *)take(sizeof(float2) * n);
-    p.Psw = (double *)take(sizeof(double) * (size_t)n * LDP);
     p.VA = (double *)take(sizeof(double) * (size_t)n * nvpad);          // every reflector, column j = v_j
     p.GB = (double *)take(sizeof(double) * (size_t)nvpad * nvpad);      // diagonal NBW blocks of VA^T VA
     p.TB = (double *)take(sizeof(double) * (size_t)(nvpad / NBB) * NBB * NBB);
@@ -1270,15 +1294,19 @@ static modal_status trd_run(modal_ctx *ctx, int n, double *A, SyevPtrs &p, int n
                                                    ctx->stream));
             MODAL_TRY(launched(ctx, "trd_panel"));
         }
-        k_panel_post<<<ceil_div((long)n * LDP, 256), 256, 0, ctx->stream>>>(n, j0, nbp, p.P, p.Psw, p.VA, p.ldva);
+        const int s = j0 + nbp, rest = n - s, pad = ceil_div(rest, 128) * 128;
+        const size_t plane = (size_t)OZ_SLICES * pad * LDP;
+        MODAL_TRY(ensure(ctx->ozw, 2 * plane * sizeof(__half) + sizeof(int) * (size_t)pad + 256));
+        __half *sa = ctx->ozw.as<__half>(), *sb = sa + plane;
+        int *ex = reinterpret_cast<int *>(sb + plane);
+        k_panel_post<<<ceil_div(nbp + pad, 32), 256, 0, ctx->stream>>>(n, j0, nbp, pad, p.P, p.VA, p.ldva, sa, sb, ex);
         MODAL_TRY(launched(ctx, "panel_post"));
-        const int s = j0 + nbp, rest = n - s;
         if (rest > 0) {
             // A22 -= V W^T + W V^T = [V W] [W V]^T on the lower triangle (tensor cores, FP64 accuracy)
-            // the same epilogue refreshes the block's (head, tail) float copy, both triangles
+            // and the block's (head, tail) float copy from it, both triangles
             double *A22 = A + (size_t)s * n + s;
-            MODAL_TRY(oz_gemm_ex(ctx, rest, rest, LDP, -1.0, p.P + (size_t)s * LDP, LDP, false, p.Psw + (size_t)s * LDP,
-                                 LDP, true, 1.0, A22, n, oz));
+            const OzOperand oa{sa, ex, rest, pad}, ob{sb, ex, rest, pad};
+            MODAL_TRY(oz_run(ctx, oa, ob, LDP, OZ_SLICES, nullptr, -1.0, 1.0, A22, n, oz));
             const int nt = ceil_div(rest, 32);
             k_trail_hilo<<<dim3(nt, nt), 256, 0, ctx->stream>>>(A, n, s, p.Ahl);
             MODAL_TRY(launched(ctx, "trail_hilo"));
