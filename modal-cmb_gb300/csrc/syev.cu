@@ -703,6 +703,14 @@ struct DcWork {
     int *err;
 };
 
+// Neighbouring entries deflate by a rotation when |t c s| <= tol, t the difference of their D,
+// c = z_n / tau, s = -z_p / tau, tau^2 = z_p^2 + z_n^2: tested without the square root and divisions
+// (on GB300's slow FP64 pipe); the rotation is formed only for the pairs that deflate.
+__device__ __forceinline__ bool dc_pair_deflates(double Dp, double zp, double Dn, double zn, double tol)
+{
+    return fabs(Dn - Dp) * fabs(zp * zn) <= tol * (zp * zp + zn * zn);
+}
+
 // Sort, deflate and compact one merge (one CTA per merge).
 // The serial part of the deflation (Dongarra-Sorensen: small z components,
 // then Givens rotations of close pairs) on D, z and the support flags of one
@@ -717,16 +725,14 @@ __device__ void dc_deflate_serial(DcWork &w, MergeInfo &M, int a, int k, double 
         for (int s = 0; s < k; s++) w.dl[a + nd++] = a + s;
     } else {
         int pj = -1;
+        bool fresh = false;  // entry pj is as it was when kf was set
         for (int nj = 0; nj < k; nj++) {
-            if (rho * fabs(z[nj]) <= tol) { w.dl[a + nd++] = a + nj; continue; }
-            if (pj < 0) { pj = nj; continue; }
-            // |t c s| <= tol with c = z_nj / tau, s = -z_pj / tau, tau^2 = z_pj^2 + z_nj^2,
-            // tested without the square root and divisions (on GB300's slow FP64 pipe);
-            // the rotation is formed only for the pairs that deflate
-            const double zp = z[pj], zn = z[nj], t = D[nj] - D[pj];
-            const double r2 = zp * zp + zn * zn;
-            if (fabs(t) * fabs(zp * zn) <= tol * r2) {
-                const double tau = sqrt(r2);
+            const int c0 = kf[nj];  // read before the kept flags, of which there are fewer, reach it
+            if (c0 == 1) { w.dl[a + nd++] = a + nj; continue; }
+            if (pj < 0) { pj = nj; fresh = true; continue; }
+            if (fresh ? c0 == 2 : dc_pair_deflates(D[pj], z[pj], D[nj], z[nj], tol)) {
+                const double zp = z[pj], zn = z[nj];
+                const double tau = sqrt(zp * zp + zn * zn);
                 const double c = zn / tau, s = -zp / tau;
                 fl[nj] |= fl[pj];  // the rotated vector has support on both halves
                 z[nj] = tau;
@@ -739,6 +745,7 @@ __device__ void dc_deflate_serial(DcWork &w, MergeInfo &M, int a, int k, double 
                 D[pj] = t2;
                 w.dl[a + nd++] = a + pj;
                 pj = nj;
+                fresh = false;
             } else {
                 // a kept entry's flag is final (later rotations only change the newer entry)
                 k1 += (fl[pj] == 1);
@@ -746,6 +753,7 @@ __device__ void dc_deflate_serial(DcWork &w, MergeInfo &M, int a, int k, double 
                 kf[kk] = fl[pj];
                 w.kl[a + kk++] = a + pj;
                 pj = nj;
+                fresh = true;
             }
         }
         if (pj >= 0) {
@@ -759,7 +767,10 @@ __device__ void dc_deflate_serial(DcWork &w, MergeInfo &M, int a, int k, double 
 }
 
 // One CTA per merge.  Shared memory (when the merge fits, DC_DEFL_SMEM): D, z
-// [k] doubles, support flags and kept flags [k] bytes.
+// [k] doubles, support flags and kept flags [k] bytes.  Which entries and pairs deflate is
+// decided in parallel on the entries as they come; the serial pass follows those decisions
+// and tests again only next to a rotation (an FP64 instruction of a lone thread takes 64 cycles).
+// n = 4,960, 13 levels: 2.6 ms; every test and the compaction in the serial pass 3.8 ms.
 __global__ void __launch_bounds__(256) k_dc_deflate(DcWork w, int use_smem)
 {
     extern __shared__ double dsm[];
@@ -810,9 +821,23 @@ __global__ void __launch_bounds__(256) k_dc_deflate(DcWork w, int use_smem)
     zm = warp_max(zm);
     if ((tid & 31) == 0) { s_mx[0][tid >> 5] = dm; s_mx[1][tid >> 5] = zm; }
     __syncthreads();
+    dm = zm = 0.0;
+    for (int t = 0; t < (int)(blockDim.x >> 5); t++) { dm = fmax(dm, s_mx[0][t]); zm = fmax(zm, s_mx[1][t]); }
+    const double tol = 8.0 * EPS * fmax(dm, zm);
+    // per entry, for the serial pass: 1 negligible z, 2 deflates with the entry before it that is not
+    // negligible, as long as that one has not been rotated
+    for (int t = tid; t < k; t += blockDim.x) {
+        int code = rho * fabs(zr[t]) <= tol ? 1 : 0;
+        if (code == 0) {
+            int pj = t - 1;
+            while (pj >= 0 && rho * fabs(zr[pj]) <= tol) pj--;
+            if (pj >= 0 && dc_pair_deflates(Dr[pj], zr[pj], Dr[t], zr[t], tol)) code = 2;
+        }
+        if (use_smem) kfsh[t] = (unsigned char)code;
+        else w.kci[a + t] = code;
+    }
+    __syncthreads();
     if (tid == 0) {
-        for (int t = 1; t < (int)(blockDim.x >> 5); t++) { dm = fmax(dm, s_mx[0][t]); zm = fmax(zm, s_mx[1][t]); }
-        const double tol = 8.0 * EPS * fmax(dm, zm);
         if (use_smem)
             dc_deflate_serial<unsigned char>(w, M, a, k, rho, zm, tol, Dsh, zsh, fsh, kfsh);
         else
@@ -826,14 +851,23 @@ __global__ void __launch_bounds__(256) k_dc_deflate(DcWork w, int use_smem)
             w.zs[a + t] = zsh[t];
             w.flg[a + t] = fsh[t];
         }
-    if (tid != 0) return;
     // compact kept values; grouped columns: first-half support, both halves, second half
-    int cg[4] = {0, 0, k1 + k2, k1};
-    for (int j = 0; j < kk; j++) {
+    for (int j = tid; j < kk; j += blockDim.x) {
         const int sl = w.kl[a + j];
         w.kd[a + j] = use_smem ? Dsh[sl - a] : w.Ds[sl];
         w.kw[a + j] = use_smem ? zsh[sl - a] : w.zs[sl];
-        w.kci[a + j] = cg[use_smem ? kfsh[j] : w.kci[a + j]]++;
+    }
+    if (tid >= 32) return;
+    int c1 = 0, c2 = k1 + k2, c3 = k1;  // next column of flags 1, 2, 3
+    const unsigned below = (1u << tid) - 1u;
+    for (int j0 = 0; j0 < kk; j0 += 32) {
+        const int j = j0 + tid, f = j < kk ? (use_smem ? kfsh[j] : w.kci[a + j]) : 0;
+        const unsigned m1 = __ballot_sync(0xffffffffu, f == 1), m2 = __ballot_sync(0xffffffffu, f == 2),
+                       m3 = __ballot_sync(0xffffffffu, f == 3);
+        if (j < kk) w.kci[a + j] = f == 1 ? c1 + __popc(m1 & below) : f == 2 ? c2 + __popc(m2 & below) : c3 + __popc(m3 & below);
+        c1 += __popc(m1);
+        c2 += __popc(m2);
+        c3 += __popc(m3);
     }
 }
 
@@ -992,23 +1026,32 @@ __global__ void __launch_bounds__(256) k_dc_vectors(DcWork w)
 
 // Final positions: roots (ascending) and deflated values merged by rank; new
 // eigenvalues written; the gathered kept rows Zc[a + kci] = Z[srt[kept]].
+// Positions of a merge's new eigenvalues in ascending order (ties by index), counted on their bit
+// patterns in an order-preserving form: an eigenvalue is formed once per CTA and compared by integer
+// instructions.  n = 4,960, 13 levels: 0.26 ms (formed and compared on the FP64 pipe by every thread 2.5 ms).
 __global__ void __launch_bounds__(256) k_dc_rank(DcWork w)
 {
+    __shared__ long long key[256];
     const MergeInfo M = w.mi[blockIdx.y];
-    const int k = M.b - M.a, kk = M.kk, nd = M.nd;
-    const int t = blockIdx.x * blockDim.x + threadIdx.x;
-    if (t >= k) return;
-    auto val = [&](int x) -> double {
-        if (x < kk) return w.kd[M.a + w.org[M.a + x]] + w.rtau[M.a + x];
-        return w.Ds[w.dl[M.a + (x - kk)]];
+    const int k = M.b - M.a, kk = M.kk, tid = threadIdx.x;
+    const int t = blockIdx.x * blockDim.x + tid;
+    if (blockIdx.x * (int)blockDim.x >= k) return;
+    auto val = [&](int x) -> long long {
+        const double v = (x < kk ? w.kd[M.a + w.org[M.a + x]] + w.rtau[M.a + x] : w.Ds[w.dl[M.a + (x - kk)]]) + 0.0;
+        const long long u = __double_as_longlong(v);
+        return u ^ ((u >> 63) & 0x7fffffffffffffffll);
     };
-    const double v = val(t);
+    const long long v = t < k ? val(t) : 0;
     int r = 0;
-    for (int x = 0; x < kk + nd; x++) {
-        const double u = val(x);
-        r += (u < v) || (u == v && x < t);
+    for (int x0 = 0; x0 < k; x0 += 256) {
+        __syncthreads();
+        if (x0 + tid < k) key[tid] = val(x0 + tid);
+        __syncthreads();
+        const int m = min(256, k - x0);
+#pragma unroll 8
+        for (int i = 0; i < m; i++) r += (key[i] < v) || (key[i] == v && x0 + i < t);
     }
-    w.rank[M.a + t] = M.a + r;
+    if (t < k) w.rank[M.a + t] = M.a + r;
 }
 
 __global__ void k_dc_lam(DcWork w)
