@@ -14,7 +14,7 @@ namespace modal {
 
 __global__ void k_project_B(int L, int P, int S, const double *__restrict__ q, const double *__restrict__ Fbuf,
                             double *__restrict__ B);
-__global__ void k_project_beta(int N, int P, int S, const int *__restrict__ triples, const double *__restrict__ B,
+__global__ void k_project_beta(int N, int P, int S, int nseg, const int *__restrict__ triples, const double *__restrict__ B,
                                double *__restrict__ beta);
 
 __global__ void k_modify_bispectrum(int size, const int *__restrict__ vec, const double *__restrict__ c,
@@ -193,7 +193,7 @@ extern "C" modal_status modal_calculate_modes(modal_ctx *c, int size, const doub
         else { set_error("modal_calculate_modes: P=%d too large", P); return MODAL_ERR_ARG; }
         k_project_B<<<ceil_div((long)P * PP, 256), 256, 0, c->stream>>>(nsl, P, 1, c->q.as<double>(), Fbuf, B);
         MODAL_TRY(launched(c, "project_B"));
-        k_project_beta<<<ceil_div(N, 256), 256, 0, c->stream>>>(N, P, 1, c->triples.as<int>(), B, c->beta.as<double>());
+        k_project_beta<<<ceil_div(N, 256), 256, 0, c->stream>>>(N, P, 1, 1, c->triples.as<int>(), B, c->beta.as<double>());
         MODAL_TRY(launched(c, "project_beta"));
     }
     c->have_beta = true;

@@ -197,9 +197,10 @@ __global__ void k_slab_base(int lmin, int lmax, long long *__restrict__ base)
     if (t == 255) base[L] = part[255];
 }
 
-// Point weights in slab and row order, from their 1D factors: seven FP64 multiplications per
-// point, which bound it.  At l <= 1000: 0.69 ms; the closed form's quotients and square root
-// took 6.3 ms.  Relative error of a weight (rms, units of 2^-53): 2.9, the closed form 3.9.
+// Point weights in slab and row order, from their 1D factors: five FP64 multiplications per
+// point (0.36 ms of the FP64 pipe at l <= 1000) over rows of up to l/2 points, a warp each: 0.65 ms;
+// the closed form's quotients and square root took 6.3 ms.  Relative error of a weight (rms, units of
+// 2^-53): 2.9, the closed form 3.9.
 __global__ void __launch_bounds__(256) k_weight_table_fp64(int lmin, int lmax, const double *__restrict__ vl,
                                                            const long long *__restrict__ base, double *__restrict__ Wd)
 {
@@ -214,10 +215,11 @@ __global__ void __launch_bounds__(256) k_weight_table_fp64(int lmin, int lmax, c
     const double *gl = vl + lmax + 1 + vl_nh(lmax) + (i + j + k0) / 2;
     const double *g1 = vl + lmax + 1 + (j + k0 - i) / 2, *g2 = vl + lmax + 1 + (i + k0 - j) / 2,
                  *g3 = vl + lmax + 1 + (i + j - k0) / 2;
-    const double vij = vl[i] * vl[j];
+    const double v1 = vl[i] * vl[j], v3 = 3.0 * v1, v6 = 6.0 * v1;  // with permsix
     for (int m = lane; m < n; m += 32) {
-        const double perm = (i == j && m == 0 && ip == 0) ? 1.0 : (i == j || (m == 0 && ip == 0)) ? 3.0 : 6.0;
-        row[m] = (perm * (gl[m] * g1[m])) * (g2[m] * g3[-m]) * (vij * vk[2 * m]);
+        const bool jk = m == 0 && ip == 0;
+        const double v = i == j ? (jk ? v1 : v3) : (jk ? v3 : v6);
+        row[m] = (gl[m] * g1[m]) * (g2[m] * g3[-m]) * (v * vk[2 * m]);
     }
 }
 
@@ -340,44 +342,49 @@ __global__ void __launch_bounds__(256) k_project_slab_fp64(int lmin, int lmax, i
     }
 }
 
-// B[s][a][bc] = sum_slab q[slab][a] Fbuf[s][slab][bc]
+// B[seg][s][a][bc] = sum over the segment's slabs of q[slab][a] Fbuf[s][slab][bc].  A thread's loop
+// is bound by latency, so the slabs are split until the GPU is full (grid.y segments, added by
+// k_project_beta), eight loads in flight and four chains.  l <= 1000, P = 20, four shapes: 0.07 ms; one
+// segment 0.25 ms.
 __global__ void k_project_B(int L, int P, int S, const double *__restrict__ q, const double *__restrict__ Fbuf,
                             double *__restrict__ B)
 {
-    const int PP = P * P;
-    size_t e = (size_t)blockIdx.x * blockDim.x + threadIdx.x;
-    if (e >= (size_t)S * P * PP) return;
+    const int PP = P * P, per = (L + gridDim.y - 1) / gridDim.y, l0 = blockIdx.y * per, l1 = min(L, l0 + per);
+    const size_t e = (size_t)blockIdx.x * blockDim.x + threadIdx.x, n = (size_t)S * P * PP;
+    if (e >= n) return;
     int s = (int)(e / ((size_t)P * PP));
     int rem = (int)(e - (size_t)s * P * PP);
     int a = rem / PP, bc = rem - a * PP;
     const double *F = Fbuf + (size_t)s * L * PP + bc;
-    // eight loads in flight, four chains (the loop is one thread's and bound by latency:
-    // 0.25 ms at l <= 1000, P = 20, four shapes; 0.35 ms as one chain)
     double acc[4] = {0.0, 0.0, 0.0, 0.0};
-    int l = 0;
-    for (; l + 8 <= L; l += 8) {
+    int l = l0;
+    for (; l + 8 <= l1; l += 8) {
         double x[8];
 #pragma unroll
         for (int u = 0; u < 8; u++) x[u] = F[(size_t)(l + u) * PP];
 #pragma unroll
         for (int u = 0; u < 8; u++) acc[u & 3] = fma(q[(size_t)(l + u) * P + a], x[u], acc[u & 3]);
     }
-    for (; l < L; l++) acc[0] = fma(q[(size_t)l * P + a], F[(size_t)l * PP], acc[0]);
-    B[e] = (acc[0] + acc[1]) + (acc[2] + acc[3]);
+    for (; l < l1; l++) acc[0] = fma(q[(size_t)l * P + a], F[(size_t)l * PP], acc[0]);
+    B[blockIdx.y * n + e] = (acc[0] + acc[1]) + (acc[2] + acc[3]);
 }
 
 // beta[s][r] = (1/6) sum of B over the six orderings of mode r's triple
-__global__ void k_project_beta(int N, int P, int S, const int *__restrict__ triples, const double *__restrict__ B,
+__global__ void k_project_beta(int N, int P, int S, int nseg, const int *__restrict__ triples, const double *__restrict__ B,
                                double *__restrict__ beta)
 {
     size_t e = (size_t)blockIdx.x * blockDim.x + threadIdx.x;
     if (e >= (size_t)S * N) return;
     int s = (int)(e / N), r = (int)(e % N);
     int p1 = triples[3 * r], p2 = triples[3 * r + 1], p3 = triples[3 * r + 2];
+    const size_t n = (size_t)S * P * P * P;
     const double *b = B + (size_t)s * P * P * P;
+    double v = 0.0;
+    for (int z = 0; z < nseg; z++, b += n) {
 #define BB(x, y, z) b[((size_t)(x) * P + (y)) * P + (z)]
-    double v = BB(p1, p2, p3) + BB(p2, p3, p1) + BB(p3, p1, p2) + BB(p3, p2, p1) + BB(p2, p1, p3) + BB(p1, p3, p2);
+        v += BB(p1, p2, p3) + BB(p2, p3, p1) + BB(p3, p1, p2) + BB(p3, p2, p1) + BB(p2, p1, p3) + BB(p1, p3, p2);
 #undef BB
+    }
     beta[e] = v / 6e0;
 }
 
@@ -447,12 +454,13 @@ modal_status proj_plan(modal_ctx *ctx, int S, const modal_shape *shapes, modal_p
         if (pl.smem > 220 * 1024) { set_error("project: lmax=%d too large for the slab tile", lmax); return MODAL_ERR_ARG; }
         pl.fpt = ceil_div(PP, 256);
         if (pl.fpt > 16) { set_error("project: P=%d too large", P); return MODAL_ERR_ARG; }
-        // F partials [S][L][P*P] | B [S][P][P*P] | slab bases [L+1] | weight table [points]
+        // F partials [S][L][P*P] | B [segments][S][P][P*P] | slab bases [L+1] | weight table [points]
         long long npts = 0;
         for (int i = lmin; i <= lmax; i++) npts += tet_row_offset(i, lmax + 1, lmax);
         pl.npts = npts;
         pl.o_B = sizeof(double) * (size_t)S * L * PP;
-        pl.o_sb = pl.o_B + sizeof(double) * (size_t)S * P * PP;
+        pl.nseg = (int)std::max<long>(1, std::min<long>(std::min(8, L / 32), 152L * 1024 / ((long)S * P * PP)));
+        pl.o_sb = pl.o_B + sizeof(double) * (size_t)pl.nseg * S * P * PP;
         pl.o_w = pl.o_sb + sizeof(long long) * (size_t)(L + 1);
         MODAL_TRY(ensure(ctx->scratch, pl.o_w + sizeof(double) * (size_t)npts));
         auto attr = [&](auto kern) -> modal_status {
@@ -508,9 +516,9 @@ modal_status proj_record(modal_ctx *ctx, const ProjPlan &pl)
     else if (pl.fpt <= 4) MODAL_TRY(run(k_project_slab_fp64<4>));
     else if (pl.fpt <= 8) MODAL_TRY(run(k_project_slab_fp64<8>));
     else MODAL_TRY(run(k_project_slab_fp64<16>));
-    k_project_B<<<ceil_div((long)S * P * PP, 256), 256, 0, ctx->stream>>>(L, P, S, ctx->q.as<double>(), Fbuf, B);
+    k_project_B<<<dim3(ceil_div((long)S * P * PP, 256), pl.nseg), 256, 0, ctx->stream>>>(L, P, S, ctx->q.as<double>(), Fbuf, B);
     MODAL_TRY(launched(ctx, "project_B"));
-    k_project_beta<<<ceil_div((long)S * N, 256), 256, 0, ctx->stream>>>(N, P, S, ctx->triples.as<int>(), B,
+    k_project_beta<<<ceil_div((long)S * N, 256), 256, 0, ctx->stream>>>(N, P, S, pl.nseg, ctx->triples.as<int>(), B,
                                                                           ctx->beta.as<double>());
     return launched(ctx, "project_beta");
 }
