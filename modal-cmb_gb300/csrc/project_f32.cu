@@ -37,8 +37,10 @@
 //
 // Measured (l <= 2000, P = 30), against the CUDA-core kernel (136 warp instructions per 32 points)
 // and the shared-memory-operand tensor-core kernel that it replaces both: 16 separable shapes 33.9 ->
-// 15.8 ms, 256 mixed shapes 532 (CUDA cores), 1864 (tensor cores) -> 226 ms; error of beta against
-// 64 bits 6.2e-8 -> 1.8e-8.
+// 15.8 ms, 256 mixed shapes 532 (CUDA cores), 1864 (tensor cores) -> 233 ms; error of beta against
+// 64 bits, median and largest over the 128 bumps and 128 separable shapes: 7.5e-8, 8.9e-7 and
+// 4.7e-8, 1.3e-7 -> 5.0e-8, 7.3e-7 and 2.5e-8, 4.6e-8.  (The largest was 2.7e-6, and the 256 shapes
+// took 225 ms, with the 1D factors of the weights and of the bumps' exponents rounded to FP32.)
 #include <algorithm>
 #include <vector>
 #include <cuda_bf16.h>
@@ -114,27 +116,39 @@ __host__ __device__ inline long long pf_slab_len(int lmin, int lmax, int j)
 //   geo(l1,l2,l3) = gL(L) g(L - 2 l1) g(L - 2 l2) g(L - 2 l3) prod (2l+1), L = l1 + l2 + l3 (always even),
 //   g(x) = sqrt(x + 1/6) / (x + 1/3), gL(L) = (L + 1/3) / (2 pi^2 (L + 1) sqrt(L + 1/6))
 // (calculate_geometric.c:59-92 regrouped), v(l) = (2l+1)^{2/3} w_l (calculate_mode_3D.c:53-62).
-// g[h] = g(2h), gl[h] = gL(2h), il2[h] = 1/(2h)^2 (bumps).
-__global__ void k_pf_tables(int lmax, int nh, const double *__restrict__ cl, float *__restrict__ g, float *__restrict__ gl,
-                            float *__restrict__ il2, float *__restrict__ v)
+// g[h] = g(2h), gl[h] = gL(2h), il2[h] = 1/(2h)^2 (bumps), as double-floats: a factor's rounding is
+// shared by every point that uses it, and a sum that cancels does not average it away.
+__global__ void k_pf_tables(int lmax, int nh, const double *__restrict__ cl, float2 *__restrict__ g, float2 *__restrict__ gl,
+                            float2 *__restrict__ il2, float2 *__restrict__ v)
 {
     const int h = blockIdx.x * blockDim.x + threadIdx.x;
+    auto df = [](double x) {
+        const float hi = (float)x;
+        return make_float2(hi, (float)(x - (double)hi));
+    };
     if (h < nh) {
         const double x = 2.0 * h;
-        g[h] = (float)(sqrt(x + 1.0 / 6.0) / (x + 1.0 / 3.0));
-        gl[h] = (float)((x + 1.0 / 3.0) / ((x + 1.0) * sqrt(x + 1.0 / 6.0)) * 0.0506605918211688857);
-        il2[h] = h > 0 ? (float)(1.0 / (x * x)) : 0.f;
+        g[h] = df(sqrt(x + 1.0 / 6.0) / (x + 1.0 / 3.0));
+        gl[h] = df((x + 1.0 / 3.0) / ((x + 1.0) * sqrt(x + 1.0 / 6.0)) * 0.0506605918211688857);
+        il2[h] = df(h > 0 ? 1.0 / (x * x) : 0.0);
     }
-    if (h <= lmax) v[h] = (h < 2) ? 0.f : (float)(pow(2.0 * h + 1.0, 5.0 / 6.0) / sqrt(cl[h]));
+    if (h <= lmax) v[h] = df((h < 2) ? 0.0 : cbrt(2.0 * h + 1.0) * sqrt(2.0 * h + 1.0) / sqrt(cl[h]));
+}
+
+// Product of double-floats, about 2^-46.
+__device__ __forceinline__ float2 df_mul(float2 a, float2 b)
+{
+    const float p = a.x * b.x;
+    return make_float2(p, fmaf(a.x, b.y, fmaf(a.y, b.x, fmaf(a.x, b.x, -p))));
 }
 
 // Point weights W(i,j,k) = permsix h~^2 prod (2l+1)^{-1/3} w_l of every row block, laid out
 // [m / 4][128 rows][4], zero outside the rows.  grid (slabs, 2 parities x blocks); 128 threads.
-// Bound by its writes (1.7 GB at l <= 2000, 0.35 ms); the factors are table look-ups instead of
-// three divisions and a square root per point, and are rounded once from FP64.
+// Bound by its writes (1.7 GB at l <= 2000); the factors are table look-ups instead of three
+// divisions and a square root per point, multiplied as double-floats and rounded once.
 __global__ void __launch_bounds__(PF_ROWS) k_pf_weights(int lmin, int lmax, int nbmax, const long long *__restrict__ base,
-                                                        const float *__restrict__ g, const float *__restrict__ gl,
-                                                        const float *__restrict__ v, float4 *__restrict__ W)
+                                                        const float2 *__restrict__ g, const float2 *__restrict__ gl,
+                                                        const float2 *__restrict__ v, float4 *__restrict__ W)
 {
     const int j = lmin + blockIdx.x, p = blockIdx.y / nbmax, b = blockIdx.y - p * nbmax;
     const PfClass c = pf_class(lmin, lmax, j, p);
@@ -149,7 +163,7 @@ __global__ void __launch_bounds__(PF_ROWS) k_pf_weights(int lmin, int lmax, int 
     const bool valid = r < c.nr;
     const int i = c.i0 + 2 * (valid ? r : c.nr - 1);
     const int ml = valid ? pf_mlast(c, j, r) : -1;
-    const float vij = v[i] * v[j];
+    const float2 vij = df_mul(v[i], v[j]);
     float4 *o = W + off * (PF_ROWS / 4) + threadIdx.x;
     for (int m4 = 0; m4 < nm; m4 += 4) {
         float w[4];
@@ -160,8 +174,10 @@ __global__ void __launch_bounds__(PF_ROWS) k_pf_weights(int lmin, int lmax, int 
             if (m >= c.m0 && m <= ml) {
                 const int k = 2 * m + c.kp;
                 const float perm = (i == j && j == k) ? 1.f : ((i == j || j == k) ? 3.f : 6.f);
-                w[x] = (perm * gl[(i + j + k) >> 1] * g[(j + k - i) >> 1]) * (g[(k + i - j) >> 1] * g[(i + j - k) >> 1]) *
-                       (vij * v[k]);
+                const float2 f = df_mul(df_mul(df_mul(gl[(i + j + k) >> 1], g[(j + k - i) >> 1]),
+                                               df_mul(g[(k + i - j) >> 1], g[(i + j - k) >> 1])),
+                                        df_mul(vij, df_mul(v[k], make_float2(perm, 0.f))));
+                w[x] = f.x + f.y;
             }
         }
         o[(size_t)(m4 / 4) * PF_ROWS] = make_float4(w[0], w[1], w[2], w[3]);
@@ -212,8 +228,10 @@ __global__ void k_pf_shapes(int S, const DShape *__restrict__ in, PfShape *__res
         f.bump[2 * a] = make_float2(bh, bh);
         f.bump[2 * a + 1] = make_float2(bl, bl);
     }
-    const float ce = (float)(-1.4426950408889634074 / (2.0 * d.sigma * d.sigma));
-    f.bump[6] = f.bump[7] = make_float2(ce, ce);
+    const double ce = -1.4426950408889634074 / (2.0 * d.sigma * d.sigma);
+    const float ceh = (float)ce, cel = (float)(ce - (double)ceh);
+    f.bump[6] = make_float2(ceh, ceh);
+    f.bump[7] = make_float2(cel, cel);
     out[s] = f;
 }
 
@@ -371,7 +389,7 @@ struct PfArgs {
     const long long *base;     // [L] weight-table offset of each slab (units of 128 floats)
     const PfShape *shapes;
     const float *tabf;
-    const float *il2;
+    const float2 *il2;
     const float4 *W;
     const __nv_bfloat16 *Bt;
     const float *qt;
@@ -535,7 +553,7 @@ __device__ __forceinline__ bool pf_pass(const PfArgs &a, const PfShape &sh, int 
         if (ms + 8 * (g4 >> 1) <= rw.mlw) w[g4] = ld_w(Wrow + (size_t)g4 * PF_ROWS);
     // row coefficients, as packed pairs: with f, g, h of each term at k, or (hi, lo) of the components
     f2 co[3 * PF_TC];
-    const float *i2 = a.il2 + ((rw.i + j + c.kp) >> 1);
+    const float2 *i2 = a.il2 + ((rw.i + j + c.kp) >> 1);
     if (nt > 0) {
         const float *tab = a.tabf + sh.tab_off + (size_t)3 * t0 * 16 * a.M8;
         const float *ti = tab + (((size_t)(rw.i & 1) * a.M8 + (rw.i >> 4)) * nt * 3) * 8 + ((rw.i >> 1) & 7);
@@ -605,7 +623,7 @@ __device__ __forceinline__ bool pf_pass(const PfArgs &a, const PfShape &sh, int 
                     } else {
                         const float k0 = (float)(2 * mg + c.kp);
                         const f2 kb = pk(k0, k0 + 2.f);
-                        float il[8];
+                        float2 il[8];
 #pragma unroll
                         for (int y = 0; y < 8; y++) il[y] = __ldg(i2 + mg + y);
 #pragma unroll
@@ -618,11 +636,14 @@ __device__ __forceinline__ bool pf_pass(const PfArgs &a, const PfShape &sh, int 
                                 v[y] = x == 0 ? mul2(d, d) : fma2(d, d, v[y]);
                             }
                         }
-                        const f2 ce = T0[3].x;
+                        const ulonglong2 ce = T0[3];
 #pragma unroll
                         for (int y = 0; y < 4; y++) {
+                            // r^2 / L^2 and the exponent, both constants with their tails
+                            const float2 ia = il[2 * y], ib = il[2 * y + 1];
+                            const f2 t = fma2(v[y], pk(ia.x, ib.x), mul2(v[y], pk(ia.y, ib.y)));
                             float e0, e1;
-                            upk(mul2(mul2(v[y], pk(il[2 * y], il[2 * y + 1])), ce), e0, e1);
+                            upk(fma2(t, ce.x, mul2(t, ce.y)), e0, e1);
                             v[y] = pk(ex2(e0), ex2(e1));
                         }
                     }
@@ -1008,8 +1029,8 @@ modal_status pf_plan(modal_ctx *ctx, ProjPlan &pl)
     const int nh = 3 * (lmax + 8) / 2 + 16;
     size_t o = 0;
     pl.o_q = o; o += al(sizeof(float) * ((size_t)L + 2 * (size_t)pl.QR) * pl.NC);
-    pl.o_v = o; o += al(sizeof(float) * (lmax + 1));
-    pl.o_g = o; o += al(sizeof(float) * 3 * (size_t)nh);
+    pl.o_v = o; o += al(sizeof(float2) * (lmax + 1));
+    pl.o_g = o; o += al(sizeof(float2) * 3 * (size_t)nh);
     pl.o_t = o; o += al(sizeof(float) * (size_t)std::max(4L, pl.tabf_total));
     pl.o_s = o; o += al(sizeof(PfShape) * (size_t)S);
     pl.o_F = o; o += al(sizeof(float) * (size_t)S * L * PP);
@@ -1035,9 +1056,9 @@ modal_status pf_record(modal_ctx *ctx, const ProjPlan &pl)
     uint8_t *b = ctx->scratch.as<uint8_t>();
     float *qp = reinterpret_cast<float *>(b + pl.o_q);
     float *qt = qp + (size_t)L * NC;
-    float *v = reinterpret_cast<float *>(b + pl.o_v);
+    float2 *v = reinterpret_cast<float2 *>(b + pl.o_v);
     const int nh = 3 * (lmax + 8) / 2 + 16;
-    float *g = reinterpret_cast<float *>(b + pl.o_g), *gl = g + nh, *il2 = gl + nh;
+    float2 *g = reinterpret_cast<float2 *>(b + pl.o_g), *gl = g + nh, *il2 = gl + nh;
     float *tabf = reinterpret_cast<float *>(b + pl.o_t), *Fbuf = reinterpret_cast<float *>(b + pl.o_F);
     PfShape *fs = reinterpret_cast<PfShape *>(b + pl.o_s);
     double *B = reinterpret_cast<double *>(b + pl.o_B);
