@@ -585,10 +585,10 @@ __global__ void __launch_bounds__(256) k_panel_post(int n, int j0, int nbp, int 
 // broadcasts it and adds its multiple of G's row u to the columns after it, the next
 // row of G in flight meanwhile.  The sums run over u in the order of the recurrence
 // as written.  Several rows per warp amortise the loads of G and fill the latency of
-// the chain; a CTA's warps take rows NBB / LARFT_WARPS apart, which evens out the
-// triangle.  Bound by the FP64 pipe (about NBB^3 / 6 multiply-adds per block over 16
-// CTAs).  Measured at n = 816 (4 blocks): 0.22 ms; one CTA per block taking the columns
-// in turn, each entry one thread's serial sum, took 3.65 ms.
+// the chain.  Bound by the FP64 pipe of the warps with the longest rows (about
+// NBB^3 / 6 multiply-adds per block over 64 warps).  Measured at n = 816 (4 blocks):
+// 0.22 ms with one warp per CTA or four; one CTA per block taking the columns in turn,
+// each entry one thread's serial sum, took 3.65 ms.
 constexpr int LARFT_ROWS = 4, LARFT_WARPS = 1;
 __global__ void __launch_bounds__(32 * LARFT_WARPS) k_larft(int nv, const double *__restrict__ G, long ldg,
                                                             const double *__restrict__ tau, double *__restrict__ T)
