@@ -580,32 +580,29 @@ __global__ void __launch_bounds__(256) k_panel_post(int n, int j0, int nbp, int 
 // Compact-WY factor of a block of reflectors (LAPACK dlarft, forward, columnwise):
 // T[t][c] = -tau_c sum_{u=t}^{c-1} T[t][u] G[u][c],  T[c][c] = tau_c, with G = V^T V
 // the block's Gram matrix (T: NBB x NBB per block).  Row t needs no other row, so
-// every row is a forward substitution of its own: a warp carries LARFT_ROWS rows,
-// the lanes hold the NBB columns (lane + 32 k), and step u finishes column u,
-// broadcasts it and adds its multiple of G's row u to the columns after it, the next
-// row of G in flight meanwhile.  The sums run over u in the order of the recurrence
-// as written.  Several rows per warp amortise the loads of G and fill the latency of
-// the chain.  Bound by the FP64 pipe of the warps with the longest rows (about
-// NBB^3 / 6 multiply-adds per block over 64 warps).  Measured at n = 816 (4 blocks):
-// 0.22 ms with one warp per CTA or four; one CTA per block taking the columns in turn,
-// each entry one thread's serial sum, took 3.65 ms.
-constexpr int LARFT_ROWS = 4, LARFT_WARPS = 1;
-__global__ void __launch_bounds__(32 * LARFT_WARPS) k_larft(int nv, const double *__restrict__ G, long ldg,
-                                                            const double *__restrict__ tau, double *__restrict__ T)
+// every row is a forward substitution of its own: a warp carries one, the lanes hold
+// the NBB columns (lane + 32 k), and step u finishes column u, broadcasts it and adds
+// its multiple of G's row u to the columns after it, the next row of G in flight
+// meanwhile.  The sums run over u in the order of the recurrence as written.  Bound by
+// the FP64 instructions of the warps with the longest rows (64 cycles each on a quarter
+// of an SM), so rows do not share a warp although they would share G's loads.  Measured
+// with one | four rows per warp: n = 816 0.07 | 0.22 ms, n = 2,000 0.09 | 0.22, n = 4,960
+// 0.20 | 0.26; one CTA per block taking the columns in turn, each entry one thread's serial
+// sum, took 3.65 ms at n = 816.
+__global__ void __launch_bounds__(32) k_larft(int nv, const double *__restrict__ G, long ldg,
+                                              const double *__restrict__ tau, double *__restrict__ T)
 {
     constexpr int NC = NBB / 32;
     const int bb = blockIdx.y, j0 = bb * NBB, w = min(NBB, nv - j0);
-    const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5;
-    const int t0 = LARFT_ROWS * (blockIdx.x + gridDim.x * warp);  // rows t0 .. t0 + LARFT_ROWS - 1
+    const int lane = threadIdx.x, t = blockIdx.x;  // the row
     const double *Gb = G + (size_t)j0 * ldg + j0;
     double *Tb = T + (size_t)bb * NBB * NBB;
-    double acc[LARFT_ROWS][NC], g[NC], tn[NC];
+    double acc[NC], g[NC], tn[NC];
 #pragma unroll
     for (int k = 0; k < NC; k++) {
         const int c = lane + 32 * k;
         tn[k] = c < w ? tau[j0 + c] : 0.0;
-#pragma unroll
-        for (int r = 0; r < LARFT_ROWS; r++) acc[r][k] = 0.0;
+        acc[k] = 0.0;
     }
     auto load = [&](int u, double *x) {  // row u of G right of the diagonal
 #pragma unroll
@@ -614,30 +611,25 @@ __global__ void __launch_bounds__(32 * LARFT_WARPS) k_larft(int nv, const double
             x[k] = (c > u && c < w) ? Gb[(size_t)u * ldg + c] : 0.0;
         }
     };
-    load(t0, g);
+    load(t, g);
 #pragma unroll
     for (int kc = 0; kc < NC; kc++) {
-        if (32 * kc + 32 <= t0) continue;
-        for (int u = max(32 * kc, t0); u < min(32 * kc + 32, w); u++) {
+        if (32 * kc + 32 <= t) continue;
+        for (int u = max(32 * kc, t); u < min(32 * kc + 32, w); u++) {
             double gn[NC];
             load(u + 1, gn);
             const int ul = u & 31;
+            const double x = __shfl_sync(0xffffffffu, u == t ? tn[kc] : -tn[kc] * acc[kc], ul);
+            if (lane == ul) acc[kc] = x;
 #pragma unroll
-            for (int r = 0; r < LARFT_ROWS; r++) {
-                const double fin = u == t0 + r ? tn[kc] : (u > t0 + r ? -tn[kc] * acc[r][kc] : 0.0);
-                const double x = __shfl_sync(0xffffffffu, fin, ul);
-                if (lane == ul) acc[r][kc] = x;
-#pragma unroll
-                for (int k = kc; k < NC; k++) acc[r][k] = fma(x, g[k], acc[r][k]);
+            for (int k = kc; k < NC; k++) {
+                acc[k] = fma(x, g[k], acc[k]);
+                g[k] = gn[k];
             }
-#pragma unroll
-            for (int k = kc; k < NC; k++) g[k] = gn[k];
         }
     }
 #pragma unroll
-    for (int r = 0; r < LARFT_ROWS; r++)
-#pragma unroll
-        for (int k = 0; k < NC; k++) Tb[(size_t)(t0 + r) * NBB + lane + 32 * k] = acc[r][k];
+    for (int k = 0; k < NC; k++) Tb[(size_t)t * NBB + lane + 32 * k] = acc[k];
 }
 
 // The T factors of the blocks of NBW reflectors from the two NBB blocks each
@@ -1460,7 +1452,7 @@ static modal_status wy_blocks(modal_ctx *ctx, int n, SyevPtrs &p)
     o.diag_tiles = NBW / 128;
     o.check = false;
     MODAL_TRY(oz_gemm_ex(ctx, nv, nv, n, 1.0, p.VA, p.ldva, true, p.VA, p.ldva, false, 0.0, p.GB, p.ldva, o));
-    k_larft<<<dim3(NBB / (LARFT_ROWS * LARFT_WARPS), nbig), 32 * LARFT_WARPS, 0, ctx->stream>>>(nv, p.GB, p.ldva, p.tau, p.TB);
+    k_larft<<<dim3(NBB, nbig), 32, 0, ctx->stream>>>(nv, p.GB, p.ldva, p.tau, p.TB);
     MODAL_TRY(launched(ctx, "larft"));
     k_tw_assemble<<<dim3(NBW * NBW / 256, nbw), 256, 0, ctx->stream>>>(nv, p.TB, p.TW);
     MODAL_TRY(launched(ctx, "tw_assemble"));
