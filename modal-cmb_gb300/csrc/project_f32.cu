@@ -145,7 +145,9 @@ __device__ __forceinline__ float2 df_mul(float2 a, float2 b)
 // Point weights W(i,j,k) = permsix h~^2 prod (2l+1)^{-1/3} w_l of every row block, laid out
 // [m / 4][128 rows][4], zero outside the rows.  grid (slabs, 2 parities x blocks); 128 threads.
 // Bound by its writes (1.7 GB at l <= 2000); the factors are table look-ups instead of three
-// divisions and a square root per point, multiplied as double-floats and rounded once.
+// divisions and a square root per point, multiplied as double-floats and rounded once.  Every v takes its
+// geometric factor along: v ~ l^{5/6} C_l^{-1/2}, and the product of three alone leaves the FP32 range
+// (C_l = 1e-19 at l = 2000) long before the weight does.
 __global__ void __launch_bounds__(PF_ROWS) k_pf_weights(int lmin, int lmax, int nbmax, const long long *__restrict__ base,
                                                         const float2 *__restrict__ g, const float2 *__restrict__ gl,
                                                         const float2 *__restrict__ v, float4 *__restrict__ W)
@@ -163,7 +165,9 @@ __global__ void __launch_bounds__(PF_ROWS) k_pf_weights(int lmin, int lmax, int 
     const bool valid = r < c.nr;
     const int i = c.i0 + 2 * (valid ? r : c.nr - 1);
     const int ml = valid ? pf_mlast(c, j, r) : -1;
-    const float2 vij = df_mul(v[i], v[j]);
+    // v(i) with permsix, for k = j and for the others
+    const float2 vj = v[j], vi1 = df_mul(v[i], make_float2(i == j ? 1.f : 3.f, 0.f)),
+                 vi = df_mul(v[i], make_float2(i == j ? 3.f : 6.f, 0.f));
     float4 *o = W + off * (PF_ROWS / 4) + threadIdx.x;
     for (int m4 = 0; m4 < nm; m4 += 4) {
         float w[4];
@@ -173,10 +177,9 @@ __global__ void __launch_bounds__(PF_ROWS) k_pf_weights(int lmin, int lmax, int 
             w[x] = 0.f;
             if (m >= c.m0 && m <= ml) {
                 const int k = 2 * m + c.kp;
-                const float perm = (i == j && j == k) ? 1.f : ((i == j || j == k) ? 3.f : 6.f);
-                const float2 f = df_mul(df_mul(df_mul(gl[(i + j + k) >> 1], g[(j + k - i) >> 1]),
-                                               df_mul(g[(k + i - j) >> 1], g[(i + j - k) >> 1])),
-                                        df_mul(vij, df_mul(v[k], make_float2(perm, 0.f))));
+                const float2 f = df_mul(df_mul(df_mul(df_mul(gl[(i + j + k) >> 1], g[(j + k - i) >> 1]), k == j ? vi1 : vi),
+                                               df_mul(g[(k + i - j) >> 1], vj)),
+                                        df_mul(g[(i + j - k) >> 1], v[k]));
                 w[x] = f.x + f.y;
             }
         }

@@ -68,3 +68,22 @@ def test_f32_batch_replays_after_another_range(mg):
         c.set_basis(2, 150, q1)
         c.set_spectrum(cl)
         assert np.array_equal(c.project_batch(shapes, mg.PREC_SPLIT), first)
+
+
+@pytest.mark.parametrize("lmax,small", [(200, 5e-22), (2000, 5e-20)])
+def test_f32_projection_of_a_small_spectrum(mg, lmax, small):
+    """C_l + N_l in units where products of three point-weight factors (2l+1)^{5/6} / sqrt(C_l) exceed
+    the FP32 range although the weights do not: within the form's 1e-6."""
+    cl = mg.synthetic_cl(lmax)
+    cl *= small / cl[2:].min()
+    shapes = mg.separable_shapes(lmax, 3, seed=11, tmin=1, tmax=2) + mg.bump_shapes(1, seed=12)
+    for s in shapes[:3]:
+        s["tab"][:, 0] *= 1e-12  # keeps the sums over points in range
+    with mg.Context(0) as c:
+        c.set_basis(2, lmax, mg.legendre_q(2, lmax, 6))
+        c.set_modes(mg.mode_triples(6))
+        c.set_spectrum(cl)
+        b64 = c.project(shapes[:3], mg.PREC_FP64)
+        b32 = c.project(shapes[:3], mg.PREC_SPLIT)
+    for s in range(3):
+        assert rel_fro(b32[s], b64[s]) <= 1e-6, (s, rel_fro(b32[s], b64[s]))
