@@ -829,6 +829,7 @@ __global__ void __launch_bounds__(PfMem<NC>::THREADS, 1) k_project_f32(const PfA
             if (w >= a.nitems) break;
             const int slab = a.order[w / a.G], s0 = (w % a.G) * a.SG, sgv = min(a.SG, a.S - s0), j = a.lmin + slab;
             for (int e = 0; e < sgv * tpt * 16; e++) Fs[e * 128 + tid] = 0.f;
+            rows_bar_or(bar, false);  // a slab without rows (l_min = l_max odd) passes no other barrier before its sums
             long long woff = a.base[slab];
             for (int p = 0; p < 2 && !stop; p++) {
                 const PfClass c = pf_class(a.lmin, a.lmax, j, p);
@@ -893,7 +894,7 @@ __global__ void __launch_bounds__(PfMem<NC>::THREADS, 1) k_project_f32(const PfA
                 }
             }
             if (stop) break;
-            // (the last barrier above orders the other threads' sums)
+            // (the last barrier passed orders the other threads' sums)
             for (int sx = 0; sx < sgv; sx++)
                 for (int tt = 0; tt < tpt; tt++) {
                     const int ti = tid + 128 * tt;

@@ -87,3 +87,18 @@ def test_f32_projection_of_a_small_spectrum(mg, lmax, small):
         b32 = c.project(shapes[:3], mg.PREC_SPLIT)
     for s in range(3):
         assert rel_fro(b32[s], b64[s]) <= 1e-6, (s, rel_fro(b32[s], b64[s]))
+
+
+@pytest.mark.parametrize("P", [2, 16, 33])
+@pytest.mark.parametrize("l", [3, 5])
+def test_f32_projection_of_one_odd_multipole(mg, P, l):
+    """l_min = l_max odd has no points (i + j + k is odd): its beta is zero whatever the context
+    computed before."""
+    with _ctx(mg, 2, 64, P) as c:
+        c.project(mg.bump_shapes(9, seed=14), mg.PREC_SPLIT)
+        c.set_basis(l, l, np.random.default_rng(P).standard_normal((1, P)))
+        c.set_spectrum(mg.synthetic_cl(l))
+        shapes = mg.bump_shapes(9, seed=15)
+        b64 = c.project(shapes, mg.PREC_FP64)
+        b32 = c.project(shapes, mg.PREC_SPLIT)
+    assert not b64.any() and not b32.any()
