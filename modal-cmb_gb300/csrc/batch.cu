@@ -185,7 +185,14 @@ modal_status modal_project_batch(modal_ctx *c, int S, const modal_shape *shapes,
     }
     c->launches += g.kernels;
     MODAL_CUDA(cudaStreamSynchronize(c->stream));
-    MODAL_TRY(oz_check(c));  // a bounded wait of the tensor-core slab kernel that expired
+    bool tail = false;
+    MODAL_TRY(oz_check(c, &tail));  // a bounded wait of the tensor-core slab kernel that expired
+    if (prec == MODAL_PREC_SPLIT && tail) {  // (rare: outside the graph)
+        MODAL_TRY(project_dev(c, S, shapes, prec, true));
+        MODAL_CUDA(cudaMemcpyAsync(g.h_beta, c->beta.ptr, sizeof(double) * (size_t)S * c->N, cudaMemcpyDeviceToHost, c->stream));
+        MODAL_CUDA(cudaStreamSynchronize(c->stream));
+        MODAL_TRY(oz_check(c));
+    }
     std::memcpy(beta, g.h_beta, sizeof(double) * (size_t)S * c->N);
     c->have_beta = true;  // beta also stays on the device for modal_alpha
     c->beta_S = S;

@@ -185,7 +185,8 @@ modal_status mij_table_dev(modal_ctx *ctx, const double *q, int lmin, int lmax, 
 modal_status gamma_fp64_dev(modal_ctx *ctx, int mu0, int nmu);
 modal_status gamma_split_dev(modal_ctx *ctx, int mu0, int nmu);
 modal_status ortho_dev(modal_ctx *ctx, int pca_flag);
-modal_status project_dev(modal_ctx *ctx, int S, const modal_shape *shapes, modal_prec prec);
+// tail: the masked form, for a batch that oz_check reports to need it.
+modal_status project_dev(modal_ctx *ctx, int S, const modal_shape *shapes, modal_prec prec, bool tail = false);
 modal_status alpha_dev(modal_ctx *ctx, int S);
 modal_status lambdainv_dev(modal_ctx *ctx);  // linv = lower triangle of orthol
 modal_status transpose_dev(modal_ctx *ctx, const double *in, double *out, int R, int C);
@@ -227,14 +228,15 @@ struct ProjPlan {
     // FP32 form (project_f32.cu): shapes per work item, operand columns, groups of 8 lattice points
     // per parity of the B operand, segments of the slab reduction, buffer offsets
     int SG = 4, NC = 32, M8 = 0, QR = 0, nseg = 1, nsm = 0, teams = 1;
-    size_t team_smem = 0, o_q = 0, o_v = 0, o_g = 0, o_t = 0, o_s = 0, o_F = 0, o_bq = 0;
+    size_t team_smem = 0, o_q = 0, o_v = 0, o_g = 0, o_t = 0, o_s = 0, o_F = 0, o_bq = 0, o_m = 0;
+    bool tail = false;    // mask the points past the rows' ends
     long tabf_total = 0;  // floats of the FP32 separable tables
     RadialArgs ra;        // radial shapes (3D transfer Gamma only)
 };
 // plan: validate, size every buffer, upload the slab schedule (may allocate);
 // stage: copy shape tables/descriptors to the device; record: enqueue the
 // device work only (no allocation, no host round trip: capturable).
-modal_status proj_plan(modal_ctx *ctx, int S, const modal_shape *shapes, modal_prec prec, ProjPlan &pl);
+modal_status proj_plan(modal_ctx *ctx, int S, const modal_shape *shapes, modal_prec prec, ProjPlan &pl, bool tail = false);
 modal_status proj_stage(modal_ctx *ctx, const ProjPlan &pl, const modal_shape *shapes);
 modal_status proj_record(modal_ctx *ctx, const ProjPlan &pl);
 // The same two steps of the single-precision form (project_f32.cu).
@@ -277,7 +279,9 @@ modal_status oz_slice(modal_ctx *ctx, int R, int K, const double *X, long ld, bo
 modal_status oz_run(modal_ctx *ctx, const OzOperand &A, const OzOperand &B, int Kpad, int s,
                     const std::vector<int2> *tile_list, double alpha, double beta, double *C, long ldc, const OzOpts &o);
 modal_status oz_reset(modal_ctx *ctx);  // clear the sticky error word of unchecked calls
-modal_status oz_check(modal_ctx *ctx);  // synchronise; MODAL_ERR_TIMEOUT if any call's wait expired
+// Synchronise; MODAL_ERR_TIMEOUT if any call's wait expired.  tail: whether the FP32 projection before had
+// shapes that may leave the FP32 range past the ends of its rows, and is to be run again with those masked.
+modal_status oz_check(modal_ctx *ctx, bool *tail = nullptr);
 modal_status oz_gemm_ex(modal_ctx *ctx, int M, int N, int K, double alpha, const double *A, long lda, bool transA,
                         const double *B, long ldb, bool transB, double beta, double *C, long ldc, const OzOpts &o);
 // C (+)= A op(B) for A [S][K] with few rows S: skinny kernels for S <= 32 (alpha 1; accumulate: C +=)

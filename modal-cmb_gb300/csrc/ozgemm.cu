@@ -689,12 +689,14 @@ modal_status oz_reset(modal_ctx *ctx)
     return MODAL_OK;
 }
 
-modal_status oz_check(modal_ctx *ctx)
+modal_status oz_check(modal_ctx *ctx, bool *tail)
 {
     if (!ctx->ozerr.ptr) return MODAL_OK;
-    int herr = 0;
-    MODAL_CUDA(cudaMemcpyAsync(&herr, ctx->ozerr.ptr, sizeof(int), cudaMemcpyDeviceToHost, ctx->stream));
+    int h[2] = {0, 0};
+    MODAL_CUDA(cudaMemcpyAsync(h, ctx->ozerr.ptr, sizeof h, cudaMemcpyDeviceToHost, ctx->stream));
     MODAL_CUDA(cudaStreamSynchronize(ctx->stream));
+    const int herr = h[0];
+    if (tail) *tail = h[1] != 0;
     if (herr) { set_error("a bounded wait in a tensor-core kernel expired (role %d: 1-4 Ozaki GEMM, 21-22 slab projection)", herr); return MODAL_ERR_TIMEOUT; }
     return MODAL_OK;
 }

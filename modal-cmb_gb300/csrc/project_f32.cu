@@ -118,10 +118,14 @@ __host__ __device__ inline long long pf_slab_len(int lmin, int lmax, int j)
 // (calculate_geometric.c:59-92 regrouped), v(l) = (2l+1)^{2/3} w_l (calculate_mode_3D.c:53-62).
 // g[h] = g(2h), gl[h] = gL(2h), il2[h] = 1/(2h)^2 (bumps), as double-floats: a factor's rounding is
 // shared by every point that uses it, and a sum that cancels does not average it away.
+// Clears the nmax maxima of k_pf_tab and the flag of k_pf_shapes.
 __global__ void k_pf_tables(int lmax, int nh, const double *__restrict__ cl, float2 *__restrict__ g, float2 *__restrict__ gl,
-                            float2 *__restrict__ il2, float2 *__restrict__ v)
+                            float2 *__restrict__ il2, float2 *__restrict__ v, int nmax, unsigned *__restrict__ fmax,
+                            int *__restrict__ tail)
 {
     const int h = blockIdx.x * blockDim.x + threadIdx.x;
+    for (int e = h; e < nmax; e += gridDim.x * blockDim.x) fmax[e] = 0u;
+    if (h == 0) *tail = 0;
     auto df = [](double x) {
         const float hi = (float)x;
         return make_float2(hi, (float)(x - (double)hi));
@@ -213,11 +217,21 @@ __global__ void k_pf_basis(int lmin, int lmax, int P, int NC, int M8, int QR, co
     }
 }
 
-__global__ void k_pf_shapes(int S, const DShape *__restrict__ in, PfShape *__restrict__ out)
+// *tail is raised where a separable shape may leave the FP32 range at some (l1, l2, l3): its value is at
+// most the sum over the terms of max|f| max|g| max|h| (k_pf_tab's maxima).
+__global__ void k_pf_shapes(int S, int lmax, const DShape *__restrict__ in, const unsigned *__restrict__ fmax,
+                            PfShape *__restrict__ out, int *__restrict__ tail)
 {
     const int s = blockIdx.x * blockDim.x + threadIdx.x;
     if (s >= S) return;
     const DShape d = in[s];
+    if (d.kind == MODAL_SHAPE_SEPARABLE) {
+        const unsigned *m = fmax + d.tab_off / (lmax + 1);
+        double bound = 0.0;
+        for (int t = 0; t < 3 * d.nterms; t += 3)
+            bound += (double)__uint_as_float(m[t]) * (double)__uint_as_float(m[t + 1]) * (double)__uint_as_float(m[t + 2]);
+        if (!(bound <= 1e37)) *tail = 1;
+    }
     PfShape f;
     f.kind = d.kind;
     f.nterms = d.nterms;
@@ -241,21 +255,28 @@ __global__ void k_pf_shapes(int S, const DShape *__restrict__ in, PfShape *__res
 // FP32 tables of the separable shapes, re-laid from the FP64 [term][f, g, h][l] tables in groups of
 // up to four terms (one pass each): group t0 at float offset 3 t0 * 2 * 8 H8, then
 // [parity of l][l / 16][term of the group][f, g, h][8]: a chunk of 32 lattice points is contiguous
-// and four consecutive points of one factor are one 16-byte load.  grid (ceil(16 H8 / 256), S).
-__global__ void k_pf_tab(int lmax, int H8, const DShape *__restrict__ shapes, const double *__restrict__ tab64,
-                         float *__restrict__ tabf)
+// and four consecutive points of one factor are one 16-byte load.  fmax[term][f, g, h]: the bits of the
+// largest |factor| at l_min .. l_max (infinities and NaN above every number).  grid (ceil(16 H8 / 256), S).
+__global__ void k_pf_tab(int lmin, int lmax, int H8, const DShape *__restrict__ shapes, const double *__restrict__ tab64,
+                         float *__restrict__ tabf, unsigned *__restrict__ fmax)
 {
     const DShape d = shapes[blockIdx.y];
     if (d.kind != MODAL_SHAPE_SEPARABLE) return;
     const int l = blockIdx.x * blockDim.x + threadIdx.x;
     if (l >= 16 * H8) return;
     const int stride = lmax + 1, m = l >> 1;
+    unsigned *mx = fmax + d.tab_off / stride;
     for (int t = 0; t < d.nterms; t++) {
         const int t0 = t & ~(PF_TC - 1), ng = min(PF_TC, d.nterms - t0);
         float *o = tabf + d.tab_off_f + (size_t)3 * t0 * 16 * H8 +
                    ((((size_t)(l & 1) * H8 + (m >> 3)) * ng + (t - t0)) * 3) * 8 + (m & 7);
         const double *f = tab64 + d.tab_off + (long)t * 3 * stride;
-        for (int x = 0; x < 3; x++) o[8 * x] = l <= lmax ? (float)f[x * stride + l] : 0.f;
+        for (int x = 0; x < 3; x++) {
+            const float v = l <= lmax ? (float)f[x * stride + l] : 0.f;
+            o[8 * x] = v;
+            const unsigned b = __reduce_max_sync(0xffffffffu, l >= lmin ? __float_as_uint(v) & 0x7fffffffu : 0u);
+            if ((threadIdx.x & 31) == 0) atomicMax(mx + 3 * t + x, b);
+        }
     }
 }
 
@@ -508,6 +529,7 @@ struct PfSync {
     int first[2];             // row threads -> issuing thread, per chunk parity: PF_PASS, PF_BLOCK, PF_END
     int qrow;                 // first basis row of the new row block
 };
+static_assert(PfMem<16>::THREADS == PfMem<32>::THREADS && PfMem<48>::THREADS == PfMem<64>::THREADS, "launch shape");
 enum { PF_PASS = 1, PF_BLOCK = 2, PF_END = 4 };  // the chunk opens a pass, a row block; no more chunks
 
 // Position in the team's chunk sequence.
@@ -540,7 +562,8 @@ __device__ __forceinline__ void pf_drain(uint32_t t, f2 (&H)[NC / 2])
 }
 
 // One pass of a row block: a bump (nt = 0), or nt = 1..4 terms of a separable shape from term t0 on.
-template <int NC>
+// TAIL: the points past a row's end are masked.
+template <int NC, bool TAIL>
 __device__ __forceinline__ bool pf_pass(const PfArgs &a, const PfShape &sh, int t0, int nt, int j, const PfClass &c,
                                         const PfRow &rw, int nch, bool block, const float4 *__restrict__ Wrow, const uint8_t *sm, PfSync *sy,
                                         uint32_t tA, uint32_t tD1, PfPos &pos, f2 (&H)[NC / 2])
@@ -549,6 +572,7 @@ __device__ __forceinline__ bool pf_pass(const PfArgs &a, const PfShape &sh, int 
     const uint32_t ready = smem_u32(sy->ready), done = smem_u32(sy->done), full = smem_u32(sy->full);
     volatile int *abort_flag = &sy->abort_flag;
     const int lane = threadIdx.x & 31, ms = pf_mstart(c);
+    const int ml = TAIL ? pf_mlast(c, j, min(PF_ROWS * rw.b + (int)(threadIdx.x & 127), c.nr - 1)) : 0;
     // the first half's weights
     float4 w[4];
 #pragma unroll
@@ -659,12 +683,20 @@ __device__ __forceinline__ bool pf_pass(const PfArgs &a, const PfShape &sh, int 
                     }
                     if (mg < c.m0) {
                         // before the rows start (below lmin the caller's tables may hold anything); past a
-                        // row's end the weight is zero and the shape finite wherever it is elsewhere
+                        // row's end the weight is zero and, unless TAIL, the shape finite
 #pragma unroll
                         for (int y = 0; y < 4; y++) {
                             float v0, v1;
                             upk(v[y], v0, v1);
                             v[y] = pk(mg + 2 * y >= c.m0 ? v0 : 0.f, mg + 2 * y + 1 >= c.m0 ? v1 : 0.f);
+                        }
+                    }
+                    if (TAIL) {
+#pragma unroll
+                        for (int y = 0; y < 4; y++) {
+                            float v0, v1;
+                            upk(v[y], v0, v1);
+                            v[y] = pk(mg + 2 * y <= ml ? v0 : 0.f, mg + 2 * y + 1 <= ml ? v1 : 0.f);
                         }
                     }
                     // v = f1 + f2 + f3 exactly, 8 significant bits each (truncating splits)
@@ -707,7 +739,7 @@ __device__ __forceinline__ bool pf_pass(const PfArgs &a, const PfShape &sh, int 
     return true;
 }
 
-template <int NC>
+template <int NC, bool TAIL>
 __global__ void __launch_bounds__(PfMem<NC>::THREADS, 1) k_project_f32(const PfArgs a)
 {
     using M = PfMem<NC>;
@@ -849,7 +881,7 @@ __global__ void __launch_bounds__(PfMem<NC>::THREADS, 1) k_project_f32(const PfA
                         bool ok = true;
                         const int nterms = sh.kind == MODAL_SHAPE_SEPARABLE ? sh.nterms : 0;
                         for (int t0 = 0; ok && (t0 == 0 || t0 < nterms); t0 += PF_TC)
-                            ok = pf_pass<NC>(a, sh, t0, min(PF_TC, nterms - t0), j, c, rw, nch, sx == 0 && t0 == 0, Wrow, pf_sm, sy, tA, tD1, pos, H);
+                            ok = pf_pass<NC, TAIL>(a, sh, t0, min(PF_TC, nterms - t0), j, c, rw, nch, sx == 0 && t0 == 0, Wrow, pf_sm, sy, tA, tD1, pos, H);
                         if (ok && sx == 0) ok = pf_wait(smem_u32(&sy->qfull), nq & 1, &sy->abort_flag);
                         if (!ok) { sy->abort_flag = 1; atomicCAS(a.err, 0, 23); }
                         // fold: F[a][c] += sum over the block's rows of q_a(i) H[i][c]
@@ -982,6 +1014,16 @@ __global__ void k_pf_beta(int N, int P, int S, int nseg, const int *__restrict__
 
 }  // namespace
 
+// use(the slab kernel of the plan)
+template <class F>
+static modal_status pf_kernel(const ProjPlan &pl, F use)
+{
+    if (pl.tail) return pl.NC == 16 ? use(k_project_f32<16, true>) : pl.NC == 32 ? use(k_project_f32<32, true>)
+                      : pl.NC == 48 ? use(k_project_f32<48, true>) : use(k_project_f32<64, true>);
+    return pl.NC == 16 ? use(k_project_f32<16, false>) : pl.NC == 32 ? use(k_project_f32<32, false>)
+         : pl.NC == 48 ? use(k_project_f32<48, false>) : use(k_project_f32<64, false>);
+}
+
 // Sizes the single-precision projection (buffers, slab schedule, launch shape).
 modal_status pf_plan(modal_ctx *ctx, ProjPlan &pl)
 {
@@ -1036,6 +1078,7 @@ modal_status pf_plan(modal_ctx *ctx, ProjPlan &pl)
     pl.o_v = o; o += al(sizeof(float2) * (lmax + 1));
     pl.o_g = o; o += al(sizeof(float2) * 3 * (size_t)nh);
     pl.o_t = o; o += al(sizeof(float) * (size_t)std::max(4L, pl.tabf_total));
+    pl.o_m = o; o += al(sizeof(unsigned) * (size_t)(pl.tab_total / (lmax + 1)));
     pl.o_s = o; o += al(sizeof(PfShape) * (size_t)S);
     pl.o_F = o; o += al(sizeof(float) * (size_t)S * L * PP);
     pl.o_B = o; o += al(sizeof(double) * (size_t)pl.nseg * S * P * PP);
@@ -1046,10 +1089,7 @@ modal_status pf_plan(modal_ctx *ctx, ProjPlan &pl)
         MODAL_CUDA(cudaFuncSetAttribute(kern, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)pl.smem));
         return MODAL_OK;
     };
-    if (pl.NC == 16) MODAL_TRY(attr(k_project_f32<16>));
-    else if (pl.NC == 32) MODAL_TRY(attr(k_project_f32<32>));
-    else if (pl.NC == 48) MODAL_TRY(attr(k_project_f32<48>));
-    else MODAL_TRY(attr(k_project_f32<64>));
+    MODAL_TRY(pf_kernel(pl, attr));
     return oz_reset(ctx);
 }
 
@@ -1068,8 +1108,11 @@ modal_status pf_record(modal_ctx *ctx, const ProjPlan &pl)
     double *B = reinterpret_cast<double *>(b + pl.o_B);
     __nv_bfloat16 *Bt = reinterpret_cast<__nv_bfloat16 *>(b + pl.o_bq);
     float4 *W = reinterpret_cast<float4 *>(b + pl.o_w);
+    unsigned *fmax = reinterpret_cast<unsigned *>(b + pl.o_m);
+    int *tail = ctx->ozerr.as<int>() + 1;
     const long long *base = ctx->pf_sched.as<long long>();
-    k_pf_tables<<<ceil_div(nh, 128), 128, 0, ctx->stream>>>(lmax, nh, ctx->cl.as<double>(), g, gl, il2, v);
+    k_pf_tables<<<ceil_div(nh, 128), 128, 0, ctx->stream>>>(lmax, nh, ctx->cl.as<double>(), g, gl, il2, v,
+                                                               (int)(pl.tab_total / (lmax + 1)), fmax, tail);
     MODAL_TRY(launched(ctx, "pf_tables"));
     const int nbmax = ceil_div((lmax - lmin) / 2 + 1, PF_ROWS);
     k_pf_weights<<<dim3(L, 2 * nbmax), PF_ROWS, 0, ctx->stream>>>(lmin, lmax, nbmax, base, g, gl, v, W);
@@ -1079,10 +1122,10 @@ modal_status pf_record(modal_ctx *ctx, const ProjPlan &pl)
     MODAL_TRY(launched(ctx, "pf_basis"));
     if (pl.tabf_total > 0) {
         k_pf_tab<<<dim3(ceil_div(16L * pl.M8, 256), S), 256, 0, ctx->stream>>>(
-            lmax, pl.M8, ctx->shape_desc.as<DShape>(), ctx->shape_tab.as<double>(), tabf);
+            lmin, lmax, pl.M8, ctx->shape_desc.as<DShape>(), ctx->shape_tab.as<double>(), tabf, fmax);
         MODAL_TRY(launched(ctx, "pf_tab"));
     }
-    k_pf_shapes<<<ceil_div(S, 64), 64, 0, ctx->stream>>>(S, ctx->shape_desc.as<DShape>(), fs);
+    k_pf_shapes<<<ceil_div(S, 64), 64, 0, ctx->stream>>>(S, lmax, ctx->shape_desc.as<DShape>(), fmax, fs, tail);
     MODAL_TRY(launched(ctx, "pf_shapes"));
     PfArgs a;
     a.lmin = lmin; a.lmax = lmax; a.P = P; a.S = S; a.SG = pl.SG; a.G = ceil_div(S, pl.SG);
@@ -1096,11 +1139,11 @@ modal_status pf_record(modal_ctx *ctx, const ProjPlan &pl)
     a.teams = pl.teams;
     a.team_smem = (uint32_t)pl.team_smem;
     const int grid = std::min(ceil_div(a.nitems, pl.teams), pl.nsm);
-    if (NC == 16) k_project_f32<16><<<grid, PfMem<16>::THREADS, pl.smem, ctx->stream>>>(a);
-    else if (NC == 32) k_project_f32<32><<<grid, PfMem<32>::THREADS, pl.smem, ctx->stream>>>(a);
-    else if (NC == 48) k_project_f32<48><<<grid, PfMem<48>::THREADS, pl.smem, ctx->stream>>>(a);
-    else k_project_f32<64><<<grid, PfMem<64>::THREADS, pl.smem, ctx->stream>>>(a);
-    MODAL_TRY(launched(ctx, "project_f32"));
+    const int threads = NC <= 32 ? PfMem<32>::THREADS : PfMem<64>::THREADS;
+    MODAL_TRY(pf_kernel(pl, [&](auto kern) {
+        kern<<<grid, threads, pl.smem, ctx->stream>>>(a);
+        return launched(ctx, "project_f32");
+    }));
     k_pf_B<<<dim3(ceil_div(PP, 128), S, pl.nseg * ceil_div(P, PB)), 128, 0, ctx->stream>>>(L, P, S, NC, pl.nseg, qp, Fbuf, B);
     MODAL_TRY(launched(ctx, "pf_B"));
     k_pf_beta<<<ceil_div((long)S * N, 256), 256, 0, ctx->stream>>>(N, P, S, pl.nseg, ctx->triples.as<int>(), B,

@@ -102,3 +102,18 @@ def test_f32_projection_of_one_odd_multipole(mg, P, l):
         b64 = c.project(shapes, mg.PREC_FP64)
         b32 = c.project(shapes, mg.PREC_SPLIT)
     assert not b64.any() and not b32.any()
+
+
+def test_f32_projection_of_a_shape_that_overflows_outside_the_triangle(mg):
+    """f(i) g(j) h(k) = 1e45 at points with k > i + j, which no sum contains, and 0 at those that count."""
+    lmax = 60
+    shape = mg.separable_shapes(lmax, 1, seed=13, tmin=2, tmax=2)[0]
+    l = np.arange(lmax + 1)
+    shape["tab"][0] = [np.where(l <= 3, 1e15, 0.0), np.where(l <= 3, 1e15, 0.0), np.where(l >= 12, 1e15, 0.0)]
+    with _ctx(mg, 2, lmax, 5) as c:
+        b64 = c.project([shape], mg.PREC_FP64)
+        b32 = c.project([shape], mg.PREC_SPLIT)
+        tame = dict(shape, tab=shape["tab"] * [[[1e-12]], [[1.0]]])  # bounded: the same values at the points that count
+        batch = [c.project_batch([x], mg.PREC_SPLIT) for x in (tame, shape, tame)]
+    assert rel_fro(b32, b64) <= 1e-6
+    assert all(np.array_equal(b, b32) for b in batch)
