@@ -120,11 +120,11 @@ __host__ __device__ inline long long pf_slab_len(int lmin, int lmax, int j)
 // shared by every point that uses it, and a sum that cancels does not average it away.
 // Clears the nmax maxima of k_pf_tab and the flag of k_pf_shapes.
 __global__ void k_pf_tables(int lmax, int nh, const double *__restrict__ cl, float2 *__restrict__ g, float2 *__restrict__ gl,
-                            float2 *__restrict__ il2, float2 *__restrict__ v, int nmax, unsigned *__restrict__ fmax,
+                            float2 *__restrict__ il2, float2 *__restrict__ v, int nmax, unsigned *__restrict__ tmax,
                             int *__restrict__ tail)
 {
     const int h = blockIdx.x * blockDim.x + threadIdx.x;
-    for (int e = h; e < nmax; e += gridDim.x * blockDim.x) fmax[e] = 0u;
+    for (int e = h; e < nmax; e += gridDim.x * blockDim.x) tmax[e] = 0u;
     if (h == 0) *tail = 0;
     auto df = [](double x) {
         const float hi = (float)x;
@@ -219,14 +219,14 @@ __global__ void k_pf_basis(int lmin, int lmax, int P, int NC, int M8, int QR, co
 
 // *tail is raised where a separable shape may leave the FP32 range at some (l1, l2, l3): its value is at
 // most the sum over the terms of max|f| max|g| max|h| (k_pf_tab's maxima).
-__global__ void k_pf_shapes(int S, int lmax, const DShape *__restrict__ in, const unsigned *__restrict__ fmax,
+__global__ void k_pf_shapes(int S, int lmax, const DShape *__restrict__ in, const unsigned *__restrict__ tmax,
                             PfShape *__restrict__ out, int *__restrict__ tail)
 {
     const int s = blockIdx.x * blockDim.x + threadIdx.x;
     if (s >= S) return;
     const DShape d = in[s];
     if (d.kind == MODAL_SHAPE_SEPARABLE) {
-        const unsigned *m = fmax + d.tab_off / (lmax + 1);
+        const unsigned *m = tmax + d.tab_off / (lmax + 1);
         double bound = 0.0;
         for (int t = 0; t < 3 * d.nterms; t += 3)
             bound += (double)__uint_as_float(m[t]) * (double)__uint_as_float(m[t + 1]) * (double)__uint_as_float(m[t + 2]);
@@ -236,8 +236,17 @@ __global__ void k_pf_shapes(int S, int lmax, const DShape *__restrict__ in, cons
     f.kind = d.kind;
     f.nterms = d.nterms;
     f.tab_off = d.tab_off_f;
-    const double c[3] = {d.c1, d.c2, d.c3};
+    // a centre beyond 2^40 is brought down to it together with the width (l / L, at most 1, no longer counts there),
+    // so that the squares below stay in the FP32 range
+    double c[3] = {d.c1, d.c2, d.c3}, cm = 0.0;
     for (int a = 0; a < 3; a++) {
+        if (isinf(c[a])) c[a] = copysign(1e300, c[a]);
+        cm = fmax(cm, fabs(c[a]));
+    }
+    const int down = cm > 0x1p40 ? ilogb(cm) - 40 : 0;
+    const double sigma = ldexp(d.sigma, -down);
+    for (int a = 0; a < 3; a++) {
+        c[a] = ldexp(c[a], -down);
         f.ch[a] = (float)c[a];
         f.cl[a] = (float)(c[a] - (double)f.ch[a]);
         const double b = (a == 2 ? 1.0 : 0.0) - c[a];
@@ -245,8 +254,9 @@ __global__ void k_pf_shapes(int S, int lmax, const DShape *__restrict__ in, cons
         f.bump[2 * a] = make_float2(bh, bh);
         f.bump[2 * a + 1] = make_float2(bl, bl);
     }
-    const double ce = -1.4426950408889634074 / (2.0 * d.sigma * d.sigma);
-    const float ceh = (float)ce, cel = (float)(ce - (double)ceh);
+    // (a width below 1e-13 is a point: its exponent is bounded, and its tail left out before it could overflow)
+    const double ce = fmax(-1.4426950408889634074 / (2.0 * sigma * sigma), -1e25);
+    const float ceh = (float)ce, cel = ce < -1e20 ? 0.f : (float)(ce - (double)ceh);
     f.bump[6] = make_float2(ceh, ceh);
     f.bump[7] = make_float2(cel, cel);
     out[s] = f;
@@ -255,17 +265,17 @@ __global__ void k_pf_shapes(int S, int lmax, const DShape *__restrict__ in, cons
 // FP32 tables of the separable shapes, re-laid from the FP64 [term][f, g, h][l] tables in groups of
 // up to four terms (one pass each): group t0 at float offset 3 t0 * 2 * 8 H8, then
 // [parity of l][l / 16][term of the group][f, g, h][8]: a chunk of 32 lattice points is contiguous
-// and four consecutive points of one factor are one 16-byte load.  fmax[term][f, g, h]: the bits of the
+// and four consecutive points of one factor are one 16-byte load.  tmax[term][f, g, h]: the bits of the
 // largest |factor| at l_min .. l_max (infinities and NaN above every number).  grid (ceil(16 H8 / 256), S).
 __global__ void k_pf_tab(int lmin, int lmax, int H8, const DShape *__restrict__ shapes, const double *__restrict__ tab64,
-                         float *__restrict__ tabf, unsigned *__restrict__ fmax)
+                         float *__restrict__ tabf, unsigned *__restrict__ tmax)
 {
     const DShape d = shapes[blockIdx.y];
     if (d.kind != MODAL_SHAPE_SEPARABLE) return;
     const int l = blockIdx.x * blockDim.x + threadIdx.x;
     if (l >= 16 * H8) return;
     const int stride = lmax + 1, m = l >> 1;
-    unsigned *mx = fmax + d.tab_off / stride;
+    unsigned *mx = tmax + d.tab_off / stride;
     for (int t = 0; t < d.nterms; t++) {
         const int t0 = t & ~(PF_TC - 1), ng = min(PF_TC, d.nterms - t0);
         float *o = tabf + d.tab_off_f + (size_t)3 * t0 * 16 * H8 +
@@ -1108,11 +1118,11 @@ modal_status pf_record(modal_ctx *ctx, const ProjPlan &pl)
     double *B = reinterpret_cast<double *>(b + pl.o_B);
     __nv_bfloat16 *Bt = reinterpret_cast<__nv_bfloat16 *>(b + pl.o_bq);
     float4 *W = reinterpret_cast<float4 *>(b + pl.o_w);
-    unsigned *fmax = reinterpret_cast<unsigned *>(b + pl.o_m);
+    unsigned *tmax = reinterpret_cast<unsigned *>(b + pl.o_m);
     int *tail = ctx->ozerr.as<int>() + 1;
     const long long *base = ctx->pf_sched.as<long long>();
     k_pf_tables<<<ceil_div(nh, 128), 128, 0, ctx->stream>>>(lmax, nh, ctx->cl.as<double>(), g, gl, il2, v,
-                                                               (int)(pl.tab_total / (lmax + 1)), fmax, tail);
+                                                               (int)(pl.tab_total / (lmax + 1)), tmax, tail);
     MODAL_TRY(launched(ctx, "pf_tables"));
     const int nbmax = ceil_div((lmax - lmin) / 2 + 1, PF_ROWS);
     k_pf_weights<<<dim3(L, 2 * nbmax), PF_ROWS, 0, ctx->stream>>>(lmin, lmax, nbmax, base, g, gl, v, W);
@@ -1122,10 +1132,10 @@ modal_status pf_record(modal_ctx *ctx, const ProjPlan &pl)
     MODAL_TRY(launched(ctx, "pf_basis"));
     if (pl.tabf_total > 0) {
         k_pf_tab<<<dim3(ceil_div(16L * pl.M8, 256), S), 256, 0, ctx->stream>>>(
-            lmin, lmax, pl.M8, ctx->shape_desc.as<DShape>(), ctx->shape_tab.as<double>(), tabf, fmax);
+            lmin, lmax, pl.M8, ctx->shape_desc.as<DShape>(), ctx->shape_tab.as<double>(), tabf, tmax);
         MODAL_TRY(launched(ctx, "pf_tab"));
     }
-    k_pf_shapes<<<ceil_div(S, 64), 64, 0, ctx->stream>>>(S, lmax, ctx->shape_desc.as<DShape>(), fmax, fs, tail);
+    k_pf_shapes<<<ceil_div(S, 64), 64, 0, ctx->stream>>>(S, lmax, ctx->shape_desc.as<DShape>(), tmax, fs, tail);
     MODAL_TRY(launched(ctx, "pf_shapes"));
     PfArgs a;
     a.lmin = lmin; a.lmax = lmax; a.P = P; a.S = S; a.SG = pl.SG; a.G = ceil_div(S, pl.SG);

@@ -117,3 +117,15 @@ def test_f32_projection_of_a_shape_that_overflows_outside_the_triangle(mg):
         batch = [c.project_batch([x], mg.PREC_SPLIT) for x in (tame, shape, tame)]
     assert rel_fro(b32, b64) <= 1e-6
     assert all(np.array_equal(b, b32) for b in batch)
+
+
+@pytest.mark.parametrize("c,sigma", [((1e17, -2e17, 5e16), 1e17), ((3e16, 0.3, 0.7), 0.1), ((0.21, 0.3141, 0.4759), 1e-21),
+                                     ((0.2, 0.3, 0.5), 1e30), ((1e40, 0.0, 0.0), 1e40)])
+def test_f32_projection_of_extreme_bumps(mg, c, sigma):
+    """Centres and widths far from 1 are numbers like any other: a constant, or zero everywhere."""
+    shape = [{"kind": mg.SHAPE_BUMP, "c": np.array(c), "sigma": sigma}]
+    with _ctx(mg, 2, 60, 5) as ctx:
+        b64 = ctx.project(shape, mg.PREC_FP64)
+        b32 = ctx.project(shape, mg.PREC_SPLIT)
+    assert np.all(np.isfinite(b64))
+    assert np.linalg.norm(b32 - b64) <= 1e-6 * np.linalg.norm(b64)
