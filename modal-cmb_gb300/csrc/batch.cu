@@ -64,7 +64,9 @@ static bool batch_matches(const BatchGraph &g, const modal_ctx *c, int S, const 
         g.N != c->N || g.sg != c->proj_sg || g.cpb != c->proj_cpb || g.tc != c->proj_tc)
         return false;
     // the slab schedule on the device may by now be another range's
-    if (prec == MODAL_PREC_SPLIT && (c->pf_lmin != c->lmin || c->pf_lmax != c->lmax)) return false;
+    if (prec == MODAL_PREC_SPLIT ? c->pf_lmin != c->lmin || c->pf_lmax != c->lmax
+                                 : c->slab_lmin != c->lmin || c->slab_lmax != c->lmax)
+        return false;
     for (int s = 0; s < S; s++)
         if (g.kinds[s] != shapes[s].kind || (shapes[s].kind == MODAL_SHAPE_SEPARABLE && g.nterms[s] != shapes[s].nterms))
             return false;

@@ -68,7 +68,8 @@ struct modal_ctx {
     modal::DevBuf scratch2;
     modal::DevBuf shape_tab;   // separable tables
     modal::DevBuf shape_desc;  // device shape descriptors
-    modal::DevBuf slab_order;  // projection slab schedule
+    modal::DevBuf slab_order;  // FP64 projection: slab schedule of (slab_lmin, slab_lmax)
+    int slab_lmin = -1, slab_lmax = -1;
     // FP32 projection: weight-table offsets and slab order of (pf_lmin, pf_lmax); table length in 128 floats
     modal::DevBuf pf_sched;
     int pf_lmin = -1, pf_lmax = -1;

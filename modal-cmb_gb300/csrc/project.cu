@@ -443,13 +443,18 @@ modal_status proj_plan(modal_ctx *ctx, int S, const modal_shape *shapes, modal_p
     if (prec == MODAL_PREC_SPLIT) {
         MODAL_TRY(pf_plan(ctx, pl));
     } else {
-        // slab schedule: heaviest slabs first
-        std::vector<int> order(L);
-        std::vector<long long> cnt(L);
-        for (int q = 0; q < L; q++) { order[q] = q; cnt[q] = tet_row_offset(lmin + q, lmax + 1, lmax); }
-        std::stable_sort(order.begin(), order.end(), [&](int a, int b) { return cnt[a] > cnt[b]; });
-        MODAL_TRY(ensure(ctx->slab_order, sizeof(int) * (size_t)L));
-        MODAL_CUDA(cudaMemcpyAsync(ctx->slab_order.ptr, order.data(), sizeof(int) * L, cudaMemcpyHostToDevice, ctx->stream));
+        // slab schedule of (lmin, lmax): heaviest slabs first
+        if (ctx->slab_lmin != lmin || ctx->slab_lmax != lmax) {
+            std::vector<int> order(L);
+            std::vector<long long> cnt(L);
+            for (int q = 0; q < L; q++) { order[q] = q; cnt[q] = tet_row_offset(lmin + q, lmax + 1, lmax); }
+            std::stable_sort(order.begin(), order.end(), [&](int a, int b) { return cnt[a] > cnt[b]; });
+            ctx->slab_lmin = ctx->slab_lmax = -1;
+            MODAL_TRY(ensure(ctx->slab_order, sizeof(int) * (size_t)L));
+            MODAL_CUDA(cudaMemcpyAsync(ctx->slab_order.ptr, order.data(), sizeof(int) * L, cudaMemcpyHostToDevice, ctx->stream));
+            ctx->slab_lmin = lmin;
+            ctx->slab_lmax = lmax;
+        }
         const int KMAX = (lmax - lmin) / 2 + 2;
         pl.smem = sizeof(double) * ((size_t)JC * KMAX + (size_t)JC * P + (size_t)JC * PJ_TCOEF64 * 3);
         if (pl.smem > 220 * 1024) { set_error("project: lmax=%d too large for the slab tile", lmax); return MODAL_ERR_ARG; }

@@ -117,3 +117,21 @@ def test_autotune_applies_and_caches(mg, tmp_path):
             ref = before_tc if tcv else before_cc
             assert np.array_equal(c3.project(shapes, 1), ref)
             assert np.array_equal(c3.project_batch(shapes, 1), ref)
+
+
+@pytest.mark.parametrize("lmax,other", [(150, 90), (90, 150)])
+def test_fp64_batch_replays_after_another_range(mg, lmax, other):
+    """The captured batch uses the slab schedule of its own range: a projection at another l_max in
+    between makes it plan again."""
+    q1, _, cl1 = mg.workload(lmax, 6)
+    q2, _, cl2 = mg.workload(other, 6)
+    shapes = _mixed(mg, lmax, 3, 6)
+    with _ctx(mg, lmax) as c:
+        c.project(_mixed(mg, lmax, 4, 60), mg.PREC_FP64)  # buffers that hold either range
+        first = c.project_batch(shapes, mg.PREC_FP64)
+        c.set_basis(2, other, q2)
+        c.set_spectrum(cl2)
+        c.project(_mixed(mg, other, 4, 6), mg.PREC_FP64)
+        c.set_basis(2, lmax, q1)
+        c.set_spectrum(cl1)
+        assert np.array_equal(c.project_batch(shapes, mg.PREC_FP64), first)
