@@ -1050,8 +1050,8 @@ modal_status pf_plan(modal_ctx *ctx, ProjPlan &pl)
         for (int s = 0; s < L; s++) order[s] = s;
         auto len = [&](int s) { return (s + 1 < L ? base[s + 1] : total) - base[s]; };
         std::stable_sort(order.begin(), order.end(), [&](int x, int y) { return len(x) > len(y); });
-        MODAL_TRY(ensure(ctx->pf_sched, (sizeof(long long) + sizeof(int)) * (size_t)L));
         ctx->pf_lmin = ctx->pf_lmax = -1;
+        MODAL_TRY(ensure(ctx->pf_sched, (sizeof(long long) + sizeof(int)) * (size_t)L));
         MODAL_CUDA(cudaMemcpyAsync(ctx->pf_sched.ptr, base.data(), sizeof(long long) * L, cudaMemcpyHostToDevice, ctx->stream));
         MODAL_CUDA(cudaMemcpyAsync(ctx->pf_sched.as<long long>() + L, order.data(), sizeof(int) * L, cudaMemcpyHostToDevice,
                                    ctx->stream));
