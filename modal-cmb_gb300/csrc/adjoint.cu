@@ -327,8 +327,10 @@ modal_status pl_contract(modal_ctx *c, int ncol, double *D, double *Z)
     const int nmu = c->nmu, L = c->L, lmin = c->lmin;
     const double *pl = c->pl.as<double>() + (size_t)lmin * nmu;
     if (!c->gl_sym) return dgemm_splitk(c, L, ncol, nmu, pl, nmu, false, D, ncol, false, Z, ncol, 0, false);
-    k_fold_nodes<<<ceil_div((long)(nmu / 2) * ncol, 256), 256, 0, c->stream>>>(nmu, ncol, D);
-    MODAL_TRY(launched(c, "fold_nodes"));
+    if (nmu > 1) {  // (a single node has no mirror)
+        k_fold_nodes<<<ceil_div((long)(nmu / 2) * ncol, 256), 256, 0, c->stream>>>(nmu, ncol, D);
+        MODAL_TRY(launched(c, "fold_nodes"));
+    }
     for (int p = 0; p < 2; p++) {
         const int rows = (L - p + 1) / 2, even = !((lmin + p) & 1);
         // even l: the sums against the first half, the middle included; odd l: the differences against

@@ -36,3 +36,26 @@ def test_vjp_routes(mg, lmax, P, N, terms):
     assert rel_fro(beta, b_ref.detach().numpy()) <= 1e-12
     (b_ref * torch.tensor(upb)).sum().backward()
     assert rel_fro(db, qt.grad.numpy()) <= 1e-11
+
+
+@pytest.mark.parametrize("P,N", [(2, 4), (6, 1)])
+def test_vjps_of_one_node(mg, P, N):
+    """A quadrature of the single node 0, antisymmetric like a Gauss-Legendre rule; both routes of each."""
+    rng = np.random.default_rng(P)
+    q, _, cl = mg.workload(7, P)
+    tri = rng.integers(0, P, size=(N, 3)).astype(np.int32)
+    shapes = mg.separable_shapes(7, 2, 23, 1, 2)
+    mu, w = np.zeros(1), np.full(1, 2.0)
+    up, upb = rng.standard_normal((N, N)), rng.standard_normal((2, N))
+    with mg.Context(0) as c:
+        c.set_basis(2, 7, q)
+        c.set_modes(tri)
+        c.set_spectrum(cl)
+        c.set_gl(mu, w)
+        dg, db = c.gamma_vjp(up), c.project_gl_vjp(shapes, upb)
+    pr = at.Problem(mu, w, 2, 7, tri, cl, shapes)
+    for got, loss in ((dg, lambda t: (pr.gamma(t) * torch.tensor(up)).sum()),
+                      (db, lambda t: (pr.beta_norm2(t)[0] * torch.tensor(upb)).sum())):
+        qt = torch.tensor(q, requires_grad=True)
+        loss(qt).backward()
+        assert rel_fro(got, qt.grad.numpy()) <= 1e-11
