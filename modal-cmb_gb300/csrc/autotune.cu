@@ -147,7 +147,8 @@ modal_status modal_autotune(modal_ctx *c, const char *cache_path)
     const int P = c->P;
 
     // ---- FP32 projection kernel: shapes per work item, row teams per SM
-    const std::string kp = "proj2 " + arch + " lmax=" + std::to_string(c->lmax) + " P=" + std::to_string(P);
+    // ("teams": records without it count persistent CTAs per SM, and one of them would run one team of three)
+    const std::string kp = "proj2 " + arch + " teams lmax=" + std::to_string(c->lmax) + " P=" + std::to_string(P);
     int pv[3] = {0, 0, 0};
     if (cache_lookup(cache_path, kp, pv, 3)) {
         c->proj_sg = pv[0];

@@ -135,3 +135,17 @@ def test_fp64_batch_replays_after_another_range(mg, lmax, other):
         c.set_basis(2, lmax, q1)
         c.set_spectrum(cl1)
         assert np.array_equal(c.project_batch(shapes, mg.PREC_FP64), first)
+
+
+def test_autotune_does_not_take_records_of_other_launch_parameters(mg, tmp_path):
+    """A record whose second number counts persistent CTAs per SM is not one of row teams per SM."""
+    path, old = os.fspath(tmp_path / "tune.txt"), os.fspath(tmp_path / "old.txt")
+    with _ctx(mg, 120, 6) as c:
+        t = c.autotune(path)
+        lines = open(path).read().splitlines()
+        with open(old, "w") as f:
+            f.write(f"proj2 {lines[0].split()[1]} lmax=120 P=6 4 1 1\n{lines[1]}\n")
+    with _ctx(mg, 120, 6) as c:
+        c.autotune(old)
+        assert len(open(old).read().splitlines()) == 3
+        assert c.tuning()["proj_tc"] == t["proj_tc"] == 0
