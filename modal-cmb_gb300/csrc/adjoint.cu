@@ -241,7 +241,44 @@ __global__ void __launch_bounds__(256) k_gamma_vjp(int N, int P, int nmu, int lm
     for (int e = threadIdx.x; e < PP; e += blockDim.x) dM[(size_t)k * PP + e] = sD[e];
 }
 
-// Projection adjoint.  With the symmetric tensor of shape s
+// Projection adjoint of few modes, one CTA per mu node k: B(k) staged in shared memory, dB(k)
+// accumulated there, nine cofactors and nine shared-memory additions per term and mode, which bound it.
+__global__ void __launch_bounds__(256) k_beta_vjp_modes(int N, int nmu, LegInfo li, int E, const int *__restrict__ triples,
+                                                        const double *__restrict__ BK, const double *__restrict__ w,
+                                                        const double *__restrict__ Gb, double *__restrict__ dB)
+{
+    extern __shared__ double sm[];
+    const int k = blockIdx.x, P = li.P, EP = E * P;
+    double *sB = sm, *sD = sm + EP;
+    for (int e = threadIdx.x; e < EP; e += blockDim.x) { sB[e] = BK[(size_t)k * li.stride + e]; sD[e] = 0.0; }
+    __syncthreads();
+    const double wk = w[k] * kInv48Pi;
+    const long SN = (long)li.nshape * N;
+    for (long e = threadIdx.x; e < SN; e += blockDim.x) {
+        const double g = Gb[e];
+        if (g == 0.0) continue;
+        const int s = (int)(e / N), n = (int)(e - (long)s * N);
+        const int nb[3] = {triples[3 * n], triples[3 * n + 1], triples[3 * n + 2]};
+        const int e0 = li.leg0[s], T = li.nterm[s];
+        const double gw = g * wk;
+        for (int t = 0; t < T; t++) {
+            const int lg = e0 + 3 * t;
+            double a[3][3];
+#pragma unroll
+            for (int x = 0; x < 3; x++)
+#pragma unroll
+                for (int y = 0; y < 3; y++) a[x][y] = sB[(lg + x) * P + nb[y]];
+#pragma unroll
+            for (int x = 0; x < 3; x++)
+#pragma unroll
+                for (int y = 0; y < 3; y++) atomicAdd(&sD[(lg + x) * P + nb[y]], gw * cof3(a, x, y));
+        }
+    }
+    __syncthreads();
+    for (int e = threadIdx.x; e < EP; e += blockDim.x) dB[(size_t)k * EP + e] = sD[e];
+}
+
+// Projection adjoint of many modes.  With the symmetric tensor of shape s
 //   Gs[q][q'][q''] = sum_n Gb_sn sum over the six orderings of mode n of delta(q q' q'', ordering),
 // the term (s, t) contributes sum_k w_k/(48 pi) sum Gs B_0[q] B_1[q'] B_2[q''], so its three
 // gradients need two FMAs per entry of Gs and node instead of nine cofactors and nine shared-memory
@@ -590,15 +627,28 @@ modal_status beta_vjp_dev(modal_ctx *c, const AdjFwd &f, const double *Gb, doubl
     MODAL_TRY(ensure(c->adj2, sizeof(double) * ((size_t)nmu * EP + (size_t)L * EP)));
     double *dB = c->adj2.as<double>(), *Z2 = dB + (size_t)nmu * EP;
     const size_t PPP = (size_t)P * P * P, vs = sizeof(double) * 5 * (size_t)P * BV_T;
-    MODAL_TRY(ensure(c->trip, sizeof(double) * f.S * PPP));
-    double *Gs = c->trip.as<double>();
-    MODAL_CUDA(cudaMemsetAsync(Gs, 0, sizeof(double) * f.S * PPP, c->stream));
-    k_beta_tensor<<<ceil_div((long)f.S * c->N, 256), 256, 0, c->stream>>>(f.S, c->N, P, c->triples.as<int>(), Gb, Gs);
-    MODAL_TRY(launched(c, "beta_tensor"));
-    MODAL_CUDA(cudaFuncSetAttribute(k_beta_vjp, cudaFuncAttributeMaxDynamicSharedMemorySize, 5 * 64 * BV_T * 8));
-    k_beta_vjp<<<dim3(ceil_div(nmu, BV_T), E / 3), BV_T, vs, c->stream>>>(nmu, P, E, f.li.stride, f.term_shape, f.term_leg, f.BK,
-                                                                         c->w.as<double>(), Gs, dB);
-    MODAL_TRY(launched(c, "beta_vjp"));
+    // Few modes: 0.2 ns per term, mode and node (0.165 at P = 40, 0.24 at P = 12).  Many: a thread's P^3
+    // steps of 140 ns, or 48 ns per CTA and SM once there are more than three.  Measured, tensor | modes, whole
+    // call: l <= 300, P = 40, 4 shapes, 10 modes 9.8 | 1.0 ms, all 11,480 10.5 | 6.5; l <= 1000, P = 20, 8 shapes, 300
+    // modes 5.02 | 4.87, 400 modes 5.01 | 5.18; l <= 1000, P = 12, 32 shapes, 43 modes 6.98 | 6.93, all 364 7.3 | 12.5.
+    int nsm = 0;
+    MODAL_CUDA(cudaDeviceGetAttribute(&nsm, cudaDevAttrMultiProcessorCount, c->device));
+    const double terms = E / 3, ctas = terms * ceil_div(nmu, BV_T) / nsm;
+    if (0.2 * terms * c->N * nmu < (double)PPP * std::max(140.0, 48.0 * ctas)) {
+        MODAL_CUDA(cudaFuncSetAttribute(k_beta_vjp_modes, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem));
+        k_beta_vjp_modes<<<nmu, 256, smem, c->stream>>>(c->N, nmu, f.li, E, c->triples.as<int>(), f.BK, c->w.as<double>(), Gb, dB);
+        MODAL_TRY(launched(c, "beta_vjp_modes"));
+    } else {
+        MODAL_TRY(ensure(c->trip, sizeof(double) * f.S * PPP));
+        double *Gs = c->trip.as<double>();
+        MODAL_CUDA(cudaMemsetAsync(Gs, 0, sizeof(double) * f.S * PPP, c->stream));
+        k_beta_tensor<<<ceil_div((long)f.S * c->N, 256), 256, 0, c->stream>>>(f.S, c->N, P, c->triples.as<int>(), Gb, Gs);
+        MODAL_TRY(launched(c, "beta_tensor"));
+        MODAL_CUDA(cudaFuncSetAttribute(k_beta_vjp, cudaFuncAttributeMaxDynamicSharedMemorySize, 5 * 64 * BV_T * 8));
+        k_beta_vjp<<<dim3(ceil_div(nmu, BV_T), E / 3), BV_T, vs, c->stream>>>(nmu, P, E, f.li.stride, f.term_shape, f.term_leg, f.BK,
+                                                                             c->w.as<double>(), Gs, dB);
+        MODAL_TRY(launched(c, "beta_vjp"));
+    }
     MODAL_TRY(pl_contract(c, EP, dB, Z2));
     k_dq_beta<<<ceil_div((long)L * P, 256), 256, 0, c->stream>>>(L, P, E, Z2, f.vecs + (size_t)P * L, dq);
     return launched(c, "dq_beta");

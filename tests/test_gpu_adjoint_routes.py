@@ -59,3 +59,23 @@ def test_vjps_of_one_node(mg, P, N):
         qt = torch.tensor(q, requires_grad=True)
         loss(qt).backward()
         assert rel_fro(got, qt.grad.numpy()) <= 1e-11
+
+
+@pytest.mark.parametrize("lmax,P,N,S", [(40, 2, 4, 15), (40, 4, 20, 20), (40, 4, 2, 20), (87, 3, 10, 12), (170, 5, 35, 16)])
+def test_projection_vjp_of_many_and_few_modes(mg, lmax, P, N, S):
+    """Shape tensors where the modes are many for the basis (all but the third case), cofactors else."""
+    rng = np.random.default_rng(7 + P)
+    tri = mg.mode_triples(P)[:N]
+    q, _, cl = mg.workload(lmax, P)
+    shapes = mg.separable_shapes(lmax, S, 25, 2, 2)
+    upb = rng.standard_normal((S, N))
+    with mg.Context(0) as c:
+        c.set_basis(2, lmax, q)
+        c.set_modes(tri)
+        c.set_spectrum(cl)
+        c.init_glint()
+        mu, w = c.get_gl()
+        db = c.project_gl_vjp(shapes, upb)
+    qt = torch.tensor(q, requires_grad=True)
+    (at.Problem(mu, w, 2, lmax, tri, cl, shapes).beta_norm2(qt)[0] * torch.tensor(upb)).sum().backward()
+    assert rel_fro(db, qt.grad.numpy()) <= 1e-11
