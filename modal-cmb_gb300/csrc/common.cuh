@@ -186,8 +186,8 @@ modal_status mij_table_dev(modal_ctx *ctx, const double *q, int lmin, int lmax, 
 modal_status gamma_fp64_dev(modal_ctx *ctx, int mu0, int nmu);
 modal_status gamma_split_dev(modal_ctx *ctx, int mu0, int nmu);
 modal_status ortho_dev(modal_ctx *ctx, int pca_flag);
-// tail: the masked form, for a batch that oz_check reports to need it.
-modal_status project_dev(modal_ctx *ctx, int S, const modal_shape *shapes, modal_prec prec, bool tail = false);
+// careful: the masked form, for a batch that oz_check reports to need it.
+modal_status project_dev(modal_ctx *ctx, int S, const modal_shape *shapes, modal_prec prec, bool careful = false);
 modal_status alpha_dev(modal_ctx *ctx, int S);
 modal_status lambdainv_dev(modal_ctx *ctx);  // linv = lower triangle of orthol
 modal_status transpose_dev(modal_ctx *ctx, const double *in, double *out, int R, int C);
@@ -230,14 +230,14 @@ struct ProjPlan {
     // per parity of the B operand, segments of the slab reduction, buffer offsets
     int SG = 4, NC = 32, M8 = 0, QR = 0, nseg = 1, nsm = 0, teams = 1;
     size_t team_smem = 0, o_q = 0, o_v = 0, o_g = 0, o_t = 0, o_s = 0, o_F = 0, o_bq = 0, o_m = 0;
-    bool tail = false;    // mask the points past the rows' ends
+    bool careful = false;  // points past the rows' ends masked, row sums compensated
     long tabf_total = 0;  // floats of the FP32 separable tables
     RadialArgs ra;        // radial shapes (3D transfer Gamma only)
 };
 // plan: validate, size every buffer, upload the slab schedule (may allocate);
 // stage: copy shape tables/descriptors to the device; record: enqueue the
 // device work only (no allocation, no host round trip: capturable).
-modal_status proj_plan(modal_ctx *ctx, int S, const modal_shape *shapes, modal_prec prec, ProjPlan &pl, bool tail = false);
+modal_status proj_plan(modal_ctx *ctx, int S, const modal_shape *shapes, modal_prec prec, ProjPlan &pl, bool careful = false);
 modal_status proj_stage(modal_ctx *ctx, const ProjPlan &pl, const modal_shape *shapes);
 modal_status proj_record(modal_ctx *ctx, const ProjPlan &pl);
 // The same two steps of the single-precision form (project_f32.cu).

@@ -397,13 +397,13 @@ __global__ void k_project_beta(int N, int P, int S, int nseg, const int *__restr
 // context stream.  The record step allocates nothing and makes no host
 // round trip, so modal_project_batch can capture it into a CUDA graph.
 
-modal_status proj_plan(modal_ctx *ctx, int S, const modal_shape *shapes, modal_prec prec, ProjPlan &pl, bool tail)
+modal_status proj_plan(modal_ctx *ctx, int S, const modal_shape *shapes, modal_prec prec, ProjPlan &pl, bool careful)
 {
     const int lmin = ctx->lmin, lmax = ctx->lmax, L = ctx->L, P = ctx->P, N = ctx->N, PP = P * P;
     pl = ProjPlan();
     pl.S = S;
     pl.prec = prec;
-    pl.tail = tail;
+    pl.careful = careful;
     pl.desc.resize(S);
     long tab_total = 0;
     for (int s = 0; s < S; s++) {
@@ -529,10 +529,10 @@ modal_status proj_record(modal_ctx *ctx, const ProjPlan &pl)
     return launched(ctx, "project_beta");
 }
 
-modal_status project_dev(modal_ctx *ctx, int S, const modal_shape *shapes, modal_prec prec, bool tail)
+modal_status project_dev(modal_ctx *ctx, int S, const modal_shape *shapes, modal_prec prec, bool careful)
 {
     ProjPlan pl;
-    MODAL_TRY(proj_plan(ctx, S, shapes, prec, pl, tail));
+    MODAL_TRY(proj_plan(ctx, S, shapes, prec, pl, careful));
     MODAL_TRY(proj_stage(ctx, pl, shapes));
     return proj_record(ctx, pl);
 }

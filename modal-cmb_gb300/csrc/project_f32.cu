@@ -217,7 +217,7 @@ __global__ void k_pf_basis(int lmin, int lmax, int P, int NC, int M8, int QR, co
     }
 }
 
-// *tail is raised where a separable shape may leave the FP32 range at some (l1, l2, l3): its value is at
+// *tail (unless nullptr) is raised where a separable shape may leave the FP32 range at some (l1, l2, l3): its value is at
 // most the sum over the terms of max|f| max|g| max|h| (k_pf_tab's maxima).
 __global__ void k_pf_shapes(int S, int lmax, const DShape *__restrict__ in, const unsigned *__restrict__ tmax,
                             PfShape *__restrict__ out, int *__restrict__ tail)
@@ -230,7 +230,7 @@ __global__ void k_pf_shapes(int S, int lmax, const DShape *__restrict__ in, cons
         double bound = 0.0;
         for (int t = 0; t < 3 * d.nterms; t += 3)
             bound += (double)__uint_as_float(m[t]) * (double)__uint_as_float(m[t + 1]) * (double)__uint_as_float(m[t + 2]);
-        if (!(bound <= 1e37)) *tail = 1;
+        if (tail && !(bound <= 1e37)) *tail = 1;
     }
     PfShape f;
     f.kind = d.kind;
@@ -366,6 +366,20 @@ __device__ __forceinline__ f2 add2(f2 a, f2 b)
     f2 r;
     asm("add.rn.f32x2 %0, %1, %2;" : "=l"(r) : "l"(a), "l"(b));
     return r;
+}
+
+__device__ __forceinline__ f2 sub2(f2 a, f2 b)
+{
+    f2 r;
+    asm("sub.rn.f32x2 %0, %1, %2;" : "=l"(r) : "l"(a), "l"(b));
+    return r;
+}
+// Kahan sum: hi - lo += x
+__device__ __forceinline__ void kahan2(f2 &hi, f2 &lo, f2 x)
+{
+    const f2 y = sub2(x, lo), t = add2(hi, y);
+    lo = sub2(sub2(t, hi), y);
+    hi = t;
 }
 
 // Shared-memory descriptor, K-major without swizzle: core matrices of 8 rows x 16 bytes, `lbo`
@@ -554,35 +568,47 @@ struct PfPos {
     }
 };
 
-// Adds an accumulator's columns of this thread's row to H.
-template <int NC>
-__device__ __forceinline__ void pf_drain(uint32_t t, f2 (&H)[NC / 2])
+// Adds an accumulator's columns of this thread's row to H; CAREFUL: with Kahan's compensation in lo[NC] (the
+// thread's row of the fold's shared memory, idle during a pass).  With it always, 16 and 256 shapes at l <= 2000,
+// P = 30 took 17.4 and 268 ms instead of 16.0 and 234.
+template <int NC, bool CAREFUL>
+__device__ __forceinline__ void pf_drain(uint32_t t, f2 (&H)[NC / 2], float *lo)
 {
-    constexpr int CH = NC <= 32 ? NC : NC / 2;  // columns per round trip
+    constexpr int CH = CAREFUL && NC <= 32 ? 16 : NC <= 32 ? NC : NC / 2;  // columns per round trip
 #pragma unroll
     for (int c0 = 0; c0 < NC; c0 += CH) {
         uint32_t r[CH];
 #pragma unroll
         for (int x = 0; x < CH; x += 8) tmem_ld8(t + c0 + x, &r[x]);
         tmem_wait_ld();
+        if (CAREFUL) {
 #pragma unroll
-        for (int x = 0; x < CH / 2; x++)
-            H[c0 / 2 + x] = add2(H[c0 / 2 + x], pk(__uint_as_float(r[2 * x]), __uint_as_float(r[2 * x + 1])));
+            for (int x = 0; x < CH; x += 4) {
+                ulonglong2 l = *reinterpret_cast<ulonglong2 *>(lo + c0 + x);
+                kahan2(H[(c0 + x) / 2], l.x, pk(__uint_as_float(r[x]), __uint_as_float(r[x + 1])));
+                kahan2(H[(c0 + x) / 2 + 1], l.y, pk(__uint_as_float(r[x + 2]), __uint_as_float(r[x + 3])));
+                *reinterpret_cast<ulonglong2 *>(lo + c0 + x) = l;
+            }
+        } else {
+#pragma unroll
+            for (int x = 0; x < CH / 2; x++)
+                H[c0 / 2 + x] = add2(H[c0 / 2 + x], pk(__uint_as_float(r[2 * x]), __uint_as_float(r[2 * x + 1])));
+        }
     }
 }
 
 // One pass of a row block: a bump (nt = 0), or nt = 1..4 terms of a separable shape from term t0 on.
-// TAIL: the points past a row's end are masked.
-template <int NC, bool TAIL>
+// CAREFUL: the points past a row's end are masked and the row sums compensated.
+template <int NC, bool CAREFUL>
 __device__ __forceinline__ bool pf_pass(const PfArgs &a, const PfShape &sh, int t0, int nt, int j, const PfClass &c,
                                         const PfRow &rw, int nch, bool block, const float4 *__restrict__ Wrow, const uint8_t *sm, PfSync *sy,
-                                        uint32_t tA, uint32_t tD1, PfPos &pos, f2 (&H)[NC / 2])
+                                        uint32_t tA, uint32_t tD1, PfPos &pos, f2 (&H)[NC / 2], float *lo)
 {
     using M = PfMem<NC>;
     const uint32_t ready = smem_u32(sy->ready), done = smem_u32(sy->done), full = smem_u32(sy->full);
     volatile int *abort_flag = &sy->abort_flag;
     const int lane = threadIdx.x & 31, ms = pf_mstart(c);
-    const int ml = TAIL ? pf_mlast(c, j, min(PF_ROWS * rw.b + (int)(threadIdx.x & 127), c.nr - 1)) : 0;
+    const int ml = CAREFUL ? pf_mlast(c, j, min(PF_ROWS * rw.b + (int)(threadIdx.x & 127), c.nr - 1)) : 0;
     // the first half's weights
     float4 w[4];
 #pragma unroll
@@ -630,7 +656,7 @@ __device__ __forceinline__ bool pf_pass(const PfArgs &a, const PfShape &sh, int 
         const ulonglong2 *T0 = reinterpret_cast<const ulonglong2 *>(sm + pos.slot * M::SLOT + M::BCH);
         // chunk cc - 2 was complete before this thread wrote the second half of cc - 1; its accumulator is
         // overwritten by the products of this chunk
-        if (n >= 2) pf_drain<NC>(tA + M::D0 + NC * (cc & 1), H);
+        if (n >= 2) pf_drain<NC, CAREFUL>(tA + M::D0 + NC * (cc & 1), H, lo);
 #pragma unroll 1
         for (int hf = 0; hf < 2; hf++) {
             if (cc > 0) {  // the products that read this half a chunk ago are done
@@ -693,7 +719,7 @@ __device__ __forceinline__ bool pf_pass(const PfArgs &a, const PfShape &sh, int 
                     }
                     if (mg < c.m0) {
                         // before the rows start (below lmin the caller's tables may hold anything); past a
-                        // row's end the weight is zero and, unless TAIL, the shape finite
+                        // row's end the weight is zero and, unless CAREFUL, the shape finite
 #pragma unroll
                         for (int y = 0; y < 4; y++) {
                             float v0, v1;
@@ -701,7 +727,7 @@ __device__ __forceinline__ bool pf_pass(const PfArgs &a, const PfShape &sh, int 
                             v[y] = pk(mg + 2 * y >= c.m0 ? v0 : 0.f, mg + 2 * y + 1 >= c.m0 ? v1 : 0.f);
                         }
                     }
-                    if (TAIL) {
+                    if (CAREFUL) {
 #pragma unroll
                         for (int y = 0; y < 4; y++) {
                             float v0, v1;
@@ -740,16 +766,16 @@ __device__ __forceinline__ bool pf_pass(const PfArgs &a, const PfShape &sh, int 
         }
     }
     // the last two chunks, then the row's other products
-    if (nch > 1) pf_drain<NC>(tA + M::D0 + NC * (pos.cc & 1), H);
+    if (nch > 1) pf_drain<NC, CAREFUL>(tA + M::D0 + NC * (pos.cc & 1), H, lo);
     if (!pf_wait(done + 8, (pos.cc - 1) & 1, abort_flag)) return false;
     tc_fence_after();
-    pf_drain<NC>(tA + M::D0 + NC * ((pos.cc - 1) & 1), H);
-    pf_drain<NC>(tD1, H);
+    pf_drain<NC, CAREFUL>(tA + M::D0 + NC * ((pos.cc - 1) & 1), H, lo);
+    pf_drain<NC, CAREFUL>(tD1, H, lo);
     tc_fence_before();
     return true;
 }
 
-template <int NC, bool TAIL>
+template <int NC, bool CAREFUL>
 __global__ void __launch_bounds__(PfMem<NC>::THREADS, 1) k_project_f32(const PfArgs a)
 {
     using M = PfMem<NC>;
@@ -888,10 +914,14 @@ __global__ void __launch_bounds__(PfMem<NC>::THREADS, 1) k_project_f32(const PfA
                         f2 H[NC / 2];
 #pragma unroll
                         for (int x = 0; x < NC / 2; x++) H[x] = 0ull;
+                        float *lo = CAREFUL ? Hs + tid * M::HLD : nullptr;
+                        if (CAREFUL)
+#pragma unroll
+                            for (int x = 0; x < NC; x += 4) *reinterpret_cast<ulonglong2 *>(lo + x) = make_ulonglong2(0ull, 0ull);
                         bool ok = true;
                         const int nterms = sh.kind == MODAL_SHAPE_SEPARABLE ? sh.nterms : 0;
                         for (int t0 = 0; ok && (t0 == 0 || t0 < nterms); t0 += PF_TC)
-                            ok = pf_pass<NC, TAIL>(a, sh, t0, min(PF_TC, nterms - t0), j, c, rw, nch, sx == 0 && t0 == 0, Wrow, pf_sm, sy, tA, tD1, pos, H);
+                            ok = pf_pass<NC, CAREFUL>(a, sh, t0, min(PF_TC, nterms - t0), j, c, rw, nch, sx == 0 && t0 == 0, Wrow, pf_sm, sy, tA, tD1, pos, H, lo);
                         if (ok && sx == 0) ok = pf_wait(smem_u32(&sy->qfull), nq & 1, &sy->abort_flag);
                         if (!ok) { sy->abort_flag = 1; atomicCAS(a.err, 0, 23); }
                         // fold: F[a][c] += sum over the block's rows of q_a(i) H[i][c]
@@ -1028,7 +1058,7 @@ __global__ void k_pf_beta(int N, int P, int S, int nseg, const int *__restrict__
 template <class F>
 static modal_status pf_kernel(const ProjPlan &pl, F use)
 {
-    if (pl.tail) return pl.NC == 16 ? use(k_project_f32<16, true>) : pl.NC == 32 ? use(k_project_f32<32, true>)
+    if (pl.careful) return pl.NC == 16 ? use(k_project_f32<16, true>) : pl.NC == 32 ? use(k_project_f32<32, true>)
                       : pl.NC == 48 ? use(k_project_f32<48, true>) : use(k_project_f32<64, true>);
     return pl.NC == 16 ? use(k_project_f32<16, false>) : pl.NC == 32 ? use(k_project_f32<32, false>)
          : pl.NC == 48 ? use(k_project_f32<48, false>) : use(k_project_f32<64, false>);
@@ -1099,6 +1129,12 @@ modal_status pf_plan(modal_ctx *ctx, ProjPlan &pl)
         MODAL_CUDA(cudaFuncSetAttribute(kern, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)pl.smem));
         return MODAL_OK;
     };
+    // A row's sum adds up to `adds` accumulators, each nearly exact.  Plain FP32 additions do as long as they are no
+    // more than the 32 points of a block, which are summed in plain FP32 where CUDA cores do it; else compensated.
+    int terms = 1;
+    for (const DShape &d : pl.desc) terms = std::max(terms, d.nterms);
+    const int adds = ceil_div(terms, PF_TC) * (ceil_div(lmax / 4 + 8, PF_KC) + 1);
+    if (adds > PF_KC) pl.careful = true;
     MODAL_TRY(pf_kernel(pl, attr));
     return oz_reset(ctx);
 }
@@ -1135,7 +1171,7 @@ modal_status pf_record(modal_ctx *ctx, const ProjPlan &pl)
             lmin, lmax, pl.M8, ctx->shape_desc.as<DShape>(), ctx->shape_tab.as<double>(), tabf, tmax);
         MODAL_TRY(launched(ctx, "pf_tab"));
     }
-    k_pf_shapes<<<ceil_div(S, 64), 64, 0, ctx->stream>>>(S, lmax, ctx->shape_desc.as<DShape>(), tmax, fs, tail);
+    k_pf_shapes<<<ceil_div(S, 64), 64, 0, ctx->stream>>>(S, lmax, ctx->shape_desc.as<DShape>(), tmax, fs, pl.careful ? nullptr : tail);
     MODAL_TRY(launched(ctx, "pf_shapes"));
     PfArgs a;
     a.lmin = lmin; a.lmax = lmax; a.P = P; a.S = S; a.SG = pl.SG; a.G = ceil_div(S, pl.SG);

@@ -129,3 +129,22 @@ def test_f32_projection_of_extreme_bumps(mg, c, sigma):
         b32 = ctx.project(shape, mg.PREC_SPLIT)
     assert np.all(np.isfinite(b64))
     assert np.linalg.norm(b32 - b64) <= 1e-6 * np.linalg.norm(b64)
+
+
+def test_f32_projection_long_row_sums_keep_small_addends(mg):
+    """Nine terms at l_max = 2000, three passes of up to 17 accumulators per row (past the 32 that are added
+    plainly): in the slab j = 1000 the point k = j outweighs each later block of 32 points by more than 2^24,
+    their sum not.  Tolerance: the roundings of a point (weight, shape, product), of the fold and of the slab
+    sum, 2^-24 each at most, several of them averaged over 500 rows: 1.5e-7."""
+    lmax = 2000
+    tab = np.zeros((9, 3, lmax + 1))
+    tab[0] = 1.0
+    tab[0, :, 1000] = 3 * 2.0**30
+    with mg.Context(0) as c:
+        c.set_basis(2, lmax, np.ones((lmax - 1, 1)))
+        c.set_modes(np.zeros((1, 3), np.int32))
+        c.set_spectrum(np.ones(lmax + 1))
+        shape = [{"kind": mg.SHAPE_SEPARABLE, "tab": tab}]
+        b64 = c.project(shape, mg.PREC_FP64)
+        b32 = c.project(shape, mg.PREC_SPLIT)
+    assert rel_fro(b32, b64) <= 1.5e-7
