@@ -229,8 +229,9 @@ struct ProjPlan {
     // FP32 form (project_f32.cu): shapes per work item, operand columns, groups of 8 lattice points
     // per parity of the B operand, segments of the slab reduction, buffer offsets
     int SG = 4, NC = 32, M8 = 0, QR = 0, nseg = 1, nsm = 0, teams = 1;
-    size_t team_smem = 0, o_q = 0, o_v = 0, o_g = 0, o_t = 0, o_s = 0, o_F = 0, o_bq = 0, o_m = 0;
-    bool careful = false;  // points past the rows' ends masked, row sums compensated
+    size_t team_smem = 0, o_q = 0, o_v = 0, o_g = 0, o_t = 0, o_s = 0, o_F = 0, o_bq = 0, o_m = 0, o_fl = 0;
+    bool careful = false;  // points past the rows' ends masked, all sums compensated
+    int grp = 16, comp = 0;  // rows that are added plainly; whether the sum of such groups is compensated
     long tabf_total = 0;  // floats of the FP32 separable tables
     RadialArgs ra;        // radial shapes (3D transfer Gamma only)
 };

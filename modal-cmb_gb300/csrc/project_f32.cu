@@ -442,6 +442,8 @@ struct PfArgs {
     const __nv_bfloat16 *Bt;
     const float *qt;
     float *Fbuf;               // [S][L][P*P]
+    float *Flo;                // CAREFUL: [CTA][team][SG][tiles per thread][16][128] corrections of F (hi in shared memory)
+    int grp, comp;             // rows that the fold adds plainly; whether it compensates the sum of such groups
     int *err;
 };
 
@@ -451,6 +453,12 @@ __device__ __forceinline__ int pf_item(const PfArgs &a, int team, int it)
 {
     const int n = (int)gridDim.x * a.teams, r = team * (int)gridDim.x + (int)blockIdx.x;
     return it * n + ((it & 1) ? n - 1 - r : r);
+}
+
+// This thread's corrections of tile x (of SG tpt) of F.
+__device__ __forceinline__ float *pf_flo(const PfArgs &a, int x, int tpt)
+{
+    return a.Flo + ((size_t)(blockIdx.x * a.teams + (threadIdx.x >> 7)) * a.SG * tpt + x) * 16 * 128 + (threadIdx.x & 127);
 }
 
 // The passes of a team in order (items x parities x row blocks x shapes x groups of terms, as the row
@@ -924,40 +932,74 @@ __global__ void __launch_bounds__(PfMem<NC>::THREADS, 1) k_project_f32(const PfA
                             ok = pf_pass<NC, CAREFUL>(a, sh, t0, min(PF_TC, nterms - t0), j, c, rw, nch, sx == 0 && t0 == 0, Wrow, pf_sm, sy, tA, tD1, pos, H, lo);
                         if (ok && sx == 0) ok = pf_wait(smem_u32(&sy->qfull), nq & 1, &sy->abort_flag);
                         if (!ok) { sy->abort_flag = 1; atomicCAS(a.err, 0, 23); }
-                        // fold: F[a][c] += sum over the block's rows of q_a(i) H[i][c]
+                        // fold: F[a][c] += sum over the block's rows of q_a(i) H[i][c], in groups of rows (pf_plan)
 #pragma unroll
                         for (int x = 0; x < NC / 2; x += 2)
                             *reinterpret_cast<ulonglong2 *>(Hs + tid * M::HLD + 2 * x) = make_ulonglong2(H[x], H[x + 1]);
                         stop = rows_bar_or(bar, !ok);
                         const int nrow = min(PF_ROWS, c.nr - b * PF_ROWS);
+                        // the thread's number is read again, so that less of the fold stays in registers through the
+                        // passes (not for 64 columns, which then spill)
+                        int ft = threadIdx.x;
+                        if (NC < 64) asm volatile("mov.u32 %0, %%tid.x;" : "=r"(ft));
                         for (int tt = 0; tt < tpt; tt++) {
+                            const int tid = ft & 127;
                             const int ti = (tid & (ntp - 1)) + 128 * tt, sp = tid / ntp;
                             if (ti >= nt) break;
                             const int bt = ti / nb4, ct = ti - bt * nb4, rend = min(nrow, (sp + 1) * rper);
                             const float *qq = Qs + 4 * bt, *hq = Hs + 4 * ct;
-                            f2 acc[4][2];
-#pragma unroll
-                            for (int x = 0; x < 4; x++) acc[x][0] = acc[x][1] = 0ull;
-#pragma unroll 8
-                            for (int q = sp * rper; q < rend; q++) {
-                                const float4 qv = *reinterpret_cast<const float4 *>(qq + q * NC);
-                                const ulonglong2 hv = *reinterpret_cast<const ulonglong2 *>(hq + q * M::HLD);
-                                const f2 qa[4] = {pk(qv.x, qv.x), pk(qv.y, qv.y), pk(qv.z, qv.z), pk(qv.w, qv.w)};
-#pragma unroll
-                                for (int x = 0; x < 4; x++) {
-                                    acc[x][0] = fma2(qa[x], hv.x, acc[x][0]);
-                                    acc[x][1] = fma2(qa[x], hv.y, acc[x][1]);
-                                }
-                            }
                             float *f = Fs + (size_t)(sx * tpt + tt) * 16 * 128 + tid;
+                            float *fl = CAREFUL ? pf_flo(a, sx * tpt + tt, tpt) : nullptr;
+                            f2 hi[4][2], lk[4][2], acc[4][2];
 #pragma unroll
                             for (int x = 0; x < 4; x++)
 #pragma unroll
                                 for (int y = 0; y < 2; y++) {
-                                    float v0, v1;
-                                    upk(acc[x][y], v0, v1);
-                                    f[(4 * x + 2 * y) * 128] += v0;
-                                    f[(4 * x + 2 * y + 1) * 128] += v1;
+                                    hi[x][y] = lk[x][y] = 0ull;
+                                    const int e = (4 * x + 2 * y) * 128;
+                                    if (CAREFUL && woff != a.base[slab]) {  // (not the slab's first row block)
+                                        hi[x][y] = pk(f[e], f[e + 128]);
+                                        lk[x][y] = pk(fl[e], fl[e + 128]);
+                                    }
+                                }
+#pragma unroll 1
+                            for (int g = sp * rper; g < rend; g += a.grp) {
+                                const int ge = min(g + a.grp, rend);
+#pragma unroll
+                                for (int x = 0; x < 4; x++) acc[x][0] = acc[x][1] = 0ull;
+#pragma unroll 8
+                                for (int q = g; q < ge; q++) {
+                                    const float4 qv = *reinterpret_cast<const float4 *>(qq + q * NC);
+                                    const ulonglong2 hv = *reinterpret_cast<const ulonglong2 *>(hq + q * M::HLD);
+                                    const f2 qa[4] = {pk(qv.x, qv.x), pk(qv.y, qv.y), pk(qv.z, qv.z), pk(qv.w, qv.w)};
+#pragma unroll
+                                    for (int x = 0; x < 4; x++) {
+                                        acc[x][0] = fma2(qa[x], hv.x, acc[x][0]);
+                                        acc[x][1] = fma2(qa[x], hv.y, acc[x][1]);
+                                    }
+                                }
+#pragma unroll
+                                for (int x = 0; x < 4; x++)
+#pragma unroll
+                                    for (int y = 0; y < 2; y++) {
+                                        if (CAREFUL || a.comp) kahan2(hi[x][y], lk[x][y], acc[x][y]);
+                                        else hi[x][y] = add2(hi[x][y], acc[x][y]);
+                                    }
+                            }
+#pragma unroll
+                            for (int x = 0; x < 4; x++)
+#pragma unroll
+                                for (int y = 0; y < 2; y++) {
+                                    const int e = (4 * x + 2 * y) * 128;
+                                    if (CAREFUL) {
+                                        upk(hi[x][y], f[e], f[e + 128]);
+                                        upk(lk[x][y], fl[e], fl[e + 128]);
+                                    } else {
+                                        float v0, v1;
+                                        upk(sub2(hi[x][y], lk[x][y]), v0, v1);
+                                        f[e] += v0;
+                                        f[e + 128] += v1;
+                                    }
                                 }
                         }
                         stop = rows_bar_or(bar, stop);  // Hs is read before the next pass writes it
@@ -973,6 +1015,8 @@ __global__ void __launch_bounds__(PfMem<NC>::THREADS, 1) k_project_f32(const PfA
                     if (ti >= nt || tid >= ntp) break;
                     const int bt = ti / nb4, ct = ti - bt * nb4;
                     const float *f = Fs + (size_t)(sx * tpt + tt) * 16 * 128 + tid;
+                    const float *fl = CAREFUL ? pf_flo(a, sx * tpt + tt, tpt) : nullptr;
+                    const bool corr = CAREFUL && woff != a.base[slab];  // (a slab without rows has no corrections)
                     float *dst = a.Fbuf + ((size_t)(s0 + sx) * L + slab) * PP;
 #pragma unroll
                     for (int x = 0; x < 4; x++)
@@ -980,9 +1024,18 @@ __global__ void __launch_bounds__(PfMem<NC>::THREADS, 1) k_project_f32(const PfA
                         for (int y = 0; y < 4; y++) {
                             const int bb = 4 * bt + x, c2 = 4 * ct + y;
                             if (bb >= P || c2 >= P) continue;
-                            float v = 0.f;
-                            for (int q = 0; q < rs; q++) v += f[(4 * x + y) * 128 + q * ntp];
-                            dst[bb * P + c2] = v;
+                            float v = 0.f, lo = 0.f;
+                            for (int q = 0; q < rs; q++) {
+                                const int e = (4 * x + y) * 128 + q * ntp;
+                                if (CAREFUL) {
+                                    const float z = f[e] - lo, t = v + z;
+                                    lo = (t - v) - z;
+                                    v = t;
+                                    if (corr) lo += fl[e];
+                                } else
+                                    v += f[e];
+                            }
+                            dst[bb * P + c2] = v - lo;
                         }
                 }
             stop = rows_bar_or(bar, false);  // the sums are read before the next item clears them
@@ -1108,6 +1161,20 @@ modal_status pf_plan(modal_ctx *ctx, ProjPlan &pl)
     pl.QR = lmax / 2 + 1;
     pl.M8 = (lmax / 2 + 1 + 7) / 8 + 4;
     MODAL_CUDA(cudaDeviceGetAttribute(&pl.nsm, cudaDevAttrMultiProcessorCount, ctx->device));
+    // How the sums between a point and F are kept.  Plain FP32 additions do where a term of the sum meets no more
+    // roundings than on CUDA cores, which add 32 points of a row and 16 rows plainly and compensate beyond (52 with
+    // the roundings of their compensated sums and stores): two for a chunk's accumulator, one per accumulator of the row,
+    // `grp` for a group of rows, seven for the groups of a block and the splits of the rows (one if compensated), one
+    // per row block.  l <= 1,700 takes no compensation, l <= 2,500 that of the groups; beyond (or for more than four
+    // terms, whose passes multiply the accumulators) the careful kernel compensates all.  Groups compensated: 16 shapes
+    // at l <= 2000, P = 30 15.56 -> 15.78 ms; with the blocks compensated as well 16.5 ms and 0.25 -> 0.31 ms at l <= 100.
+    int terms = 1;
+    for (const DShape &d : pl.desc) terms = std::max(terms, d.nterms);
+    const int adds = ceil_div(terms, PF_TC) * (ceil_div(lmax / 4 + 8, PF_KC) + 1) - 1,
+              blocks = 2 * ceil_div(lmax / 2 + 1, PF_ROWS) - 1, limit = 52;
+    pl.comp = 2 + adds + 16 + 7 + blocks > limit;
+    pl.grp = pl.comp && 2 + adds + 16 + 1 + blocks > limit ? 8 : 16;
+    if (pl.comp && 2 + adds + pl.grp + 1 + blocks > limit) pl.careful = true;
     // segments of the reduction over slabs: about four CTAs per SM
     const long ctas = (long)ceil_div(PP, 128) * S * ceil_div(P, PB);
     pl.nseg = (int)std::max(1L, std::min(std::min(16L, (long)ceil_div(L, 32)), 4L * pl.nsm / ctas));
@@ -1121,6 +1188,7 @@ modal_status pf_plan(modal_ctx *ctx, ProjPlan &pl)
     pl.o_m = o; o += al(sizeof(unsigned) * (size_t)(pl.tab_total / (lmax + 1)));
     pl.o_s = o; o += al(sizeof(PfShape) * (size_t)S);
     pl.o_F = o; o += al(sizeof(float) * (size_t)S * L * PP);
+    pl.o_fl = o; o += al(pl.careful ? (size_t)pl.nsm * pl.teams * pl.SG * fper : 0);
     pl.o_B = o; o += al(sizeof(double) * (size_t)pl.nseg * S * P * PP);
     pl.o_bq = o; o += al(sizeof(__nv_bfloat16) * 2 * 3 * 8 * (size_t)pl.M8 * pl.NC);
     pl.o_w = o; o += al(sizeof(float) * PF_ROWS * (size_t)ctx->pf_total);
@@ -1129,12 +1197,6 @@ modal_status pf_plan(modal_ctx *ctx, ProjPlan &pl)
         MODAL_CUDA(cudaFuncSetAttribute(kern, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)pl.smem));
         return MODAL_OK;
     };
-    // A row's sum adds up to `adds` accumulators, each nearly exact.  Plain FP32 additions do as long as they are no
-    // more than the 32 points of a block, which are summed in plain FP32 where CUDA cores do it; else compensated.
-    int terms = 1;
-    for (const DShape &d : pl.desc) terms = std::max(terms, d.nterms);
-    const int adds = ceil_div(terms, PF_TC) * (ceil_div(lmax / 4 + 8, PF_KC) + 1);
-    if (adds > PF_KC) pl.careful = true;
     MODAL_TRY(pf_kernel(pl, attr));
     return oz_reset(ctx);
 }
@@ -1178,6 +1240,9 @@ modal_status pf_record(modal_ctx *ctx, const ProjPlan &pl)
     a.nitems = L * a.G;
     a.M8 = pl.M8;
     a.QR = pl.QR;
+    a.Flo = reinterpret_cast<float *>(b + pl.o_fl);
+    a.grp = pl.grp;
+    a.comp = pl.comp;
     a.order = reinterpret_cast<const int *>(base + L);
     a.base = base;
     a.shapes = fs; a.tabf = tabf; a.il2 = il2; a.W = W; a.Bt = Bt; a.qt = qt; a.Fbuf = Fbuf;

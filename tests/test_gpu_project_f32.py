@@ -116,7 +116,8 @@ def test_f32_projection_of_a_shape_that_overflows_outside_the_triangle(mg):
         tame = dict(shape, tab=shape["tab"] * [[[1e-12]], [[1.0]]])  # bounded: the same values at the points that count
         batch = [c.project_batch([x], mg.PREC_SPLIT) for x in (tame, shape, tame)]
     assert rel_fro(b32, b64) <= 1e-6
-    assert all(np.array_equal(b, b32) for b in batch)
+    assert np.array_equal(batch[1], b32) and np.array_equal(batch[0], batch[2])
+    assert rel_fro(batch[0], b64) <= 1e-6
 
 
 @pytest.mark.parametrize("c,sigma", [((1e17, -2e17, 5e16), 1e17), ((3e16, 0.3, 0.7), 0.1), ((0.21, 0.3141, 0.4759), 1e-21),
@@ -148,3 +149,37 @@ def test_f32_projection_long_row_sums_keep_small_addends(mg):
         b64 = c.project(shape, mg.PREC_FP64)
         b32 = c.project(shape, mg.PREC_SPLIT)
     assert rel_fro(b32, b64) <= 1.5e-7
+
+
+@pytest.mark.parametrize("P", [30, 33])
+def test_f32_projection_fold_keeps_small_addends(mg, P):
+    """Every slab's first row, l = 2, outweighs each other one by 2^24 or more.  Tolerance: rows are added in
+    groups of 16 before the compensated sum, 15 additions that round by half a unit, 2^-25, at most."""
+    lmax = 1000
+    tab = np.ones((1, 3, lmax + 1))
+    tab[:, 0, 2] = 3 * 2.0**30
+    with mg.Context(0) as c:
+        c.set_basis(2, lmax, mg.legendre_q(2, lmax, P))
+        c.set_modes(np.zeros((1, 3), np.int32))
+        c.set_spectrum(np.ones(lmax + 1))
+        shape = [{"kind": mg.SHAPE_SEPARABLE, "tab": tab}]
+        b64 = c.project(shape, mg.PREC_FP64)
+        b32 = c.project(shape, mg.PREC_SPLIT)
+    assert rel_fro(b32, b64) <= 15 * 2.0**-25
+
+
+@pytest.mark.parametrize("P", [30, 33])
+def test_f32_projection_fold_keeps_small_addends(mg, P):
+    """Every slab's first row, l = 2, outweighs each other one by 2^24 or more.  Tolerance: rows are added in
+    groups of 16 before the compensated sum, 15 additions that round by half a unit, 2^-25, at most."""
+    lmax = 1000
+    tab = np.ones((1, 3, lmax + 1))
+    tab[:, 0, 2] = 3 * 2.0**30
+    with mg.Context(0) as c:
+        c.set_basis(2, lmax, mg.legendre_q(2, lmax, P))
+        c.set_modes(np.zeros((1, 3), np.int32))
+        c.set_spectrum(np.ones(lmax + 1))
+        shape = [{"kind": mg.SHAPE_SEPARABLE, "tab": tab}]
+        b64 = c.project(shape, mg.PREC_FP64)
+        b32 = c.project(shape, mg.PREC_SPLIT)
+    assert rel_fro(b32, b64) <= 15 * 2.0**-25
