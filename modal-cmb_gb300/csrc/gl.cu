@@ -1,19 +1,10 @@
 // gl.cu -- Gauss-Legendre quadrature, the P_l(mu) table, the shifted Legendre
 // basis and the asymptotic geometric factor, all FP64 on the GPU.
 #include "common.cuh"
+#include "divsmall.cuh"
 #include "legendre.cuh"
 
 namespace modal {
-
-// n / c for a small positive integer c and r = 1 / c rounded: Markstein's correction of n r (P. W.
-// Markstein, "Computation of elementary functions on the IBM RISC System/6000 processor", IBM J.
-// Res. Develop. 34 (1990)).  Three dependent operations instead of a division's dozen, and the same
-// bits: the residual is exact, and a quotient by c < 2^13 is never within 2^-14 ulp of a midpoint.
-__device__ __forceinline__ double div_small(double n, double c, double r)
-{
-    const double q = n * r;
-    return fma(fma(-q, c, n), r, q);
-}
 
 // ---------------------------------------------------------------------------
 // Gauss-Legendre nodes/weights (replaces asy, gl_integration.c:46-168; same
