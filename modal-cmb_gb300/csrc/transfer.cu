@@ -232,12 +232,30 @@ __global__ void k_transfer_node_weights(int nmu, int xsize, int nx, const double
     w2[e] = (xi < nx ? x2 : cx[xi] * x2) * w[k];
 }
 
-// out[m][n]: six entries of T_sum and, one x at a time, of the first nx tables with the zero rule.
-// T: [nx] tables of the first samples, then T_sum (if last), zstride apart.
+// y_x of one (m, n), summed as k_gamma_transfer sums it: a pair's permanent per node, nodes in order.
+// p: P times the primordial triple, q: the late triple, A: the sample's [nmu][nu] table.
+__device__ __noinline__ double transfer_sample(int nmu, int nu, const int *p, const int *q, const double *__restrict__ A,
+                                               const double *__restrict__ w)
+{
+    double acc = 0.0;
+    for (int k = 0; k < nmu; k++, A += nu) {
+        const double *r1 = A + p[0], *r2 = A + p[1], *r3 = A + p[2];
+        const double a21 = r2[q[0]], a22 = r2[q[1]], a23 = r2[q[2]], a31 = r3[q[0]], a32 = r3[q[1]], a33 = r3[q[2]];
+        const double t1 = fma(a23, a32, a22 * a33), t2 = fma(a23, a31, a21 * a33), t3 = fma(a22, a31, a21 * a32);
+        acc = fma(w[k], fma(r1[q[2]], t3, fma(r1[q[1]], t2, r1[q[0]] * t1)), acc);
+    }
+    return acc;
+}
+
+// out[m][n]: six entries of T_sum and, one x at a time, of the first nx tables with the zero rule, which
+// within 1e-6 (relative) of its threshold goes by the sum of the permanents: both routes then drop the same
+// samples.  T: [nx] tables of the first samples, then T_sum (if last), zstride apart.
 __global__ void __launch_bounds__(256) k_transfer_gather(int N, int Nprim, int P, int U, long ldT, int nx, int last, size_t zstride,
                                                          const int *__restrict__ triples, const int *__restrict__ prim,
                                                          const double *__restrict__ cx, const double *__restrict__ T,
-                                                         double scale, double *__restrict__ out)
+                                                         int nmu, const double *__restrict__ mt2, const double *__restrict__ w,
+                                                         const double *__restrict__ xvec, double scale,
+                                                         double *__restrict__ out)
 {
     const long e = (long)blockIdx.x * blockDim.x + threadIdx.x;
     if (e >= (long)N * Nprim) return;
@@ -253,6 +271,8 @@ __global__ void __launch_bounds__(256) k_transfer_gather(int N, int Nprim, int P
         double y = 0.0;
 #pragma unroll
         for (int s = 0; s < 6; s++) y += T[x * zstride + at[s]];
+        if (fabs(fabs(y) - 1e-18) <= 1e-24)
+            y = xvec[x] * xvec[x] * transfer_sample(nmu, U, p, q, mt2 + (size_t)x * nmu * U, w);
         if (fabs(y) > 1e-18) y = 0.0;
         res = fma(cx[x], y, res);
     }
@@ -387,8 +407,8 @@ static modal_status transfer_triple_dev(modal_ctx *c, double scale)
         MODAL_TRY(triple_sum_dev(c, n, Zn, n, T + nx * n));
     }
     k_transfer_gather<<<ceil_div((long)N * Nprim, 256), 256, 0, c->stream>>>(
-        N, Nprim, c->P, U, (long)UV, nx, K2 > 0, n, c->triples.as<int>(), c->tr_prim.as<int>(), cx, T, scale,
-        c->tr_out.as<double>());
+        N, Nprim, c->P, U, (long)UV, nx, K2 > 0, n, c->triples.as<int>(), c->tr_prim.as<int>(), cx, T, nmu,
+        c->tr_mt.as<double>(), c->w.as<double>(), c->tr_x.as<double>(), scale, c->tr_out.as<double>());
     return launched(c, "transfer_gather");
 }
 
