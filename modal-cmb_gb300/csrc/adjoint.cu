@@ -358,12 +358,16 @@ __global__ void k_fold_nodes(int nmu, int ncol, double *__restrict__ D)
 }
 
 // Z[l - lmin][c] = sum_k pl[l][k] D[k][c], D overwritten.  Antisymmetric nodes: P_l(-x) = (-1)^l P_l(x)
-// leaves the sums (even l) or differences (odd l) of mirrored rows against half the nodes.
+// leaves the sums (even l) or differences (odd l) of mirrored rows against half the nodes, which pays for its
+// launches and shorter sums where the FP64 pipe is the bound: Gamma's adjoint at l <= 1000 with 78 columns 1.77 ms
+// folded, 1.58 not, the projection's with 240 2.42 and 2.54 (whole calls); l <= 600, 3 columns 1.00 and 0.37, l <= 20
+// 0.090 and 0.082.
 modal_status pl_contract(modal_ctx *c, int ncol, double *D, double *Z)
 {
     const int nmu = c->nmu, L = c->L, lmin = c->lmin;
     const double *pl = c->pl.as<double>() + (size_t)lmin * nmu;
-    if (!c->gl_sym) return dgemm_splitk(c, L, ncol, nmu, pl, nmu, false, D, ncol, false, Z, ncol, 0, false);
+    if (!c->gl_sym || (double)L * ncol * nmu < 2.5e8)
+        return dgemm_splitk(c, L, ncol, nmu, pl, nmu, false, D, ncol, false, Z, ncol, 0, false);
     if (nmu > 1) {  // (a single node has no mirror)
         k_fold_nodes<<<ceil_div((long)(nmu / 2) * ncol, 256), 256, 0, c->stream>>>(nmu, ncol, D);
         MODAL_TRY(launched(c, "fold_nodes"));
