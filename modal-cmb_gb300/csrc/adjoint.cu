@@ -30,6 +30,7 @@
 //   dJ/dGamma = sum_s c_s alpha_s alpha_s^T, dJ/dbeta_s = -2 c_s alpha_s, c_s = 1/(S <S_s,S_s>).
 #include <algorithm>
 #include <cmath>
+#include <cstring>
 #include <vector>
 #include "common.cuh"
 #include "triple.cuh"
@@ -531,15 +532,18 @@ modal_status adj_forward(modal_ctx *c, int S, const modal_shape *shapes, AdjFwd 
                                    cudaMemcpyHostToDevice, c->stream));
         off += n;
     }
-    MODAL_CUDA(cudaMemcpyAsync(b + o_loff, leg_off.data(), sizeof(long) * E, cudaMemcpyHostToDevice, c->stream));
-    MODAL_CUDA(cudaMemcpyAsync(b + o_ca, ca.data(), sizeof(int) * ncol, cudaMemcpyHostToDevice, c->stream));
-    MODAL_CUDA(cudaMemcpyAsync(b + o_cb, cb.data(), sizeof(int) * ncol, cudaMemcpyHostToDevice, c->stream));
-    MODAL_CUDA(cudaMemcpyAsync(b + o_leg0, leg0.data(), sizeof(int) * S, cudaMemcpyHostToDevice, c->stream));
-    MODAL_CUDA(cudaMemcpyAsync(b + o_nt, nterm.data(), sizeof(int) * S, cudaMemcpyHostToDevice, c->stream));
-    MODAL_CUDA(cudaMemcpyAsync(b + o_kb, kb.data(), sizeof(int) * S, cudaMemcpyHostToDevice, c->stream));
-    MODAL_CUDA(cudaMemcpyAsync(b + o_ts, tshape.data(), sizeof(int) * tshape.size(), cudaMemcpyHostToDevice, c->stream));
-    MODAL_CUDA(cudaMemcpyAsync(b + o_ts + sizeof(int) * tshape.size(), tleg.data(), sizeof(int) * tleg.size(),
-                               cudaMemcpyHostToDevice, c->stream));
+    // the index tables lie side by side: one copy
+    std::vector<uint8_t> idx(o_wl - o_loff);
+    auto put = [&](size_t at, const void *src, size_t bytes) { std::memcpy(idx.data() + (at - o_loff), src, bytes); };
+    put(o_loff, leg_off.data(), sizeof(long) * E);
+    put(o_ca, ca.data(), sizeof(int) * ncol);
+    put(o_cb, cb.data(), sizeof(int) * ncol);
+    put(o_leg0, leg0.data(), sizeof(int) * S);
+    put(o_nt, nterm.data(), sizeof(int) * S);
+    put(o_kb, kb.data(), sizeof(int) * S);
+    put(o_ts, tshape.data(), sizeof(int) * tshape.size());
+    put(o_ts + sizeof(int) * tshape.size(), tleg.data(), sizeof(int) * tleg.size());
+    MODAL_CUDA(cudaMemcpyAsync(b + o_loff, idx.data(), idx.size(), cudaMemcpyHostToDevice, c->stream));
     f.term_shape = reinterpret_cast<const int *>(b + o_ts);
     f.term_leg = f.term_shape + tshape.size();
     double *wl = reinterpret_cast<double *>(b + o_wl);
@@ -573,12 +577,15 @@ modal_status adj_forward(modal_ctx *c, int S, const modal_shape *shapes, AdjFwd 
     int nsm = 0;
     MODAL_CUDA(cudaDeviceGetAttribute(&nsm, cudaDevAttrMultiProcessorCount, c->device));
     const int Zn = (int)std::max<long>(1, std::min<long>(std::min(4, nmu / 64), 8L * nsm / ((long)ceil_div(N, 128) * S)));
-    MODAL_TRY(ensure(c->trip, sizeof(double) * (size_t)Zn * S * N));
+    if (Zn > 1) MODAL_TRY(ensure(c->trip, sizeof(double) * (size_t)Zn * S * N));
+    double *part = Zn > 1 ? c->trip.as<double>() : f.beta;
     const dim3 g2(ceil_div(N, 128), S, Zn);
-    k_beta_gl<<<g2, 128, 0, c->stream>>>(N, nmu, f.li, c->triples.as<int>(), c->w.as<double>(), f.BK, c->trip.as<double>());
+    k_beta_gl<<<g2, 128, 0, c->stream>>>(N, nmu, f.li, c->triples.as<int>(), c->w.as<double>(), f.BK, part);
     MODAL_TRY(launched(c, "beta_gl"));
-    k_beta_sum<<<ceil_div((long)S * N, 256), 256, 0, c->stream>>>((long)S * N, Zn, c->trip.as<double>(), f.beta);
-    MODAL_TRY(launched(c, "beta_sum"));
+    if (Zn > 1) {
+        k_beta_sum<<<ceil_div((long)S * N, 256), 256, 0, c->stream>>>((long)S * N, Zn, part, f.beta);
+        MODAL_TRY(launched(c, "beta_sum"));
+    }
     k_norm_gl<<<S, 128, 0, c->stream>>>(nmu, f.li, c->w.as<double>(), f.BK, f.norm2);
     MODAL_TRY(launched(c, "norm_gl"));
     // the host-side tables above are pageable and go out of scope on return
@@ -592,8 +599,9 @@ modal_status gamma_vjp_dev(modal_ctx *c, const double *G, double *dq)
     const int P = c->P, PP = P * P, nmu = c->nmu, L = c->L, U = P * (P + 1) / 2;
     // by distinct triple products where that takes fewer FP64 instructions (U^3/2 per node against
     // about 45 per pair of modes, and nine shared-memory additions): the full list of 364 modes at
-    // P = 12, n_mu = 1501 takes 1 ms instead of 49
-    if (0.5 * U * (U * (U + 1.0)) < 45.0 * c->N * (double)c->N && 4.0 * U * U * (U + 1.0) <= 16e9) {
+    // P = 12, n_mu = 1501 takes 1 ms instead of 49.  Five launches more are for nothing up to 20 modes and 128 nodes
+    // (20 modes at l <= 60: 0.181 and 0.175 ms, whole calls; 4 modes at l <= 150: 0.292 and 0.295)
+    if ((c->N > 20 || nmu > 128) && 0.5 * U * (U * (U + 1.0)) < 45.0 * c->N * (double)c->N && 4.0 * U * U * (U + 1.0) <= 16e9) {
         MODAL_TRY(mt_ready(c));
         MODAL_TRY(ensure(c->adj2, sizeof(double) * ((size_t)nmu + L) * U));
         double *dX = c->adj2.as<double>(), *Z = dX + (size_t)nmu * U;
