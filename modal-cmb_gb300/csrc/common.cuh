@@ -203,7 +203,7 @@ struct DShape {
     int kind, nterms;
     long tab_off;  // FP64 tables: [term][f, g, h][l] from this double offset
     double c1, c2, c3, sigma;
-    long tab_off_f = 0;  // FP32 form (k_pf_tab's layout) from this float offset
+    long tab_off_f = 0;  // FP32 form (pf_tab's layout) from this float offset
 };
 
 // Internal shape kind of the 3D transfer Gamma: the radial integral s_n(l1,l2,l3)

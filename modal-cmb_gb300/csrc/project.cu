@@ -426,7 +426,7 @@ modal_status proj_plan(modal_ctx *ctx, int S, const modal_shape *shapes, modal_p
         }
     }
     pl.tab_total = tab_total;
-    {   // FP32 layout (k_pf_tab): per term and factor 16 H8 entries, H8 = groups of 8 lattice points per parity
+    {   // FP32 layout (pf_tab): per term and factor 16 H8 entries, H8 = groups of 8 lattice points per parity
         const long H8 = (lmax / 2 + 1 + 7) / 8 + 4;
         long off = 0;
         for (int s = 0; s < S; s++)

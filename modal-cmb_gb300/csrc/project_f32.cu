@@ -65,7 +65,7 @@ struct __align__(16) PfShape {
     // and -log2(e) / (2 sigma^2), every value twice (packed operands)
     float2 bump[8];
     int kind, nterms;
-    long tab_off;        // separable tables from this float offset (k_pf_tab)
+    long tab_off;        // separable tables from this float offset (pf_tab)
     float ch[3], cl[3];  // bump centre as hi + lo
 };
 
@@ -118,14 +118,9 @@ __host__ __device__ inline long long pf_slab_len(int lmin, int lmax, int j)
 // (calculate_geometric.c:59-92 regrouped), v(l) = (2l+1)^{2/3} w_l (calculate_mode_3D.c:53-62).
 // g[h] = g(2h), gl[h] = gL(2h), il2[h] = 1/(2h)^2 (bumps), as double-floats: a factor's rounding is
 // shared by every point that uses it, and a sum that cancels does not average it away.
-// Clears the nmax maxima of k_pf_tab and the flag of k_pf_shapes.
-__global__ void k_pf_tables(int lmax, int nh, const double *__restrict__ cl, float2 *__restrict__ g, float2 *__restrict__ gl,
-                            float2 *__restrict__ il2, float2 *__restrict__ v, int nmax, unsigned *__restrict__ tmax,
-                            int *__restrict__ tail)
+__device__ __forceinline__ void pf_tables(int h, int lmax, int nh, const double *__restrict__ cl, float2 *__restrict__ g,
+                                          float2 *__restrict__ gl, float2 *__restrict__ il2, float2 *__restrict__ v)
 {
-    const int h = blockIdx.x * blockDim.x + threadIdx.x;
-    for (int e = h; e < nmax; e += gridDim.x * blockDim.x) tmax[e] = 0u;
-    if (h == 0) *tail = 0;
     auto df = [](double x) {
         const float hi = (float)x;
         return make_float2(hi, (float)(x - (double)hi));
@@ -194,10 +189,10 @@ __global__ void __launch_bounds__(PF_ROWS) k_pf_weights(int lmin, int lmax, int 
 // B operand image: [parity kp][m / 8][piece][column c < NC][8] BF16 pieces of q_c(2m + kp), zero
 // outside the basis; and the padded FP32 basis rows of the slab reduction, qp[l - lmin][NC], and of
 // the fold, qt[parity of l][l / 2][NC] (rows outside the basis zero).
-__global__ void k_pf_basis(int lmin, int lmax, int P, int NC, int M8, int QR, const double *__restrict__ q,
-                           __nv_bfloat16 *__restrict__ Bt, float *__restrict__ qp, float *__restrict__ qt)
+__device__ __forceinline__ void pf_basis(long e, int lmin, int lmax, int P, int NC, int M8, int QR,
+                                         const double *__restrict__ q, __nv_bfloat16 *__restrict__ Bt, float *__restrict__ qp,
+                                         float *__restrict__ qt)
 {
-    const long e = (long)blockIdx.x * blockDim.x + threadIdx.x;
     const int c = (int)(e % NC);
     const long x = e / NC;
     if (x < 2L * M8 * 8) {
@@ -217,21 +212,8 @@ __global__ void k_pf_basis(int lmin, int lmax, int P, int NC, int M8, int QR, co
     }
 }
 
-// *tail (unless nullptr) is raised where a separable shape may leave the FP32 range at some (l1, l2, l3): its value is at
-// most the sum over the terms of max|f| max|g| max|h| (k_pf_tab's maxima).
-__global__ void k_pf_shapes(int S, int lmax, const DShape *__restrict__ in, const unsigned *__restrict__ tmax,
-                            PfShape *__restrict__ out, int *__restrict__ tail)
+__device__ __forceinline__ PfShape pf_shape(const DShape &d)
 {
-    const int s = blockIdx.x * blockDim.x + threadIdx.x;
-    if (s >= S) return;
-    const DShape d = in[s];
-    if (d.kind == MODAL_SHAPE_SEPARABLE) {
-        const unsigned *m = tmax + d.tab_off / (lmax + 1);
-        double bound = 0.0;
-        for (int t = 0; t < 3 * d.nterms; t += 3)
-            bound += (double)__uint_as_float(m[t]) * (double)__uint_as_float(m[t + 1]) * (double)__uint_as_float(m[t + 2]);
-        if (tail && !(bound <= 1e37)) *tail = 1;
-    }
     PfShape f;
     f.kind = d.kind;
     f.nterms = d.nterms;
@@ -259,35 +241,72 @@ __global__ void k_pf_shapes(int S, int lmax, const DShape *__restrict__ in, cons
     const float ceh = (float)ce, cel = ce < -1e20 ? 0.f : (float)(ce - (double)ceh);
     f.bump[6] = make_float2(ceh, ceh);
     f.bump[7] = make_float2(cel, cel);
-    out[s] = f;
+    return f;
 }
 
-// FP32 tables of the separable shapes, re-laid from the FP64 [term][f, g, h][l] tables in groups of
+// FP32 table of term t of a separable shape, re-laid from the FP64 [term][f, g, h][l] tables in groups of
 // up to four terms (one pass each): group t0 at float offset 3 t0 * 2 * 8 H8, then
 // [parity of l][l / 16][term of the group][f, g, h][8]: a chunk of 32 lattice points is contiguous
 // and four consecutive points of one factor are one 16-byte load.  tmax[term][f, g, h]: the bits of the
-// largest |factor| at l_min .. l_max (infinities and NaN above every number).  grid (ceil(16 H8 / 256), S).
-__global__ void k_pf_tab(int lmin, int lmax, int H8, const DShape *__restrict__ shapes, const double *__restrict__ tab64,
-                         float *__restrict__ tabf, unsigned *__restrict__ tmax)
+// largest |factor| at l_min .. l_max (infinities and NaN above every number).  One block of 256 threads.
+__device__ __forceinline__ void pf_tab(int t, int lmin, int lmax, int H8, const DShape &d, const double *__restrict__ tab64,
+                                       float *__restrict__ tabf, unsigned *__restrict__ tmax)
 {
-    const DShape d = shapes[blockIdx.y];
-    if (d.kind != MODAL_SHAPE_SEPARABLE) return;
-    const int l = blockIdx.x * blockDim.x + threadIdx.x;
-    if (l >= 16 * H8) return;
-    const int stride = lmax + 1, m = l >> 1;
-    unsigned *mx = tmax + d.tab_off / stride;
-    for (int t = 0; t < d.nterms; t++) {
-        const int t0 = t & ~(PF_TC - 1), ng = min(PF_TC, d.nterms - t0);
+    __shared__ unsigned mx[3];
+    if (threadIdx.x < 3) mx[threadIdx.x] = 0u;
+    __syncthreads();
+    const int stride = lmax + 1, t0 = t & ~(PF_TC - 1), ng = min(PF_TC, d.nterms - t0);
+    const double *f = tab64 + d.tab_off + (long)t * 3 * stride;
+    unsigned b[3] = {0u, 0u, 0u};
+    for (int l = threadIdx.x; l < 16 * H8; l += 256) {
+        const int m = l >> 1;
         float *o = tabf + d.tab_off_f + (size_t)3 * t0 * 16 * H8 +
                    ((((size_t)(l & 1) * H8 + (m >> 3)) * ng + (t - t0)) * 3) * 8 + (m & 7);
-        const double *f = tab64 + d.tab_off + (long)t * 3 * stride;
+#pragma unroll
         for (int x = 0; x < 3; x++) {
             const float v = l <= lmax ? (float)f[x * stride + l] : 0.f;
             o[8 * x] = v;
-            const unsigned b = __reduce_max_sync(0xffffffffu, l >= lmin ? __float_as_uint(v) & 0x7fffffffu : 0u);
-            if ((threadIdx.x & 31) == 0) atomicMax(mx + 3 * t + x, b);
+            if (l >= lmin) b[x] = max(b[x], __float_as_uint(v) & 0x7fffffffu);
         }
     }
+#pragma unroll
+    for (int x = 0; x < 3; x++) {
+        const unsigned w = __reduce_max_sync(0xffffffffu, b[x]);
+        if ((threadIdx.x & 31) == 0) atomicMax(mx + x, w);
+    }
+    __syncthreads();
+    if (threadIdx.x < 3) tmax[d.tab_off / stride + 3 * t + threadIdx.x] = mx[threadIdx.x];
+}
+
+// What the weights and the slab kernel read, in one launch (four of their own made small batches
+// slower): blocks for the 1D factors, for the basis, and one per shape and term.
+struct PfSetup {
+    int lmin, lmax, P, NC, M8, QR, nh, maxt, nbt, nbb;
+    const double *cl, *q, *tab64;
+    const DShape *desc;
+    float2 *g, *gl, *il2, *v;
+    __nv_bfloat16 *Bt;
+    float *qp, *qt, *tabf;
+    unsigned *tmax;
+    PfShape *shapes;
+};
+__global__ void __launch_bounds__(256) k_pf_setup(const PfSetup a)
+{
+    int b = blockIdx.x;
+    if (b < a.nbt) {
+        pf_tables(b * 256 + threadIdx.x, a.lmax, a.nh, a.cl, a.g, a.gl, a.il2, a.v);
+        return;
+    }
+    b -= a.nbt;
+    if (b < a.nbb) {
+        pf_basis((long)b * 256 + threadIdx.x, a.lmin, a.lmax, a.P, a.NC, a.M8, a.QR, a.q, a.Bt, a.qp, a.qt);
+        return;
+    }
+    b -= a.nbb;
+    const int s = b / a.maxt, t = b - s * a.maxt;
+    const DShape d = a.desc[s];
+    if (d.kind == MODAL_SHAPE_SEPARABLE && t < d.nterms) pf_tab(t, a.lmin, a.lmax, a.M8, d, a.tab64, a.tabf, a.tmax);
+    if (t == 0 && threadIdx.x == 0) a.shapes[s] = pf_shape(d);
 }
 
 // ---- PTX of this kernel -------------------------------------------------
@@ -1009,34 +1028,31 @@ __global__ void __launch_bounds__(PfMem<NC>::THREADS, 1) k_project_f32(const PfA
             }
             if (stop) break;
             // (the last barrier passed orders the other threads' sums)
+            // One entry per thread and step: with a tile's sixteen by the thread that folds it, few tiles left 16 of
+            // the 128 threads to write all (15,000 cycles a work item at P = 6).
             for (int sx = 0; sx < sgv; sx++)
                 for (int tt = 0; tt < tpt; tt++) {
-                    const int ti = tid + 128 * tt;
-                    if (ti >= nt || tid >= ntp) break;
-                    const int bt = ti / nb4, ct = ti - bt * nb4;
-                    const float *f = Fs + (size_t)(sx * tpt + tt) * 16 * 128 + tid;
-                    const float *fl = CAREFUL ? pf_flo(a, sx * tpt + tt, tpt) : nullptr;
+                    const float *F = Fs + (size_t)(sx * tpt + tt) * 16 * 128;
+                    const float *L0 = CAREFUL ? pf_flo(a, sx * tpt + tt, tpt) - tid : nullptr;
                     const bool corr = CAREFUL && woff != a.base[slab];  // (a slab without rows has no corrections)
                     float *dst = a.Fbuf + ((size_t)(s0 + sx) * L + slab) * PP;
-#pragma unroll
-                    for (int x = 0; x < 4; x++)
-#pragma unroll
-                        for (int y = 0; y < 4; y++) {
-                            const int bb = 4 * bt + x, c2 = 4 * ct + y;
-                            if (bb >= P || c2 >= P) continue;
-                            float v = 0.f, lo = 0.f;
-                            for (int q = 0; q < rs; q++) {
-                                const int e = (4 * x + y) * 128 + q * ntp;
-                                if (CAREFUL) {
-                                    const float z = f[e] - lo, t = v + z;
-                                    lo = (t - v) - z;
-                                    v = t;
-                                    if (corr) lo += fl[e];
-                                } else
-                                    v += f[e];
-                            }
-                            dst[bb * P + c2] = v - lo;
+                    for (int u = tid; u < 16 * ntp; u += 128) {
+                        const int t0 = u & (ntp - 1), xy = u / ntp, ti = t0 + 128 * tt;
+                        const int bt = ti / nb4, bb = 4 * bt + (xy >> 2), c2 = 4 * (ti - bt * nb4) + (xy & 3);
+                        if (ti >= nt || bb >= P || c2 >= P) continue;
+                        float v = 0.f, lo = 0.f;
+                        for (int q = 0; q < rs; q++) {
+                            const int e = xy * 128 + t0 + q * ntp;
+                            if (CAREFUL) {
+                                const float z = F[e] - lo, t = v + z;
+                                lo = (t - v) - z;
+                                v = t;
+                                if (corr) lo += L0[e];
+                            } else
+                                v += F[e];
                         }
+                        dst[bb * P + c2] = v - lo;
+                    }
                 }
             stop = rows_bar_or(bar, false);  // the sums are read before the next item clears them
         }
@@ -1087,10 +1103,27 @@ __global__ void __launch_bounds__(128) k_pf_B(int L, int P, int S, int NC, int n
         if (b0 + x < P) B[(((size_t)seg * S + s) * P + b0 + x) * PP + e] = (double)hi[x] - (double)lo[x];
 }
 
-// beta[s][r] = (1/6) sum over the segments and the six orderings of mode r of B
+// beta[s][r] = (1/6) sum over the segments and the six orderings of mode r of B.  *tail: whether (raise) a
+// separable shape may leave the FP32 range at some (l1, l2, l3): its value is at most the sum over the terms of
+// max|f| max|g| max|h| (pf_tab's maxima).
 __global__ void k_pf_beta(int N, int P, int S, int nseg, const int *__restrict__ triples, const double *__restrict__ B,
-                          double *__restrict__ beta)
+                          double *__restrict__ beta, int lmax, const DShape *__restrict__ desc,
+                          const unsigned *__restrict__ tmax, bool raise, int *__restrict__ tail)
 {
+    if (blockIdx.x == 0) {
+        bool far = false;
+        for (int s = threadIdx.x; raise && s < S; s += blockDim.x) {
+            const DShape d = desc[s];
+            if (d.kind != MODAL_SHAPE_SEPARABLE) continue;
+            const unsigned *m = tmax + d.tab_off / (lmax + 1);
+            double bound = 0.0;
+            for (int t = 0; t < 3 * d.nterms; t += 3)
+                bound += (double)__uint_as_float(m[t]) * (double)__uint_as_float(m[t + 1]) * (double)__uint_as_float(m[t + 2]);
+            far |= !(bound <= 1e37);
+        }
+        far = __syncthreads_or(far);
+        if (threadIdx.x == 0) *tail = far;
+    }
     const size_t e = (size_t)blockIdx.x * blockDim.x + threadIdx.x;
     if (e >= (size_t)S * N) return;
     const int s = (int)(e / N), r = (int)(e % N);
@@ -1219,22 +1252,21 @@ modal_status pf_record(modal_ctx *ctx, const ProjPlan &pl)
     unsigned *tmax = reinterpret_cast<unsigned *>(b + pl.o_m);
     int *tail = ctx->ozerr.as<int>() + 1;
     const long long *base = ctx->pf_sched.as<long long>();
-    k_pf_tables<<<ceil_div(nh, 128), 128, 0, ctx->stream>>>(lmax, nh, ctx->cl.as<double>(), g, gl, il2, v,
-                                                               (int)(pl.tab_total / (lmax + 1)), tmax, tail);
-    MODAL_TRY(launched(ctx, "pf_tables"));
+    PfSetup u;
+    u.lmin = lmin; u.lmax = lmax; u.P = P; u.NC = NC; u.M8 = pl.M8; u.QR = pl.QR; u.nh = nh;
+    u.maxt = 1;
+    for (const DShape &d : pl.desc) u.maxt = std::max(u.maxt, d.nterms);
+    u.nbt = ceil_div(std::max(nh, lmax + 1), 256);
+    u.nbb = ceil_div((long)std::max(std::max(16 * pl.M8, L), 2 * pl.QR) * NC, 256);
+    u.cl = ctx->cl.as<double>(); u.q = ctx->q.as<double>(); u.tab64 = ctx->shape_tab.as<double>();
+    u.desc = ctx->shape_desc.as<DShape>();
+    u.g = g; u.gl = gl; u.il2 = il2; u.v = v; u.Bt = Bt; u.qp = qp; u.qt = qt; u.tabf = tabf; u.tmax = tmax;
+    u.shapes = fs;
+    k_pf_setup<<<u.nbt + u.nbb + S * u.maxt, 256, 0, ctx->stream>>>(u);
+    MODAL_TRY(launched(ctx, "pf_setup"));
     const int nbmax = ceil_div((lmax - lmin) / 2 + 1, PF_ROWS);
     k_pf_weights<<<dim3(L, 2 * nbmax), PF_ROWS, 0, ctx->stream>>>(lmin, lmax, nbmax, base, g, gl, v, W);
     MODAL_TRY(launched(ctx, "pf_weights"));
-    const long nb = (long)std::max(std::max(16 * pl.M8, L), 2 * pl.QR) * NC;
-    k_pf_basis<<<ceil_div(nb, 256), 256, 0, ctx->stream>>>(lmin, lmax, P, NC, pl.M8, pl.QR, ctx->q.as<double>(), Bt, qp, qt);
-    MODAL_TRY(launched(ctx, "pf_basis"));
-    if (pl.tabf_total > 0) {
-        k_pf_tab<<<dim3(ceil_div(16L * pl.M8, 256), S), 256, 0, ctx->stream>>>(
-            lmin, lmax, pl.M8, ctx->shape_desc.as<DShape>(), ctx->shape_tab.as<double>(), tabf, tmax);
-        MODAL_TRY(launched(ctx, "pf_tab"));
-    }
-    k_pf_shapes<<<ceil_div(S, 64), 64, 0, ctx->stream>>>(S, lmax, ctx->shape_desc.as<DShape>(), tmax, fs, pl.careful ? nullptr : tail);
-    MODAL_TRY(launched(ctx, "pf_shapes"));
     PfArgs a;
     a.lmin = lmin; a.lmax = lmax; a.P = P; a.S = S; a.SG = pl.SG; a.G = ceil_div(S, pl.SG);
     a.nitems = L * a.G;
@@ -1258,7 +1290,8 @@ modal_status pf_record(modal_ctx *ctx, const ProjPlan &pl)
     k_pf_B<<<dim3(ceil_div(PP, 128), S, pl.nseg * ceil_div(P, PB)), 128, 0, ctx->stream>>>(L, P, S, NC, pl.nseg, qp, Fbuf, B);
     MODAL_TRY(launched(ctx, "pf_B"));
     k_pf_beta<<<ceil_div((long)S * N, 256), 256, 0, ctx->stream>>>(N, P, S, pl.nseg, ctx->triples.as<int>(), B,
-                                                                     ctx->beta.as<double>());
+                                                                     ctx->beta.as<double>(), lmax,
+                                                                     ctx->shape_desc.as<DShape>(), tmax, !pl.careful, tail);
     return launched(ctx, "pf_beta");
 }
 
