@@ -577,9 +577,10 @@ modal_status modal_project(modal_ctx *c, int S, const modal_shape *shapes, modal
     c->beta_S = S;
     if (beta) MODAL_TRY(d2h(c, beta, c->beta.ptr, sizeof(double) * (size_t)S * c->N));
     MODAL_TRY(sync(c));
+    if (prec != MODAL_PREC_SPLIT) return MODAL_OK;
     bool tail = false;
     MODAL_TRY(oz_check(c, &tail));  // a bounded wait of the tensor-core slab kernel that expired
-    if (prec != MODAL_PREC_SPLIT || !tail) return MODAL_OK;
+    if (!tail) return MODAL_OK;
     {
         StageTimer t(c, MODAL_T_PROJECT);
         MODAL_TRY(project_dev(c, S, shapes, prec, true));

@@ -29,7 +29,7 @@ struct BatchGraph {
     cudaGraphExec_t exec = nullptr;
     double *h_tab = nullptr;
     DShape *h_desc = nullptr;
-    double *h_beta = nullptr;
+    double *h_beta = nullptr;  // [S][N], then (single precision) the error word and the flag of the projection
     ProjPlan plan;
     long kernels = 0;  // kernel nodes per replay
     void clear()
@@ -83,7 +83,7 @@ static modal_status batch_capture(modal_ctx *c, int S, const modal_shape *shapes
     const size_t tab_bytes = sizeof(double) * (size_t)(g.plan.tab_total > 0 ? g.plan.tab_total : 1);
     MODAL_CUDA(cudaHostAlloc(reinterpret_cast<void **>(&g.h_tab), tab_bytes, cudaHostAllocDefault));
     MODAL_CUDA(cudaHostAlloc(reinterpret_cast<void **>(&g.h_desc), sizeof(DShape) * (size_t)S, cudaHostAllocDefault));
-    MODAL_CUDA(cudaHostAlloc(reinterpret_cast<void **>(&g.h_beta), sizeof(double) * (size_t)S * c->N,
+    MODAL_CUDA(cudaHostAlloc(reinterpret_cast<void **>(&g.h_beta), sizeof(double) * ((size_t)S * c->N + 1),
                              cudaHostAllocDefault));
     MODAL_CUDA(cudaStreamSynchronize(c->stream));  // the plan's uploads are done before capture starts
     const long l0 = c->launches;
@@ -99,6 +99,8 @@ static modal_status batch_capture(modal_ctx *c, int S, const modal_shape *shapes
     if (st == MODAL_OK) st = proj_record(c, g.plan);
     if (st == MODAL_OK) {
         e = cudaMemcpyAsync(g.h_beta, c->beta.ptr, sizeof(double) * (size_t)S * c->N, cudaMemcpyDeviceToHost, c->stream);
+        if (e == cudaSuccess && prec == MODAL_PREC_SPLIT)
+            e = cudaMemcpyAsync(g.h_beta + (size_t)S * c->N, c->ozerr.ptr, 2 * sizeof(int), cudaMemcpyDeviceToHost, c->stream);
         if (e != cudaSuccess) {
             set_error("modal_project_batch: result copy in capture: %s", cudaGetErrorString(e));
             st = MODAL_ERR_CUDA;
@@ -187,9 +189,10 @@ modal_status modal_project_batch(modal_ctx *c, int S, const modal_shape *shapes,
     }
     c->launches += g.kernels;
     MODAL_CUDA(cudaStreamSynchronize(c->stream));
-    bool tail = false;
-    MODAL_TRY(oz_check(c, &tail));  // a bounded wait of the tensor-core slab kernel that expired
-    if (prec == MODAL_PREC_SPLIT && tail) {  // (rare: outside the graph)
+    int flags[2] = {0, 0};
+    if (prec == MODAL_PREC_SPLIT) std::memcpy(flags, g.h_beta + (size_t)S * c->N, sizeof flags);
+    MODAL_TRY(oz_status(flags[0]));  // a bounded wait of the tensor-core slab kernel that expired
+    if (flags[1]) {  // (rare: outside the graph)
         MODAL_TRY(project_dev(c, S, shapes, prec, true));
         MODAL_CUDA(cudaMemcpyAsync(g.h_beta, c->beta.ptr, sizeof(double) * (size_t)S * c->N, cudaMemcpyDeviceToHost, c->stream));
         MODAL_CUDA(cudaStreamSynchronize(c->stream));

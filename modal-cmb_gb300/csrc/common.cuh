@@ -284,6 +284,7 @@ modal_status oz_reset(modal_ctx *ctx);  // clear the sticky error word of unchec
 // Synchronise; MODAL_ERR_TIMEOUT if any call's wait expired.  tail: whether the FP32 projection before had
 // shapes that may leave the FP32 range past the ends of its rows, and is to be run again with those masked.
 modal_status oz_check(modal_ctx *ctx, bool *tail = nullptr);
+modal_status oz_status(int herr);  // of an error word that the host holds
 modal_status oz_gemm_ex(modal_ctx *ctx, int M, int N, int K, double alpha, const double *A, long lda, bool transA,
                         const double *B, long ldb, bool transB, double beta, double *C, long ldc, const OzOpts &o);
 // C (+)= A op(B) for A [S][K] with few rows S: skinny kernels for S <= 32 (alpha 1; accumulate: C +=)

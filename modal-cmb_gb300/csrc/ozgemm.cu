@@ -695,9 +695,13 @@ modal_status oz_check(modal_ctx *ctx, bool *tail)
     int h[2] = {0, 0};
     MODAL_CUDA(cudaMemcpyAsync(h, ctx->ozerr.ptr, sizeof h, cudaMemcpyDeviceToHost, ctx->stream));
     MODAL_CUDA(cudaStreamSynchronize(ctx->stream));
-    const int herr = h[0];
     if (tail) *tail = h[1] != 0;
-    if (herr) { set_error("a bounded wait in a tensor-core kernel expired (role %d: 1-4 Ozaki GEMM, 21-22 slab projection)", herr); return MODAL_ERR_TIMEOUT; }
+    return oz_status(h[0]);
+}
+
+modal_status oz_status(int herr)
+{
+    if (herr) { set_error("a bounded wait in a tensor-core kernel expired (role %d: 1-4 Ozaki GEMM, 21 and 23 slab projection)", herr); return MODAL_ERR_TIMEOUT; }
     return MODAL_OK;
 }
 

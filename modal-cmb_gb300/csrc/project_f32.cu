@@ -1189,11 +1189,19 @@ modal_status pf_plan(modal_ctx *ctx, ProjPlan &pl)
     auto team = [&](int sg) { return (pl.smem + sg * fper + 127) & ~(size_t)127; };
     while (pl.SG > 1 && pl.teams * team(pl.SG) > most) pl.SG--;
     while (pl.teams > 1 && pl.teams * team(pl.SG) > most) pl.teams--;
+    MODAL_CUDA(cudaDeviceGetAttribute(&pl.nsm, cudaDevAttrMultiProcessorCount, ctx->device));
+    if (!want) {
+        // fewer shapes per item where whole rounds of items over the teams take a tenth fewer shapes each
+        auto rounds = [&](int sg) { return (long)ceil_div((long)L * ceil_div(S, sg), pl.nsm * pl.teams) * sg; };
+        int sg = pl.SG;
+        for (int x = pl.SG - 1; x >= 1; x--)
+            if (rounds(x) < rounds(sg)) sg = x;
+        if (10 * rounds(sg) <= 9 * rounds(pl.SG)) pl.SG = sg;
+    }
     pl.team_smem = team(pl.SG);
     pl.smem = (size_t)pl.teams * pl.team_smem;
     pl.QR = lmax / 2 + 1;
     pl.M8 = (lmax / 2 + 1 + 7) / 8 + 4;
-    MODAL_CUDA(cudaDeviceGetAttribute(&pl.nsm, cudaDevAttrMultiProcessorCount, ctx->device));
     // How the sums between a point and F are kept.  Plain FP32 additions do where a term of the sum meets no more
     // roundings than on CUDA cores, which add 32 points of a row and 16 rows plainly and compensate beyond (52 with
     // the roundings of their compensated sums and stores): two for a chunk's accumulator, one per accumulator of the row,
