@@ -536,7 +536,7 @@ modal_status modal_set_pca_floor(modal_ctx *c, double floor)
 modal_status modal_set_proj_kernel(modal_ctx *c, int tensor_cores)
 {
     if (!c || (tensor_cores != 0 && tensor_cores != 1)) {
-        set_error("modal_set_proj_kernel: 0 (CUDA cores) or 1 (tensor cores)");
+        set_error("modal_set_proj_kernel: 0 or 1");
         return MODAL_ERR_ARG;
     }
     c->proj_tc = tensor_cores;

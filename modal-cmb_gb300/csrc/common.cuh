@@ -42,7 +42,7 @@ struct modal_ctx {
     long captures = 0;                   // graphs captured so far
     // tuned launch configurations (0: built-in defaults; set by modal_autotune)
     int proj_sg = 0, proj_cpb = 0, gamma_kc = 0;
-    int proj_tc = 0;  // 1: FP32 projection on the tensor cores where P <= 32 (0: CUDA-core kernel)
+    int proj_tc = 0;  // modal_set_proj_kernel's preference; one kernel serves both
     int beta_S = 0;
 
     // device state

@@ -149,3 +149,13 @@ def test_autotune_does_not_take_records_of_other_launch_parameters(mg, tmp_path)
         c.autotune(old)
         assert len(open(old).read().splitlines()) == 3
         assert c.tuning()["proj_tc"] == t["proj_tc"] == 0
+
+
+def test_batch_is_not_captured_again_for_the_kernel_preference(mg):
+    """Both settings of the preference run the same kernel: the graph serves both, with the same bits."""
+    shapes = _mixed(mg, 160, 3)
+    with _ctx(mg) as c:
+        first = c.project_batch(shapes, mg.PREC_SPLIT)
+        n = c.captures
+        c.set_proj_kernel(True)
+        assert np.array_equal(c.project_batch(shapes, mg.PREC_SPLIT), first) and c.captures == n
