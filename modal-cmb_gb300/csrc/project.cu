@@ -465,7 +465,8 @@ modal_status proj_plan(modal_ctx *ctx, int S, const modal_shape *shapes, modal_p
         for (int i = lmin; i <= lmax; i++) npts += tet_row_offset(i, lmax + 1, lmax);
         pl.npts = npts;
         pl.o_B = sizeof(double) * (size_t)S * L * PP;
-        pl.nseg = (int)std::max<long>(1, std::min<long>(std::min(8, L / 32), 152L * 1024 / ((long)S * P * PP)));
+        MODAL_CUDA(cudaDeviceGetAttribute(&pl.nsm, cudaDevAttrMultiProcessorCount, ctx->device));
+        pl.nseg = (int)std::max<long>(1, std::min<long>(std::min(8, L / 32), 1024L * pl.nsm / ((long)S * P * PP)));
         pl.o_sb = pl.o_B + sizeof(double) * (size_t)pl.nseg * S * P * PP;
         pl.o_w = pl.o_sb + sizeof(long long) * (size_t)(L + 1);
         MODAL_TRY(ensure(ctx->scratch, pl.o_w + sizeof(double) * (size_t)npts));
