@@ -25,7 +25,8 @@
 // there; the other five share a second accumulator for the whole row, where a truncation is 2^-8 of
 // that.  (Two TF32 pieces in one accumulator were tried first: 1.3e-7 from the FP64 beta at
 // l <= 2000, P = 30, against 5e-8 of the FP32 FMAs this replaces.)  The row's thread adds every
-// chunk's accumulator into its H row; F is folded on the CUDA cores once per 128 rows.
+// chunk's accumulator into its H row; F is folded on the CUDA cores once per 128 rows.  These sums are plain
+// FP32 where a term meets no more roundings than on CUDA cores and compensated where it would (pf_plan).
 //
 // What bounds it: issue slots of the row warps (evaluation, split, fold) and, with 12 row warps per
 // SM, the latencies between them; so every operand is fetched ahead (ring of three chunks, the
@@ -33,14 +34,14 @@
 // halves of 16 points.  One CTA per SM: three teams (two for P > 32) of four row warps, each with its
 // own items, and one warp per team that copies and issues; the row warps take registers over from
 // the issuing warps (setmaxnreg 152 / 56 of 128), since a spill to this kernel's small L1 costs an
-// L2 round trip.  TMEM per team: 48 columns of A, two leading accumulators and one for the rest.
+// L2 round trip.  (Whatever the fold keeps in registers through the passes moves the time by 5%.)  TMEM per team: 48 columns of A, two leading accumulators and one for the rest.
 //
 // Measured (l <= 2000, P = 30), against the CUDA-core kernel (136 warp instructions per 32 points)
 // and the shared-memory-operand tensor-core kernel that it replaces both: 16 separable shapes 33.9 ->
-// 15.8 ms, 256 mixed shapes 532 (CUDA cores), 1864 (tensor cores) -> 233 ms; error of beta against
+// 15.9 ms, 256 mixed shapes 532 (CUDA cores), 1864 (tensor cores) -> 237 ms; error of beta against
 // 64 bits, median and largest over the 128 bumps and 128 separable shapes: 7.5e-8, 8.9e-7 and
-// 4.7e-8, 1.3e-7 -> 5.0e-8, 7.3e-7 and 2.5e-8, 4.6e-8.  (The largest was 2.7e-6, and the 256 shapes
-// took 225 ms, with the 1D factors of the weights and of the bumps' exponents rounded to FP32.)
+// 4.7e-8, 1.3e-7 -> 5.0e-8, 7.2e-7 and 2.5e-8, 4.6e-8.  (The largest was 2.7e-6, and the 256 shapes
+// took 8 ms less, with the 1D factors of the weights and of the bumps' exponents rounded to FP32.)
 #include <algorithm>
 #include <vector>
 #include <cuda_bf16.h>

@@ -762,7 +762,8 @@ __device__ void dc_deflate_serial(DcWork &w, MergeInfo &M, int a, int k, double 
 // [k] doubles, support flags and kept flags [k] bytes.  Which entries and pairs deflate is
 // decided in parallel on the entries as they come; the serial pass follows those decisions
 // and tests again only next to a rotation (an FP64 instruction of a lone thread takes 64 cycles).
-// n = 4,960, 13 levels: 2.6 ms; every test and the compaction in the serial pass 3.8 ms.
+// n = 4,960, 13 levels, Gamma of the plain FP64 form: 2.6 ms (of the split form, which deflates more pairs, 4.1);
+// every test and the compaction in the serial pass 3.8 ms.
 __global__ void __launch_bounds__(256) k_dc_deflate(DcWork w, int use_smem)
 {
     extern __shared__ double dsm[];
@@ -884,7 +885,8 @@ __global__ void k_dc_rotate(DcWork w)
 // Secular roots: one warp per position p; root j = p - a of the merge holding p.
 // Bound by FP64 instructions (64 cycles each per warp on a quarter of an SM): for small merges those
 // of an iteration outside the sum, so the four sums share their last levels and a step takes one
-// square root and one division.  n = 4,960, 13 levels: 3.7 ms, with four separate sums and both roots 4.1 ms
+// square root and one division.  n = 4,960, 13 levels, Gamma of the plain FP64 form (of the split form): 3.7 ms (4.4), with
+// four separate sums and both roots 4.1 ms
 // (n = 220: 0.48 ms before).
 __global__ void __launch_bounds__(256) k_dc_secular(DcWork w)
 {

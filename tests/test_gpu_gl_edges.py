@@ -15,3 +15,9 @@ def test_gl_nodes_edges(mg, orc, n):
     assert np.max(np.abs(x - xo)) <= 5e-16
     assert np.max(np.abs(w - wo) / wo) <= 1e-13
     assert np.array_equal(x, -x[::-1]) and np.array_equal(w, w[::-1])
+
+
+@pytest.mark.parametrize("n", [1, 2, 3, 31, 33, 95, 96, 97])
+def test_gl_nodes_chunk_edges(mg, orc, n):
+    """The recurrence works in chunks of 32 steps: a first step past a whole chunk, and one short of it."""
+    test_gl_nodes_edges(mg, orc, n)
