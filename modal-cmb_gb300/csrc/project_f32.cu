@@ -1178,21 +1178,19 @@ modal_status pf_plan(modal_ctx *ctx, ProjPlan &pl)
         ctx->pf_total = total;
     }
     pl.NC = P <= 16 ? 16 : (P <= 32 ? 32 : (P <= 48 ? 48 : 64));
-    // teams per SM and shapes per work item: as asked for, or as many as fit in shared memory
+    // teams per SM and shapes per work item: as asked for at most, as many as fit in shared memory
     const int nb4 = (P + 3) / 4, tpt = ceil_div((long)nb4 * nb4, 128);
     const size_t slot = 192 * (size_t)pl.NC + 384 * PF_TC, fper = sizeof(float) * 16 * PF_ROWS * (size_t)tpt;
     pl.smem = PF_SLOTS * slot + sizeof(float) * PF_ROWS * (size_t)(2 * pl.NC + 4) + 128;
-    const int want = (ctx->proj_sg == 4 || ctx->proj_sg == 8) ? ctx->proj_sg : 0;
     const size_t most = 226 * 1024;
     const int teams = pl.NC <= 32 ? 3 : 2;
     pl.teams = ctx->proj_cpb > 0 ? std::min(ctx->proj_cpb, teams) : teams;
-    pl.SG = want ? want : 4;
+    pl.SG = ctx->proj_sg == 8 ? 8 : 4;
     auto team = [&](int sg) { return (pl.smem + sg * fper + 127) & ~(size_t)127; };
     while (pl.SG > 1 && pl.teams * team(pl.SG) > most) pl.SG--;
     while (pl.teams > 1 && pl.teams * team(pl.SG) > most) pl.teams--;
     MODAL_CUDA(cudaDeviceGetAttribute(&pl.nsm, cudaDevAttrMultiProcessorCount, ctx->device));
-    if (!want) {
-        // fewer shapes per item where whole rounds of items over the teams take a tenth fewer shapes each
+    {   // fewer shapes per item where whole rounds of items over the teams take a tenth fewer shapes each
         auto rounds = [&](int sg) { return (long)ceil_div((long)L * ceil_div(S, sg), pl.nsm * pl.teams) * sg; };
         int sg = pl.SG;
         for (int x = pl.SG - 1; x >= 1; x--)

@@ -183,3 +183,24 @@ def test_f32_projection_fold_keeps_small_addends(mg, P):
         b64 = c.project(shape, mg.PREC_FP64)
         b32 = c.project(shape, mg.PREC_SPLIT)
     assert rel_fro(b32, b64) <= 15 * 2.0**-25
+
+
+@pytest.mark.parametrize("P", [5, 20, 40, 60])
+@pytest.mark.parametrize("terms", [36, 40, 48, 60])
+def test_f32_projection_sum_modes(mg, terms, P):
+    """The four ways of the sums, by the number of roundings that the terms' passes add at l_max = 130: plain,
+    groups of 16 rows compensated, groups of 8, everything compensated; for each operand width, and again with a
+    term that overflows outside the triangle (masked and compensated)."""
+    lmax = 130
+    shapes = mg.separable_shapes(lmax, 2, seed=16, tmin=terms, tmax=terms) + mg.bump_shapes(1, seed=17)
+    l = np.arange(lmax + 1)
+    far = [dict(s, tab=s["tab"].copy()) for s in shapes[:2]] + shapes[2:]
+    for s in far[:2]:
+        s["tab"][0] = [np.where(l <= 3, 1e15, 0.0), np.where(l <= 3, 1e15, 0.0), np.where(l >= 12, 1e15, 0.0)]
+    with _ctx(mg, 2, lmax, P) as c:
+        for sh in (shapes, far):
+            b64 = c.project(sh, mg.PREC_FP64)
+            b32 = c.project(sh, mg.PREC_SPLIT)
+            assert np.array_equal(b32, c.project_batch(sh, mg.PREC_SPLIT))
+            for s in range(3):
+                assert rel_fro(b32[s], b64[s]) <= (1e-6 if P <= 32 else 2e-6), (s, rel_fro(b32[s], b64[s]))
